@@ -235,6 +235,12 @@ __device__ __forceinline__ void acc_add(dacc& a, df x) {
   a.hi = s.hi;
   a.lo = __fadd_rn(a.lo, __fadd_rn(s.lo, x.lo));
 }
+// a += x * y
+__device__ __forceinline__ void acc_fma(dacc& a, df x, df y) {
+  const df p = two_prod(x.hi, y.hi), s = two_sum(a.hi, p.hi);
+  a.hi = s.hi;
+  a.lo = __fadd_rn(a.lo, __fmaf_rn(x.hi, y.lo, __fmaf_rn(x.lo, y.hi, __fadd_rn(s.lo, p.lo))));
+}
 __device__ __forceinline__ df acc_val(const dacc& a) { return two_sum(a.hi, a.lo); }
 struct dacc3 {
   dacc x, y, z;
@@ -243,6 +249,12 @@ __device__ __forceinline__ void acc_add3(dacc3& a, const df3& v) {
   acc_add(a.x, v.x);
   acc_add(a.y, v.y);
   acc_add(a.z, v.z);
+}
+// a += s * v
+__device__ __forceinline__ void acc_fma3(dacc3& a, df s, const df3& v) {
+  acc_fma(a.x, s, v.x);
+  acc_fma(a.y, s, v.y);
+  acc_fma(a.z, s, v.z);
 }
 __device__ __forceinline__ df3 acc_val3(const dacc3& a) { return {acc_val(a.x), acc_val(a.y), acc_val(a.z)}; }
 

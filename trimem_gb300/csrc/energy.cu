@@ -392,20 +392,25 @@ EP make_ep(const tm_energy* e) {
 }
 
 void energy_eval(tm_energy* e, tm_mesh* m, const double* P, bool want_grad, bool want_vprops, double* d_grad,
-                 cudaStream_t s) {
+                 cudaStream_t s, double* d_energy) {
+  if (e->stencil == 2 && !want_vprops) {
+    energy_eval_df(e, m, P, want_grad, d_grad, d_energy, nullptr, s, nullptr);
+    return;
+  }
   energy_eval_marked(e, m, P, want_grad, want_vprops, d_grad, s, nullptr);
+  if (d_energy)
+    TM_CUDA(cudaMemcpyAsync(d_energy, &e->glob.get()->comps[6], sizeof(double), cudaMemcpyDeviceToDevice, s));
 }
 
 static void eval_fp64_launches(tm_energy* e, tm_mesh* m, const double* P, bool want_grad, bool want_vprops,
                                double* d_grad, cudaStream_t s, cudaEvent_t* ev);
 
-// the launches of one evaluation in the energy's stencil precision
+// the launches of one FP32 or FP64 evaluation (the double-word path is short
+// enough to need no graph)
 static void eval_launches(tm_energy* e, tm_mesh* m, const double* P, bool want_grad, double* d_grad,
                           cudaStream_t s) {
   if (e->stencil == 1)
     energy_eval32(e, m, P, want_grad, false, d_grad, s, nullptr);
-  else if (e->stencil == 2)
-    energy_eval_df(e, m, P, want_grad, d_grad, s, nullptr);
   else
     eval_fp64_launches(e, m, P, want_grad, false, d_grad, s, nullptr);
 }
@@ -498,10 +503,6 @@ void energy_eval_marked(tm_energy* e, tm_mesh* m, const double* P, bool want_gra
     energy_eval32(e, m, P, want_grad, want_vprops, d_grad, s, ev);
     return;
   }
-  if (e->stencil == 2 && !want_vprops) {
-    energy_eval_df(e, m, P, want_grad, d_grad, s, ev);
-    return;
-  }
   eval_fp64_launches(e, m, P, want_grad, want_vprops, d_grad, s, ev);
 }
 
@@ -575,11 +576,21 @@ void tm_energy::ensure(int nv_, int ne_, int nf_) {
   vprops.ensure(6 * (size_t)std::max(nv, 1));
   pos32.ensure(3 * (size_t)std::max(nv, 1));
   int nb = std::max(1, (nv + tmg::VB - 1) / tmg::VB);
-  partials.ensure(8 * (size_t)nb);
+  partials.ensure(8 * (size_t)nb * 8);  // up to eight lanes per vertex
+  moved.ensure(nb);
   grad.ensure(3 * (size_t)std::max(nv, 1));
   work.ensure(64);
   glob.ensure(1);
   TM_CUDA(cudaMemsetAsync(glob.get(), 0, sizeof(tmg::Globals), stream));
+}
+
+int tm_energy::sm_count() {
+  if (!sms) {
+    int dev = 0;
+    TM_CUDA(cudaGetDevice(&dev));
+    TM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  }
+  return sms;
 }
 
 void tm_energy::to_host(double* dst, const double* src, size_t n) {
@@ -782,9 +793,7 @@ int tm_energy_eval_device(tm_energy* e, tm_mesh* m, const double* d_points, doub
   TM_API_BEGIN
   if (!e || !m || !d_points) fail(TM_ERR_ARG, "NULL argument");
   cudaStream_t s = stream ? (cudaStream_t)stream : e->stream;
-  tmg::energy_eval(e, m, d_points, d_grad != nullptr, false, d_grad, s);
-  if (d_energy)
-    TM_CUDA(cudaMemcpyAsync(d_energy, &e->glob.get()->comps[6], sizeof(double), cudaMemcpyDeviceToDevice, s));
+  tmg::energy_eval(e, m, d_points, d_grad != nullptr, false, d_grad, s, d_energy);
   TM_API_END
 }
 
@@ -795,7 +804,10 @@ int tm_energy_eval_timed(tm_energy* e, tm_mesh* m, const double* d_points, doubl
   cudaStream_t s = stream ? (cudaStream_t)stream : e->stream;
   cudaEvent_t ev[5];
   for (int k = 0; k < 5; ++k) TM_CUDA(cudaEventCreate(&ev[k]));
-  tmg::energy_eval_marked(e, m, d_points, d_grad != nullptr, false, d_grad, s, ev);
+  if (e->stencil == 2)
+    tmg::energy_eval_df(e, m, d_points, d_grad != nullptr, d_grad, nullptr, nullptr, s, ev);
+  else
+    tmg::energy_eval_marked(e, m, d_points, d_grad != nullptr, false, d_grad, s, ev);
   TM_CUDA(cudaEventSynchronize(ev[4]));
   for (int k = 0; k < 4; ++k) TM_CUDA(cudaEventElapsedTime(&ms5[k], ev[k], ev[k + 1]));
   TM_CUDA(cudaEventElapsedTime(&ms5[4], ev[0], ev[4]));

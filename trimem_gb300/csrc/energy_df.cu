@@ -5,8 +5,8 @@
 // kernels of energy.cu keep it ~85% busy.  These kernels compute the same
 // quantities with double-word numbers (df64.cuh: pairs of floats, ~48-bit
 // significands) on the FP32 pipe:
-//   * positions are split once per evaluation into float hi / lo parts
-//     (one float4 each per vertex); edge vectors are double-word differences,
+//   * positions are split once per evaluation into float hi / lo parts (one
+//     32-byte sector per vertex); edge vectors are double-word differences,
 //     so |x| >> |x_b - x_a| costs no accuracy;
 //   * products are exact TwoProds, sums collect their rounding errors in one
 //     float (Dot2 / Sum2 style) and are renormalised once, normalisations
@@ -19,6 +19,19 @@
 //     and the penalty assembly.
 // The results agree with the FP64 oracle to ~1e-13 relative (the parity
 // tests hold them to 1e-10); they are not bitwise equal to the FP64 kernels.
+//
+// An evaluation is a chain of five kernels (positions, faces + repulsion,
+// edges + queued repulsion, vertices, gradient).  What bounds it: on large
+// meshes issue slots (each double-word operation is 7-20 FP32 instructions)
+// and gathers over the 1-ring, on small ones the kernels' latencies.  Against
+// the former chain of eight kernels on two streams (a graph replay, 64- and
+// 32-byte records gathered in 16-byte pieces, cross products per ring slot):
+// 113 to 85 us at 163,842 vertices (the gradient 41 to 25), 59 to 41 at
+// 40,962, 43 to 24 at 642, 85 to 37 for an open tube of 7,566 vertices with
+// Verlet rows; the errors against 64 bits are the same (gradient 6.7e-13 at
+// 163,842 vertices, energy 1.9e-14).  A variant with all stages in one
+// cooperative kernel (grid barriers instead of launches) was slower at every
+// size: 32 us at 642 vertices, 40 at 10,242, 150 at 163,842.
 #include <algorithm>
 #include <cmath>
 
@@ -32,36 +45,105 @@ namespace tmg {
 
 namespace {
 
-// Face record, four float4 per face:
-//   [0] (nx, ny)  [1] (nz, A)  [2] (V, cot a)  [3] (cot b, cot c)
-// with n the unit normal, A the area, V the signed volume about the origin
-// and the cotangents of the corners in the face's stored vertex order.
-// Edge record, two float4 per edge:
-//   [0] (l, theta)  [1] (dB/dl, s/l)
-// with s = +1 on interior edges and -1 on boundary edges.
+// Face record, four float4 (two sectors) per face:
+//   [0] (nx, ny)  [1] (nz, A)  [2] (cot a, cot b)  [3] (cot c, -)
+// with n the unit normal, A the area and the cotangents of the corners in
+// the face's stored vertex order; (A, V), V the signed volume about the
+// origin, again in a compact record for the ring sums.
+// Edge records, one float4 each: (l theta, bond value) for the ring sums and
+// (theta / l, kt dB/dl / l) for the gradient.
 // Every entry is a double-word (hi, lo).
 
-__global__ void k_split_dw(int nv, const double* __restrict__ P, float4* __restrict__ X, float* __restrict__ P32) {
-  int v = blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= nv) return;
-  float hx, hy, hz, lx, ly, lz;
-  split_bits(P[3 * v], &hx, &lx);
-  split_bits(P[3 * v + 1], &hy, &ly);
-  split_bits(P[3 * v + 2], &hz, &lz);
-  X[v] = make_float4(hx, hy, hz, 0.0f);
-  X[nv + v] = make_float4(lx, ly, lz, 0.0f);
-  // the float copy of the positions read by the repulsion prefilter
-  P32[3 * v] = hx;
-  P32[3 * v + 1] = hy;
-  P32[3 * v + 2] = hz;
+// What the stages of one evaluation work on.
+struct DwEval {
+  Topo t;
+  const double* P;  // positions
+  float4* X;        // PosDW records
+  float* P32;       // float copy of the positions (repulsion prefilter)
+  float4 *fd, *fav, *eg, *elt;
+  const float4* sct;
+  EP ep;
+  EPD epd;
+  // repulsion: rep 0 none, 1 with near rows or Verlet rows, 2 without
+  int rep, use_near, excl_fresh;
+  NLView nl;
+  const double* xb;  // positions the near rows were built at
+  double thr2;
+  float thr;
+  int* moved;  // per block of the split stage: some vertex left its skin
+  int nmoved;
+  double *pot, *repg;
+  int *slow, *nslow;
+  double* partial;
+  Globals* g;
+  double* energy;  // energy of the evaluation, may be NULL
+  double* grad;    // NULL: energy only
+};
+
+// The velocity-Verlet update that precedes an evaluation inside an HMC move
+// (kick with the last two forces, drift): per vertex, so the split stage
+// does it on the fly instead of a pass of its own over x, p and g.
+struct DwMove {
+  double *x, *p;
+  const double *g0, *g1;  // g1 NULL: drift only, with g0
+  double dt, im;
+};
+
+__device__ __forceinline__ df3 pos_of(const float4* X, int v) { return PosDW{X}.at(v); }
+__device__ __forceinline__ df3 pos_of(const float4* X, int v, df* kr) { return PosDW{X}.at(v, kr); }
+
+// ---- stage 1: positions ------------------------------------------------------
+// Returns whether the vertex has left the skin of the near rows (the test of
+// k_moved, decided in float when the float distance is clearly inside: the
+// margin is four times the rounding of the two positions).
+template <bool MOVE>
+__device__ __forceinline__ bool split_vertex(const DwEval& a, const DwMove& mv, int v) {
+  double x[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const size_t i = 3 * (size_t)v + k;
+    if (MOVE) {
+      double pn = mv.p[i], f = -mv.g0[i];
+      if (mv.g1) {
+        const double f1 = -mv.g1[i];
+        pn = pn + 0.5 * (f + f1) * mv.dt;
+        mv.p[i] = pn;
+        f = f1;
+      }
+      x[k] = mv.x[i] + (pn * mv.dt + 0.5 * f * (mv.dt * mv.dt)) * mv.im;
+      mv.x[i] = x[k];
+    } else {
+      x[k] = a.P[i];
+    }
+  }
+  float h[3], l[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) split_bits(x[k], &h[k], &l[k]);
+  st32(a.X + 2 * (size_t)v, make_float4(h[0], h[1], h[2], 0.0f), make_float4(l[0], l[1], l[2], 0.0f));
+  if (!a.rep) return false;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) a.P32[3 * (size_t)v + k] = h[k];
+  if (!a.use_near) return false;
+  double b[3];
+  float s = 0.0f, m = 0.0f;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    b[k] = __ldg(a.xb + 3 * (size_t)v + k);
+    float bh, bl;
+    split_bits(b[k], &bh, &bl);
+    const float d = h[k] - bh;
+    s = fmaf(d, d, s);
+    m = fmaxf(m, fmaxf(fabsf(h[k]), fabsf(bh)));
+  }
+  const float in = a.thr - 1e-6f * m;
+  if (in > 0.0f && s < 0.999f * in * in) return false;
+  const double dx = x[0] - b[0], dy = x[1] - b[1], dz = x[2] - b[2];
+  return !(dx * dx + dy * dy + dz * dz < a.thr2);  // NaN counts as moved
 }
 
-// fav: (area, volume) again as (hi, lo, hi, lo), compact for k_vertex_dw
-__global__ void __launch_bounds__(256) k_face_dw(Topo t, PosDW X, float4* __restrict__ fd, float4* __restrict__ fav) {
-  int f = blockIdx.x * blockDim.x + threadIdx.x;
-  if (f >= t.nf) return;
-  const int a = t.fv[3 * f], b = t.fv[3 * f + 1], c = t.fv[3 * f + 2];
-  const df3 pa = X.at(a), pb = X.at(b), pc = X.at(c);
+// ---- stage 2: faces, and the repulsion of the vertices -----------------------
+__device__ __forceinline__ void face_dw(const DwEval& q, int a, int b, int c, int f) {
+  const df3 pa = pos_of(q.X, a), pb = pos_of(q.X, b), pc = pos_of(q.X, c);
   const df3 eab = sub3(pb, pa), eac = sub3(pc, pa), ebc = sub3(pc, pb);
   const df3 N = cross3(eab, eac);
   const df n2 = dot3(N, N);
@@ -73,14 +155,180 @@ __global__ void __launch_bounds__(256) k_face_dw(Topo t, PosDW X, float4* __rest
   const df c0 = mul_s(dot3(eab, eac), r);
   const df c1 = neg(mul_s(dot3(eab, ebc), r));
   const df c2 = mul_s(dot3(eac, ebc), r);
-  float4* o = fd + 4 * (size_t)f;
-  o[0] = make_float4(nx.hi, nx.lo, ny.hi, ny.lo);
-  o[1] = make_float4(nz.hi, nz.lo, A.hi, A.lo);
-  o[2] = make_float4(V.hi, V.lo, c0.hi, c0.lo);
-  o[3] = make_float4(c1.hi, c1.lo, c2.hi, c2.lo);
-  fav[f] = make_float4(A.hi, A.lo, V.hi, V.lo);
+  float4* o = q.fd + 4 * (size_t)f;
+  st32(o, make_float4(nx.hi, nx.lo, ny.hi, ny.lo), make_float4(nz.hi, nz.lo, A.hi, A.lo));
+  st32(o + 2, make_float4(c0.hi, c0.lo, c1.hi, c1.lo), make_float4(c2.hi, c2.lo, 0.0f, 0.0f));
+  q.fav[f] = make_float4(A.hi, A.lo, V.hi, V.lo);
 }
 
+// Whether the near rows serve this evaluation: 0 no, 1 rows and exclusion
+// flags, 2 rows with the exclusion tested (the topology has changed since).
+// Called by whole blocks.
+__device__ __forceinline__ int near_mode_of(const DwEval& q) {
+  if (!q.use_near) return 0;
+  bool mv = false;
+  for (int b = threadIdx.x; b < q.nmoved; b += blockDim.x) mv = mv || ((volatile int*)q.moved)[b] != 0;
+  if (__syncthreads_or(mv)) return 0;
+  if (q.nl.nflag[1] != 0) return 0;
+  return q.nl.nflag[2] == *q.nl.dtopo ? 1 : 2;
+}
+
+// Pair term of the repulsion and (grad) its derivative over l times the
+// distance vector
+struct RepTerm {
+  double pot, gx, gy, gz;
+};
+template <bool GRAD>
+__device__ __forceinline__ RepTerm rep_term(const EP& ep, double l, d3 dv) {
+  const double lmc = l - ep.rlc1;
+  const double ilmc = 1.0 / lmc, il = 1.0 / l;
+  const double ex = exp(l * ilmc) * ipow(il, ep.rr);
+  RepTerm r{ex, 0.0, 0.0, 0.0};
+  if (GRAD) {
+    const double fac = -(ep.rlc1 * (ilmc * ilmc) + ep.rr * il) * (ex * il);
+    r.gx = fac * dv.x;
+    r.gy = fac * dv.y;
+    r.gz = fac * dv.z;
+  }
+  return r;
+}
+
+// The repulsion of vertex v by its RL lanes (1 or NEAR_HITS): each lane tests
+// every RL-th row entry (one coalesced load of the row instead of one
+// thread's serial walk).  Near rows: the accepted pairs go to the group's
+// slots in shared memory, one lane evaluates each, and they are added in the
+// reference's visiting order (the rows' own order depends on when they were
+// built).  Verlet rows keep their order between rebuilds: each lane sums its
+// own pairs, then a fixed shuffle tree.  Vertices that need the cell walk
+// are queued.
+struct RepSlots {
+  long long key[NEAR_HITS];
+  double s[NEAR_HITS];
+};
+template <bool GRAD, int RL>
+__device__ __forceinline__ void rep_vertex(const DwEval& q, int v, int sub, int near_mode, RepSlots* slots) {
+  const NLView& nl = q.nl;
+  const EP& ep = q.ep;
+  static_assert(RL == 1 || RL == NEAR_HITS, "one lane per accepted pair");
+  const unsigned gmask = ((1u << RL) - 1u) << (threadIdx.x & 31 & ~(RL - 1));
+  const d3 p = ld3p(q.P, v);
+  const PairTest pt = make_pair_test(nl, v, ep.rlc1, ep.rT);
+  TableExcl x{q.t, nl.excl};
+  RepTerm sum{0.0, 0.0, 0.0, 0.0};
+  auto add = [&](int, double l, d3 dv) {
+    const RepTerm r = rep_term<GRAD>(ep, l, dv);
+    sum.pot += r.pot;
+    sum.gx += r.gx;
+    sum.gy += r.gy;
+    sum.gz += r.gz;
+  };
+  if (nl.kind == 0 && !near_mode) {  // candidate rows or the cell walk
+    bool fast = false;
+    if (sub == 0) {
+      int co[3];
+      fast = in_build_cell(nl, v, p, co);
+      if (fast) {
+        visit_candidates(pt, nl, q.P, v, p, x, add);
+      } else {
+        q.slow[atomicAdd(q.nslow, 1)] = v;
+      }
+    }
+    if (!fast) return;
+  } else if (nl.kind == 0 && RL == 1) {
+    int co[3];
+    in_build_cell(nl, v, p, co);
+    if (!visit_near(pt, nl, q.P, v, p, near_mode, co, x, add)) {
+      q.slow[atomicAdd(q.nslow, 1)] = v;
+      return;
+    }
+  } else if (nl.kind == 0) {
+    const int* row = nl.nent + (size_t)v * TM_NEAR_CAP;
+    const int n = nl.ncnt[v];
+    int co[3];
+    bool have_co = false;
+    int total = 0;
+    for (int e0 = 0; e0 < n; e0 += RL) {
+      const int e = e0 + sub;
+      bool acc = false;
+      long long key = 0;
+      double s = 0.0;
+      if (e < n) {
+        const int c = row[e], j = c & 0x7fffffff;
+        d3 pj;
+        if (!(near_mode == 1 && c < 0) && pair_within(pt, nl, q.P, p, j, &pj, &s)) {
+          if (!have_co) in_build_cell(nl, v, p, co);
+          have_co = true;
+          const int ox = nl.bcoord[3 * j] - co[0], oy = nl.bcoord[3 * j + 1] - co[1], oz = nl.bcoord[3 * j + 2] - co[2];
+          acc = ox >= -1 && ox <= 1 && oy >= -1 && oy <= 1 && oz >= -1 && oz <= 1 &&
+                !(near_mode == 2 && nl.excl > 0 && x(v, j));
+          key = ((long long)((ox + 1) * 9 + (oy + 1) * 3 + (oz + 1)) << 32) | (long long)j;
+        }
+      }
+      const unsigned b = __ballot_sync(gmask, acc);
+      const int pos = total + __popc(b & ((1u << (threadIdx.x & 31)) - 1u));
+      if (acc && pos < NEAR_HITS) {
+        slots->key[pos] = key;
+        slots->s[pos] = s;
+      }
+      total += __popc(b);
+    }
+    if (total > NEAR_HITS) {
+      if (sub == 0) q.slow[atomicAdd(q.nslow, 1)] = v;
+      return;
+    }
+    if (total > 0) {
+      __syncwarp(gmask);
+      RepTerm r{0.0, 0.0, 0.0, 0.0};
+      int rank = -1;
+      if (sub < total) {
+        const long long k = slots->key[sub];
+        rank = 0;
+        for (int o = 0; o < total; ++o) rank += slots->key[o] < k ? 1 : 0;
+        r = rep_term<GRAD>(ep, __dsqrt_rn(slots->s[sub]), exact_diff(p, ld3p(q.P, (int)(k & 0xffffffff))));
+      }
+      __syncwarp(gmask);
+      for (int h = 0; h < total; ++h) {
+        const int src = __ffs(__ballot_sync(gmask, rank == h)) - 1;
+        sum.pot += __shfl_sync(gmask, r.pot, src);
+        if (GRAD) {
+          sum.gx += __shfl_sync(gmask, r.gx, src);
+          sum.gy += __shfl_sync(gmask, r.gy, src);
+          sum.gz += __shfl_sync(gmask, r.gz, src);
+        }
+      }
+    }
+  } else {
+    const int lo = nl.vrow[v], hi = nl.vrow[v + 1];
+    for (int e = lo + sub; e < hi; e += RL) {
+      const int j = nl.vcol[e];
+      d3 pj;
+      double s;
+      if (!pair_within(pt, nl, q.P, p, j, &pj, &s)) continue;
+      // the rows leave out the pairs excluded when they were built
+      if (!q.excl_fresh && nl.excl > 0 && x(v, j)) continue;
+      add(j, __dsqrt_rn(s), exact_diff(p, pj));
+    }
+    __syncwarp(gmask);
+    const unsigned any = __ballot_sync(gmask, sum.pot != 0.0);
+    if (RL > 1 && any) {  // (no FP64 shuffle tree where no lane has a pair)
+#pragma unroll
+      for (int o = RL / 2; o > 0; o >>= 1) {
+        sum.pot += __shfl_down_sync(gmask, sum.pot, o);
+        if (GRAD) {
+          sum.gx += __shfl_down_sync(gmask, sum.gx, o);
+          sum.gy += __shfl_down_sync(gmask, sum.gy, o);
+          sum.gz += __shfl_down_sync(gmask, sum.gz, o);
+        }
+      }
+    }
+  }
+  if (sub == 0) {
+    q.pot[v] = sum.pot;
+    if (GRAD) st3(q.repg, v, 2.0 * mk(sum.gx, sum.gy, sum.gz));
+  }
+}
+
+// ---- stage 3: edges, and the queued repulsion --------------------------------
 // Flat-bottom bond of an edge shorter than lc1 (src/mesh_tether.h:29-85)
 // in double-word arithmetic: value e^(l/(l-lc1)) / l^r, derivative
 // -(lc1/(l-lc1)^2 + r/l) e^(l/(l-lc1)) / l^r (plus the l > lc0 branch when
@@ -103,29 +351,27 @@ __device__ __forceinline__ void edge_bond_short_dw(const EP& ep, const EPD& epd,
   *fac = mul_s(mul_s(f, ilr), ex);
 }
 
-// elt: (l theta, bond value) as (hi, lo, hi, lo), compact for k_vertex_dw
-__global__ void __launch_bounds__(256) k_edge_dw(Topo t, PosDW X, const float4* __restrict__ fd,
-                                                float4* __restrict__ ed, float4* __restrict__ elt, EP ep, EPD epd,
-                                                const float4* __restrict__ sct) {
-  int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= t.ne) return;
-  const int4 E = t.edge[e];
-  const df3 ev = sub3(X.at(E.y), X.at(E.x));
+
+__device__ __forceinline__ void edge_dw(const DwEval& q, int4 E, int e) {
+  const EP& ep = q.ep;
+  const EPD& epd = q.epd;
+  const df3 ev = sub3(pos_of(q.X, E.y), pos_of(q.X, E.x));
   const df l2 = dot3(ev, ev);
   const df il = rsqrt_dw(l2);
   const df l = mul_s(l2, il);
   df th = df_make(0.0f);
   const bool interior = E.z >= 0 && E.w >= 0;
   if (interior) {
-    const float4 a0 = __ldg(fd + 4 * (size_t)E.z), a1 = __ldg(fd + 4 * (size_t)E.z + 1);
-    const float4 b0 = __ldg(fd + 4 * (size_t)E.w), b1 = __ldg(fd + 4 * (size_t)E.w + 1);
+    float4 a0, a1, b0, b1;
+    ld32(q.fd + 4 * (size_t)E.z, a0, a1);
+    ld32(q.fd + 4 * (size_t)E.w, b0, b1);
     const df3 n0 = {{a0.x, a0.y}, {a0.z, a0.w}, {a1.x, a1.y}};
     const df3 n1 = {{b0.x, b0.y}, {b0.z, b0.w}, {b1.x, b1.y}};
     // n0 x n1 lies along the shared edge: its projection on the unit edge
     // is the signed sine, with the sign of the reference's test
     // (n0 x n1) . e >= 0
     const df sd = mul_s(dot3(cross3(n0, n1), ev), il);
-    th = angle_dw(sd, dot3(n0, n1), sct);
+    th = angle_dw(sd, dot3(n0, n1), q.sct);
   }
   // flat-bottom edge penalty: above the flat bottom products only, below it
   // the exponential (a warp with any short edge takes that branch; on the
@@ -150,48 +396,102 @@ __global__ void __launch_bounds__(256) k_edge_dw(Topo t, PosDW X, const float4* 
       db = df_from(f);
     }
   }
-  const df ils = interior ? il : neg(il);
-  ed[2 * (size_t)e] = make_float4(l.hi, l.lo, th.hi, th.lo);
-  ed[2 * (size_t)e + 1] = make_float4(db.hi, db.lo, ils.hi, ils.lo);
-  const df lt = mul_s(l, th);
-  elt[e] = make_float4(lt.hi, lt.lo, val.hi, val.lo);
+  const df lt = mul_s(l, th), tl = mul_s(th, il), kd = mul_s(mul_s(epd.kt, db), il);
+  q.eg[e] = make_float4(tl.hi, tl.lo, kd.hi, kd.lo);
+  q.elt[e] = make_float4(lt.hi, lt.lo, val.hi, val.lo);
 }
 
-// Per-vertex ring sums, the six properties, the curvature weights
-// (kb rho, 2/3 kb rho^2) for the gradient, and the global sums: a
-// double-word shuffle tree per warp, FP64 over the warps of a block in warp
-// order, and the last block (atomic ticket) reduces the block partials in
-// block order and assembles energy and the penalty factors.  Fixed order
-// throughout: results are bit-reproducible.
-__global__ void __launch_bounds__(VB, 4) k_vertex_dw(Topo t, const float4* __restrict__ fav,
-                                                 const float4* __restrict__ elt, const double* __restrict__ reppot,
-                                                 EP ep, EPD epd, float4* __restrict__ rk, double* __restrict__ partial,
-                                                 Globals* g) {
-  constexpr int NW = VB / 32;
-  __shared__ float2 wsum[6][NW];
-  __shared__ double redd[6];
-  __shared__ bool last;
-  const int v = blockIdx.x * VB + threadIdx.x;
-  df pr[6];
+// One warp per queued vertex: lane l < 27 scans neighbour cell l (the
+// reference's x-outer / z-inner order), then the lanes' sums are combined by
+// a fixed shuffle tree, so the result does not depend on timing.
+template <bool GRAD>
+__device__ __forceinline__ void rep_queue(const DwEval& q, int warp, int nwarps) {
+  const int n = *(volatile int*)q.nslow;
+  const int lane = threadIdx.x & 31;
+  const NLView& nl = q.nl;
+  const NLGeom& G = *nl.geom;
+  TableExcl x{q.t, nl.excl};
+  for (int i = warp; i < n; i += nwarps) {
+    const int v = ((volatile int*)q.slow)[i];
+    const d3 p = ld3p(q.P, v);
+    const PairTest pt = make_pair_test(nl, v, q.ep.rlc1, q.ep.rT);
+    RepTerm sum{0.0, 0.0, 0.0, 0.0};
+    int co[3];
+    in_build_cell(nl, v, p, co);
+    if (lane < 27) {
+      const int ii = co[0] + lane / 9 - 1, jj = co[1] + (lane / 3) % 3 - 1, kk = co[2] + lane % 3 - 1;
+      if (ii >= 0 && ii < G.shape[0] && jj >= 0 && jj < G.shape[1] && kk >= 0 && kk < G.shape[2]) {
+        const long long cid = ii * G.stride[0] + jj * G.stride[1] + kk * G.stride[2];
+        int st = 0;
+        const int cnt = cell_find(nl, cell_key(cid, 0), &st);
+        auto add = [&](int, double l, d3 dv) {
+          const RepTerm r = rep_term<GRAD>(q.ep, l, dv);
+          sum.pot += r.pot;
+          sum.gx += r.gx;
+          sum.gy += r.gy;
+          sum.gz += r.gz;
+        };
+        for (int c = 0; c < cnt; ++c) {
+          const int j = nl.cell_verts[st + c];
+          if (j != v) visit_pair(pt, nl, q.P, v, p, j, x, add);
+        }
+      }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      sum.pot += __shfl_down_sync(0xffffffffu, sum.pot, o);
+      if (GRAD) {
+        sum.gx += __shfl_down_sync(0xffffffffu, sum.gx, o);
+        sum.gy += __shfl_down_sync(0xffffffffu, sum.gy, o);
+        sum.gz += __shfl_down_sync(0xffffffffu, sum.gz, o);
+      }
+    }
+    if (lane == 0) {
+      q.pot[v] = sum.pot;
+      if (GRAD) st3(q.repg, v, 2.0 * mk(sum.gx, sum.gy, sum.gz));
+    }
+  }
+}
+
+// ---- stage 4: vertices and global sums ---------------------------------------
+// Sum of x over the L lanes of a vertex (adjacent lanes, L a power of two);
+// every lane ends with the same sum.  Called by whole warps.
+template <int L>
+__device__ __forceinline__ df lane_sum(df x) {
+#pragma unroll
+  for (int q = L / 2; q > 0; q >>= 1)
+    x = add_s(x, df{__shfl_xor_sync(0xffffffffu, x.hi, q), __shfl_xor_sync(0xffffffffu, x.lo, q)});
+  return x;
+}
+
+// The six properties of vertex v from its ring into pr (lane 0 of the
+// vertex's L lanes, each with a run of ceil(d / L) ring slots), and the
+// curvature weight kb c/a for the gradient into the free entries of the
+// position record.
+template <int L>
+__device__ __forceinline__ void vertex_dw(const DwEval& q, int v, int sub, df* pr) {
+  const Topo& t = q.t;
+  dacc A = {0.0f, 0.0f}, Vo = A, LT = A, T = A;
+#pragma unroll
   for (int k = 0; k < 6; ++k) pr[k] = df_make(0.0f);
   if (v < t.nv) {
     const int d = t.val[v];
-    dacc A = {0.0f, 0.0f}, Vo = A, LT = A, T = A;
-    // slots in groups of six (one group at the usual valence): all loads of
-    // a group are issued before the sums, which keep the slot order
-    constexpr int G = 6;
-    for (int m0 = 0; m0 < d; m0 += G) {
+    const int run = (d + L - 1) / L, m1 = min(d, (sub + 1) * run);
+    // slots in groups (one group at the usual valence): all loads of a group
+    // are issued before the sums, which keep the slot order
+    constexpr int G = (6 + L - 1) / L;
+    for (int m0 = sub * run; m0 < m1; m0 += G) {
       int4 s[G];
 #pragma unroll
-      for (int k = 0; k < G; ++k) s[k] = m0 + k < d ? t.slot[(size_t)(m0 + k) * t.nv + v] : make_int4(0, -1, 0, 0);
+      for (int k = 0; k < G; ++k) s[k] = m0 + k < m1 ? t.slot[(size_t)(m0 + k) * t.nv + v] : make_int4(0, -1, 0, 0);
       float4 av[G], lb[G];
 #pragma unroll
       for (int k = 0; k < G; ++k) {
         const int f = slot_face(s[k].y);
         av[k] = lb[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         if (f >= 0) {
-          av[k] = __ldg(fav + f);
-          lb[k] = __ldg(elt + s[k].z);
+          av[k] = __ldg(q.fav + f);
+          lb[k] = __ldg(q.elt + s[k].z);
         }
       }
 #pragma unroll
@@ -200,178 +500,323 @@ __global__ void __launch_bounds__(VB, 4) k_vertex_dw(Topo t, const float4* __res
         acc_add(A, lo_hi(av[k].x, av[k].y));
         acc_add(Vo, lo_hi(av[k].z, av[k].w));
         acc_add(LT, lo_hi(lb[k].x, lb[k].y));
-        if (ep.btype == 0) {
+        if (q.ep.btype == 0) {
           acc_add(T, lo_hi(lb[k].z, lb[k].w));
         } else {
-          const df q = sub_s(mul_s(lo_hi(av[k].x, av[k].y), epd.inv_a0), df_make(1.0f));
-          acc_add(T, mul_s(q, q));
+          const df z = sub_s(mul_s(lo_hi(av[k].x, av[k].y), q.epd.inv_a0), df_make(1.0f));
+          acc_add(T, mul_s(z, z));
         }
       }
     }
-    const df a = mul_s(acc_val(A), third());
-    const df c = ldexp2(acc_val(LT), 0.25f);
-    const df ia = rcp_dw(a);
-    const df rho = mul_s(c, ia);
+  }
+  const df sA = lane_sum<L>(acc_val(A)), sV = lane_sum<L>(acc_val(Vo)), sLT = lane_sum<L>(acc_val(LT)),
+           sT = lane_sum<L>(acc_val(T));
+  if (v < t.nv && sub == 0) {
+    const df a = mul_s(sA, third());
+    const df c = ldexp2(sLT, 0.25f);
+    const df rho = mul_s(c, rcp_dw(a));
     pr[0] = a;
-    pr[1] = mul_s(acc_val(Vo), third());
+    pr[1] = mul_s(sV, third());
     pr[2] = c;
     pr[3] = ldexp2(mul_s(c, rho), 2.0f);  // 2 c^2 / a
-    pr[4] = mul_s(acc_val(T), epd.inv_tdiv);
-    split_bits(reppot[v], &pr[5].hi, &pr[5].lo);  // integer operations, no FP64
-    const df kr = mul_s(epd.kb, rho), kq = mul_s(epd.kb23, mul_s(rho, rho));
-    rk[v] = make_float4(kr.hi, kr.lo, kq.hi, kq.lo);
+    pr[4] = mul_s(sT, q.epd.inv_tdiv);
+    if (q.rep) split_bits(__ldg(q.pot + v), &pr[5].hi, &pr[5].lo);
+    const df kr = mul_s(q.epd.kb, rho);
+    q.X[2 * (size_t)v].w = kr.hi;
+    q.X[2 * (size_t)v + 1].w = kr.lo;
   }
-  // warp tree (lane 0 ends with the warp's sum), then FP64 over the warps
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1)
-#pragma unroll
-    for (int k = 0; k < 6; ++k) {
-      const df o = {__shfl_down_sync(0xffffffffu, pr[k].hi, off), __shfl_down_sync(0xffffffffu, pr[k].lo, off)};
-      pr[k] = add_s(pr[k], o);
-    }
+}
+
+// Sums of the six properties over a block into partial[0..5] (FP64).  Warp
+// sums by halving (each step a lane keeps half of its values and adds the
+// partner's): 8 additions per lane instead of the 30 of six shuffle trees,
+// which were half of the vertex stage's instructions.  The lanes' bits 4..2
+// select the property they end with.  Then property k is summed over the
+// warps in warp order by thread k, with one FP64 conversion per block
+// (GB300's FP64 pipe is the scarce one).
+template <int NW>
+__device__ __forceinline__ void block_props(const df* pr, float2 (*wsum)[NW], double* partial) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  if (lane == 0)
-    for (int k = 0; k < 6; ++k) wsum[k][w] = make_float2(pr[k].hi, pr[k].lo);
+  auto swap_add = [](bool up, const df& a, const df& b, int o) {  // keep a (up: b), add the partner's same one
+    const df keep = up ? b : a, send = up ? a : b;
+    return add_s(keep, df{__shfl_xor_sync(0xffffffffu, send.hi, o), __shfl_xor_sync(0xffffffffu, send.lo, o)});
+  };
+  const df zero = df_make(0.0f);
+  const df q0 = swap_add(lane & 16, pr[0], pr[3], 16), q1 = swap_add(lane & 16, pr[1], pr[4], 16),
+           q2 = swap_add(lane & 16, pr[2], pr[5], 16);
+  const df r0 = swap_add(lane & 8, q0, q2, 8), r1 = swap_add(lane & 8, q1, zero, 8);
+  df r = swap_add(lane & 4, r0, r1, 4);
+#pragma unroll
+  for (int o = 2; o > 0; o >>= 1)
+    r = add_s(r, df{__shfl_xor_sync(0xffffffffu, r.hi, o), __shfl_xor_sync(0xffffffffu, r.lo, o)});
+  const int prop = (lane & 16 ? 3 : 0) + (lane & 8 ? 2 : (lane & 4 ? 1 : 0));
+  if ((lane & 3) == 0 && (lane & 12) != 12) wsum[prop][w] = make_float2(r.hi, r.lo);
   __syncthreads();
-  // property k of the block: thread k sums the warps in warp order (one
-  // FP64 conversion per block: GB300's FP64 pipe is the scarce one)
   if (threadIdx.x < 6) {
     df s = df_make(0.0f);
-    for (int q = 0; q < NW; ++q) s = add_s(s, lo_hi(wsum[threadIdx.x][q].x, wsum[threadIdx.x][q].y));
-    partial[8 * (size_t)blockIdx.x + threadIdx.x] = df_to(s);
+    for (int k = 0; k < NW; ++k) s = add_s(s, lo_hi(wsum[threadIdx.x][k].x, wsum[threadIdx.x][k].y));
+    partial[threadIdx.x] = df_to(s);
   }
+}
+// Property w (warp w < 6) over nb block partials: lane l takes blocks l,
+// l + 32, ... in order, then a fixed shuffle tree
+__device__ __forceinline__ void total_props(const double* partial, int nb, double* redd) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (w < 6) {
+    double acc = 0.0;
+    for (int b = lane; b < nb; b += 32) acc += __ldcg(partial + 8 * (size_t)b + w);
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, off);
+    if (lane == 0) redd[w] = acc;
+  }
+}
+
+// ---- stage 5: gradient ---------------------------------------------------------
+// Gradient gather per vertex i over its ring (slot m: face (i, j = r_m,
+// k = r_{m-1})), the reference's gather (src/mesh_properties.cpp:51-148 with
+// src/kernel.h:124-137) with every term written along the edge vectors
+// d_j = x_j - x_i and the face normals n, so that each slot needs two scaled
+// vectors and no cross product (the area gradient in its cotangent form and
+// the volume gradient through the normal, Meyer, Desbrun, Schroeder & Barr,
+// "Discrete differential-geometry operators for triangulated 2-manifolds",
+// 2003).  With h = alpha / 2, alpha = gA - 2/3 kb (rho_i^2 + rho_j^2 +
+// rho_k^2), and w = gC/2 + kb (rho_i + rho_j):
+//   area       -h (cot_k d_j + cot_j d_k)       [= h n x (x_k - x_j)]
+//   volume     gV/3 A n                         [= gV/6 d_j x d_k; the
+//              x_i x (d_k - d_j) / 6 parts cancel around a closed fan]
+//   length     -(w theta + kt dB/dl) / l d_j    for edge (i, j)
+//   dihedral   (w_ij cot_j + w_ik cot_k - w_jk (cot_j + cot_k)) n
+// Positions enter relative to x_i, so the sums stay near the size of the
+// result.  Per slot a lane gathers four sectors: the neighbour's position
+// and weight, the face's two, the edge's 16 bytes.
+// L lanes share a vertex, each with a run of ceil(d / L) slots; the part of
+// a run's first face on d_k (the previous run's last vector) is added
+// directly, later ones complete the coefficient of the vector before.
+__device__ __forceinline__ df cot_of(const float4& F2, const float4& F3, int c) {
+  return c == 0 ? lo_hi(F2.x, F2.y) : (c == 1 ? lo_hi(F2.z, F2.w) : lo_hi(F3.x, F3.y));
+}
+// 2/3 kb rho^2 from kb rho (epd.kq = 2 s / (3 kb), epd.iks = 1 / s with s the
+// power of two at kb: no under- or overflow of the square)
+__device__ __forceinline__ df kq_of(const EPD& epd, df kr) {
+  return mul_s(mul_s(ldexp2(kr, epd.iks), kr), epd.kq);
+}
+
+template <bool CLOSED, int L>
+__device__ __forceinline__ void grad_dw(const DwEval& q, int i, int sub, df gA, df gV, df gC) {
+  const Topo& t = q.t;
+  const EPD& epd = q.epd;
+  dacc3 acc = {{0.0f, 0.0f}, {0.0f, 0.0f}, {0.0f, 0.0f}};
+  dacc3 vtel = acc;
+  df3 xi = {df_make(0.0f), df_make(0.0f), df_make(0.0f)};
+  if (i < t.nv) {
+    const df gV3 = mul_s(gV, third());
+    const df hgC = half(gC);
+    df kri;
+    xi = pos_of(q.X, i, &kri);
+    const df ai = sub_s(gA, kq_of(epd, kri));
+    const df wi = add_s(hgC, kri);
+    const int d = t.val[i];
+    const int run = (d + L - 1) / L, mb = sub * run, m1 = min(d, mb + run);
+    const size_t nv = t.nv;
+    if (mb < m1) {
+      const int4 sp = t.slot[(size_t)(mb == 0 ? d - 1 : mb - 1) * nv + i];
+      df krk;
+      df3 dk = sub3(pos_of(q.X, sp.x, &krk), xi);
+      df qk = kq_of(epd, krk);
+      df uk = add_s(hgC, krk);
+      df wk = add_s(wi, krk);  // weight of edge (i, k)
+      bool fprev = slot_face(sp.y) >= 0;
+      int4 sc = t.slot[(size_t)mb * nv + i];
+      dacc s = {0.0f, 0.0f};  // coefficient of d_k still open
+      for (int m = mb; m < m1; ++m) {
+        // the next slot's row is fetched one slot ahead; on an open fan it
+        // also tells whether edge (i, j) has a face on either side
+        int4 sn = sc;
+        if (!CLOSED || m + 1 < m1) sn = t.slot[(size_t)(m + 1 == d ? 0 : m + 1) * nv + i];
+        df krj;
+        const df3 dj = sub3(pos_of(q.X, sc.x, &krj), xi);
+        const df qj = kq_of(epd, krj);
+        const df wj = add_s(wi, krj);
+        const int f = slot_face(sc.y);
+        const float4 E = __ldg(q.eg + sc.z);
+        dacc sj = {0.0f, 0.0f};
+        if (CLOSED || f >= 0) {
+          float4 F0, F1, F2, F3;
+          ld32(q.fd + 4 * (size_t)f, F0, F1);
+          ld32(q.fd + 4 * (size_t)f + 2, F2, F3);
+          const int ci = slot_corner(sc.y);
+          const df cj = cot_of(F2, F3, ci == 2 ? 0 : ci + 1), ck = cot_of(F2, F3, ci == 0 ? 2 : ci - 1);
+          df alpha = sub_s(sub_s(ai, qj), qk);
+          if (q.ep.btype == 1) {
+            const df z = sub_s(mul_s(lo_hi(F1.z, F1.w), epd.inv_a0), df_make(1.0f));
+            alpha = add_s(alpha, ldexp2(mul_s(mul_s(epd.kt, z), epd.inv_a0), 2.0f));
+          }
+          const df h = half(neg(alpha));
+          // edge (i, k): this face completes its coefficient
+          acc_fma(s, h, cj);
+          acc_fma3(acc, acc_val(s), dk);
+          // edge (i, j): length and area terms
+          acc_fma(sj, neg(wj), lo_hi(E.x, E.y));
+          if (q.ep.btype == 0) acc_add(sj, neg(lo_hi(E.z, E.w)));
+          acc_fma(sj, h, ck);
+          // along n
+          dacc c = {0.0f, 0.0f};
+          acc_fma(c, gV3, lo_hi(F1.z, F1.w));
+          bool in_ij = true, in_ik = true, in_jk = true;
+          if (!CLOSED) {
+            in_ij = slot_face(sn.y) >= 0;
+            in_ik = fprev;
+            const int4 ejk = t.edge[sc.w];
+            in_jk = ejk.z >= 0 && ejk.w >= 0;
+          }
+          if (in_ij) acc_fma(c, wj, cj);
+          if (in_ik) acc_fma(c, wk, ck);
+          if (in_jk) acc_fma(c, neg(add_s(uk, krj)), add_s(cj, ck));
+          acc_fma3(acc, acc_val(c), {{F0.x, F0.y}, {F0.z, F0.w}, {F1.x, F1.y}});
+          if (!CLOSED) acc_add3(vtel, sub3(dk, dj));
+        } else {
+          // no face: the edge before it has no more terms
+          acc_fma3(acc, acc_val(s), dk);
+        }
+        fprev = f >= 0;
+        s = sj;
+        dk = dj;
+        qk = qj;
+        uk = add_s(hgC, krj);
+        wk = wj;
+        sc = sn;
+      }
+      acc_fma3(acc, acc_val(s), dk);  // the run's last edge
+    }
+  }
+  df3 r = acc_val3(acc);
+  if (L > 1) r = {lane_sum<L>(r.x), lane_sum<L>(r.y), lane_sum<L>(r.z)};
+  if (!CLOSED) {
+    df3 tel = acc_val3(vtel);
+    if (L > 1) tel = {lane_sum<L>(tel.x), lane_sum<L>(tel.y), lane_sum<L>(tel.z)};
+    const df3 tx = scale3(mul_s(gV, sixth()), cross3(xi, tel));
+    r = {add_s(r.x, tx.x), add_s(r.y, tx.y), add_s(r.z, tx.z)};
+  }
+  if (i >= t.nv || sub != 0) return;
+  double o[3] = {df_to(r.x), df_to(r.y), df_to(r.z)};
+  if (q.rep) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      o[k] = o[k] + q.ep.kr * __ldg(q.repg + 3 * (size_t)i + k);
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 3; ++k) q.grad[3 * (size_t)i + k] = o[k];
+}
+
+// ---- the five kernels ----------------------------------------------------------
+// Each stage is a kernel; the repulsion runs as extra blocks of the face and
+// edge kernels (its queue between the two), so the kernels form one chain.
+// Every kernel but the first is launched with programmatic stream
+// serialisation: it may start while the one before drains, fetches its
+// topology rows (which no evaluation writes) and only then waits.
+__device__ __forceinline__ void wait_previous() { cudaGridDependencySynchronize(); }
+__device__ __forceinline__ void let_next_start() { cudaTriggerProgrammaticLaunchCompletion(); }
+
+constexpr int SB = 256;  // threads per block of the split, face and edge kernels
+
+template <bool MOVE>
+__global__ void __launch_bounds__(SB) k_split_dw(const __grid_constant__ DwEval q, const __grid_constant__ DwMove mv) {
+  let_next_start();
+  const int v = blockIdx.x * SB + threadIdx.x;
+  const bool m = v < q.t.nv && split_vertex<MOVE>(q, mv, v);
+  if (q.use_near) {
+    const int any = __syncthreads_or(m);
+    if (threadIdx.x == 0) q.moved[blockIdx.x] = any;
+  }
+  if (v == 0) *q.nslow = 0;
+}
+
+// blocks [0, nrep): repulsion, RL lanes per vertex; the others: faces
+template <bool GRAD, int RL>
+__global__ void __launch_bounds__(SB) k_face_dw(const __grid_constant__ DwEval q, int nrep) {
+  __shared__ RepSlots slots[RL > 1 ? SB / RL : 1];
+  let_next_start();
+  if ((int)blockIdx.x < nrep) {
+    wait_previous();
+    const int nm = near_mode_of(q);
+    const int v = (blockIdx.x * SB + threadIdx.x) / RL;
+    if (v < q.t.nv) rep_vertex<GRAD, RL>(q, v, threadIdx.x % RL, nm, &slots[RL > 1 ? threadIdx.x / RL : 0]);
+    return;
+  }
+  const int f = (blockIdx.x - nrep) * SB + threadIdx.x;
+  int a = 0, b = 0, c = 0;
+  if (f < q.t.nf) {
+    a = __ldg(q.t.fv + 3 * (size_t)f);
+    b = __ldg(q.t.fv + 3 * (size_t)f + 1);
+    c = __ldg(q.t.fv + 3 * (size_t)f + 2);
+  }
+  wait_previous();
+  if (f < q.t.nf) face_dw(q, a, b, c, f);
+}
+
+// blocks [0, nqueue): the queued repulsion, one warp per vertex
+template <bool GRAD>
+__global__ void __launch_bounds__(SB) k_edge_dw(const __grid_constant__ DwEval q, int nqueue) {
+  let_next_start();
+  if ((int)blockIdx.x < nqueue) {
+    wait_previous();
+    rep_queue<GRAD>(q, (blockIdx.x * SB + threadIdx.x) >> 5, nqueue * (SB / 32));
+    return;
+  }
+  const int e = (blockIdx.x - nqueue) * SB + threadIdx.x;
+  int4 E = make_int4(0, 0, -1, -1);
+  if (e < q.t.ne) E = __ldg(q.t.edge + e);
+  wait_previous();
+  if (e < q.t.ne) edge_dw(q, E, e);
+}
+
+// The last block (atomic ticket) reduces the block partials in block order
+// and assembles energy and penalty factors.  Fixed order throughout: results
+// are bit-reproducible.
+template <int L>
+__global__ void __launch_bounds__(VB) k_vertex_dw(const __grid_constant__ DwEval q) {
+  __shared__ float2 wsum[6][VB / 32];
+  __shared__ double redd[6];
+  __shared__ bool last;
+  let_next_start();
+  wait_previous();
+  df pr[6];
+  vertex_dw<L>(q, (blockIdx.x * VB + threadIdx.x) / L, threadIdx.x % L, pr);
+  block_props<VB / 32>(pr, wsum, q.partial + 8 * (size_t)blockIdx.x);
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
-    const unsigned int tk = atomicAdd(&g->ticket, 1u);
+    const unsigned int tk = atomicAdd(&q.g->ticket, 1u);
     last = (tk == gridDim.x - 1);
   }
   __syncthreads();
   if (!last) return;
   __threadfence();
-  // last block: warp k reduces property k over the block partials (lane l
-  // takes blocks l, l + 32, ... in order, then a fixed shuffle tree)
-  if (w < 6) {
-    double acc = 0.0;
-    for (int b = lane; b < (int)gridDim.x; b += 32) acc += ((volatile double*)partial)[8 * (size_t)b + w];
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, off);
-    if (lane == 0) redd[w] = acc;
-  }
+  total_props(q.partial, gridDim.x, redd);
   __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int k = 0; k < 6; ++k) g->props[k] = redd[k];
-    assemble(ep, g);
-    g->ticket = 0;
-  }
+  if (threadIdx.x < 32) assemble_warp(q.ep, redd, q.g, q.energy);
 }
 
-// Gradient gather per vertex i over its ring (slot m: face (i, j = r_m,
-// k = r_{m-1})), the reference's gather (src/mesh_properties.cpp:51-148 with
-// src/kernel.h:124-137) regrouped per face and edge, with alpha =
-// gA - 2/3 kb (rho_i^2 + rho_j^2 + rho_k^2) and w = gC/2 + kb (rho_i + rho_j):
-//   area       (alpha / 2) n x (x_k - x_j)
-//   volume     (gV / 6) x_j x x_k, summed as d_j x d_k with d = x - x_i
-//              (the x_i x (d_k - d_j) parts cancel around a closed fan)
-//   length     -(w theta + kt dB/dl) / l (x_j - x_i) for edge (i, j)
-//   dihedral   along n: w_ij cot_j + w_ik cot_k - w_jk (cot_j + cot_k)
-// Positions enter relative to x_i, so the sums stay near the size of the
-// result.
-__device__ __forceinline__ df cot_of(const float4& F2, const float4& F3, int c) {
-  return c == 0 ? lo_hi(F2.z, F2.w) : (c == 1 ? lo_hi(F3.x, F3.y) : lo_hi(F3.z, F3.w));
+template <bool CLOSED, int L>
+__global__ void __launch_bounds__(128, 5) k_grad_dw(const __grid_constant__ DwEval q) {
+  wait_previous();
+  const Globals* g = q.g;
+  grad_dw<CLOSED, L>(q, (blockIdx.x * 128 + threadIdx.x) / L, threadIdx.x % L, {g->gdf[0], g->gdf[1]}, {g->gdf[2], g->gdf[3]},
+                            {g->gdf[4], g->gdf[5]});
 }
 
-template <bool CLOSED>
-__global__ void __launch_bounds__(128, 5) k_grad_dw(Topo t, PosDW X, const float4* __restrict__ fd,
-                                                const float4* __restrict__ ed, const float4* __restrict__ rk,
-                                                const double* __restrict__ repg, const Globals* __restrict__ g,
-                                                EP ep, EPD epd, double* __restrict__ grad) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= t.nv) return;
-  const df gA = {g->gdf[0], g->gdf[1]}, gV = {g->gdf[2], g->gdf[3]}, gC = {g->gdf[4], g->gdf[5]};
-  const df hgC = half(gC);
-  const df3 xi = X.at(i);
-  const float4 q4 = __ldg(rk + i);
-  const df ai = sub_s(gA, lo_hi(q4.z, q4.w));
-  const df wi = add_s(hgC, lo_hi(q4.x, q4.y));
-  dacc3 acc = {{0.0f, 0.0f}, {0.0f, 0.0f}, {0.0f, 0.0f}};
-  dacc3 vcr = acc, vtel = acc;
-  const int d = t.val[i];
-  if (d > 0) {
-    const size_t nv = t.nv;
-    const int4 sp = t.slot[(size_t)(d - 1) * nv + i];
-    df3 dk = sub3(X.at(sp.x), xi);
-    float4 qk = __ldg(rk + sp.x);
-    df wprev = df_make(0.0f);  // w of edge (i, k) and whether it is interior
-    bool prev_int = false;
-    for (int m = 0; m < d; ++m) {
-      const int4 sc = t.slot[(size_t)m * nv + i];
-      const df3 dj = sub3(X.at(sc.x), xi);
-      const float4 qj = __ldg(rk + sc.x);
-      const int f = slot_face(sc.y);
-      const float4 e0 = __ldg(ed + 2 * (size_t)sc.z), e1 = __ldg(ed + 2 * (size_t)sc.z + 1);
-      const bool int_ij = e1.z > 0.0f;
-      const df w = add_s(wi, lo_hi(qj.x, qj.y));
-      if (f >= 0) {
-        const float4 F0 = __ldg(fd + 4 * (size_t)f), F1 = __ldg(fd + 4 * (size_t)f + 1);
-        const float4 F2 = __ldg(fd + 4 * (size_t)f + 2), F3 = __ldg(fd + 4 * (size_t)f + 3);
-        const float4 ejk = __ldg(ed + 2 * (size_t)sc.w + 1);
-        const df3 n = {{F0.x, F0.y}, {F0.z, F0.w}, {F1.x, F1.y}};
-        const int ci = slot_corner(sc.y);
-        const int cjx = ci == 2 ? 0 : ci + 1, ckx = ci == 0 ? 2 : ci - 1;
-        const df cj = cot_of(F2, F3, cjx), ck = cot_of(F2, F3, ckx);
-        // face (i, j, k): area and volume terms
-        df alpha = sub_s(sub_s(ai, lo_hi(qj.z, qj.w)), lo_hi(qk.z, qk.w));
-        if (ep.btype == 1) {
-          const df q = sub_s(mul_s(lo_hi(F1.z, F1.w), epd.inv_a0), df_make(1.0f));
-          alpha = add_s(alpha, ldexp2(mul_s(mul_s(epd.kt, q), epd.inv_a0), 2.0f));
-        }
-        const df3 dkj = sub3(dk, dj);
-        acc_add3(acc, scale3(half(alpha), cross3(n, dkj)));
-        acc_add3(vcr, cross3(dj, dk));
-        if (!CLOSED) acc_add3(vtel, dkj);
-        // edge (i, j): length term
-        df cl = mul_s(w, lo_hi(e0.z, e0.w));
-        if (ep.btype == 0) cl = add_s(cl, mul_s(epd.kt, lo_hi(e1.x, e1.y)));
-        acc_add3(acc, scale3(neg(mul_s(cl, dabs(lo_hi(e1.z, e1.w)))), dj));
-        // dihedral terms of edges (i, j), (i, k) and (j, k) along n
-        df cn = df_make(0.0f);
-        if (int_ij) cn = mul_s(w, cj);
-        if (prev_int && m > 0) cn = add_s(cn, mul_s(wprev, ck));
-        if (ejk.z > 0.0f)
-          cn = sub_s(cn, mul_s(add_s(add_s(hgC, lo_hi(qj.x, qj.y)), lo_hi(qk.x, qk.y)), add_s(cj, ck)));
-        acc_add3(acc, scale3(cn, n));
-      }
-      wprev = w;
-      prev_int = int_ij && f >= 0;
-      dk = dj;
-      qk = qj;
-    }
-    // the last edge (i, r_{d-1}) is edge (i, k) of the first face (whose
-    // record is read again rather than kept in registers through the loop)
-    const int4 s0 = t.slot[i];
-    const int f0 = slot_face(s0.y);
-    if (prev_int && f0 >= 0) {
-      const float4 F0 = __ldg(fd + 4 * (size_t)f0), F1 = __ldg(fd + 4 * (size_t)f0 + 1);
-      const float4 F2 = __ldg(fd + 4 * (size_t)f0 + 2), F3 = __ldg(fd + 4 * (size_t)f0 + 3);
-      const int ci = slot_corner(s0.y);
-      const df ck0 = cot_of(F2, F3, ci == 0 ? 2 : ci - 1);
-      const df3 n0 = {{F0.x, F0.y}, {F0.z, F0.w}, {F1.x, F1.y}};
-      acc_add3(acc, scale3(mul_s(wprev, ck0), n0));
-    }
-  }
-  df3 vol = acc_val3(vcr);
-  if (!CLOSED) {
-    const df3 tx = cross3(xi, acc_val3(vtel));
-    vol = {add_s(vol.x, tx.x), add_s(vol.y, tx.y), add_s(vol.z, tx.z)};
-  }
-  const df gV6 = mul_s(gV, sixth());
-  acc_add3(acc, scale3(gV6, vol));
-  const df3 r = acc_val3(acc);
-  const d3 rg = ld3(repg, i);
-  grad[3 * i] = df_to(r.x) + ep.kr * rg.x;
-  grad[3 * i + 1] = df_to(r.y) + ep.kr * rg.y;
-  grad[3 * i + 2] = df_to(r.z) + ep.kr * rg.z;
+__global__ void k_split_only(int nv, const double* __restrict__ P, float4* __restrict__ X, float* __restrict__ P32) {
+  const int v = blockIdx.x * blockDim.x + threadIdx.x;
+  if (v >= nv) return;
+  float hx, hy, hz, lx, ly, lz;
+  split_bits(P[3 * v], &hx, &lx);
+  split_bits(P[3 * v + 1], &hy, &ly);
+  split_bits(P[3 * v + 2], &hz, &lz);
+  st32(X + 2 * (size_t)v, make_float4(hx, hy, hz, 0.0f), make_float4(lx, ly, lz, 0.0f));
+  P32[3 * v] = hx;
+  P32[3 * v + 1] = hy;
+  P32[3 * v + 2] = hz;
 }
 
 inline int nblk(long n, int b) { return (int)((n + b - 1) / b); }
@@ -388,7 +833,11 @@ EPD make_epd(const EP& ep) {
   epd.kb = host_df(ep.kb);
   epd.kt = host_df(ep.kt);
   epd.kr = host_df(ep.kr);
-  epd.kb23 = host_df(ep.kb * (2.0 / 3.0));
+  int ex = 0;
+  std::frexp(ep.kb, &ex);
+  ex = std::min(std::max(ex, -100), 100);
+  epd.iks = (float)std::ldexp(1.0, -ex);
+  epd.kq = host_df(ep.kb != 0.0 ? std::ldexp(2.0 / 3.0, ex) / ep.kb : 0.0);
   epd.a0 = host_df(ep.a0);
   epd.inv_a0 = host_df(1.0 / ep.a0);
   epd.inv_tdiv = host_df(1.0 / ep.tdiv);
@@ -403,54 +852,102 @@ const float4* split_positions_dw(tm_energy* e, int nv, const double* P, cudaStre
   const size_t n = std::max(nv, 1);
   e->pos32.ensure(3 * n);
   e->posdw.ensure(2 * n);
-  if (nv) k_split_dw<<<nblk(nv, 256), 256, 0, s>>>(nv, P, e->posdw.get(), e->pos32.get());
+  if (nv) k_split_only<<<nblk(nv, 256), 256, 0, s>>>(nv, P, e->posdw.get(), e->pos32.get());
   TM_LAUNCH();
   return e->posdw.get();
 }
 
-void energy_eval_df(tm_energy* e, tm_mesh* m, const double* P, bool want_grad, double* d_grad, cudaStream_t s,
-                    cudaEvent_t* ev) {
+namespace {
+// launch with programmatic stream serialisation (see wait_previous)
+template <class... A, class... B>
+void launch_after(void (*k)(A...), int grid, int block, cudaStream_t s, B... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  TM_CUDA(cudaLaunchKernelEx(&cfg, k, args...));
+}
+}  // namespace
+
+void energy_eval_df(tm_energy* e, tm_mesh* m, const double* P, bool want_grad, double* d_grad, double* d_energy,
+                    const Leap* leap, cudaStream_t s, cudaEvent_t* ev) {
   e->ensure(m->nv, m->ne, m->nf);
   const size_t nv = std::max(m->nv, 1);
   e->pos32.ensure(3 * nv);
   e->posdw.ensure(2 * nv);
-  Topo t = m->topo();
-  EP ep = make_ep(e);
-  const EPD epd = make_epd(ep);
-  PosDW X{e->posdw.get(), (int)nv};
-  float4* fd = reinterpret_cast<float4*>(e->face.get());   // 64 bytes per face
-  float4* ed = reinterpret_cast<float4*>(e->edge.get());   // 32 bytes per edge
-  float4* eb = reinterpret_cast<float4*>(e->ebond.get());  // (l theta, bond) per edge, 16 bytes
-  float4* fav = reinterpret_cast<float4*>(e->fav.get());   // (area, volume) per face, 16 bytes
-  float4* rho = reinterpret_cast<float4*>(e->rho.get());   // (kb rho, 2/3 kb rho^2) per vertex
+  DwEval q{};
+  q.t = m->topo();
+  q.P = P;
+  q.X = e->posdw.get();
+  q.P32 = e->pos32.get();
+  q.fd = reinterpret_cast<float4*>(e->face.get());    // 64 bytes per face
+  q.eg = reinterpret_cast<float4*>(e->edge.get());    // (theta / l, kt dB/dl / l) per edge, 16 bytes
+  q.elt = reinterpret_cast<float4*>(e->ebond.get());  // (l theta, bond) per edge, 16 bytes
+  q.fav = reinterpret_cast<float4*>(e->fav.get());    // (area, volume) per face, 16 bytes
+  q.sct = e->sctf.get();
+  q.ep = make_ep(e);
+  q.epd = make_epd(q.ep);
+  q.nl = e->nl.view;
+  q.nl.pos32 = q.P32;
+  q.rep = q.ep.rlc1 > 0 ? 1 : 0;  // no pair can be closer than a non-positive cut-off
+  q.use_near = q.rep && q.nl.kind == 0 && q.nl.nent && e->nl.near_nv == m->nv && e->nl.near_lc1 == q.ep.rlc1;
+  q.excl_fresh = e->nl.built_topo == m->topo_version;
+  q.xb = e->nl.xb.get();
+  q.thr2 = e->nl.near_move2;
+  q.thr = (float)std::sqrt(std::max(q.thr2, 0.0));
+  q.moved = e->moved.get();
+  q.pot = e->reppot.get();
+  q.repg = e->repg.get();
+  q.slow = e->slow.get();
+  q.nslow = q.slow + nv;
+  q.partial = e->partials.get();
+  q.g = e->glob.get();
+  q.energy = d_energy;
+  q.grad = want_grad ? d_grad : nullptr;
+  DwMove mv{};
+  if (leap) mv = DwMove{leap->x, leap->p, leap->g0, leap->g1, leap->dt, leap->im};
+  const Topo& t = q.t;
+  const int nsb = std::max(1, nblk(t.nv, SB));
+  q.nmoved = nsb;
   if (ev) TM_CUDA(cudaEventRecord(ev[0], s));
-  if (m->nv) k_split_dw<<<nblk(m->nv, 256), 256, 0, s>>>(m->nv, P, e->posdw.get(), e->pos32.get());
-  TM_LAUNCH();
-  const bool conc = ev == nullptr;  // repulsion overlaps the face and edge kernels
-  if (conc) fork_repulsion(e, m, P, want_grad, s, true);
-  if (t.nf) k_face_dw<<<nblk(t.nf, 256), 256, 0, s>>>(t, X, fd, fav);
-  TM_LAUNCH();
-  if (ev) TM_CUDA(cudaEventRecord(ev[1], s));
-  if (t.ne) k_edge_dw<<<nblk(t.ne, 256), 256, 0, s>>>(t, X, fd, ed, eb, ep, epd, e->sctf.get());
-  TM_LAUNCH();
-  if (ev) TM_CUDA(cudaEventRecord(ev[2], s));
-  if (conc)
-    join_repulsion(e, s, true);
+  if (leap)
+    k_split_dw<true><<<nsb, SB, 0, s>>>(q, mv);
   else
-    fork_repulsion(e, m, P, want_grad, s, false);
-  int nb = std::max(1, nblk(t.nv, VB));
-  k_vertex_dw<<<nb, VB, 0, s>>>(t, fav, eb, e->reppot.get(), ep, epd, rho, e->partials.get(), e->glob.get());
+    k_split_dw<false><<<nsb, SB, 0, s>>>(q, mv);
   TM_LAUNCH();
+  // Verlet rows that hold a few entries per vertex are shared by eight lanes
+  // (the tube of 7,566 vertices with 1,220 active pairs: 38.6 us per
+  // evaluation against 57.5); near rows and sparse rows, where almost every
+  // entry is skipped without a test, are walked by one (163,842 vertices:
+  // 85 us against 105).
+  const int RL = q.nl.kind == 1 && e->nl.vtotal >= 2LL * t.nv ? 8 : 1;
+  const int nrep = q.rep ? nblk((long)t.nv * RL, SB) : 0;
+  auto* kf = RL == 8 ? (want_grad ? k_face_dw<true, 8> : k_face_dw<false, 8>)
+                       : (want_grad ? k_face_dw<true, 1> : k_face_dw<false, 1>);
+  launch_after(kf, std::max(1, nrep + nblk(t.nf, SB)), SB, s, q, nrep);
+  if (ev) TM_CUDA(cudaEventRecord(ev[1], s));
+  const int nqueue = q.rep && q.nl.kind == 0 ? e->sm_count() : 0;
+  launch_after(want_grad ? k_edge_dw<true> : k_edge_dw<false>, std::max(1, nqueue + nblk(t.ne, SB)), SB, s, q,
+               nqueue);
+  if (ev) TM_CUDA(cudaEventRecord(ev[2], s));
+  // Eight lanes per vertex shorten the chain of one thread's walk over its
+  // ring, one lane per vertex issues fewer instructions.  Whole evaluations
+  // of spheres on a GB300, eight lanes against one: 642 vertices 23.9 / 27.4
+  // us, 2,562 25.3 / 28.5, 10,242 30.8 / 30.2, 16,002 34.8 / 29.3; an open
+  // tube of 7,566 vertices (more arithmetic per slot) 36.9 / 38.5.
+  const bool lanes = t.nv <= 8000;
+  launch_after(lanes ? k_vertex_dw<8> : k_vertex_dw<1>, std::max(1, nblk((long)t.nv * (lanes ? 8 : 1), VB)), VB, s, q);
   if (ev) TM_CUDA(cudaEventRecord(ev[3], s));
   if (want_grad && t.nv) {
-    if (m->closed)
-      k_grad_dw<true><<<nblk(t.nv, 128), 128, 0, s>>>(t, X, fd, ed, rho, e->repg.get(), e->glob.get(), ep, epd,
-                                                      d_grad);
-    else
-      k_grad_dw<false><<<nblk(t.nv, 128), 128, 0, s>>>(t, X, fd, ed, rho, e->repg.get(), e->glob.get(), ep, epd,
-                                                       d_grad);
+    auto* kg = lanes ? (m->closed ? k_grad_dw<true, 8> : k_grad_dw<false, 8>)
+                     : (m->closed ? k_grad_dw<true, 1> : k_grad_dw<false, 1>);
+    launch_after(kg, nblk((long)t.nv * (lanes ? 8 : 1), 128), 128, s, q);
   }
-  TM_LAUNCH();
   if (ev) TM_CUDA(cudaEventRecord(ev[4], s));
 }
 

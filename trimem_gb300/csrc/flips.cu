@@ -1079,7 +1079,7 @@ static int flip_sweep(tm_mesh* m, tm_energy* e, const double* P, double ratio, u
   const EPD epd = make_epd(ep);
   // the positions as double-words for the filter pass of the property
   // changes, and the float copy read by the repulsion prefilter
-  const PosDW X{split_positions_dw(e, m->nv, P, s), std::max(m->nv, 1)};
+  const PosDW X{split_positions_dw(e, m->nv, P, s)};
   NLView nlv = e->nl.view;
   nlv.pos32 = e->pos32.get();
   TopoW t = m->topo_w();
@@ -1234,7 +1234,7 @@ static int flip_sweep(tm_mesh* m, tm_energy* e, const double* P, double ratio, u
   }
   m->host_topo_stale = true;
   if (hs.acc > 0) {
-    ++m->topo_version;
+    m->new_topology();
     k_set_int<<<1, 1, 0, s>>>(m->d_topo_ver.get(), (int)(m->topo_version & 0x7fffffff));
     TM_LAUNCH();
   }

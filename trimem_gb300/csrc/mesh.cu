@@ -10,6 +10,7 @@
 // Flips edit the halfedge arrays; the face/edge/ring tables are rebuilt
 // from them afterwards.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <unordered_map>
@@ -267,6 +268,11 @@ void tm_mesh::sync_host_topology() {
   host_topo_stale = false;
 }
 
+unsigned long long tmg::next_topology_id() {
+  static std::atomic<unsigned long long> next{0};
+  return ++next;
+}
+
 tm_mesh::~tm_mesh() {
   if (h_pts) cudaFreeHost(h_pts);
   if (stream) cudaStreamDestroy(stream);
@@ -384,7 +390,9 @@ static void upload_topology(tm_mesh* m) {
   m->d_scratch.ensure(4096);
   m->d_status.ensure(4);
   m->d_topo_ver.ensure(1);
-  TM_CUDA(cudaMemsetAsync(m->d_topo_ver.get(), 0, sizeof(int), m->stream));
+  m->new_topology();  // exclusion flags kept with neighbour rows are not trusted
+  const int ver = (int)(m->topo_version & 0x7fffffff);
+  TM_CUDA(cudaMemcpyAsync(m->d_topo_ver.get(), &ver, sizeof(int), cudaMemcpyHostToDevice, m->stream));
   cudaStream_t s = m->stream;
   if (nh) {
     TM_CUDA(cudaMemcpyAsync(m->d_to.get(), m->h_to.data(), sizeof(int) * nh, cudaMemcpyHostToDevice, s));
@@ -559,11 +567,6 @@ int tm_mesh_set_topology(tm_mesh* m, const int32_t* to, const int32_t* next, con
   for (int h = 0; h < nh; ++h) m->closed = m->closed && face[h] >= 0;
   upload_topology(m);
   m->host_topo_stale = false;
-  // a new topology: exclusion flags kept with neighbour rows are not trusted
-  ++m->topo_version;
-  const int ver = (int)(m->topo_version & 0x7fffffff);
-  TM_CUDA(cudaMemcpyAsync(m->d_topo_ver.get(), &ver, sizeof(int), cudaMemcpyHostToDevice, m->stream));
-  TM_CUDA(cudaStreamSynchronize(m->stream));
   TM_API_END
 }
 

@@ -782,6 +782,8 @@ void nlist_make(tm_nlist* nl, tm_mesh* m, const tm_params& p, const double* P, c
   if (p.n_search != 0 && p.n_search != 1) fail(TM_ERR_ARG, "Unknown neighbour search algorithm.");
   if (p.exclusion_level < 0 || p.exclusion_level > 2) fail(TM_ERR_ARG, "Unsupported exclusion level");
   nl->prm = p;
+  nl->built_topo = m->topo_version;
+  nl->vtotal = 0;
   int nv = m->nv;
   nl->nv = nv;
   NLView& V = nl->view;
@@ -818,6 +820,7 @@ void nlist_make(tm_nlist* nl, tm_mesh* m, const tm_params& p, const double* P, c
       TM_CUDA(cudaMemsetAsync(nl->cnt.get() + nv, 0, sizeof(int), s));
       exclusive_scan_int(nl->cnt.get(), nl->vrow.get(), nv + 1, &total, nl->tmp, s);
       nl->vcol.ensure(std::max(total, 1));
+      nl->vtotal = total;
       nl->d_res.ensure(std::max(total, 1));
       k_cell_pairs<<<nblk(nv, 256), 256, 0, s>>>(nv, P, V, t, nl->vcoord.get(), nl->vcid.get(), p.rlist, 0, 1,
                                                  nullptr, nl->vrow.get(), nl->d_res.get(), nullptr, nl->vcol.get());
@@ -841,6 +844,8 @@ void nlist_make_batch(tm_nlist* nl, tm_mesh* m, int R, const int* d_vrep, const 
   if (excl < 0 || excl > 2) fail(TM_ERR_ARG, "Unsupported exclusion level");
   int nv = m->nv;
   nl->nv = nv;
+  nl->built_topo = m->topo_version;
+  nl->vtotal = 0;
   nl->prm.n_search = verlet ? 1 : 0;
   nl->prm.exclusion_level = excl;
   NLView& V = nl->view;
@@ -874,6 +879,7 @@ void nlist_make_batch(tm_nlist* nl, tm_mesh* m, int R, const int* d_vrep, const 
       TM_CUDA(cudaMemsetAsync(nl->cnt.get() + nv, 0, sizeof(int), s));
       exclusive_scan_int(nl->cnt.get(), nl->vrow.get(), nv + 1, &total, nl->tmp, s);
       nl->vcol.ensure(std::max(total, 1));
+      nl->vtotal = total;
       nl->d_res.ensure(std::max(total, 1));
       k_verlet_batch<<<nblk(nv, 256), 256, 0, s>>>(nv, P, V, t, nl->vcoord.get(), d_rlist, 1, nullptr,
                                                    nl->vrow.get(), nl->d_res.get(), nl->vcol.get());

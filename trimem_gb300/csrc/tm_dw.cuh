@@ -12,19 +12,45 @@ namespace tmg {
 __device__ __forceinline__ df third() { return {3.333333433e-01f, -9.934107481e-09f}; }
 __device__ __forceinline__ df sixth() { return {1.666666716e-01f, -4.967053740e-09f}; }
 
-// positions as double-words: hi parts p[v] = (x, y, z, 0), lo parts p[nv + v]
+// 32 bytes of read-only data in one load instruction, 32-byte aligned: one
+// sector per lane instead of two 16-byte requests
+__device__ __forceinline__ void ld32(const float4* p, float4& a, float4& b) {
+  asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+      : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+      : "l"(p));
+}
+// 32 bytes in one store instruction (a whole sector), 32-byte aligned
+__device__ __forceinline__ void st32(float4* p, const float4& a, const float4& b) {
+  asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "f"(a.x), "f"(a.y), "f"(a.z), "f"(a.w),
+               "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
+               : "memory");
+}
+
+// Positions as double-words, one 32-byte sector per vertex: hi parts
+// p[2v] = (x, y, z, .), lo parts p[2v + 1] = (x, y, z, .).  The two w
+// entries are the vertex stage's: hi and lo of kb c/a, so that a gradient's
+// gather of a neighbour's position brings its curvature weight along.
 struct PosDW {
   const float4* __restrict__ p;
-  int nv;
   __device__ __forceinline__ df3 at(int v) const {
-    const float4 h = __ldg(p + v), l = __ldg(p + nv + v);
+    float4 h, l;
+    ld32(p + 2 * (size_t)v, h, l);
+    return {{h.x, l.x}, {h.y, l.y}, {h.z, l.z}};
+  }
+  // position and weight
+  __device__ __forceinline__ df3 at(int v, df* kr) const {
+    float4 h, l;
+    ld32(p + 2 * (size_t)v, h, l);
+    *kr = {h.w, l.w};
     return {{h.x, l.x}, {h.y, l.y}, {h.z, l.z}};
   }
 };
 
 // double-word parameters (hi / lo from the host)
 struct EPD {
-  df kb, kt, kr, kb23, a0, inv_a0, inv_tdiv, lc0, lc1, br1, br2;
+  df kb, kt, kr, a0, inv_a0, inv_tdiv, lc0, lc1, br1, br2;
+  df kq;      // 2 s / (3 kb) with s the power of two at kb, 0 without bending
+  float iks;  // 1 / s
 };
 __device__ __forceinline__ bool df_less(df a, df b) { return a.hi < b.hi || (a.hi == b.hi && a.lo < b.lo); }
 __device__ __forceinline__ df ipow_dw(df x, int n) {
@@ -96,8 +122,8 @@ __device__ __forceinline__ void split_bits(double x, float* hi, float* lo) {
 struct EP;
 // double-word copies of the energy parameters (energy_df.cu)
 EPD make_epd(const EP& ep);
-// positions split into double-words (hi parts [nv], lo parts [nv] of
-// e->posdw) and the float copy e->pos32, on stream s; returns e->posdw
+// positions split into double-words (e->posdw, see PosDW) and the float copy
+// e->pos32, on stream s; returns e->posdw
 const float4* split_positions_dw(tm_energy* e, int nv, const double* P, cudaStream_t s);
 
 }  // namespace tmg

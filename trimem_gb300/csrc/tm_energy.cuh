@@ -139,7 +139,7 @@ __device__ __forceinline__ bool pair_within(const PairTest& t, const NLView& nl,
     float s32 = dx * dx + dy * dy + dz * dz;
     if (s32 > t.bound) return false;
   }
-  d3 pj = ld3(P, j);
+  d3 pj = ld3p(P, j);
   double dx = __dsub_rn(p.x, pj.x), dy = __dsub_rn(p.y, pj.y), dz = __dsub_rn(p.z, pj.z);
   double s = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
   *pj_out = pj;
@@ -203,14 +203,18 @@ constexpr int NEAR_HITS = 8;
 template <class F, class X>
 __device__ __forceinline__ bool visit_near(const PairTest& pt, const NLView& nl, const double* P, int v, d3 p,
                                            int mode, const int* co, const X& is_excluded, F& fn) {
-  const int* row = nl.nent + (size_t)v * TM_NEAR_CAP;
+  // four entries per load (a row starts on a 192-byte boundary)
+  const int4* row4 = reinterpret_cast<const int4*>(nl.nent + (size_t)v * TM_NEAR_CAP);
   const int n = nl.ncnt[v];
   long long key[NEAR_HITS];
   double dist[NEAR_HITS];
   d3 dif[NEAR_HITS];
   int hits = 0;
+  int4 r4 = make_int4(0, 0, 0, 0);
   for (int q = 0; q < n; ++q) {
-    int c = row[q];
+    if ((q & 3) == 0) r4 = row4[q >> 2];
+    const int c = r4.x;
+    r4 = make_int4(r4.y, r4.z, r4.w, 0);
     if (mode == 1 && c < 0) continue;
     int j = c & 0x7fffffff;
     d3 pj;
@@ -321,6 +325,46 @@ __device__ __forceinline__ void assemble(const EP& ep, Globals* g) {
   }
 }
 
+// assemble by one warp from the six sums in shared memory, the reset of the
+// ticket and, when asked, the energy into *energy: lanes 0..2 take one quadratic penalty each, so the chain of
+// FP64 operations (two divisions and about ten more, each some tens of
+// cycles on GB300) is a third of one thread's; the same operations in the
+// same order as assemble.
+__device__ __forceinline__ void assemble_warp(const EP& ep, const double* sum6, Globals* g, double* energy = nullptr) {
+  const int lane = threadIdx.x & 31;
+  const int k3 = lane < 3 ? lane : 0;
+  const double p = sum6[k3];
+  const double kap = k3 == 0 ? ep.ka : (k3 == 1 ? ep.kv : ep.kc);
+  const double ref = k3 == 0 ? ep.refA : (k3 == 1 ? ep.refV : ep.refC);
+  const double d = p / ref - 1.0;
+  const double c = kap * d * d;
+  const double gk = 2.0 * kap / ref * d;
+  const double c1 = __shfl_sync(0xffffffffu, c, 1), c2 = __shfl_sync(0xffffffffu, c, 2);
+  if (lane < 3) {
+    g->comps[lane] = c;
+    (&g->gA)[lane] = gk;
+    const float h = (float)gk;
+    g->gdf[2 * lane] = h;
+    g->gdf[2 * lane + 1] = (float)(gk - (double)h);
+  }
+  if (lane < 6) g->props[lane] = sum6[lane];
+  if (lane == 0) {
+    const double cB = ep.kb * sum6[3], cT = ep.kt * sum6[4], cR = ep.kr * sum6[5];
+    double tot = 0.0;
+    tot += c;
+    tot += c1;
+    tot += c2;
+    tot += cT;
+    tot += cR;
+    tot += cB;
+    g->comps[3] = cB;
+    g->comps[4] = cT;
+    g->comps[5] = cR;
+    g->comps[6] = tot;
+    g->ticket = 0;
+    if (energy) *energy = tot;
+  }
+}
 
 // Energy of a set of global properties (src/kernel.h:110-122, summation
 // order area, volume, area-difference, tether, repulsion, bending).

@@ -138,6 +138,7 @@ __device__ __forceinline__ int excl_of(const NLView& nl, int v) { return nl.rexc
 #endif
 
 struct TopoW;
+unsigned long long next_topology_id();  // 1, 2, ... over the process
 
 }  // namespace tmg
 
@@ -161,7 +162,10 @@ struct tm_mesh {
   tmg::DevBuf<int> d_status;
   tmg::DevBuf<int> d_topo_ver;  // device copy of topo_version (low 31 bits)
   cudaStream_t stream = nullptr;
-  unsigned long long topo_version = 0;  // advanced by every flip sweep that flips
+  // identifies the connectivity: unique over all meshes of the process, a new
+  // one for every flip sweep that flips
+  unsigned long long topo_version = 0;
+  void new_topology() { topo_version = tmg::next_topology_id(); }
   tmg::Topo topo() const;
   tmg::TopoW topo_w();
   void rebuild_tables(cudaStream_t s);  // faces, edges, rings from halfedges
@@ -184,6 +188,8 @@ struct tm_nlist {
   tmg::DevBuf<double> xb;  // positions when the near rows were built
   double near_lc1 = 0.0, near_move2 = 0.0;
   int near_nv = -1;
+  long long vtotal = 0;  // Verlet row entries
+  unsigned long long built_topo = 0;  // topology (tm_mesh::topo_version) of the last build
   // last query result
   std::vector<double> res_d;
   std::vector<int> res_i, res_j;
@@ -213,8 +219,9 @@ struct tm_energy {
   int nv = 0, ne = 0, nf = 0;
   tmg::DevBuf<double> face, edge, ebond, fav, rho, repg, reppot, vprops, partials, grad, work;
   tmg::DevBuf<int> slow;  // vertices that left their build cell (+ count)
+  tmg::DevBuf<int> moved;  // double-word path: per block, some vertex left its skin
   tmg::DevBuf<float> pos32, poslo;
-  tmg::DevBuf<float4> posdw;  // double-word stencils: hi parts [nv], lo parts [nv]
+  tmg::DevBuf<float4> posdw;  // double-word stencils: hi and lo parts, 2 per vertex (PosDW)
   tmg::DevBuf<tmg::Globals> glob;
   tmg::DevBuf<double2> sct;  // {sin, cos}(k / 128), k < TM_SCT_N
   tmg::DevBuf<float4> sctf;  // the same as double-words (sin hi, sin lo, cos hi, cos lo)
@@ -242,6 +249,8 @@ struct tm_energy {
   unsigned long long eval_tick = 0;
   EvalGraph flip_graph;  // one group of flip-sweep windows
   int flip_coop = 0;     // claim + winner as one cooperative launch: 0 unknown, 1 yes, -1 no
+  int sms = 0;
+  int sm_count();
   void ensure(int nv_, int ne_, int nf_);
   // copies n doubles from device memory to host memory dst and synchronises
   void to_host(double* dst, const double* src, size_t n);
@@ -250,8 +259,9 @@ struct tm_energy {
 
 namespace tmg {
 // energy.cu
+// (d_energy, when given, receives the energy)
 void energy_eval(tm_energy* e, tm_mesh* m, const double* d_points, bool want_grad, bool want_vprops,
-                 double* d_grad, cudaStream_t s);
+                 double* d_grad, cudaStream_t s, double* d_energy = nullptr);
 // same, recording ev[0..4] around the face, edge, vertex and gradient kernels
 void energy_eval_marked(tm_energy* e, tm_mesh* m, const double* d_points, bool want_grad, bool want_vprops,
                         double* d_grad, cudaStream_t s, cudaEvent_t* ev);
@@ -288,9 +298,17 @@ void energy_eval_batch32(tm_energy* e, tm_mesh* m, const double* d_points, doubl
                          const BatchStreams* bs, cudaStream_t s);
 void batch32_class_kernel(int which, const BatchClass& c, int blk, tm_energy* e, tm_mesh* m, const double* P,
                           double* d_grad, const EP* eps, const int* vrep, const Globals* gs, cudaStream_t s);
-// double-float stencil variant (stencil mode 2)
+// velocity-Verlet update that precedes an evaluation: kick with g0 and g1
+// (drift only, with g0, when g1 is NULL), drift of x; im = 1 / mass
+struct Leap {
+  double *x, *p;
+  const double *g0, *g1;
+  double dt, im;
+};
+// double-word stencils (stencil mode 2).  leap: update the positions first
+// (d_points is then leap->x).  ev: five events around the stages.
 void energy_eval_df(tm_energy* e, tm_mesh* m, const double* d_points, bool want_grad, double* d_grad,
-                    cudaStream_t s, cudaEvent_t* ev);
+                    double* d_energy, const Leap* leap, cudaStream_t s, cudaEvent_t* ev);
 // FP32-stencil variant (stencil mode 1); per-vertex properties are not
 // produced by it
 void energy_eval32(tm_energy* e, tm_mesh* m, const double* d_points, bool want_grad, bool want_vprops,

@@ -29,6 +29,11 @@ __device__ __forceinline__ double norm(d3 a) { return sqrt(dot(a, a)); }
 __device__ __forceinline__ d3 ld3(const double* p, int i) {
   return {__ldg(p + 3 * i), __ldg(p + 3 * i + 1), __ldg(p + 3 * i + 2)};
 }
+// the same without the read-only path, for positions that the running kernel
+// may have written itself
+__device__ __forceinline__ d3 ld3p(const double* p, int i) {
+  return {p[3 * (size_t)i], p[3 * (size_t)i + 1], p[3 * (size_t)i + 2]};
+}
 __device__ __forceinline__ void st3(double* p, int i, d3 v) {
   p[3 * i] = v.x;
   p[3 * i + 1] = v.y;

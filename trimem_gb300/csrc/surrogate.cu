@@ -302,13 +302,20 @@ __global__ void __launch_bounds__(128) k_dense(const __grid_constant__ CUtensorM
         const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&hv);
         uint4 ov;
         __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&ov);
+        float zv[8];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           const int n = c * 8 + 2 * q;
           float2 hf = __bfloat1622float2(h2[q]);
           const float z0 = acc[n] + bias[n], z1 = acc[n + 1] + bias[n + 1];
           o2[q] = __floats2bfloat162_rn(hf.x + silu(z0), hf.y + silu(z1));
-          if (zout) *reinterpret_cast<float2*>(zout + (size_t)(m0 + r) * H + n) = make_float2(z0, z1);
+          zv[2 * q] = z0;
+          zv[2 * q + 1] = z1;
+        }
+        if (zout) {
+          float4* z4 = reinterpret_cast<float4*>(zout + (size_t)(m0 + r) * H + c * 8);
+          z4[0] = make_float4(zv[0], zv[1], zv[2], zv[3]);
+          z4[1] = make_float4(zv[4], zv[5], zv[6], zv[7]);
         }
         *reinterpret_cast<uint4*>(out + (size_t)(m0 + r) * H + c * 8) = ov;
       }
@@ -513,8 +520,8 @@ void surrogate_grad(tm_surrogate* sg, tm_energy* e, tm_mesh* m, const double* P,
 //   messages dh_j += sum_i (W_e e_ij + b_e) * dm_i over the rings of j,
 //            dW_e += (dm_i * h_j) e_ij^T, db_e += dm_i * h_j
 //   input    dz = dh * SiLU'(z), dW_in += dz u^T, db_in += dz
-// Parameter gradients are summed per block and then over the blocks in
-// block order (no floating-point atomics: a step is bit-reproducible).
+// Parameter gradients are summed per block and then over the blocks in a
+// fixed order (no floating-point atomics: a step is bit-reproducible).
 // --------------------------------------------------------------------------
 namespace {
 
@@ -546,53 +553,55 @@ __global__ void __launch_bounds__(TB) k_t_embed(int nv, const float* __restrict_
   float x[FV];
 #pragma unroll
   for (int k = 0; k < FV; ++k) x[k] = u[(size_t)FV * i + k];
-  float o[8];
+  float y[8], o[8];
 #pragma unroll
   for (int q = 0; q < 8; ++q) {
     const int c = 8 * sub + q;
-    float y = th[P_BIN + c];
+    const float4 w0 = *reinterpret_cast<const float4*>(th + P_WIN + c * FV);
+    const float4 w1 = *reinterpret_cast<const float4*>(th + P_WIN + c * FV + 4);
+    const float w[FV] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+    y[q] = th[P_BIN + c];
 #pragma unroll
-    for (int k = 0; k < FV; ++k) y += th[P_WIN + c * FV + k] * x[k];
-    z[(size_t)H * i + c] = y;
-    o[q] = silu(y);
+    for (int k = 0; k < FV; ++k) y[q] += w[k] * x[k];
+    o[q] = silu(y[q]);
   }
+  float4* z4 = reinterpret_cast<float4*>(z + (size_t)H * i + 8 * sub);
+  z4[0] = make_float4(y[0], y[1], y[2], y[3]);
+  z4[1] = make_float4(y[4], y[5], y[6], y[7]);
   reinterpret_cast<uint4*>(h)[(size_t)i * (H / 8) + sub] = pack8(o);
 }
 
 // messages m_i = sum_j (W_e e_ij + b_e) * h_j over the exported rings
-// (nbr / ef slot-major [D][n]); 16 threads per vertex, 4 channels each
+// (nbr / ef slot-major [D][n]); 8 threads per vertex, 8 channels (16 bytes of
+// h_j) each: half the index and feature loads of 16 threads with 4 channels.
+// The next neighbour's index is in flight while the current one is summed.
 __global__ void __launch_bounds__(TB) k_t_agg(int nv, int D, const int* __restrict__ nbr, const float* __restrict__ ef,
                                               const float* __restrict__ th, int r,
                                               const __nv_bfloat16* __restrict__ h, __nv_bfloat16* __restrict__ mout) {
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  const int i = g >> 4, sub = g & 15;
+  const int i = g >> 3, sub = g & 7;
   if (i >= nv) return;
-  float4 w[4];
-  float b[4];
+  float4 w[8];
+  float b[8], acc[8];
 #pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    const int ch = 4 * sub + c;
-    w[c] = *reinterpret_cast<const float4*>(th + p_we(r) + ch * FE);
-    b[c] = th[p_be(r) + ch];
+  for (int c = 0; c < 8; ++c) {
+    w[c] = *reinterpret_cast<const float4*>(th + p_we(r) + (8 * sub + c) * FE);
+    b[c] = th[p_be(r) + 8 * sub + c];
+    acc[c] = 0.f;
   }
-  const uint2* h2 = reinterpret_cast<const uint2*>(h);
-  float acc[4] = {0.f, 0.f, 0.f, 0.f};
-  for (int m = 0; m < D; ++m) {
+  const uint4* h4 = reinterpret_cast<const uint4*>(h);
+  int j = nbr[i];
+  for (int m = 0; j >= 0; ++m) {
     const size_t o = (size_t)m * nv + i;
-    const int j = nbr[o];
-    if (j < 0) break;
+    const int jn = m + 1 < D ? nbr[o + nv] : -1;
     const float4 e = *reinterpret_cast<const float4*>(ef + FE * o);
-    const uint2 hv = h2[(size_t)j * (H / 4) + sub];
-    const float2 h01 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&hv.x));
-    const float2 h23 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&hv.y));
-    const float hj[4] = {h01.x, h01.y, h23.x, h23.y};
+    float hj[8];
+    unpack8(h4[(size_t)j * (H / 8) + sub], hj);
 #pragma unroll
-    for (int c = 0; c < 4; ++c) acc[c] += (b[c] + w[c].x * e.x + w[c].y * e.y + w[c].z * e.z + w[c].w * e.w) * hj[c];
+    for (int c = 0; c < 8; ++c) acc[c] += (b[c] + w[c].x * e.x + w[c].y * e.y + w[c].z * e.z + w[c].w * e.w) * hj[c];
+    j = jn;
   }
-  uint2 o;
-  *reinterpret_cast<__nv_bfloat162*>(&o.x) = __floats2bfloat162_rn(acc[0], acc[1]);
-  *reinterpret_cast<__nv_bfloat162*>(&o.y) = __floats2bfloat162_rn(acc[2], acc[3]);
-  reinterpret_cast<uint2*>(mout)[(size_t)i * (H / 4) + sub] = o;
+  reinterpret_cast<uint4*>(mout)[(size_t)i * (H / 8) + sub] = pack8(acc);
 }
 
 // Sum of a per-thread value over the block's threads in thread order,
@@ -609,20 +618,29 @@ __device__ __forceinline__ float block_sum(float v, float* sh) {
   return r;
 }
 
-// Per-channel sums over the vertices of a block, where thread t holds
-// channels 8 (t & 7) .. 8 (t & 7) + 7 of vertex t >> 3 (32 vertices): the
-// column sums in vertex order into out[0..63].
-__device__ __forceinline__ void block_channel_sum(const float* v8, float* sh, float* out) {
-  const int sub = threadIdx.x & 7, vi = threadIdx.x >> 3;
+// Sums of NVAL values a thread over the threads of a block with the same
+// sub = threadIdx.x & (S - 1), written to out[sub * NVAL + k] for the caller's
+// layout through put(sub, k, sum): the lanes of a warp by a fixed shuffle
+// tree, then the warps in warp order.  One pass at the end of a persistent
+// block instead of one per tile of vertices.
+template <int S, int NVAL, class Put>
+__device__ __forceinline__ void block_group_sum(float* v, float* sh, const Put& put) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-  for (int q = 0; q < 8; ++q) sh[vi * H + 8 * sub + q] = v8[q];
-  __syncthreads();
-  if (threadIdx.x < H) {
-    float s = 0.f;
-    for (int k = 0; k < TB / 8; ++k) s += sh[k * H + threadIdx.x];
-    out[threadIdx.x] = s;
+  for (int k = 0; k < NVAL; ++k) {
+#pragma unroll
+    for (int o = 16; o >= S; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
   }
+  if (lane < S)
+#pragma unroll
+    for (int k = 0; k < NVAL; ++k) sh[(warp * NVAL + k) * S + lane] = v[k];
   __syncthreads();
+  for (int q = threadIdx.x; q < S * NVAL; q += TB) {
+    float s = 0.f;
+#pragma unroll
+    for (int w = 0; w < TB / 32; ++w) s += sh[w * S * NVAL + q];
+    put(q % S, q / S, s);
+  }
 }
 
 // output head, loss and dL/dF: 8 threads per vertex
@@ -652,10 +670,12 @@ __global__ void __launch_bounds__(TB) k_t_out(int nv, int D, const int* __restri
   cn += th[P_BN];
   float Fx = cn * nrm[4 * (size_t)ii], Fy = cn * nrm[4 * (size_t)ii + 1], Fz = cn * nrm[4 * (size_t)ii + 2];
   const float bo = th[P_BO];
-  for (int m = 0; m < D; ++m) {
+  // the eight lanes of a vertex share its ring, so they leave the loop together
+  int j = nbr[ii];
+  for (int m = 0; j >= 0; ++m) {
     const size_t o = (size_t)m * nv + ii;
-    const int j = nbr[o];
-    if (j < 0) break;
+    const int jn = m + 1 < D ? nbr[o + nv] : -1;
+    const float ux = dirs[3 * o], uy = dirs[3 * o + 1], uz = dirs[3 * o + 2];
     float hj[8];
     unpack8(h4[(size_t)j * (H / 8) + sub], hj);
     float c = 0.f;
@@ -664,9 +684,10 @@ __global__ void __launch_bounds__(TB) k_t_out(int nv, int D, const int* __restri
 #pragma unroll
     for (int q = 1; q < 8; q <<= 1) c += __shfl_xor_sync(gmask, c, q);
     c += bo;
-    Fx += c * dirs[3 * o];
-    Fy += c * dirs[3 * o + 1];
-    Fz += c * dirs[3 * o + 2];
+    Fx += c * ux;
+    Fy += c * uy;
+    Fz += c * uz;
+    j = jn;
   }
   Fx *= fs;
   Fy *= fs;
@@ -689,187 +710,253 @@ __global__ void __launch_bounds__(TB) k_t_out(int nv, int D, const int* __restri
 }
 
 // Backward of the output head: dh of the last round (FP32) and the block
-// partials of (w_o, b_o, w_n, b_n) (part: 130 floats per block)
+// partials of (w_o, b_o, w_n, b_n) (part: 130 floats per block).  Persistent
+// blocks: the parameter sums stay in registers over the block's vertices.
 __global__ void __launch_bounds__(TB) k_t_outback(int nv, int D, const int* __restrict__ nbr,
                                                   const float* __restrict__ dirs, const float* __restrict__ nrm,
                                                   const float* __restrict__ th, float fs,
                                                   const __nv_bfloat16* __restrict__ h, const float* __restrict__ dF,
                                                   float* __restrict__ dh, float* __restrict__ part) {
-  __shared__ float sh[(TB / 8) * H];
-  __shared__ float sred[TB];
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  const int i = g >> 3, sub = g & 7;
-  const bool act = i < nv;
-  const int ii = act ? i : 0;
+  __shared__ float sh[(TB / 32) * 18 * 8];
+  const int sub = threadIdx.x & 7;
   const uint4* h4 = reinterpret_cast<const uint4*>(h);
-  float hi[8], acc[8], pwo[8], pwn[8];
-  unpack8(h4[(size_t)ii * (H / 8) + sub], hi);
-  const float dfx = act ? dF[3 * (size_t)ii] : 0.f, dfy = act ? dF[3 * (size_t)ii + 1] : 0.f,
-              dfz = act ? dF[3 * (size_t)ii + 2] : 0.f;
-  const float dci = fs * (dfx * nrm[4 * (size_t)ii] + dfy * nrm[4 * (size_t)ii + 1] + dfz * nrm[4 * (size_t)ii + 2]);
-  float pbo = 0.f;
+  float wo[8], wn[8], sum[18];  // sum: w_o (8 channels), w_n (8), b_o, b_n
 #pragma unroll
   for (int q = 0; q < 8; ++q) {
-    acc[q] = dci * th[P_WN + 8 * sub + q];
-    pwn[q] = dci * hi[q];
-    pwo[q] = 0.f;
+    wo[q] = th[P_WO + 8 * sub + q];
+    wn[q] = th[P_WN + 8 * sub + q];
   }
-  for (int m = 0; act && m < D; ++m) {
-    const size_t o = (size_t)m * nv + ii;
-    const int j = nbr[o];
-    if (j < 0) break;
-    const float ux = dirs[3 * o], uy = dirs[3 * o + 1], uz = dirs[3 * o + 2];
-    const float dcij = fs * (dfx * ux + dfy * uy + dfz * uz);
-    const float dcji = -fs * (dF[3 * (size_t)j] * ux + dF[3 * (size_t)j + 1] * uy + dF[3 * (size_t)j + 2] * uz);
-    float hj[8];
-    unpack8(h4[(size_t)j * (H / 8) + sub], hj);
+#pragma unroll
+  for (int q = 0; q < 18; ++q) sum[q] = 0.f;
+  for (int i = (blockIdx.x * TB + threadIdx.x) >> 3; i < nv; i += gridDim.x * (TB / 8)) {
+    float hi[8], acc[8], t[8];
+    int j = nbr[i];
+    unpack8(h4[(size_t)i * (H / 8) + sub], hi);
+    const float dfx = dF[3 * (size_t)i], dfy = dF[3 * (size_t)i + 1], dfz = dF[3 * (size_t)i + 2];
+    const float dci = fs * (dfx * nrm[4 * (size_t)i] + dfy * nrm[4 * (size_t)i + 1] + dfz * nrm[4 * (size_t)i + 2]);
+    float pbo = 0.f;
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
-      acc[q] += (dcij + dcji) * th[P_WO + 8 * sub + q] * hj[q];
-      pwo[q] += dcij * hi[q] * hj[q];
+      acc[q] = dci * wn[q];
+      t[q] = 0.f;
     }
-    if (sub == 0) pbo += dcij;
-  }
-  if (act)
+    for (int m = 0; j >= 0; ++m) {
+      const size_t o = (size_t)m * nv + i;
+      const int jn = m + 1 < D ? nbr[o + nv] : -1;
+      const float ux = dirs[3 * o], uy = dirs[3 * o + 1], uz = dirs[3 * o + 2];
+      float hj[8];
+      unpack8(h4[(size_t)j * (H / 8) + sub], hj);
+      const float dcij = fs * (dfx * ux + dfy * uy + dfz * uz);
+      const float dcji = -fs * (dF[3 * (size_t)j] * ux + dF[3 * (size_t)j + 1] * uy + dF[3 * (size_t)j + 2] * uz);
 #pragma unroll
-    for (int q = 0; q < 8; ++q) dh[(size_t)H * i + 8 * sub + q] = acc[q];
-  float* pb = part + 130 * (size_t)blockIdx.x;
-  block_channel_sum(pwo, sh, pb);
-  block_channel_sum(pwn, sh, pb + 65);
-  const float sbo = block_sum(pbo, sred);
-  const float sbn = block_sum(sub == 0 ? dci : 0.f, sred);
-  if (threadIdx.x == 0) {
-    pb[64] = sbo;
-    pb[129] = sbn;
+      for (int q = 0; q < 8; ++q) {
+        acc[q] += (dcij + dcji) * wo[q] * hj[q];
+        t[q] += dcij * hj[q];
+      }
+      pbo += dcij;
+      j = jn;
+    }
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      sum[q] += t[q] * hi[q];
+      sum[8 + q] += dci * hi[q];
+    }
+    sum[16] += pbo;
+    sum[17] += dci;
+    float4* d4 = reinterpret_cast<float4*>(dh + (size_t)H * i + 8 * sub);
+    d4[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+    d4[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
   }
+  float* pb = part + 130 * (size_t)blockIdx.x;
+  block_group_sum<8, 18>(sum, sh, [&](int sb, int k, float v) {
+    if (k < 8) pb[8 * sb + k] = v;
+    else if (k < 16) pb[65 + 8 * sb + k - 8] = v;
+    else if (sb == 0) pb[k == 16 ? 64 : 129] = v;
+  });
 }
 
 // Backward of dense layer r over tiles of 64 vertices (persistent blocks):
 // dz = dh1 * SiLU'(z); dh0 = dh1 + dz W[:, :64]; dm = dz W[:, 64:];
-// block partials of dW (64 x 128, row n, column k) and db (64).  Thread t
-// owns column k = t & 127 and half of the rows (vertices for d[h | m],
-// output channels for dW): shared-memory reads of W and [h | m] are
-// consecutive across a warp, those of dz are broadcasts.
-constexpr int DT = 64;  // vertices per tile
-constexpr int DENSE_BACK_SMEM = (DT * H + DT * 2 * H + H * 2 * H) * sizeof(float);
-__global__ void __launch_bounds__(TB) k_t_dense_back(int nv, const float* __restrict__ th, int r,
-                                                     const float* __restrict__ z, const __nv_bfloat16* __restrict__ h,
-                                                     const __nv_bfloat16* __restrict__ mm,
-                                                     const float* __restrict__ dh1, float* __restrict__ dh0,
-                                                     float* __restrict__ dm, float* __restrict__ part) {
-  extern __shared__ float sm[];
-  float* sdz = sm;              // [DT][H]
-  float* sa = sdz + DT * H;     // [DT][2H]: [h | m]
-  float* sw = sa + DT * 2 * H;  // [H][2H]: W rounded to bf16
-  const int t = threadIdx.x;
-  const int k = t & (2 * H - 1), half = t >> 7;  // column, and rows half * 32 .. + 31
-  for (int q = t; q < H * 2 * H; q += TB) sw[q] = __bfloat162float(__float2bfloat16_rn(th[p_w(r) + q]));
-  float gw[32];
+// block partials of dW (64 x 128, row n, column k) and db (64).  Both are
+// FP32 matrix products (the gradients keep FP32 operands), bound by the FMA
+// pipe once the operands reach it: thread t owns rows rg + 8 q (vertices) or
+// 8 rg + q (channels), q < 8, and columns 4 kg .. + 3 of each product, so that
+// 32 FMAs share three 16-byte shared loads, each one wavefront a warp (four
+// row groups and eight column groups a warp; sdz rows are padded by four
+// floats to keep the row groups on different banks).  40,962 vertices: one
+// column and 32 rows a thread, one shared load per FMA, took 142 us a layer.
+constexpr int DT = 64;        // vertices per tile
+constexpr int ZP = H + 4;     // padded row of sdz
+constexpr int DENSE_BACK_SMEM = (DT * ZP + DT * 2 * H + H * 2 * H) * sizeof(float);
+__global__ void __launch_bounds__(TB, 2) k_t_dense_back(int nv, const float* __restrict__ th, int r,
+                                                        const float* __restrict__ z,
+                                                        const __nv_bfloat16* __restrict__ h,
+                                                        const __nv_bfloat16* __restrict__ mm,
+                                                        const float* __restrict__ dh1, float* __restrict__ dh0,
+                                                        float* __restrict__ dm, float* __restrict__ part) {
+  extern __shared__ float4 sm4[];
+  float* sdz = reinterpret_cast<float*>(sm4);  // [DT][ZP]
+  float* sa = sdz + DT * ZP;                   // [DT][2H]: [h | m]
+  float* sw = sa + DT * 2 * H;                 // [H][2H]: W rounded to bf16
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int rg = (warp & 1) * 4 + (lane & 3);         // row group 0 .. 7
+  const int kc = 4 * ((warp >> 1) * 8 + (lane >> 2));  // first column, 0 .. 124
+  for (int q = t; q < H * 2 * H / 4; q += TB) {
+    const float4 w = reinterpret_cast<const float4*>(th + p_w(r))[q];
+    reinterpret_cast<float4*>(sw)[q] =
+        make_float4(__bfloat162float(__float2bfloat16_rn(w.x)), __bfloat162float(__float2bfloat16_rn(w.y)),
+                    __bfloat162float(__float2bfloat16_rn(w.z)), __bfloat162float(__float2bfloat16_rn(w.w)));
+  }
+  float gw[8][4];
 #pragma unroll
-  for (int q = 0; q < 32; ++q) gw[q] = 0.f;
+  for (int q = 0; q < 8; ++q)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) gw[q][c] = 0.f;
   float gb = 0.f;
+  const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
   const int ntile = (nv + DT - 1) / DT;
   for (int tile = blockIdx.x; tile < ntile; tile += gridDim.x) {
-    const int v0 = tile * DT;
+    const int v0 = tile * DT, nrow = min(DT, nv - v0);
     __syncthreads();  // the previous tile's reads are done (and sw is written)
-    for (int q = t; q < DT * H; q += TB) {
-      const int v = v0 + q / H;
-      sdz[q] = v < nv ? dh1[(size_t)v0 * H + q] * dsilu(z[(size_t)v0 * H + q]) : 0.f;
+    for (int q = t; q < DT * H / 4; q += TB) {
+      const int vr = q / (H / 4), c = q % (H / 4);
+      float4 d = zero4;
+      if (vr < nrow) {
+        const float4 zz = reinterpret_cast<const float4*>(z + (size_t)v0 * H)[q];
+        d = reinterpret_cast<const float4*>(dh1 + (size_t)v0 * H)[q];
+        d = make_float4(d.x * dsilu(zz.x), d.y * dsilu(zz.y), d.z * dsilu(zz.z), d.w * dsilu(zz.w));
+      }
+      *reinterpret_cast<float4*>(sdz + vr * ZP + 4 * c) = d;
     }
-    for (int q = t; q < DT * 2 * H; q += TB) {
-      const int vr = q / (2 * H), c = q % (2 * H), v = v0 + vr;
-      float a = 0.f;
-      if (v < nv) a = __bfloat162float(c < H ? h[(size_t)v * H + c] : mm[(size_t)v * H + c - H]);
-      sa[q] = a;
+    for (int q = t; q < DT * 2 * H / 8; q += TB) {  // eight bf16 at a time: h, then m
+      const int vr = q / (2 * H / 8), c = q % (2 * H / 8);
+      float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      if (vr < nrow) {
+        const size_t row = (size_t)(v0 + vr) * (H / 8);
+        unpack8(c < H / 8 ? reinterpret_cast<const uint4*>(h)[row + c]
+                          : reinterpret_cast<const uint4*>(mm)[row + c - H / 8], f);
+      }
+      float4* d = reinterpret_cast<float4*>(sa + vr * 2 * H + 8 * c);
+      d[0] = make_float4(f[0], f[1], f[2], f[3]);
+      d[1] = make_float4(f[4], f[5], f[6], f[7]);
     }
     __syncthreads();
-    // d[h | m][v][k] = sum_n dz[v][n] W[n][k] for this thread's 32 vertices
+    // d[h | m][v][k] = sum_n dz[v][n] W[n][k], vertices rg + 8 q
     {
-      float o[32];
+      float o[8][4];
 #pragma unroll
-      for (int q = 0; q < 32; ++q) o[q] = 0.f;
-      for (int n = 0; n < H; ++n) {
-        const float w = sw[n * 2 * H + k];
+      for (int q = 0; q < 8; ++q)
 #pragma unroll
-        for (int q = 0; q < 32; ++q) o[q] += sdz[(half * 32 + q) * H + n] * w;
+        for (int c = 0; c < 4; ++c) o[q][c] = 0.f;
+#pragma unroll 2
+      for (int n = 0; n < H; n += 4) {
+        float4 w[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) w[u] = *reinterpret_cast<const float4*>(sw + (n + u) * 2 * H + kc);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const float4 d = *reinterpret_cast<const float4*>(sdz + (rg + 8 * q) * ZP + n);
+          const float dd[4] = {d.x, d.y, d.z, d.w};
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            o[q][0] += dd[u] * w[u].x;
+            o[q][1] += dd[u] * w[u].y;
+            o[q][2] += dd[u] * w[u].z;
+            o[q][3] += dd[u] * w[u].w;
+          }
+        }
       }
 #pragma unroll
-      for (int q = 0; q < 32; ++q) {
-        const int v = v0 + half * 32 + q;
-        if (v >= nv) break;
-        if (k < H)
-          dh0[(size_t)v * H + k] = dh1[(size_t)v * H + k] + o[q];
-        else
-          dm[(size_t)v * H + k - H] = o[q];
+      for (int q = 0; q < 8; ++q) {
+        if (rg + 8 * q >= nrow) break;
+        const size_t v = v0 + rg + 8 * q;
+        float4 x = make_float4(o[q][0], o[q][1], o[q][2], o[q][3]);
+        if (kc < H) {
+          const float4 y = *reinterpret_cast<const float4*>(dh1 + v * H + kc);
+          *reinterpret_cast<float4*>(dh0 + v * H + kc) = make_float4(y.x + x.x, y.y + x.y, y.z + x.z, y.w + x.w);
+        } else {
+          *reinterpret_cast<float4*>(dm + v * H + kc - H) = x;
+        }
       }
     }
-    // dW[n][k] += sum over the tile's vertices of dz[v][n] a[v][k], rows
-    // n = half * 32 .. + 31
+    // dW[n][k] += sum over the tile's vertices of dz[v][n] a[v][k], channels
+    // n = 8 rg + q
+#pragma unroll 4
     for (int vr = 0; vr < DT; ++vr) {
-      const float a = sa[vr * 2 * H + k];
+      const float4 a = *reinterpret_cast<const float4*>(sa + vr * 2 * H + kc);
+      const float4 d0 = *reinterpret_cast<const float4*>(sdz + vr * ZP + 8 * rg);
+      const float4 d1 = *reinterpret_cast<const float4*>(sdz + vr * ZP + 8 * rg + 4);
+      const float dd[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
 #pragma unroll
-      for (int q = 0; q < 32; ++q) gw[q] += sdz[vr * H + half * 32 + q] * a;
+      for (int q = 0; q < 8; ++q) {
+        gw[q][0] += dd[q] * a.x;
+        gw[q][1] += dd[q] * a.y;
+        gw[q][2] += dd[q] * a.z;
+        gw[q][3] += dd[q] * a.w;
+      }
     }
     if (t < H)
-      for (int vr = 0; vr < DT; ++vr) gb += sdz[vr * H + t];
+      for (int vr = 0; vr < DT; ++vr) gb += sdz[vr * ZP + t];
   }
   float* pb = part + (size_t)(H * 2 * H + H) * blockIdx.x;
 #pragma unroll
-  for (int q = 0; q < 32; ++q) pb[(half * 32 + q) * 2 * H + k] = gw[q];
+  for (int q = 0; q < 8; ++q)
+    *reinterpret_cast<float4*>(pb + (8 * rg + q) * 2 * H + kc) = make_float4(gw[q][0], gw[q][1], gw[q][2], gw[q][3]);
   if (t < H) pb[H * 2 * H + t] = gb;
 }
 
 // Backward of the messages of round r, per vertex v (16 threads, 4
 // channels each): as a sender dh[v] += sum_i (W_e e_iv + b_e) * dm_i over
 // v's ring (e_iv is e_vi with the antisymmetric feature 2 negated); as a
-// receiver the block partials of dW_e and db_e (320 floats per block).
-__global__ void __launch_bounds__(TB) k_t_msg_back(int nv, int D, const int* __restrict__ nbr,
-                                                   const float* __restrict__ ef, const float* __restrict__ th, int r,
-                                                   const __nv_bfloat16* __restrict__ h, const float* __restrict__ dm,
-                                                   float* __restrict__ dh, float* __restrict__ part) {
-  __shared__ float sh[TB];
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  const int i = g >> 4, sub = g & 15;
-  const bool act = i < nv;
-  const int ii = act ? i : 0;
+// receiver the block partials of dW_e and db_e (320 floats per block), summed
+// in registers over the vertices of a persistent block.
+__global__ void __launch_bounds__(TB, 3) k_t_msg_back(int nv, int D, const int* __restrict__ nbr,
+                                                      const float* __restrict__ ef, const float* __restrict__ th,
+                                                      int r, const __nv_bfloat16* __restrict__ h,
+                                                      const float* __restrict__ dm, float* __restrict__ dh,
+                                                      float* __restrict__ part) {
+  __shared__ float sh[(TB / 32) * 20 * 16];
+  const int sub = threadIdx.x & 15;
   float4 w[4];
-  float b[4], dmi[4], add[4] = {0.f, 0.f, 0.f, 0.f}, gwe[4][FE], gbe[4];
+  float b[4], sum[20];  // sum[5 c + k]: dW_e (k < 4) and db_e of channel c
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
-    const int ch = 4 * sub + c;
-    w[c] = *reinterpret_cast<const float4*>(th + p_we(r) + ch * FE);
-    b[c] = th[p_be(r) + ch];
-    dmi[c] = dm[(size_t)H * ii + ch];
-    gbe[c] = 0.f;
-#pragma unroll
-    for (int k = 0; k < FE; ++k) gwe[c][k] = 0.f;
+    w[c] = *reinterpret_cast<const float4*>(th + p_we(r) + (4 * sub + c) * FE);
+    b[c] = th[p_be(r) + 4 * sub + c];
   }
+#pragma unroll
+  for (int q = 0; q < 20; ++q) sum[q] = 0.f;
   const uint2* h2 = reinterpret_cast<const uint2*>(h);
-  for (int m = 0; act && m < D; ++m) {
-    const size_t o = (size_t)m * nv + ii;
-    const int j = nbr[o];
-    if (j < 0) break;
-    const float4 e = *reinterpret_cast<const float4*>(ef + FE * o);  // e_vj
-    const uint2 hv = h2[(size_t)j * (H / 4) + sub];
-    const float2 h01 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&hv.x));
-    const float2 h23 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&hv.y));
-    const float hj[4] = {h01.x, h01.y, h23.x, h23.y};
-    const float4 dmj = *reinterpret_cast<const float4*>(dm + (size_t)H * j + 4 * sub);
-    const float dj[4] = {dmj.x, dmj.y, dmj.z, dmj.w};
+  const float4* dm4 = reinterpret_cast<const float4*>(dm);
+  for (int i = (blockIdx.x * TB + threadIdx.x) >> 4; i < nv; i += gridDim.x * (TB / 16)) {
+    int j = nbr[i];
+    const float4 di = dm4[(size_t)i * (H / 4) + sub];
+    const float dmi[4] = {di.x, di.y, di.z, di.w};
+    float add[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int m = 0; j >= 0; ++m) {
+      const size_t o = (size_t)m * nv + i;
+      const int jn = m + 1 < D ? nbr[o + nv] : -1;
+      const float4 e = *reinterpret_cast<const float4*>(ef + FE * o);  // e_vj
+      const uint2 hv = h2[(size_t)j * (H / 4) + sub];
+      const float4 dmj = dm4[(size_t)j * (H / 4) + sub];
+      const float2 h01 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&hv.x));
+      const float2 h23 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&hv.y));
+      const float hj[4] = {h01.x, h01.y, h23.x, h23.y};
+      const float dj[4] = {dmj.x, dmj.y, dmj.z, dmj.w};
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      // receiver: m_v gathers (W_e e_vj + b_e) * h_j
-      const float q = dmi[c] * hj[c];
-      gbe[c] += q;
-      gwe[c][0] += q * e.x;
-      gwe[c][1] += q * e.y;
-      gwe[c][2] += q * e.z;
-      gwe[c][3] += q * e.w;
-      // sender: m_j gathers (W_e e_jv + b_e) * h_v, e_jv = e_vj with feature 2 negated
-      add[c] += (b[c] + w[c].x * e.x + w[c].y * e.y - w[c].z * e.z + w[c].w * e.w) * dj[c];
+      for (int c = 0; c < 4; ++c) {
+        // receiver: m_v gathers (W_e e_vj + b_e) * h_j
+        const float q = dmi[c] * hj[c];
+        sum[5 * c] += q * e.x;
+        sum[5 * c + 1] += q * e.y;
+        sum[5 * c + 2] += q * e.z;
+        sum[5 * c + 3] += q * e.w;
+        sum[5 * c + 4] += q;
+        // sender: m_j gathers (W_e e_jv + b_e) * h_v, e_jv = e_vj with feature 2 negated
+        add[c] += (b[c] + w[c].x * e.x + w[c].y * e.y - w[c].z * e.z + w[c].w * e.w) * dj[c];
+      }
+      j = jn;
     }
-  }
-  if (act) {
     float4* d4 = reinterpret_cast<float4*>(dh + (size_t)H * i + 4 * sub);
     float4 cur = *d4;
     cur.x += add[0];
@@ -878,91 +965,118 @@ __global__ void __launch_bounds__(TB) k_t_msg_back(int nv, int D, const int* __r
     cur.w += add[3];
     *d4 = cur;
   }
-  // block partials: thread (vertex, sub) holds 4 channels x (4 + 1) values;
-  // sum over the block's 16 vertices per channel in vertex order
   float* pb = part + (H * FE + H) * (size_t)blockIdx.x;
-  for (int k = 0; k < FE + 1; ++k) {
-    for (int c = 0; c < 4; ++c) {
-      sh[threadIdx.x] = k < FE ? gwe[c][k] : gbe[c];
-      __syncthreads();
-      if (threadIdx.x < 16) {
-        float s = 0.f;
-        for (int v = 0; v < TB / 16; ++v) s += sh[v * 16 + threadIdx.x];
-        const int ch = 4 * threadIdx.x + c;
-        if (k < FE)
-          pb[ch * FE + k] = s;
-        else
-          pb[H * FE + ch] = s;
-      }
-      __syncthreads();
-    }
-  }
+  block_group_sum<16, 20>(sum, sh, [&](int sb, int k, float v) {
+    const int ch = 4 * sb + k / 5;
+    if (k % 5 < FE)
+      pb[ch * FE + k % 5] = v;
+    else
+      pb[H * FE + ch] = v;
+  });
 }
 
 // Backward of the input layer: dz = dh * SiLU'(z), block partials of
-// dW_in (64 x 8) and db_in (576 floats per block); 8 threads per vertex
-__global__ void __launch_bounds__(TB) k_t_embed_back(int nv, const float* __restrict__ u, const float* __restrict__ z,
-                                                     const float* __restrict__ dh, float* __restrict__ part) {
-  __shared__ float sh[(TB / 8) * H];
-  __shared__ float col[H];
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  const int i = g >> 3, sub = g & 7;
-  const bool act = i < nv;
-  const int ii = act ? i : 0;
-  float x[FV], dz[8];
+// dW_in (64 x 8) and db_in (576 floats per block); 8 threads per vertex,
+// persistent blocks
+__global__ void __launch_bounds__(TB, 2) k_t_embed_back(int nv, const float* __restrict__ u,
+                                                        const float* __restrict__ z, const float* __restrict__ dh,
+                                                        float* __restrict__ part) {
+  __shared__ float sh[(TB / 32) * 72 * 8];
+  const int sub = threadIdx.x & 7;
+  float sum[72];  // sum[9 q + k]: dW_in (k < 8) and db_in of channel 8 sub + q
 #pragma unroll
-  for (int k = 0; k < FV; ++k) x[k] = act ? u[(size_t)FV * ii + k] : 0.f;
+  for (int q = 0; q < 72; ++q) sum[q] = 0.f;
+  for (int i = (blockIdx.x * TB + threadIdx.x) >> 3; i < nv; i += gridDim.x * (TB / 8)) {
+    float x[FV];
 #pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    const size_t o = (size_t)H * ii + 8 * sub + q;
-    dz[q] = act ? dh[o] * dsilu(z[o]) : 0.f;
+    for (int k = 0; k < FV; ++k) x[k] = u[(size_t)FV * i + k];
+    const float4* z4 = reinterpret_cast<const float4*>(z + (size_t)H * i + 8 * sub);
+    const float4* d4 = reinterpret_cast<const float4*>(dh + (size_t)H * i + 8 * sub);
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+      const float4 zz = z4[p], dd = d4[p];
+      const float dz[4] = {dd.x * dsilu(zz.x), dd.y * dsilu(zz.y), dd.z * dsilu(zz.z), dd.w * dsilu(zz.w)};
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+#pragma unroll
+        for (int k = 0; k < FV; ++k) sum[9 * (4 * p + q) + k] += dz[q] * x[k];
+        sum[9 * (4 * p + q) + FV] += dz[q];
+      }
+    }
   }
   float* pb = part + (H * FV + H) * (size_t)blockIdx.x;
-  float v8[8];
-  for (int k = 0; k < FV; ++k) {
-#pragma unroll
-    for (int q = 0; q < 8; ++q) v8[q] = dz[q] * x[k];
-    block_channel_sum(v8, sh, col);
-    if (threadIdx.x < H) pb[threadIdx.x * FV + k] = col[threadIdx.x];
+  block_group_sum<8, 72>(sum, sh, [&](int sb, int k, float v) {
+    const int ch = 8 * sb + k / 9;
+    if (k % 9 < FV)
+      pb[ch * FV + k % 9] = v;
+    else
+      pb[H * FV + ch] = v;
+  });
+}
+
+// All parameter gradients of a pass in one launch: group g's column k is the
+// sum over its nb block partials part[b * stride + k], written to grad[dst + k]
+// (32 columns a block, eight threads a column, each every eighth partial in
+// order, then the eight in order).  The last block sums the loss partials.
+// With ADAM the parameter is updated where its gradient is (Kingma & Ba 2015,
+// with bias correction) and the dense weights' bf16 copies (what the forward
+// reads) are refreshed from the FP32 master.  One thread a column over all
+// partials, a launch per group, took 718 us of the 1,265 us step at 40,962
+// vertices; with it, persistent blocks and the tiled products the step is 466.
+struct RedGroup {
+  const float* part;
+  int nb, n, dst, blk0;  // partials, columns (= stride), first parameter, first block
+};
+struct RedArgs {
+  RedGroup g[2 + 2 * NR];
+  int ng;
+  const float* lossp;
+  int nl;
+  float *loss, *grad;
+};
+struct AdamArgs {
+  float *th, *m1, *m2;
+  float lr, b1, b2, eps, c1, c2;
+  __nv_bfloat16* wd;
+};
+template <bool ADAM>
+__global__ void __launch_bounds__(256) k_t_reduce(const __grid_constant__ RedArgs R, const __grid_constant__ AdamArgs A) {
+  __shared__ float sh[256];
+  const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+  if (blockIdx.x + 1 == gridDim.x) {
+    float s = 0.f;
+    for (int b = threadIdx.x; b < R.nl; b += 256) s += R.lossp[b];
+    s = block_sum(s, sh);
+    if (threadIdx.x == 0) *R.loss = s;
+    return;
   }
-  block_channel_sum(dz, sh, col);
-  if (threadIdx.x < H) pb[H * FV + threadIdx.x] = col[threadIdx.x];
-}
-
-// grad[dst + k] = sum over nb blocks (in block order) of part[b * stride + k]
-__global__ void k_t_reduce(const float* __restrict__ part, int nb, int stride, int n, float* __restrict__ grad,
-                           int dst) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= n) return;
+  int gi = 0;
+  while (gi + 1 < R.ng && (int)blockIdx.x >= R.g[gi + 1].blk0) ++gi;
+  const RedGroup G = R.g[gi];
+  const int k = ((int)blockIdx.x - G.blk0) * 32 + x;
   float s = 0.f;
-  for (int b = 0; b < nb; ++b) s += part[(size_t)b * stride + k];
-  grad[dst + k] = s;
-}
-// the output head's partials: (w_o 64, b_o 1, w_n 64, b_n 1) map onto
-// theta's last 130 entries in the same order
-__global__ void k_t_loss(const float* __restrict__ lossp, int nb, float* __restrict__ loss) {
-  if (threadIdx.x || blockIdx.x) return;
-  float s = 0.f;
-  for (int b = 0; b < nb; ++b) s += lossp[b];
-  *loss = s;
-}
-
-// Adam (Kingma & Ba 2015) with bias correction; the dense weights' bf16
-// copies (what the forward reads) are refreshed from the FP32 master
-__global__ void k_t_adam(int n, float* __restrict__ th, const float* __restrict__ g, float* __restrict__ m1,
-                         float* __restrict__ m2, float lr, float b1, float b2, float eps, float c1, float c2,
-                         __nv_bfloat16* __restrict__ wd) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= n) return;
-  const float gk = g[k];
-  const float a = b1 * m1[k] + (1.0f - b1) * gk;
-  const float b = b2 * m2[k] + (1.0f - b2) * gk * gk;
-  m1[k] = a;
-  m2[k] = b;
-  const float x = th[k] - lr * (a * c1) / (sqrtf(b * c2) + eps);
-  th[k] = x;
-  for (int r = 0; r < NR; ++r)
-    if (k >= p_w(r) && k < p_w(r) + H * 2 * H) wd[(size_t)r * H * 2 * H + (k - p_w(r))] = __float2bfloat16_rn(x);
+  if (k < G.n) {
+#pragma unroll 8
+    for (int b = y; b < G.nb; b += 8) s += G.part[(size_t)b * G.n + k];
+  }
+  sh[threadIdx.x] = s;
+  __syncthreads();
+  if (y || k >= G.n) return;
+  s = 0.f;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) s += sh[32 * q + x];
+  const int p = G.dst + k;
+  R.grad[p] = s;
+  if (ADAM) {
+    const float a = A.b1 * A.m1[p] + (1.0f - A.b1) * s;
+    const float b = A.b2 * A.m2[p] + (1.0f - A.b2) * s * s;
+    A.m1[p] = a;
+    A.m2[p] = b;
+    const float v = A.th[p] - A.lr * (a * A.c1) / (sqrtf(b * A.c2) + A.eps);
+    A.th[p] = v;
+    for (int r = 0; r < NR; ++r)
+      if (p >= p_w(r) && p < p_w(r) + H * 2 * H) A.wd[(size_t)r * H * 2 * H + (p - p_w(r))] = __float2bfloat16_rn(v);
+  }
 }
 
 }  // namespace
@@ -978,7 +1092,8 @@ struct tm_strain {
   DevBuf<__nv_bfloat16> mb;      // [NR][nv][H]
   DevBuf<float> dha, dhb, dm, dF, part, lossp;
   DevBuf<int> status;
-  int nb_dense = 0;
+  // persistent blocks of the backward kernels (at most one per tile)
+  int nb_dense = 0, nb_msg = 0, nb_out = 0, nb_emb = 0;
   alignas(64) CUtensorMap map_h[NR];
   alignas(64) CUtensorMap map_m[NR];
   alignas(64) CUtensorMap map_w[NR];
@@ -986,18 +1101,19 @@ struct tm_strain {
 
 namespace {
 
-int dense_back_blocks() {
-  static int nbk = 0;
-  if (!nbk) {
-    TM_CUDA(cudaFuncSetAttribute(k_t_dense_back, cudaFuncAttributeMaxDynamicSharedMemorySize, DENSE_BACK_SMEM));
-    int per_sm = 0, nsm = 0, dev = 0;
-    TM_CUDA(cudaGetDevice(&dev));
-    TM_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    TM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_t_dense_back, TB, DENSE_BACK_SMEM));
-    nbk = std::max(1, per_sm) * nsm;
-  }
-  return nbk;
+// blocks of kernel k that fit on the GPU at once
+template <class K>
+int resident_blocks(K* k, int smem) {
+  int per_sm = 0, nsm = 0, dev = 0;
+  if (smem > 48 * 1024) TM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  TM_CUDA(cudaGetDevice(&dev));
+  TM_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  TM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, TB, smem));
+  return std::max(1, per_sm) * nsm;
 }
+
+// floats of nb partials of n columns, each group's on a 16-byte boundary
+size_t part_floats(int nb, int n) { return ((size_t)nb * n + 3) & ~(size_t)3; }
 
 struct TrainInputs {
   const float *u, *nrm, *ef, *dirs, *tgt;
@@ -1006,16 +1122,18 @@ struct TrainInputs {
 };
 
 // forward pass (kept intermediates) and, with want_grad, the backward pass
-// and the gradient into st->grad; F (n x 3, may be NULL) receives the force
-void train_pass(tm_strain* st, const TrainInputs& in, float inv_norm, bool want_grad, float* F, cudaStream_t s) {
+// and the gradient into st->grad, with the update of adam when it is given;
+// F (n x 3, may be NULL) receives the force
+void train_pass(tm_strain* st, const TrainInputs& in, float inv_norm, bool want_grad, float* F, const AdamArgs* adam,
+                cudaStream_t s) {
   const int nv = st->nv, D = in.D;
   const size_t NH = (size_t)nv * H;
   const float* th = st->th.get();
-  const int nb8 = nblk((long)nv * 8, TB), nb16 = nblk((long)nv * 16, TB);
+  const int nb8 = nblk((long)nv * 8, TB);
   k_t_embed<<<nb8, TB, 0, s>>>(nv, in.u, th, st->z.get(), st->hb.get());
   TM_LAUNCH();
   for (int r = 0; r < NR; ++r) {
-    k_t_agg<<<nb16, TB, 0, s>>>(nv, D, in.nbr, in.ef, th, r, st->hb.get() + r * NH, st->mb.get() + r * NH);
+    k_t_agg<<<nb8, TB, 0, s>>>(nv, D, in.nbr, in.ef, th, r, st->hb.get() + r * NH, st->mb.get() + r * NH);
     TM_LAUNCH();
     dense_launch(st->map_h[r], st->map_m[r], st->map_w[r], th + p_b(r), st->hb.get() + (r + 1) * NH, nv,
                  st->status.get(), s, WAIT_POLLS, st->z.get() + (r + 1) * NH);
@@ -1023,39 +1141,46 @@ void train_pass(tm_strain* st, const TrainInputs& in, float inv_norm, bool want_
   k_t_out<<<nb8, TB, 0, s>>>(nv, D, in.nbr, in.dirs, in.nrm, in.tgt, th, st->fscale, inv_norm,
                               st->hb.get() + NR * NH, F, st->dF.get(), st->lossp.get());
   TM_LAUNCH();
-  k_t_loss<<<1, 1, 0, s>>>(st->lossp.get(), nb8, st->loss.get());
-  TM_LAUNCH();
-  if (!want_grad) return;
-  float* g = st->grad.get();
+  RedArgs R{};
+  int nblocks = 0;
   float* part = st->part.get();
-  // output head
-  k_t_outback<<<nb8, TB, 0, s>>>(nv, D, in.nbr, in.dirs, in.nrm, th, st->fscale, st->hb.get() + NR * NH,
-                                  st->dF.get(), st->dha.get(), part);
-  TM_LAUNCH();
-  k_t_reduce<<<1, 256, 0, s>>>(part, nb8, 130, 130, g, P_WO);
-  TM_LAUNCH();
-  // rounds, last to first: dense layer, then messages
-  float* dcur = st->dha.get();
-  float* dnext = st->dhb.get();
-  const int nbd = st->nb_dense;
-  for (int r = NR - 1; r >= 0; --r) {
-    k_t_dense_back<<<nbd, TB, DENSE_BACK_SMEM, s>>>(nv, th, r, st->z.get() + (r + 1) * NH, st->hb.get() + r * NH,
-                                                     st->mb.get() + r * NH, dcur, dnext, st->dm.get(), part);
+  auto group = [&](int nb, int n, int dst) {  // partials of the next parameter group
+    R.g[R.ng++] = RedGroup{part, nb, n, dst, nblocks};
+    nblocks += nblk(n, 32);
+    float* p = part;
+    part += part_floats(nb, n);
+    return p;
+  };
+  R.lossp = st->lossp.get();
+  R.nl = nb8;
+  R.loss = st->loss.get();
+  R.grad = st->grad.get();
+  if (want_grad) {
+    // output head
+    k_t_outback<<<st->nb_out, TB, 0, s>>>(nv, D, in.nbr, in.dirs, in.nrm, th, st->fscale, st->hb.get() + NR * NH,
+                                           st->dF.get(), st->dha.get(), group(st->nb_out, 130, P_WO));
     TM_LAUNCH();
-    k_t_reduce<<<nblk(H * 2 * H + H, 256), 256, 0, s>>>(part, nbd, H * 2 * H + H, H * 2 * H, g, p_w(r));
+    // rounds, last to first: dense layer, then messages
+    float* dcur = st->dha.get();
+    float* dnext = st->dhb.get();
+    for (int r = NR - 1; r >= 0; --r) {
+      k_t_dense_back<<<st->nb_dense, TB, DENSE_BACK_SMEM, s>>>(
+          nv, th, r, st->z.get() + (r + 1) * NH, st->hb.get() + r * NH, st->mb.get() + r * NH, dcur, dnext,
+          st->dm.get(), group(st->nb_dense, H * 2 * H + H, p_w(r)));
+      TM_LAUNCH();
+      k_t_msg_back<<<st->nb_msg, TB, 0, s>>>(nv, D, in.nbr, in.ef, th, r, st->hb.get() + r * NH, st->dm.get(), dnext,
+                                              group(st->nb_msg, H * FE + H, p_we(r)));
+      TM_LAUNCH();
+      std::swap(dcur, dnext);
+    }
+    // input layer
+    k_t_embed_back<<<st->nb_emb, TB, 0, s>>>(nv, in.u, st->z.get(), dcur, group(st->nb_emb, H * FV + H, P_WIN));
     TM_LAUNCH();
-    k_t_reduce<<<1, 256, 0, s>>>(part + H * 2 * H, nbd, H * 2 * H + H, H, g, p_b(r));
-    TM_LAUNCH();
-    k_t_msg_back<<<nb16, TB, 0, s>>>(nv, D, in.nbr, in.ef, th, r, st->hb.get() + r * NH, st->dm.get(), dnext, part);
-    TM_LAUNCH();
-    k_t_reduce<<<nblk(H * FE + H, 256), 256, 0, s>>>(part, nb16, H * FE + H, H * FE + H, g, p_we(r));
-    TM_LAUNCH();
-    std::swap(dcur, dnext);
   }
-  // input layer
-  k_t_embed_back<<<nb8, TB, 0, s>>>(nv, in.u, st->z.get(), dcur, part);
-  TM_LAUNCH();
-  k_t_reduce<<<nblk(H * FV + H, 256), 256, 0, s>>>(part, nb8, H * FV + H, H * FV + H, g, P_WIN);
+  if (adam)
+    k_t_reduce<true><<<nblocks + 1, 256, 0, s>>>(R, *adam);
+  else
+    k_t_reduce<false><<<nblocks + 1, 256, 0, s>>>(R, AdamArgs{});
   TM_LAUNCH();
 }
 
@@ -1213,10 +1338,13 @@ int tm_surrogate_train_create(int64_t n_vertices, int32_t max_valence, const flo
   st->dhb.ensure(NH);
   st->dm.ensure(NH);
   st->dF.ensure(3 * (size_t)nv);
-  st->nb_dense = dense_back_blocks();
-  const size_t nb8 = nblk((long)nv * 8, TB), nb16 = nblk((long)nv * 16, TB);
-  st->part.ensure(std::max({nb8 * (H * FV + H), nb8 * 130, nb16 * (H * FE + H),
-                            (size_t)st->nb_dense * (H * 2 * H + H)}));
+  const int nb8 = nblk((long)nv * 8, TB), nb16 = nblk((long)nv * 16, TB);
+  st->nb_dense = std::min(resident_blocks(k_t_dense_back, DENSE_BACK_SMEM), nblk(nv, DT));
+  st->nb_msg = std::min(resident_blocks(k_t_msg_back, 0), nb16);
+  st->nb_out = std::min(resident_blocks(k_t_outback, 0), nb8);
+  st->nb_emb = std::min(resident_blocks(k_t_embed_back, 0), nb8);
+  st->part.ensure(part_floats(st->nb_out, 130) + NR * part_floats(st->nb_dense, H * 2 * H + H) +
+                  NR * part_floats(st->nb_msg, H * FE + H) + part_floats(st->nb_emb, H * FV + H));
   st->lossp.ensure(nb8);
   st->status.ensure(1);
   TM_CUDA(cudaMemcpy(st->th.get(), weights + BLOB_HEADER, sizeof(float) * NPARAM, cudaMemcpyHostToDevice));
@@ -1259,7 +1387,7 @@ int tm_surrogate_train_grad(tm_strain* st, const float* d_u, const float* d_nrm,
   cudaStream_t s = (cudaStream_t)stream;
   TM_CUDA(cudaMemsetAsync(st->status.get(), 0, sizeof(int), s));
   const float inv_norm = 1.0f / (3.0f * (float)st->nv * target_rms * target_rms);
-  train_pass(st, in, inv_norm, d_grad != nullptr, d_force, s);
+  train_pass(st, in, inv_norm, d_grad != nullptr, d_force, nullptr, s);
   if (d_loss) TM_CUDA(cudaMemcpyAsync(d_loss, st->loss.get(), sizeof(float), cudaMemcpyDeviceToDevice, s));
   if (d_grad)
     TM_CUDA(cudaMemcpyAsync(d_grad, st->grad.get(), sizeof(float) * NPARAM, cudaMemcpyDeviceToDevice, s));
@@ -1281,13 +1409,13 @@ int tm_surrogate_train_step(tm_strain* st, const float* d_u, const float* d_nrm,
     fail(TM_ERR_ARG, "invalid training hyperparameters");
   cudaStream_t s = (cudaStream_t)stream;
   const float inv_norm = 1.0f / (3.0f * (float)st->nv * target_rms * target_rms);
-  train_pass(st, in, inv_norm, true, nullptr, s);
+  // the step counts once the pass is queued, as its update does
+  const double k = (double)(st->step + 1);
+  const AdamArgs adam{st->th.get(), st->m1.get(), st->m2.get(), lr, beta1, beta2, eps,
+                      (float)(1.0 / (1.0 - std::pow((double)beta1, k))),
+                      (float)(1.0 / (1.0 - std::pow((double)beta2, k))), st->wd.get()};
+  train_pass(st, in, inv_norm, true, nullptr, &adam, s);
   st->step += 1;
-  const float c1 = (float)(1.0 / (1.0 - std::pow((double)beta1, (double)st->step)));
-  const float c2 = (float)(1.0 / (1.0 - std::pow((double)beta2, (double)st->step)));
-  k_t_adam<<<nblk(NPARAM, 256), 256, 0, s>>>(NPARAM, st->th.get(), st->grad.get(), st->m1.get(), st->m2.get(), lr,
-                                            beta1, beta2, eps, c1, c2, st->wd.get());
-  TM_LAUNCH();
   if (d_loss) TM_CUDA(cudaMemcpyAsync(d_loss, st->loss.get(), sizeof(float), cudaMemcpyDeviceToDevice, s));
   TM_API_END
 }

@@ -37,6 +37,7 @@
 
 #include "df64.cuh"
 #include "tm_dw.cuh"
+#include "tm_chain.cuh"
 #include "tm_energy.cuh"
 #include "tm_internal.h"
 #include "tm_math.cuh"
@@ -490,8 +491,8 @@ __device__ __forceinline__ void vertex_dw(const DwEval& q, int v, int sub, df* p
         const int f = slot_face(s[k].y);
         av[k] = lb[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         if (f >= 0) {
-          av[k] = __ldg(q.fav + f);
-          lb[k] = __ldg(q.elt + s[k].z);
+          av[k] = q.fav[f];
+          lb[k] = q.elt[s[k].z];
         }
       }
 #pragma unroll
@@ -520,7 +521,7 @@ __device__ __forceinline__ void vertex_dw(const DwEval& q, int v, int sub, df* p
     pr[2] = c;
     pr[3] = ldexp2(mul_s(c, rho), 2.0f);  // 2 c^2 / a
     pr[4] = mul_s(sT, q.epd.inv_tdiv);
-    if (q.rep) split_bits(__ldg(q.pot + v), &pr[5].hi, &pr[5].lo);
+    if (q.rep) split_bits(q.pot[v], &pr[5].hi, &pr[5].lo);
     const df kr = mul_s(q.epd.kb, rho);
     q.X[2 * (size_t)v].w = kr.hi;
     q.X[2 * (size_t)v + 1].w = kr.lo;
@@ -638,7 +639,7 @@ __device__ __forceinline__ void grad_dw(const DwEval& q, int i, int sub, df gA, 
         const df qj = kq_of(epd, krj);
         const df wj = add_s(wi, krj);
         const int f = slot_face(sc.y);
-        const float4 E = __ldg(q.eg + sc.z);
+        const float4 E = q.eg[sc.z];
         dacc sj = {0.0f, 0.0f};
         if (CLOSED || f >= 0) {
           float4 F0, F1, F2, F3;
@@ -702,7 +703,7 @@ __device__ __forceinline__ void grad_dw(const DwEval& q, int i, int sub, df gA, 
   if (q.rep) {
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      o[k] = o[k] + q.ep.kr * __ldg(q.repg + 3 * (size_t)i + k);
+      o[k] = o[k] + q.ep.kr * q.repg[3 * (size_t)i + k];
     }
   }
 #pragma unroll
@@ -715,8 +716,6 @@ __device__ __forceinline__ void grad_dw(const DwEval& q, int i, int sub, df gA, 
 // Every kernel but the first is launched with programmatic stream
 // serialisation: it may start while the one before drains, fetches its
 // topology rows (which no evaluation writes) and only then waits.
-__device__ __forceinline__ void wait_previous() { cudaGridDependencySynchronize(); }
-__device__ __forceinline__ void let_next_start() { cudaTriggerProgrammaticLaunchCompletion(); }
 
 constexpr int SB = 256;  // threads per block of the split, face and edge kernels
 
@@ -856,23 +855,6 @@ const float4* split_positions_dw(tm_energy* e, int nv, const double* P, cudaStre
   TM_LAUNCH();
   return e->posdw.get();
 }
-
-namespace {
-// launch with programmatic stream serialisation (see wait_previous)
-template <class... A, class... B>
-void launch_after(void (*k)(A...), int grid, int block, cudaStream_t s, B... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(block);
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  TM_CUDA(cudaLaunchKernelEx(&cfg, k, args...));
-}
-}  // namespace
 
 void energy_eval_df(tm_energy* e, tm_mesh* m, const double* P, bool want_grad, double* d_grad, double* d_energy,
                     const Leap* leap, cudaStream_t s, cudaEvent_t* ev) {

@@ -1,18 +1,26 @@
 // Neighbour lists: cell list and Verlet list (src/nlists/cell_list.h,
 // verlet_list.h, nlist.cpp).
 //
-// Cell list build (every rebuild, all on the device except the box):
-//   1. bounding box by a fixed-order min/max reduction, with the reference's
-//      initial values {DBL_MAX,0,0} / {-1,0,0} (cell_list.h:46-47), copied
-//      to the host, which derives r_list/shape/strides exactly like
-//      cell_list.h:56-65
-//   2. cell id per vertex with C truncation (cell_list.h:71-78), inserted
-//      into an open-addressing hash table of the non-empty cells
-//      (2x the vertex count, power of two) -> per-cell counts
-//   3. exclusive scan of the counts -> cell start offsets
-//   4. scatter of the vertex ids, then each cell sorted by vertex id, so a
-//      cell lists its vertices in ascending order like the reference's
-//      std::map<int, std::vector<int>>
+// Cell list build (every rebuild, all on the device; five kernels in one
+// chain of programmatic dependent launches, each a pass over the vertices):
+//   k_box     bounding-box partials with the reference's initial values
+//             {DBL_MAX,0,0} / {-1,0,0} (cell_list.h:46-47); on the side the
+//             hash table is cleared and the near rows' skin is tested
+//   k_insert  every block finishes the box and derives r_list/shape/strides
+//             exactly like cell_list.h:56-65; cell id per vertex with C
+//             truncation (cell_list.h:71-78), inserted into an open-addressing
+//             hash table of the non-empty cells (2x the vertex count, power of
+//             two), which counts the members
+//   k_alloc   a cell's first arrival takes the cell's run of the member array
+//             (the order of the runs is not observable)
+//   k_scatter members into their cell's run in order of arrival
+//   k_rank    rank of each member by vertex id, so a cell lists its vertices
+//             in ascending order like the reference's
+//             std::map<int, std::vector<int>>
+// What bounds it is the chain's length: at 10,242 vertices a rebuild was 13
+// launches and 60 us, with passes over all table slots, a three-kernel scan
+// of them and one thread sorting a cell (a ten-iteration minimisation, eleven
+// rebuilds with two of the near rows: 5.55 ms then, 4.89 now).
 // Queries bin the query point with its CURRENT position but look up the
 // cells' build-time members, as the reference does (cell_list.h:131-219).
 // Distances are rounded operation by operation (no FMA), so pair sets match
@@ -25,6 +33,7 @@
 #include <cstring>
 #include <memory>
 
+#include "tm_chain.cuh"
 #include "tm_energy.cuh"
 #include "tm_internal.h"
 #include "tm_math.cuh"
@@ -85,144 +94,154 @@ __device__ bool nl_excluded(const Topo& t, int excl, int v, int j) {
 namespace {
 
 constexpr int BB = 256;
+constexpr int NBOX = 296;  // most box partials of one mesh: two blocks per SM
 
-__global__ void k_bbox(int nv, const double* P, double* part) {
-  __shared__ double s[6][BB];
-  double lo[3] = {DBL_MAX, 0.0, 0.0}, hi[3] = {-1.0, 0.0, 0.0};
-  for (int i = blockIdx.x * BB + threadIdx.x; i < nv; i += gridDim.x * BB)
+// smaller / larger by the reference's comparisons (a NaN never replaces)
+__device__ __forceinline__ double box_min(double a, double b) { return b < a ? b : a; }
+__device__ __forceinline__ double box_max(double a, double b) { return b > a ? b : a; }
+
+// skin test of the near rows: they go stale once some vertex has moved lc1/2
+// or more from where they were built (thr2 rounded down; NaN moves)
+struct NearCheck {
+  const double* xb;  // NULL: no rows to test
+  double thr2;
+  int* flag;
+  const EP* eps;  // batch: the replica's skin
+};
+
+// Box partials, one per block: a block takes every gridDim-th 256 vertices
+// (batch: exactly its 256, which belong to one replica)
+__global__ void __launch_bounds__(BB) k_box(int nv, const double* __restrict__ P, const int* __restrict__ vrep,
+                                            double* __restrict__ part, CellEntry* __restrict__ T, size_t tsize,
+                                            int* cursor, NearCheck nc) {
+  __shared__ double s[6][BB / 32];
+  let_next_start();
+  const int first = blockIdx.x * BB + threadIdx.x, step = gridDim.x * BB;
+  if (first == 0) *cursor = 0;
+  for (size_t i = first; i < tsize; i += step) T[i] = CellEntry{-1, 0, 0};
+  const bool check = nc.xb && !nc.flag[1];
+  double m[6] = {DBL_MAX, 0.0, 0.0, -1.0, 0.0, 0.0};
+  for (int i = first; i < nv; i += step) {
+    const int rep = vrep ? vrep[i] : 0;
+    if (rep < 0) continue;  // padding vertex of a batch: in no box, never moves
+    const double x[3] = {P[3 * (size_t)i], P[3 * (size_t)i + 1], P[3 * (size_t)i + 2]};
+#pragma unroll
     for (int k = 0; k < 3; ++k) {
-      double x = P[3 * i + k];
-      if (x < lo[k]) lo[k] = x;
-      if (x > hi[k]) hi[k] = x;
+      m[k] = box_min(m[k], x[k]);
+      m[3 + k] = box_max(m[3 + k], x[k]);
     }
-  for (int k = 0; k < 3; ++k) {
-    s[k][threadIdx.x] = lo[k];
-    s[3 + k][threadIdx.x] = hi[k];
+    if (check) {
+      double thr2 = nc.thr2;
+      if (vrep) thr2 = 0.25 * nc.eps[rep].rlc1 * nc.eps[rep].rlc1 * (1.0 - 1e-12);
+      const double dx = x[0] - nc.xb[3 * (size_t)i], dy = x[1] - nc.xb[3 * (size_t)i + 1],
+                   dz = x[2] - nc.xb[3 * (size_t)i + 2];
+      if (!(dx * dx + dy * dy + dz * dz < thr2)) nc.flag[1] = 1;
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 6; ++k) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const double y = __shfl_xor_sync(0xffffffffu, m[k], o);
+      m[k] = k < 3 ? box_min(m[k], y) : box_max(m[k], y);
+    }
+    if ((threadIdx.x & 31) == 0) s[k][threadIdx.x >> 5] = m[k];
   }
   __syncthreads();
-  for (int o = BB / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o)
-      for (int k = 0; k < 3; ++k) {
-        double a = s[k][threadIdx.x + o];
-        if (a < s[k][threadIdx.x]) s[k][threadIdx.x] = a;
-        double b = s[3 + k][threadIdx.x + o];
-        if (b > s[3 + k][threadIdx.x]) s[3 + k][threadIdx.x] = b;
-      }
-    __syncthreads();
+  if (threadIdx.x < 6) {
+    double r = s[threadIdx.x][0];
+    for (int w = 1; w < BB / 32; ++w)
+      r = threadIdx.x < 3 ? box_min(r, s[threadIdx.x][w]) : box_max(r, s[threadIdx.x][w]);
+    part[6 * (size_t)blockIdx.x + threadIdx.x] = r;
   }
-  if (threadIdx.x == 0)
-    for (int k = 0; k < 6; ++k) part[6 * blockIdx.x + k] = s[k][0];
 }
 
-// Bounding box with the reference's initial values, then r_list, shape and
-// strides exactly like src/nlists/cell_list.h:56-65.  One block reduces the
-// block partials (min/max are exact, so the order does not matter).
-__device__ void k_bbox_final_body(int nb, const double* part, double rlist, NLGeom* G);
-__global__ void k_bbox_final(int nb, const double* part, double rlist, NLGeom* G) {
-  k_bbox_final_body(nb, part, rlist, G);
-}
-__device__ void k_bbox_final_body(int nb, const double* part, double rlist, NLGeom* G) {
-  __shared__ double s[6][BB];
-  double lo[3] = {DBL_MAX, 0.0, 0.0}, hi[3] = {-1.0, 0.0, 0.0};
-  for (int b = threadIdx.x; b < nb; b += BB)
-    for (int k = 0; k < 3; ++k) {
-      double a = part[6 * b + k], c = part[6 * b + 3 + k];
-      if (a < lo[k]) lo[k] = a;
-      if (c > hi[k]) hi[k] = c;
+// Bounding box from nb partials, then r_list, shape and strides exactly like
+// src/nlists/cell_list.h:56-65 (min/max are exact, so the order does not
+// matter).  Called by a whole block.
+__device__ void box_geometry(int nb, const double* part, double rlist, NLGeom& G) {
+  __shared__ double s[6];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (w < 6) {
+    double r = w == 0 ? DBL_MAX : (w == 3 ? -1.0 : 0.0);
+    for (int b = lane; b < nb; b += 32) {
+      const double y = part[6 * (size_t)b + w];
+      r = w < 3 ? box_min(r, y) : box_max(r, y);
     }
-  for (int k = 0; k < 3; ++k) {
-    s[k][threadIdx.x] = lo[k];
-    s[3 + k][threadIdx.x] = hi[k];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const double y = __shfl_xor_sync(0xffffffffu, r, o);
+      r = w < 3 ? box_min(r, y) : box_max(r, y);
+    }
+    if (lane == 0) s[w] = r;
   }
   __syncthreads();
-  for (int o = BB / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o)
-      for (int k = 0; k < 3; ++k) {
-        double a = s[k][threadIdx.x + o];
-        if (a < s[k][threadIdx.x]) s[k][threadIdx.x] = a;
-        double c = s[3 + k][threadIdx.x + o];
-        if (c > s[3 + k][threadIdx.x]) s[3 + k][threadIdx.x] = c;
-      }
-    __syncthreads();
-  }
-  if (threadIdx.x) return;
-  const double box_eps = 1.0e-6;
-  for (int k = 0; k < 3; ++k) {
-    double dim = __dadd_rn(__dsub_rn(s[3 + k][0], s[k][0]), box_eps);
-    int nk = (int)__ddiv_rn(dim, rlist);
-    G->rl[k] = nk > 0 ? __ddiv_rn(dim, (double)nk) : dim;
-    G->inv_rl[k] = 1.0 / G->rl[k];
-    G->inv_rlf[k] = (float)G->inv_rl[k];
-    G->bminf[k] = (float)s[k][0];
-    G->shape[k] = nk > 0 ? nk : 1;
-    G->bmin[k] = s[k][0];
-  }
-  G->stride[0] = 1;
-  G->stride[1] = G->shape[0];
-  G->stride[2] = (long long)G->shape[0] * G->shape[1];
-}
-
-// batch: one partial box per 256-vertex block (blocks never straddle
-// replicas), then one block per replica reduces its blocks
-__global__ void k_bbox_blocks(int nv, const double* P, const int* vrep, double* part) {
-  __shared__ double s[6][BB];
-  double lo[3] = {DBL_MAX, 0.0, 0.0}, hi[3] = {-1.0, 0.0, 0.0};
-  int i = blockIdx.x * BB + threadIdx.x;
-  if (i < nv && vrep[i] >= 0)
-    for (int k = 0; k < 3; ++k) {
-      double x = P[3 * i + k];
-      if (x < lo[k]) lo[k] = x;
-      if (x > hi[k]) hi[k] = x;
-    }
-  for (int k = 0; k < 3; ++k) {
-    s[k][threadIdx.x] = lo[k];
-    s[3 + k][threadIdx.x] = hi[k];
+  if (threadIdx.x < 3) {
+    const int k = threadIdx.x;
+    const double box_eps = 1.0e-6;
+    const double dim = __dadd_rn(__dsub_rn(s[3 + k], s[k]), box_eps);
+    const int nk = (int)__ddiv_rn(dim, rlist);
+    G.rl[k] = nk > 0 ? __ddiv_rn(dim, (double)nk) : dim;
+    G.inv_rl[k] = 1.0 / G.rl[k];
+    G.inv_rlf[k] = (float)G.inv_rl[k];
+    G.bminf[k] = (float)s[k];
+    G.shape[k] = nk > 0 ? nk : 1;
+    G.bmin[k] = s[k];
   }
   __syncthreads();
-  for (int o = BB / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o)
-      for (int k = 0; k < 3; ++k) {
-        double a = s[k][threadIdx.x + o];
-        if (a < s[k][threadIdx.x]) s[k][threadIdx.x] = a;
-        double b = s[3 + k][threadIdx.x + o];
-        if (b > s[3 + k][threadIdx.x]) s[3 + k][threadIdx.x] = b;
-      }
-    __syncthreads();
+  if (threadIdx.x == 0) {
+    G.stride[0] = 1;
+    G.stride[1] = G.shape[0];
+    G.stride[2] = (long long)G.shape[0] * G.shape[1];
   }
-  if (threadIdx.x == 0)
-    for (int k = 0; k < 6; ++k) part[6 * blockIdx.x + k] = s[k][0];
+  __syncthreads();
 }
 
-__global__ void k_bbox_final_batch(const int2* rblocks, const double* part, const double* rlist, NLGeom* geoms) {
-  int r = blockIdx.x;
-  int2 rb = rblocks[r];
-  k_bbox_final_body(rb.y - rb.x, part + 6 * rb.x, rlist[r], geoms + r);
-}
-
-__global__ void k_table_init(CellEntry* T, size_t n) {
-  size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  if (i < n) {
-    T[i].key = -1;
-    T[i].start = 0;
-    T[i].count = 0;
+// (int)(x / rl) as the reference truncates it: the product with 1 / rl is
+// within 3 ulps of the quotient, so the truncation differs only next to an
+// integer (or out of range), where the division decides
+__device__ __forceinline__ int cell_coord(double x, double rl, double inv_rl) {
+  const double q = x * inv_rl;
+  if (q > 0.0 && q < 1.0e6) {
+    const int c = (int)q;
+    const double r = q - (double)c;
+    if (r > 1.0e-9 && r < 1.0 - 1.0e-9) return c;
   }
+  return (int)__ddiv_rn(x, rl);
 }
 
-__global__ void k_cell_insert(int nv, const double* P, NLView nl, CellEntry* T, long long* vcid, int* vcoord,
-                              int* vslot, int* status) {
-  int v = blockIdx.x * blockDim.x + threadIdx.x;
+// cell of every vertex and its hash slot; vrank takes the order of arrival
+// in the cell.  rblocks: the box partials of each replica of a batch.
+__global__ void __launch_bounds__(BB) k_insert(int nv, const double* __restrict__ P, NLView nl, CellEntry* T,
+                                               const double* part, int nb,
+                                               const int2* __restrict__ rblocks, double rlist,
+                                               const double* __restrict__ rlists, NLGeom* geoms, long long* vcid,
+                                               int* vcoord, int* vslot, int* vrank, int* status) {
+  __shared__ NLGeom G;
+  let_next_start();
+  const int v = blockIdx.x * BB + threadIdx.x;
+  const int brep = nl.vrep ? nl.vrep[blockIdx.x * BB] : 0;  // the block's replica (its first vertex is real)
+  int b0 = 0;
+  if (nl.vrep) {
+    const int2 rb = rblocks[brep];
+    b0 = rb.x;
+    nb = rb.y - rb.x;
+    rlist = rlists[brep];
+  }
+  wait_previous();
+  box_geometry(nb, part + 6 * (size_t)b0, rlist, G);
+  if (threadIdx.x == 0 && (int)blockIdx.x == b0) geoms[brep] = G;
   if (v >= nv) return;
-  int rep = rep_of(nl, v);
+  const int rep = rep_of(nl, v);
   if (rep < 0) {  // padding vertex of a batch: in no cell
     vslot[v] = -1;
     vcid[v] = -1;
     vcoord[3 * v] = vcoord[3 * v + 1] = vcoord[3 * v + 2] = -1000000;
     return;
   }
-  const NLGeom& G = nl.geom[rep];
   long long id = 0;
   for (int k = 0; k < 3; ++k) {
-    int c = (int)__ddiv_rn(__dsub_rn(P[3 * v + k], G.bmin[k]), G.rl[k]);
+    const int c = cell_coord(__dsub_rn(P[3 * (size_t)v + k], G.bmin[k]), G.rl[k], G.inv_rl[k]);
     vcoord[3 * v + k] = c;
     id += (long long)c * G.stride[k];
   }
@@ -241,46 +260,57 @@ __global__ void k_cell_insert(int nv, const double* P, NLView nl, CellEntry* T, 
   }
   if (slot < 0) {
     atomicExch(status, 1);
-    vslot[v] = 0;
+    vslot[v] = -1;
     return;
   }
   vslot[v] = slot;
-  atomicAdd(&T[slot].count, 1);
+  vrank[v] = atomicAdd(&T[slot].count, 1);
 }
 
-__global__ void k_counts(const CellEntry* T, int n, int* cnt) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) cnt[i] = T[i].count;
-}
-__global__ void k_set_start(CellEntry* T, int n, const int* start) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) T[i].start = start[i];
-}
-__global__ void k_scatter(int nv, const int* vslot, const CellEntry* T, int* fill, int* cell_verts) {
-  int v = blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= nv) return;
-  int s = vslot[v];
-  if (s < 0) return;
-  int pos = T[s].start + atomicAdd(&fill[s], 1);
-  cell_verts[pos] = v;
-}
-// sort each cell's members ascending and record each vertex's rank in its cell
-__global__ void k_sort_cells(const CellEntry* T, int n, int* cell_verts, int* vrank) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  int c = T[i].count;
-  if (c < 1) return;
-  int* a = cell_verts + T[i].start;
-  for (int x = 1; x < c; ++x) {
-    int key = a[x];
-    int y = x - 1;
-    while (y >= 0 && a[y] > key) {
-      a[y + 1] = a[y];
-      --y;
-    }
-    a[y + 1] = key;
+// a cell's first arrival takes the cell's run of members (one atomic a warp)
+__global__ void __launch_bounds__(BB) k_alloc(int nv, const int* vslot, const int* vrank,
+                                              CellEntry* T, int* cursor) {
+  let_next_start();
+  wait_previous();
+  const int v = blockIdx.x * BB + threadIdx.x, lane = threadIdx.x & 31;
+  const int slot = v < nv ? vslot[v] : -1;
+  const bool first = slot >= 0 && vrank[v] == 0;
+  const int n = first ? T[slot].count : 0;
+  int incl = n;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
   }
-  for (int x = 0; x < c; ++x) vrank[a[x]] = x;
+  int base = 0;
+  if (lane == 31 && incl > 0) base = atomicAdd(cursor, incl);
+  base = __shfl_sync(0xffffffffu, base, 31);
+  if (first) T[slot].start = base + incl - n;
+}
+__global__ void __launch_bounds__(BB) k_scatter(int nv, const int* vslot, const int* vrank,
+                                                const CellEntry* T, int* members) {
+  let_next_start();
+  wait_previous();
+  const int v = blockIdx.x * BB + threadIdx.x;
+  if (v >= nv) return;
+  const int s = vslot[v];
+  if (s >= 0) members[T[s].start + vrank[v]] = v;
+}
+// rank of each vertex among its cell's members (ascending vertex id)
+__global__ void __launch_bounds__(BB) k_rank(int nv, const int* vslot, const CellEntry* T,
+                                             const int* members, int* cell_verts,
+                                             int* vrank) {
+  let_next_start();
+  wait_previous();
+  const int v = blockIdx.x * BB + threadIdx.x;
+  if (v >= nv) return;
+  const int s = vslot[v];
+  if (s < 0) return;
+  const CellEntry c = T[s];
+  int r = 0;
+  for (int q = 0; q < c.count; ++q) r += members[c.start + q] < v ? 1 : 0;
+  cell_verts[c.start + r] = v;
+  vrank[v] = r;
 }
 
 // Position of the pair {v, u} in the reference's distance_matrix traversal
@@ -482,118 +512,123 @@ __global__ void k_cand(int nv, NLView nl, const int* vcoord, int pass, int* cnt,
 // table (the cells that meet the ball of radius rn), with a flag for pairs
 // excluded on the current topology.  A row longer than TM_NEAR_CAP marks the
 // rows unusable (flag[3]).
-constexpr int NB = 128;  // threads per block of k_near
-__global__ void __launch_bounds__(NB) k_near(int nv, const double* P, NLView nl, Topo t, int excl, double rn,
-                                             double rn2, int* flag, int* ncnt, int* nent, double* xb,
-                                             const EP* eps) {
-  // the row of each thread, staged in shared memory (stride 49: no bank
-  // conflicts) while the exclusion flags are set
-  __shared__ int srow[NB][TM_NEAR_CAP + 1];
+// Eight lanes share a vertex: each looks up every eighth of the up to 343
+// cells around the ball (most are empty, so the time is the chain of hash
+// probes) and walks the rings of every eighth ring vertex for the exclusion
+// flags.  A row's order does not matter to its readers, which visit accepted
+// pairs by their cell and id; it is the same from run to run.  10,242
+// vertices: 290 us with one thread per vertex.
+constexpr int NB = 128;   // threads per block of k_near
+constexpr int NL8 = 8;    // lanes per vertex
+constexpr int NEAR_BLOCKS = 8 * 152;  // resident blocks, looping over the vertices
+__global__ void __launch_bounds__(NB) k_near(int nv, const double* __restrict__ P, NLView nl, Topo t, int excl,
+                                             double rn, double rn2, int* flag, const int* dtopo, int* ncnt,
+                                             int* nent, double* xb, const EP* eps) {
+  __shared__ int srow[NB / NL8][TM_NEAR_CAP + 1];
+  let_next_start();
+  wait_previous();
   if (flag[1] == 0) return;  // rows still valid
-  int a = blockIdx.x * blockDim.x + threadIdx.x;
-  if (a >= nv) return;
-  const int rep = rep_of(nl, a);
-  if (rep < 0) {  // padding vertex of a batch
-    ncnt[a] = 0;
-    return;
-  }
-  if (eps) {  // batch: the replica's cut-off
-    rn = 2.0 * eps[rep].rlc1;
-    rn2 = rn * rn * (1.0 + 1e-12);
-  }
-  const NLGeom& G = nl.geom[rep];
-  d3 pa = ld3(P, a);
-  const double* pp = &pa.x;
-  int lo[3], hi[3];
-  // position in cell units (float) for the box-distance pruning; a cell is
-  // skipped only when it is farther than rn after every axis distance is
-  // shortened by 1e-3 cell widths plus 8 float ulps of the coordinate, far
-  // above the float rounding of the cell coordinate
-  float u[3], rlf[3], mg[3];
-  for (int k = 0; k < 3; ++k) {
-    lo[k] = max(0, (int)floor((pp[k] - rn - G.bmin[k]) * G.inv_rl[k]) - 1);
-    hi[k] = min(G.shape[k] - 1, (int)floor((pp[k] + rn - G.bmin[k]) * G.inv_rl[k]) + 1);
-    u[k] = (float)((pp[k] - G.bmin[k]) * G.inv_rl[k]);
-    rlf[k] = (float)G.rl[k];
-    mg[k] = 1e-3f + 9.6e-7f * fabsf(u[k]);
-  }
-  const float rnf2 = (float)rn2 * 1.0001f;
-  int* row = srow[threadIdx.x];
-  int n = 0;
-  for (int ii = lo[0]; ii <= hi[0]; ++ii) {
-    float dx = fmaxf(fmaxf((float)ii - u[0], u[0] - (float)(ii + 1)) - mg[0], 0.0f) * rlf[0];
-    for (int jj = lo[1]; jj <= hi[1]; ++jj) {
-      float dy = fmaxf(fmaxf((float)jj - u[1], u[1] - (float)(jj + 1)) - mg[1], 0.0f) * rlf[1];
-      float gxy = dx * dx + dy * dy;
-      if (gxy > rnf2) continue;
-      for (int kk = lo[2]; kk <= hi[2]; ++kk) {
-        float dz = fmaxf(fmaxf((float)kk - u[2], u[2] - (float)(kk + 1)) - mg[2], 0.0f) * rlf[2];
-        if (gxy + dz * dz > rnf2) continue;
-        long long cid = ii * G.stride[0] + jj * G.stride[1] + kk * G.stride[2];
-        int st = 0;
-        int c = cell_lookup(nl, cell_key(cid, rep), &st);
-        for (int q = 0; q < c; ++q) {
-          int b = nl.cell_verts[st + q];
-          if (b == a) continue;
-          d3 pb = ld3(P, b);
-          double ex = pa.x - pb.x, ey = pa.y - pb.y, ez = pa.z - pb.z;
-          if (ex * ex + ey * ey + ez * ez >= rn2) continue;
-          if (n < TM_NEAR_CAP) row[n] = b;
-          ++n;
+  const int sub = threadIdx.x % NL8, lane = threadIdx.x & 31;
+  const unsigned gmask = ((1u << NL8) - 1u) << (lane & ~(NL8 - 1)), below = (1u << lane) - 1u;
+  int* row = srow[threadIdx.x / NL8];
+  for (int a = (blockIdx.x * NB + threadIdx.x) / NL8; a < nv; a += gridDim.x * (NB / NL8)) {
+    const int rep = rep_of(nl, a);
+    if (rep < 0) {  // padding vertex of a batch
+      if (sub == 0) ncnt[a] = 0;
+      continue;
+    }
+    if (eps) {  // batch: the replica's cut-off
+      rn = 2.0 * eps[rep].rlc1;
+      rn2 = rn * rn * (1.0 + 1e-12);
+    }
+    const NLGeom& G = nl.geom[rep];
+    const d3 pa = ld3(P, a);
+    const double* pp = &pa.x;
+    int lo[3], hi[3];
+    // position in cell units (float) for the box-distance pruning; a cell is
+    // skipped only when it is farther than rn after every axis distance is
+    // shortened by 1e-3 cell widths plus 8 float ulps of the coordinate, far
+    // above the float rounding of the cell coordinate
+    float u[3], rlf[3], mg[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      lo[k] = max(0, (int)floor((pp[k] - rn - G.bmin[k]) * G.inv_rl[k]) - 1);
+      hi[k] = min(G.shape[k] - 1, (int)floor((pp[k] + rn - G.bmin[k]) * G.inv_rl[k]) + 1);
+      u[k] = (float)((pp[k] - G.bmin[k]) * G.inv_rl[k]);
+      rlf[k] = (float)G.rl[k];
+      mg[k] = 1e-3f + 9.6e-7f * fabsf(u[k]);
+    }
+    const float rnf2 = (float)rn2 * 1.0001f;
+    const int ny = hi[1] - lo[1] + 1, nz = hi[2] - lo[2] + 1;
+    const int ncell = hi[0] >= lo[0] && ny > 0 && nz > 0 ? (hi[0] - lo[0] + 1) * ny * nz : 0;
+    int n = 0;
+    for (int c0 = 0; c0 < ncell; c0 += NL8) {
+      const int c = c0 + sub;
+      int cnt = 0, st = 0;
+      if (c < ncell) {
+        const int kk = lo[2] + c % nz, ij = c / nz;
+        const int jj = lo[1] + ij % ny, ii = lo[0] + ij / ny;
+        const float dx = fmaxf(fmaxf((float)ii - u[0], u[0] - (float)(ii + 1)) - mg[0], 0.0f) * rlf[0];
+        const float dy = fmaxf(fmaxf((float)jj - u[1], u[1] - (float)(jj + 1)) - mg[1], 0.0f) * rlf[1];
+        const float dz = fmaxf(fmaxf((float)kk - u[2], u[2] - (float)(kk + 1)) - mg[2], 0.0f) * rlf[2];
+        if (!(dx * dx + dy * dy + dz * dz > rnf2))
+          cnt = cell_lookup(nl, cell_key(ii * G.stride[0] + jj * G.stride[1] + kk * G.stride[2], rep), &st);
+      }
+      for (int q = 0; __any_sync(gmask, q < cnt); ++q) {
+        bool acc = false;
+        int b = a;
+        if (q < cnt) {
+          b = nl.cell_verts[st + q];
+          const d3 pb = ld3(P, b);
+          const double ex = pa.x - pb.x, ey = pa.y - pb.y, ez = pa.z - pb.z;
+          acc = b != a && !(ex * ex + ey * ey + ez * ez >= rn2);
         }
+        const unsigned bal = __ballot_sync(gmask, acc);
+        const int pos = n + __popc(bal & below);
+        if (acc && pos < TM_NEAR_CAP) row[pos] = b;
+        n += __popc(bal);
       }
     }
-  }
-  if (n > TM_NEAR_CAP) atomicOr(&flag[3], 1);
-  n = min(n, TM_NEAR_CAP);
-  // exclusion flags (nl_excluded): an entry is excluded when it is in the
-  // ring of a or, at level 2, in the ring of a ring vertex of a; the rings
-  // are walked once and their vertices looked up in the row
-  if (nl.rexcl) excl = nl.rexcl[rep];  // batch: the replica's level
-  if (excl > 0 && n > 0) {
-    const int d = t.val[a];
-    for (int m = 0; m < d; ++m) {
-      const int w = t.nbr[(size_t)m * t.nv + a];
-      for (int e = 0; e < n; ++e)
-        if (row[e] == w) row[e] |= (int)0x80000000u;
-      if (excl > 1) {
-        const int dw = t.val[w];
-        for (int q = 0; q < dw; ++q) {
-          const int x = t.nbr[(size_t)q * t.nv + w];
-          for (int e = 0; e < n; ++e)
-            if ((row[e] & 0x7fffffff) == x) row[e] |= (int)0x80000000u;
+    if (sub == 0 && n > TM_NEAR_CAP) atomicOr(&flag[3], 1);
+    n = min(n, TM_NEAR_CAP);
+    __syncwarp(gmask);
+    // exclusion flags (nl_excluded): an entry is excluded when it is in the
+    // ring of a or, at level 2, in the ring of a ring vertex of a; the rings
+    // are walked once and their vertices looked up in the row
+    const int level = nl.rexcl ? nl.rexcl[rep] : excl;  // batch: the replica's level
+    if (level > 0 && n > 0) {
+      const int d = t.val[a];
+      auto mark = [&](int w) {
+        for (int e = 0; e < n; ++e)
+          if ((row[e] & 0x7fffffff) == w) atomicOr(&row[e], (int)0x80000000u);
+      };
+      for (int m = sub; m < d; m += NL8) {
+        const int w = t.nbr[(size_t)m * t.nv + a];
+        mark(w);
+        if (level > 1) {
+          const int dw = t.val[w];
+          for (int q = 0; q < dw; ++q) mark(t.nbr[(size_t)q * t.nv + w]);
         }
       }
+      __syncwarp(gmask);
+    }
+    int* out = nent + (size_t)a * TM_NEAR_CAP;
+    for (int e = sub; e < n; e += NL8) out[e] = row[e];
+    if (sub == 0) ncnt[a] = n;
+    if (sub < 3) xb[3 * (size_t)a + sub] = pp[sub];
+    __syncwarp(gmask);  // the row is reused
+  }
+  // the last block (it follows every block's reads of the flag): usable
+  // unless a row overflowed; record the topology version
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(&flag[4], 1) == (int)gridDim.x - 1) {
+      flag[1] = atomicExch(&flag[3], 0);
+      flag[2] = *dtopo;
+      flag[4] = 0;
     }
   }
-  int* out = nent + (size_t)a * TM_NEAR_CAP;
-  for (int e = 0; e < n; ++e) out[e] = row[e];
-  ncnt[a] = n;
-  xb[3 * a] = pa.x;
-  xb[3 * a + 1] = pa.y;
-  xb[3 * a + 2] = pa.z;
-}
-// after a build: usable unless a row overflowed; record the topology version
-__global__ void k_near_done(int* flag, const int* dtopo) {
-  if (threadIdx.x || blockIdx.x) return;
-  if (flag[1] == 0) return;
-  flag[1] = flag[3];
-  flag[2] = *dtopo;
-  flag[3] = 0;
-}
-// before a cell-list rebuild: the rows go stale once some vertex has moved
-// lc1/2 or more from where they were built (thr2 rounded down; NaN moves)
-__global__ void k_near_check(int nv, const double* __restrict__ P, const double* __restrict__ xb, double thr2,
-                             int* flag, const int* __restrict__ vrep, const EP* __restrict__ eps) {
-  int v = blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= nv || flag[1]) return;
-  if (vrep) {  // batch: the replica's skin, padding vertices never move
-    int r = vrep[v];
-    if (r < 0) return;
-    thr2 = 0.25 * eps[r].rlc1 * eps[r].rlc1 * (1.0 - 1e-12);
-  }
-  double dx = P[3 * v] - xb[3 * v], dy = P[3 * v + 1] - xb[3 * v + 1], dz = P[3 * v + 2] - xb[3 * v + 2];
-  if (!(dx * dx + dy * dy + dz * dz < thr2)) flag[1] = 1;
 }
 
 // distance_matrix of the Verlet list: rows in vertex order, d < rd
@@ -678,10 +713,21 @@ inline int nblk(long n, int b) { return (int)((n + b - 1) / b); }
 
 }  // namespace
 
-// Steps 2-4 of the cell-list build and the candidate rows (shared by single
-// meshes and batches; V.geom and V.vrep are set by the caller).
-static void build_cells(tm_nlist* nl, NLView& V, int nv, const double* P, cudaStream_t s, bool candidates) {
-  // 2. hash table of the non-empty cells: 2x the vertex count, power of two
+// What a build needs beside the mesh: one box (rlist) or one per replica of
+// a batch (vrep in the view, rblocks, rlists)
+struct BoxInput {
+  double rlist;
+  const int2* rblocks;
+  const double* rlists;
+  int boxes;
+};
+
+// The cell list (header comment) and the candidate rows, shared by single
+// meshes and batches; V.vrep is set by the caller.  near: test the near
+// rows' skin on the side.
+static void build_cells(tm_nlist* nl, NLView& V, int nv, const double* P, const BoxInput& in, const NearCheck& near,
+                        cudaStream_t s, bool candidates) {
+  // hash table of the non-empty cells: 2x the vertex count, power of two
   size_t tsize = 64;
   while (tsize < 2 * (size_t)std::max(nv, 1)) tsize <<= 1;
   nl->table.ensure(tsize);
@@ -690,34 +736,27 @@ static void build_cells(tm_nlist* nl, NLView& V, int nv, const double* P, cudaSt
   nl->vcoord.ensure(3 * (size_t)std::max(nv, 1));
   nl->vslot.ensure(std::max(nv, 1));
   nl->vrank.ensure(std::max(nv, 1));
-  nl->cnt.ensure(tsize + 1);
-  nl->fill.ensure(tsize);
+  nl->fill.ensure((size_t)std::max(nv, 1));
   nl->cell_verts.ensure(std::max(nv, 1));
   nl->d_count.ensure(4);
-  k_table_init<<<nblk((long)tsize, 256), 256, 0, s>>>(nl->table.get(), tsize);
-  TM_LAUNCH();
+  const int vb = std::max(1, nblk(nv, BB));
+  const int nb = V.vrep ? vb : std::min(NBOX, vb);
+  nl->bbox.ensure(6 * (size_t)nb);
+  nl->geom.ensure(in.boxes);
+  V.geom = nl->geom.get();
   V.table = nl->table.get();
   V.cell_verts = nl->cell_verts.get();
   V.bcoord = nl->vcoord.get();  // build-time cell of every vertex
-  if (nv > 0) {
-    k_cell_insert<<<nblk(nv, 256), 256, 0, s>>>(nv, P, V, nl->table.get(), nl->vcid.get(), nl->vcoord.get(),
-                                                nl->vslot.get(), nl->d_count.get());
-    TM_LAUNCH();
-    // 3. offsets
-    k_counts<<<nblk((long)tsize, 256), 256, 0, s>>>(nl->table.get(), (int)tsize, nl->cnt.get());
-    TM_LAUNCH();
-    exclusive_scan_int(nl->cnt.get(), nl->fill.get(), (int)tsize, nullptr, nl->tmp, s);
-    k_set_start<<<nblk((long)tsize, 256), 256, 0, s>>>(nl->table.get(), (int)tsize, nl->fill.get());
-    TM_LAUNCH();
-    // 4. scatter + per-cell sort (members ascending, rank of each vertex)
-    TM_CUDA(cudaMemsetAsync(nl->fill.get(), 0, sizeof(int) * tsize, s));
-    k_scatter<<<nblk(nv, 256), 256, 0, s>>>(nv, nl->vslot.get(), nl->table.get(), nl->fill.get(),
-                                            nl->cell_verts.get());
-    TM_LAUNCH();
-    k_sort_cells<<<nblk((long)tsize, 256), 256, 0, s>>>(nl->table.get(), (int)tsize, nl->cell_verts.get(),
-                                                        nl->vrank.get());
-    TM_LAUNCH();
-  }
+  int* status = nl->d_count.get();
+  int* cursor = status + 1;
+  k_box<<<nb, BB, 0, s>>>(nv, P, V.vrep, nl->bbox.get(), nl->table.get(), tsize, cursor, near);
+  TM_LAUNCH();
+  launch_after(k_insert, vb, BB, s, nv, P, V, nl->table.get(), nl->bbox.get(), nb, in.rblocks, in.rlist, in.rlists,
+               nl->geom.get(), nl->vcid.get(), nl->vcoord.get(), nl->vslot.get(), nl->vrank.get(), status);
+  launch_after(k_alloc, vb, BB, s, nv, nl->vslot.get(), nl->vrank.get(), nl->table.get(), cursor);
+  launch_after(k_scatter, vb, BB, s, nv, nl->vslot.get(), nl->vrank.get(), nl->table.get(), nl->fill.get());
+  launch_after(k_rank, vb, BB, s, nv, nl->vslot.get(), nl->table.get(), nl->fill.get(), nl->cell_verts.get(),
+               nl->vrank.get());
   if (candidates && nv > 0) {
     // candidate rows for the queries of points that stay in their build cell
     nl->crow.ensure((size_t)nv + 1);
@@ -747,31 +786,29 @@ static void build_cells(tm_nlist* nl, NLView& V, int nv, const double* P, cudaSt
 // current cell and visits them in the reference's order.  The rows do not
 // depend on the cell list, so a cell-list rebuild rebuilds them only when a
 // vertex has moved lc1/2 since they were built (decided on the device).
-static void refresh_near(tm_nlist* nl, tm_mesh* m, NLView& V, const double* P, double lc1, cudaStream_t s,
-                         const EP* eps = nullptr) {
-  int nv = nl->nv;
-  Topo t = m->topo();
-  double rn = 2.0 * lc1;
+static NearCheck prepare_near(tm_nlist* nl, int nv, double lc1, cudaStream_t s, const EP* eps = nullptr) {
   if (nl->near_nv != nv || nl->near_lc1 != lc1) {
     nl->nent.ensure((size_t)nv * TM_NEAR_CAP);
     nl->ncnt.ensure(nv);
     nl->xb.ensure(3 * (size_t)nv);
-    nl->nflag.ensure(4);
-    int init[4] = {0, 1, 0, 0};  // stale until built
+    nl->nflag.ensure(5);
+    int init[5] = {0, 1, 0, 0, 0};  // stale until built
     TM_CUDA(cudaMemcpyAsync(nl->nflag.get(), init, sizeof(init), cudaMemcpyHostToDevice, s));
     TM_CUDA(cudaStreamSynchronize(s));
     nl->near_nv = nv;
     nl->near_lc1 = lc1;
     nl->near_move2 = 0.25 * lc1 * lc1 * (1.0 - 1e-12);
   }
+  return NearCheck{nl->xb.get(), nl->near_move2, nl->nflag.get(), eps};
+}
+// after build_cells with the check of prepare_near
+static void refresh_near(tm_nlist* nl, tm_mesh* m, NLView& V, const double* P, double lc1, cudaStream_t s,
+                         const EP* eps = nullptr) {
+  const int nv = nl->nv;
+  const double rn = 2.0 * lc1;
   int* flag = nl->nflag.get();
-  k_near_check<<<nblk(nv, 256), 256, 0, s>>>(nv, P, nl->xb.get(), nl->near_move2, flag, V.vrep, eps);
-  TM_LAUNCH();
-  k_near<<<nblk(nv, NB), NB, 0, s>>>(nv, P, V, t, V.excl, rn, rn * rn * (1.0 + 1e-12), flag, nl->ncnt.get(),
-                                       nl->nent.get(), nl->xb.get(), eps);
-  TM_LAUNCH();
-  k_near_done<<<1, 32, 0, s>>>(flag, m->d_topo_ver.get());
-  TM_LAUNCH();
+  launch_after(k_near, std::min(NEAR_BLOCKS, nblk((long)nv * NL8, NB)), NB, s, nv, P, V, m->topo(), V.excl, rn,
+               rn * rn * (1.0 + 1e-12), flag, m->d_topo_ver.get(), nl->ncnt.get(), nl->nent.get(), nl->xb.get(), eps);
   V.nent = nl->nent.get();
   V.ncnt = nl->ncnt.get();
   V.nflag = flag;
@@ -790,21 +827,12 @@ void nlist_make(tm_nlist* nl, tm_mesh* m, const tm_params& p, const double* P, c
   V = NLView{};
   V.kind = 0;
   V.excl = p.exclusion_level;
-  // 1. box and cell geometry (device only, no host round trip)
-  int nb = std::max(1, std::min(1024, nblk(nv, BB)));
-  nl->bbox.ensure(6 * (size_t)nb + 6);
-  nl->geom.ensure(1);
-  V.geom = nl->geom.get();
-  if (nv > 0) {
-    k_bbox<<<nb, BB, 0, s>>>(nv, P, nl->bbox.get());
-    TM_LAUNCH();
-  }
-  k_bbox_final<<<1, BB, 0, s>>>(nv > 0 ? nb : 0, nl->bbox.get(), p.rlist, nl->geom.get());
-  TM_LAUNCH();
   // with near rows the candidate rows are not needed: the rare fallback
   // (a vertex moved lc1/2 since the rows were built) takes the cell walk
   const bool near = p.n_search == 0 && p.rep_lc1 > 0 && p.rlist >= p.rep_lc1 && nv > 0;
-  build_cells(nl, V, nv, P, s, p.n_search == 0 && !near);
+  NearCheck nc{};
+  if (near) nc = prepare_near(nl, nv, p.rep_lc1, s);
+  build_cells(nl, V, nv, P, BoxInput{p.rlist, nullptr, nullptr, 1}, nc, s, p.n_search == 0 && !near);
   if (near) refresh_near(nl, m, V, P, p.rep_lc1, s);
   if (p.n_search == 1) {
     // Verlet CSR from the cell list at cut-off rlist, rows in the reference's
@@ -854,20 +882,11 @@ void nlist_make_batch(tm_nlist* nl, tm_mesh* m, int R, const int* d_vrep, const 
   V.excl = excl;
   V.rexcl = d_rexcl;
   V.vrep = d_vrep;
-  int nb = std::max(1, nblk(nv, BB));
-  nl->bbox.ensure(6 * (size_t)nb);
-  nl->geom.ensure(R);
-  V.geom = nl->geom.get();
-  if (nv > 0) {
-    k_bbox_blocks<<<nb, BB, 0, s>>>(nv, P, d_vrep, nl->bbox.get());
-    TM_LAUNCH();
-  }
-  k_bbox_final_batch<<<R, BB, 0, s>>>(d_rblocks, nl->bbox.get(), d_rlist, nl->geom.get());
-  TM_LAUNCH();
+  const BoxInput in{0.0, d_rblocks, d_rlist, R};
   if (verlet) {
     // Verlet rows at each replica's cut-off, ordered like the single-mesh
     // rows (the reference's insertion order)
-    build_cells(nl, V, nv, P, s, false);
+    build_cells(nl, V, nv, P, in, NearCheck{}, s, false);
     nl->vrow.ensure((size_t)nv + 1);
     Topo t = m->topo();
     int total = 0;
@@ -899,9 +918,11 @@ void nlist_make_batch(tm_nlist* nl, tm_mesh* m, int R, const int* d_vrep, const 
   // candidate rows as well: unrelaxed replicas can move a skin's width
   // within a few steps, and then the candidate rows keep most vertices off
   // the cell walk
-  build_cells(nl, V, nv, P, s, true);
   // near rows with each replica's cut-off (the lc1 argument only tags the
   // rows: any positive value)
+  NearCheck nc{};
+  if (near && nv > 0) nc = prepare_near(nl, nv, 1.0, s, d_eps);
+  build_cells(nl, V, nv, P, in, nc, s, true);
   if (near && nv > 0) refresh_near(nl, m, V, P, 1.0, s, d_eps);
 }
 

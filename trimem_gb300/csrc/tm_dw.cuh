@@ -13,9 +13,10 @@ __device__ __forceinline__ df third() { return {3.333333433e-01f, -9.934107481e-
 __device__ __forceinline__ df sixth() { return {1.666666716e-01f, -4.967053740e-09f}; }
 
 // 32 bytes of read-only data in one load instruction, 32-byte aligned: one
-// sector per lane instead of two 16-byte requests
+// sector per lane instead of two 16-byte requests (volatile: stays below the
+// wait for the kernel that writes the data)
 __device__ __forceinline__ void ld32(const float4* p, float4& a, float4& b) {
-  asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+  asm volatile("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
       : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
       : "l"(p));
 }

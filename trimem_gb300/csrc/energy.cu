@@ -601,7 +601,17 @@ void tm_energy::to_host(double* dst, const double* src, size_t n) {
   TM_CUDA(cudaStreamSynchronize(stream));
 }
 
+double* tm_energy::host_scalars() {
+  if (!pinned && cudaMallocHost(&pinned, 16 * sizeof(double)) != cudaSuccess) {
+    cudaGetLastError();
+    pinned = nullptr;
+    fail(TM_ERR_NOMEM, "page-locked allocation failed");
+  }
+  return pinned;
+}
+
 tm_energy::~tm_energy() {
+  if (pinned) cudaFreeHost(pinned);
   for (auto& g : eval_graphs)
     if (g.exec) cudaGraphExecDestroy(g.exec);
   if (flip_graph.exec) cudaGraphExecDestroy(flip_graph.exec);

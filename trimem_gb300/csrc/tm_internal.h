@@ -231,6 +231,11 @@ struct tm_energy {
   tmg::DevBuf<unsigned char> fw_winner, fw_state;
   tmg::DevBuf<double> fw_dpn;
   tmg::DevBuf<float> fw_dpf;
+  tmg::DevBuf<double> mwork;  // minimisation workspace, kept between calls
+  // a few page-locked doubles that kernels write for the host (one call at a
+  // time, like every other workspace of the handle)
+  double* pinned = nullptr;
+  double* host_scalars();
   cudaStream_t stream = nullptr;
   // second stream: the repulsion pass runs there, concurrent with the
   // edge kernels, between a fork and a join event

@@ -22,11 +22,13 @@
 // dense weights W^r are bf16 with FP32 accumulation in tensor memory; the
 // small layers are FP32.
 //
-// The dense layer is one CTA per 128 vertices: TMA loads [h | m] (two
-// 128 x 64 bf16 boxes) and W^r (two 64 x 64 boxes) into 128-byte-swizzled
-// shared memory, one thread issues 8 tcgen05.mma (M 128, N 64, K 16), the
-// accumulator (128 lanes x 64 FP32 columns) is read back by four warps and
-// the epilogue adds bias, SiLU and the residual h (from the swizzled tile).
+// A round is one CTA per 128 vertices (k_layer): TMA loads h (a 128 x 64 bf16
+// box) and W^r (two 64 x 64 boxes) into 128-byte-swizzled shared memory while
+// the threads gather the messages m into the other operand tile; one thread
+// issues 8 tcgen05.mma (M 128, N 64, K 16), the accumulator (128 lanes x 64
+// FP32 columns) is read back by eight warps, the epilogue adds bias, SiLU and
+// the residual h (in the swizzled tile), and TMA stores the tile.  k_dense is
+// the dense layer alone, on given [h | m] (tm_dense_silu_bf16).
 #include <cuda_bf16.h>
 #include <cudaTypedefs.h>
 
@@ -78,12 +80,11 @@ struct tm_surrogate {
   SurW hw{};
   DevBuf<SurW> w;
   DevBuf<__nv_bfloat16> wd;  // dense weights [NR][H][2H] (row n, column k)
-  DevBuf<float> u, nrm;
-  DevBuf<__nv_bfloat16> hb[2], mb;
+  DevBuf<float> nrm;
+  DevBuf<__nv_bfloat16> hb[2];
   DevBuf<double> gloc;
   DevBuf<int> status;
   alignas(64) CUtensorMap map_h[2];
-  alignas(64) CUtensorMap map_m;
   alignas(64) CUtensorMap map_w[NR];
 };
 
@@ -96,57 +97,97 @@ inline int nblk(long n, int b) { return (int)((n + b - 1) / b); }
 
 __device__ __forceinline__ float silu(float x) { return x / (1.0f + __expf(-x)); }
 
-// vertex features, normal and embedding (one thread per vertex)
-__global__ void k_sfeat(Topo t, const FaceF* __restrict__ fd, const EdgeF* __restrict__ ed,
-                        const float* __restrict__ rho, const SurW* __restrict__ W, float* __restrict__ u,
-                        float* __restrict__ nrm, __nv_bfloat16* __restrict__ h) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= t.nv) return;
-  const float lbar = W->lbar, abar = W->abar;
-  int d = t.val[i];
-  float A = 0.f, ls = 0.f, l2 = 0.f, ths = 0.f, th2 = 0.f;
-  f3 N = {0.f, 0.f, 0.f};
-  for (int m = 0; m < d; ++m) {
-    int4 s = t.slot[(size_t)m * t.nv + i];
-    int f = slot_face(s.y);
-    if (f >= 0) {
-      FaceF F = fd[f];
-      A += F.A;
-      N += F.A * f3{F.nx, F.ny, F.nz};
+__device__ __forceinline__ uint4 pack8(const float* f) {
+  uint4 v;
+  __nv_bfloat162* b = reinterpret_cast<__nv_bfloat162*>(&v);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) b[q] = __floats2bfloat162_rn(f[2 * q], f[2 * q + 1]);
+  return v;
+}
+
+// the input layer's weights of channels 8 sub .. 8 sub + 7, in registers
+struct Embed8 {
+  float w[8][FV], b[8];
+  __device__ __forceinline__ Embed8(const float* win, const float* bin, int sub) {
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const float4* r = reinterpret_cast<const float4*>(win + (8 * sub + q) * FV);
+      const float4 w0 = r[0], w1 = r[1];
+      w[q][0] = w0.x, w[q][1] = w0.y, w[q][2] = w0.z, w[q][3] = w0.w;
+      w[q][4] = w1.x, w[q][5] = w1.y, w[q][6] = w1.z, w[q][7] = w1.w;
+      b[q] = bin[8 * sub + q];
     }
-    EdgeF E = ed[s.z];
-    float lr = E.l / lbar;
-    ls += lr;
-    l2 += lr * lr;
-    ths += E.th;
-    th2 += E.th * E.th;
   }
-  float inv_d = d > 0 ? 1.0f / d : 0.0f;
-  float x[FV];
-  float rl = rho[i] * lbar;
-  x[0] = (A / 3.0f) / abar - 1.0f;
-  x[1] = rl;
-  x[2] = rl * rl;
-  x[3] = (d - 6) * (1.0f / 6.0f);
-  x[4] = ths * inv_d;
-  x[5] = sqrtf(th2 * inv_d);
-  x[6] = ls * inv_d - 1.0f;
-  x[7] = sqrtf(fmaxf(l2 * inv_d - (ls * inv_d) * (ls * inv_d), 0.0f));
-  for (int k = 0; k < FV; ++k) u[(size_t)FV * i + k] = x[k];
-  float nn = fnorm(N);
-  float in = nn > 0.f ? 1.0f / nn : 0.0f;
-  nrm[4 * (size_t)i] = N.x * in;
-  nrm[4 * (size_t)i + 1] = N.y * in;
-  nrm[4 * (size_t)i + 2] = N.z * in;
-  nrm[4 * (size_t)i + 3] = 0.f;
-  __nv_bfloat162* h2 = reinterpret_cast<__nv_bfloat162*>(h + (size_t)H * i);
-  for (int c = 0; c < H; c += 2) {
-    float y0 = W->bin[c], y1 = W->bin[c + 1];
-    for (int k = 0; k < FV; ++k) {
-      y0 += W->win[c * FV + k] * x[k];
-      y1 += W->win[(c + 1) * FV + k] * x[k];
+  __device__ __forceinline__ void operator()(const float* x, float* y) const {
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      y[q] = b[q];
+#pragma unroll
+      for (int k = 0; k < FV; ++k) y[q] += w[q][k] * x[k];
     }
-    h2[c / 2] = __floats2bfloat162_rn(silu(y0), silu(y1));
+  }
+};
+
+// vertex features and normal (one thread per vertex), then the embedding of
+// the block's vertices by eight threads each, with the weights in registers
+// and whole rows of h per store (one thread per vertex with 32 four-byte
+// stores took 53 us at 163,842 vertices, now 35)
+constexpr int SFB = 128;
+__global__ void __launch_bounds__(SFB) k_sfeat(Topo t, const FaceF* __restrict__ fd, const EdgeF* __restrict__ ed,
+                                               const float* __restrict__ rho, const SurW* __restrict__ W,
+                                               float* __restrict__ u, float* __restrict__ nrm,
+                                               __nv_bfloat16* __restrict__ h) {
+  __shared__ float sx[SFB][FV + 1];
+  const int i = blockIdx.x * SFB + threadIdx.x;
+  if (i < t.nv) {
+    const float lbar = W->lbar, abar = W->abar;
+    const int d = t.val[i];
+    float A = 0.f, ls = 0.f, l2 = 0.f, ths = 0.f, th2 = 0.f;
+    f3 N = {0.f, 0.f, 0.f};
+    int4 s = d > 0 ? t.slot[i] : make_int4(0, -1, 0, 0);
+    for (int m = 0; m < d; ++m) {
+      const int4 sn = m + 1 < d ? t.slot[(size_t)(m + 1) * t.nv + i] : s;
+      const int f = slot_face(s.y);
+      if (f >= 0) {
+        FaceF F = fd[f];
+        A += F.A;
+        N += F.A * f3{F.nx, F.ny, F.nz};
+      }
+      EdgeF E = ed[s.z];
+      float lr = E.l / lbar;
+      ls += lr;
+      l2 += lr * lr;
+      ths += E.th;
+      th2 += E.th * E.th;
+      s = sn;
+    }
+    float inv_d = d > 0 ? 1.0f / d : 0.0f;
+    float* x = sx[threadIdx.x];
+    float rl = rho[i] * lbar;
+    x[0] = (A / 3.0f) / abar - 1.0f;
+    x[1] = rl;
+    x[2] = rl * rl;
+    x[3] = (d - 6) * (1.0f / 6.0f);
+    x[4] = ths * inv_d;
+    x[5] = sqrtf(th2 * inv_d);
+    x[6] = ls * inv_d - 1.0f;
+    x[7] = sqrtf(fmaxf(l2 * inv_d - (ls * inv_d) * (ls * inv_d), 0.0f));
+    float nn = fnorm(N);
+    float in = nn > 0.f ? 1.0f / nn : 0.0f;
+    reinterpret_cast<float4*>(nrm)[i] = make_float4(N.x * in, N.y * in, N.z * in, 0.f);
+  }
+  __syncthreads();
+  const int v0 = blockIdx.x * SFB, n = min(SFB, t.nv - v0);
+  if (u)
+    for (int q = threadIdx.x; q < n * FV; q += SFB) u[(size_t)FV * v0 + q] = sx[q / FV][q % FV];
+  const int sub = threadIdx.x & 7;
+  const Embed8 emb(W->win, W->bin, sub);
+  for (int v = threadIdx.x >> 3; v < n; v += SFB / 8) {
+    float y[8];
+    emb(sx[v], y);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) y[q] = silu(y[q]);
+    reinterpret_cast<uint4*>(h)[(size_t)(v0 + v) * (H / 8) + sub] = pack8(y);
   }
 }
 
@@ -166,58 +207,6 @@ __device__ __forceinline__ void unpack8(uint4 v, float* f) {
     f[2 * q + 1] = x.y;
   }
 }
-__device__ __forceinline__ uint4 pack8(const float* f) {
-  uint4 v;
-  __nv_bfloat162* b = reinterpret_cast<__nv_bfloat162*>(&v);
-#pragma unroll
-  for (int q = 0; q < 4; ++q) b[q] = __floats2bfloat162_rn(f[2 * q], f[2 * q + 1]);
-  return v;
-}
-
-// m_i = sum_j (W_e e_ij + b_e) * h_j: sixteen threads per vertex, four
-// channels (8 bytes of h_j) per thread; the next ring slot is loaded while
-// the current neighbour is summed
-__global__ void __launch_bounds__(256) k_agg(Topo t, const EdgeF* __restrict__ ed, const float* __restrict__ rho,
-                                             const SurW* __restrict__ W, int r, const __nv_bfloat16* __restrict__ h,
-                                             __nv_bfloat16* __restrict__ mout) {
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  const int i = g >> 4, sub = g & 15;
-  if (i >= t.nv) return;
-  float4 w[4];
-  float b[4];
-#pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    const int ch = 4 * sub + c;
-    w[c] = *reinterpret_cast<const float4*>(&W->we[r][ch * FE]);
-    b[c] = W->be[r][ch];
-  }
-  const float lbar = W->lbar, ri = rho[i];
-  const uint2* h2 = reinterpret_cast<const uint2*>(h);
-  float acc[4] = {0.f, 0.f, 0.f, 0.f};
-  const int d = t.val[i];
-  int4 s = d > 0 ? t.slot[i] : make_int4(0, 0, 0, 0);
-  for (int m = 0; m < d; ++m) {
-    const int4 sn = m + 1 < d ? t.slot[(size_t)(m + 1) * t.nv + i] : s;
-    const int j = s.x;
-    const uint2 hv = h2[(size_t)j * (H / 4) + sub];
-    float ef[FE];
-    edge_feat(ed[s.z], ri, rho[j], lbar, ef);
-    const float2 h01 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&hv.x));
-    const float2 h23 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&hv.y));
-    const float hj[4] = {h01.x, h01.y, h23.x, h23.y};
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      float gt = b[c] + w[c].x * ef[0] + w[c].y * ef[1] + w[c].z * ef[2] + w[c].w * ef[3];
-      acc[c] += gt * hj[c];
-    }
-    s = sn;
-  }
-  uint2 o;
-  *reinterpret_cast<__nv_bfloat162*>(&o.x) = __floats2bfloat162_rn(acc[0], acc[1]);
-  *reinterpret_cast<__nv_bfloat162*>(&o.y) = __floats2bfloat162_rn(acc[2], acc[3]);
-  reinterpret_cast<uint2*>(mout)[(size_t)i * (H / 4) + sub] = o;
-}
-
 // h_out = h + SiLU([h | m] W^T + b) for 128 vertices per CTA on the tensor cores
 constexpr int DENSE_SMEM = 1024 + 49152 + 64;
 
@@ -230,8 +219,7 @@ constexpr int WAIT_POLLS = 1 << 22;
 __global__ void __launch_bounds__(128) k_dense(const __grid_constant__ CUtensorMap mh,
                                                const __grid_constant__ CUtensorMap mm,
                                                const __grid_constant__ CUtensorMap mw, const float* __restrict__ bias,
-                                               __nv_bfloat16* __restrict__ out, int M, int* status, int wait_polls,
-                                               float* __restrict__ zout) {
+                                               __nv_bfloat16* __restrict__ out, int M, int* status, int wait_polls) {
   using namespace tmg::tc;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -302,20 +290,12 @@ __global__ void __launch_bounds__(128) k_dense(const __grid_constant__ CUtensorM
         const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&hv);
         uint4 ov;
         __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&ov);
-        float zv[8];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
           const int n = c * 8 + 2 * q;
           float2 hf = __bfloat1622float2(h2[q]);
           const float z0 = acc[n] + bias[n], z1 = acc[n + 1] + bias[n + 1];
           o2[q] = __floats2bfloat162_rn(hf.x + silu(z0), hf.y + silu(z1));
-          zv[2 * q] = z0;
-          zv[2 * q + 1] = z1;
-        }
-        if (zout) {
-          float4* z4 = reinterpret_cast<float4*>(zout + (size_t)(m0 + r) * H + c * 8);
-          z4[0] = make_float4(zv[0], zv[1], zv[2], zv[3]);
-          z4[1] = make_float4(zv[4], zv[5], zv[6], zv[7]);
         }
         *reinterpret_cast<uint4*>(out + (size_t)(m0 + r) * H + c * 8) = ov;
       }
@@ -331,18 +311,235 @@ __global__ void __launch_bounds__(128) k_dense(const __grid_constant__ CUtensorM
   if (warp == 0) tmem_dealloc(tmem, 64);
 }
 
+// One round for 128 vertices per CTA: m_i = sum_j (W_e e_ij + b_e) * h_j into
+// the second operand tile, then h_out = h + SiLU([h | m] W^T + b) as in
+// k_dense.  What bounds it is the gather of h_j (six rows of 128 bytes per
+// vertex, from L2): eight threads share a vertex with eight channels (16
+// bytes) each, lane k of the eight loads ring slot k (index and edge features
+// once per slot, the next vertex's while the current one is summed) and hands
+// them around, and four gathers are in flight per thread.  The message weights
+// stay in registers over a thread's four vertices.  Separate kernels with 16
+// threads per vertex, every one of them loading every slot's features, took
+// 70 + 29 us a round at 163,842 vertices, this one 64; three CTAs per SM (80
+// registers, 50 bytes spilled) beat two (112) by 13 us a round.
+struct LayerIn {
+  // inference: rings and edge records of the mesh
+  Topo t;
+  const EdgeF* ed;
+  const float* rho;
+  float lbar;
+  // training: exported rings [D][n]
+  const int* nbr;
+  const float4* ef;
+  int D;
+  const float *we, *be, *bias;  // W_e (64 x 4), b_e, dense bias
+  const uint4* h;               // activations in, 8 x 16 bytes per vertex
+  float* z;                     // training: pre-activations out
+  int M;
+  int* status;
+};
+struct RingSlot {
+  int j, edge, lim;  // neighbour (-1: none), its edge, ring slots of the vertex
+};
+constexpr int LT = 256;
+constexpr int LAYER_SMEM = DENSE_SMEM;
+template <bool TRAIN>
+__device__ __forceinline__ RingSlot ring_slot(const LayerIn& q, int i, int m) {
+  if (TRAIN) return {i < q.M && m < q.D ? q.nbr[(size_t)m * q.M + i] : -1, 0, q.D};
+  if (i >= q.M || m >= TM_MAXVAL) return {-1, 0, 0};
+  const int d = q.t.val[i];
+  const int4 s = q.t.slot[(size_t)m * q.M + i];
+  return {m < d ? s.x : -1, s.z, d};
+}
+// e_ij of slot m
+template <bool TRAIN>
+__device__ __forceinline__ float4 ring_feat(const LayerIn& q, const RingSlot& r, int i, int m) {
+  if (r.j < 0) return make_float4(0.f, 0.f, 0.f, 0.f);
+  if (TRAIN) return q.ef[(size_t)m * q.M + i];
+  float e[FE];
+  edge_feat(q.ed[r.edge], q.rho[i], q.rho[r.j], q.lbar, e);
+  return make_float4(e[0], e[1], e[2], e[3]);
+}
+
+template <bool TRAIN>
+__global__ void __launch_bounds__(LT, 3) k_layer(const __grid_constant__ CUtensorMap mh,
+                                                 const __grid_constant__ CUtensorMap mw,
+                                                 const __grid_constant__ CUtensorMap mout,
+                                                 const __grid_constant__ CUtensorMap mm,
+                                                 const __grid_constant__ LayerIn q) {
+  using namespace tmg::tc;
+  constexpr unsigned FULL = 0xffffffffu;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* A0 = base;           // h tile, 128 rows x 128 B; later the result
+  uint8_t* A1 = base + 16384;   // m tile
+  uint8_t* B0 = base + 32768;   // W[:, 0:64], 64 rows x 128 B
+  uint8_t* B1 = base + 40960;   // W[:, 64:128]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(base + 49152);
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(base + 49152 + 16);
+  int* issued = reinterpret_cast<int*>(base + 49152 + 20);  // the MMA was issued
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int m0 = blockIdx.x * BM;
+  if (threadIdx.x == 0) {
+    mbar_init(&bars[0], 1);
+    mbar_init(&bars[1], 1);
+    mbar_fence_init();
+    *issued = 0;
+    mbar_expect_tx(&bars[0], 32768);
+    tma_load_2d(A0, &mh, &bars[0], 0, m0);
+    tma_load_2d(B0, &mw, &bars[0], 0, 0);
+    tma_load_2d(B1, &mw, &bars[0], 64, 0);
+  }
+  if (warp == 0) {
+    __syncwarp();
+    tmem_alloc(tslot, 64);
+    tmem_relinquish();
+  }
+  // messages: rows 32 it + (thread >> 3), it < 4
+  {
+    const int sub = threadIdx.x & 7, grp = threadIdx.x >> 3;
+    float4 w[8];
+    float b[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      w[c] = *reinterpret_cast<const float4*>(q.we + (8 * sub + c) * FE);
+      b[c] = q.be[8 * sub + c];
+    }
+    RingSlot r = ring_slot<TRAIN>(q, m0 + grp, sub);
+    float4 e = ring_feat<TRAIN>(q, r, m0 + grp, sub);
+    for (int it = 0; it < 4; ++it) {
+      const int row = 32 * it + grp, i = m0 + row;
+      RingSlot rn = {-1, 0, 0};
+      if (it < 3) rn = ring_slot<TRAIN>(q, i + 32, sub);
+      float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      for (int m = 0;;) {  // eight slots at a time; the ring ends at the first absent one
+        const unsigned have = (__ballot_sync(FULL, r.j >= 0) >> (lane & 24)) & 0xffu;
+        const int cnt = have == 0xffu ? 8 : __ffs(~have) - 1;
+        const int most = __reduce_max_sync(FULL, cnt);
+#pragma unroll
+        for (int k0 = 0; k0 < 8; k0 += 4) {
+          if (k0 >= most) break;
+          uint4 hv[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const int j = __shfl_sync(FULL, r.j, k0 + k, 8);
+            hv[k] = make_uint4(0u, 0u, 0u, 0u);
+            if (k0 + k < cnt) hv[k] = q.h[(size_t)j * (H / 8) + sub];
+          }
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const float4 f = make_float4(__shfl_sync(FULL, e.x, k0 + k, 8), __shfl_sync(FULL, e.y, k0 + k, 8),
+                                         __shfl_sync(FULL, e.z, k0 + k, 8), __shfl_sync(FULL, e.w, k0 + k, 8));
+            float hj[8];
+            unpack8(hv[k], hj);
+            if (k0 + k < cnt) {
+#pragma unroll
+              for (int c = 0; c < 8; ++c)
+                acc[c] += (b[c] + w[c].x * f.x + w[c].y * f.y + w[c].z * f.z + w[c].w * f.w) * hj[c];
+            }
+          }
+        }
+        m += 8;
+        const bool more = cnt == 8 && m < r.lim;
+        if (!__any_sync(FULL, more)) break;
+        r.j = -1;
+        if (more) r = ring_slot<TRAIN>(q, i, m + sub);
+        e = ring_feat<TRAIN>(q, r, i, m + sub);
+      }
+      *reinterpret_cast<uint4*>(A1 + (row >> 3) * 1024 + (row & 7) * 128 + ((sub ^ (row & 7)) * 16)) = pack8(acc);
+      r = rn;
+      if (it < 3) e = ring_feat<TRAIN>(q, r, i + 32, sub);
+    }
+  }
+  fence_async_smem();
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tslot;
+  if (threadIdx.x == 0) {
+    if (mbar_wait(&bars[0], 0, WAIT_POLLS)) {
+      constexpr uint32_t idesc = idesc_bf16_f32(BM, H);
+#pragma unroll
+      for (int kc = 0; kc < 2; ++kc) {
+        const uint32_t a = smem_u32(kc ? A1 : A0), b = smem_u32(kc ? B1 : B0);
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          mma_bf16(tmem, sdesc_sw128(a + 32 * k, 1024), sdesc_sw128(b + 32 * k, 1024), idesc, (kc | k) != 0);
+      }
+      mma_commit(&bars[1]);
+      *issued = 1;
+    } else {
+      atomicExch(q.status, 1);  // tile loads did not arrive in time
+      // the copies are still this CTA's: let them land before it exits
+      if (!mbar_wait(&bars[0], 0, WAIT_POLLS)) atomicExch(q.status, 3);
+    }
+  }
+  __syncthreads();
+  const bool done = __syncthreads_and(*issued && mbar_wait(&bars[1], 0, WAIT_POLLS));
+  tc_fence_after();
+  if (done) {
+    // warp w: rows 32 (w & 3) + lane, columns 32 (w >> 2) .. + 31
+    const int r = (warp & 3) * 32 + lane, n0 = (warp >> 2) * 32;
+    float acc[32];
+    tmem_ld32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + n0, acc);
+    uint8_t* rowp = A0 + (r >> 3) * 1024 + (r & 7) * 128;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      uint4* hp = reinterpret_cast<uint4*>(rowp + (((n0 / 8 + c) ^ (r & 7)) * 16));
+      float hf[8], o[8];
+      unpack8(*hp, hf);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const float z = acc[8 * c + k] + q.bias[n0 + 8 * c + k];
+        acc[8 * c + k] = z;
+        o[k] = hf[k] + silu(z);
+      }
+      *hp = pack8(o);
+    }
+    if (TRAIN && m0 + r < q.M) {
+      float4* z4 = reinterpret_cast<float4*>(q.z + (size_t)(m0 + r) * H + n0);
+#pragma unroll
+      for (int c = 0; c < 8; ++c) z4[c] = make_float4(acc[4 * c], acc[4 * c + 1], acc[4 * c + 2], acc[4 * c + 3]);
+    }
+    fence_async_smem();
+  } else if (threadIdx.x == 0) {
+    atomicExch(q.status, 2);  // the MMA completion did not arrive in time
+    // an MMA that was issued still writes the accumulator: wait for it
+    // before the tensor memory is freed
+    if (*issued && !mbar_wait(&bars[1], 0, WAIT_POLLS)) atomicExch(q.status, 3);
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (threadIdx.x == 0 && done) {
+    tma_store_2d(&mout, A0, 0, m0);
+    if (TRAIN) tma_store_2d(&mm, A1, 0, m0);
+    tma_store_wait();
+  }
+  if (warp == 0) {
+    __syncwarp();
+    tmem_dealloc(tmem, 64);
+  }
+}
+
 // output head: g = g_local - s (sum_j c_ij d_ij + c_i N_i), eight threads
-// per vertex with eight channels each; the channel sums are reduced within
-// the eight threads in a fixed order
-__global__ void k_out(Topo t, Split S, const float* __restrict__ nrm, const SurW* __restrict__ W,
-                      const __nv_bfloat16* __restrict__ h, const double* __restrict__ gloc, double* __restrict__ g) {
+// per vertex with eight channels each; lane k of the eight holds ring slot
+// k's neighbour and direction, the eight slots' products are gathered in
+// flight together and reduced so that lane k ends with slot k's sum (7
+// shuffles for eight slots, the same pairs as eight butterflies), and three
+// lanes add the slots in order.  Every lane computing every direction, 24
+// shuffles: 53 us at 163,842 vertices, now 38.
+__global__ void __launch_bounds__(256) k_out(Topo t, Split S, const float* __restrict__ nrm,
+                                             const SurW* __restrict__ W, const __nv_bfloat16* __restrict__ h,
+                                             const double* __restrict__ gloc, double* __restrict__ g) {
+  __shared__ float4 term[256];  // (c_ij / |e|, e) of each slot
+  constexpr unsigned FULL = 0xffffffffu;
   const int gt = blockIdx.x * blockDim.x + threadIdx.x;
   const int i = gt >> 3, sub = gt & 7;
-  if (i >= t.nv) return;
-  const unsigned gmask = 0xffu << (threadIdx.x & 24);  // the eight threads of this vertex
+  const bool act = i < t.nv;
+  const int ii = act ? i : 0, d = act ? t.val[i] : 0;
   const uint4* h4 = reinterpret_cast<const uint4*>(h);
   float hi[8], pi[8];
-  unpack8(h4[(size_t)i * (H / 8) + sub], hi);
+  unpack8(h4[(size_t)ii * (H / 8) + sub], hi);
   float cn = 0.f;
 #pragma unroll
   for (int c = 0; c < 8; ++c) {
@@ -350,30 +547,48 @@ __global__ void k_out(Topo t, Split S, const float* __restrict__ nrm, const SurW
     cn += W->wn[8 * sub + c] * hi[c];
   }
 #pragma unroll
-  for (int o = 1; o < 8; o <<= 1) cn += __shfl_xor_sync(gmask, cn, o);
+  for (int o = 1; o < 8; o <<= 1) cn += __shfl_xor_sync(FULL, cn, o);
   cn += W->bn;
-  f3 F = cn * f3{nrm[4 * (size_t)i], nrm[4 * (size_t)i + 1], nrm[4 * (size_t)i + 2]};
   const float bo = W->bo;
-  const int d = t.val[i];
-  for (int m = 0; m < d; ++m) {
-    const int j = t.nbr[(size_t)m * t.nv + i];
-    float hj[8];
-    unpack8(h4[(size_t)j * (H / 8) + sub], hj);
-    float c = 0.f;
+  float F = cn * nrm[4 * (size_t)ii + (sub < 3 ? sub : 3)];  // lane k < 3: component k
+  const float4* mine = term + (threadIdx.x & ~7);
+  for (int m = 0; __any_sync(FULL, m < d); m += 8) {
+    const int cnt = min(8, d - m);
+    int j = -1;
+    f3 e = {0.f, 0.f, 0.f};
+    if (sub < cnt) {
+      j = t.nbr[(size_t)(m + sub) * t.nv + ii];
+      e = S.diff(j, ii);
+    }
+    float c[8];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) c += pi[q] * hj[q];
+    for (int k = 0; k < 8; ++k) {
+      const int jk = __shfl_sync(FULL, j, k, 8);
+      c[k] = 0.f;
+      if (k < cnt) {
+        float hj[8];
+        unpack8(h4[(size_t)jk * (H / 8) + sub], hj);
 #pragma unroll
-    for (int o = 1; o < 8; o <<= 1) c += __shfl_xor_sync(gmask, c, o);
-    c += bo;
-    f3 e = S.diff(j, i);
-    F += (c / fnorm(e)) * e;
+        for (int q = 0; q < 8; ++q) c[k] += pi[q] * hj[q];
+      }
+    }
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) {  // keep the slots whose bit o is this lane's
+      const bool up = (sub & o) != 0;
+#pragma unroll
+      for (int k = 0; k < 8 / (2 * o); ++k) {
+        const float keep = up ? c[2 * k + 1] : c[2 * k], send = up ? c[2 * k] : c[2 * k + 1];
+        c[k] = keep + __shfl_xor_sync(FULL, send, o);
+      }
+    }
+    const float s = j >= 0 ? (c[0] + bo) / fnorm(e) : 0.f;
+    term[threadIdx.x] = make_float4(e.x, e.y, e.z, s);
+    __syncwarp();
+    if (sub < 3)
+      for (int k = 0; k < cnt; ++k) F += mine[k].w * (sub == 0 ? mine[k].x : (sub == 1 ? mine[k].y : mine[k].z));
+    __syncwarp();
   }
-  if (sub == 0) {
-    const float sc = W->fscale;
-    g[3 * (size_t)i] = gloc[3 * (size_t)i] - (double)(sc * F.x);
-    g[3 * (size_t)i + 1] = gloc[3 * (size_t)i + 1] - (double)(sc * F.y);
-    g[3 * (size_t)i + 2] = gloc[3 * (size_t)i + 2] - (double)(sc * F.z);
-  }
+  if (act && sub < 3) g[3 * (size_t)i + sub] = gloc[3 * (size_t)i + sub] - (double)(W->fscale * F);
 }
 
 // training inputs: ring neighbours, edge features and unit edge directions,
@@ -431,14 +646,25 @@ void make_map(CUtensorMap* map, const void* ptr, uint64_t rows, uint64_t cols, u
 }
 
 void dense_launch(const CUtensorMap& mh, const CUtensorMap& mm, const CUtensorMap& mw, const float* bias,
-                  __nv_bfloat16* out, int M, int* status, cudaStream_t s, int wait_polls = WAIT_POLLS,
-                  float* zout = nullptr) {
+                  __nv_bfloat16* out, int M, int* status, cudaStream_t s, int wait_polls) {
   static bool attr = false;
   if (!attr) {
     TM_CUDA(cudaFuncSetAttribute(k_dense, cudaFuncAttributeMaxDynamicSharedMemorySize, DENSE_SMEM));
     attr = true;
   }
-  if (M > 0) k_dense<<<nblk(M, BM), BM, DENSE_SMEM, s>>>(mh, mm, mw, bias, out, M, status, wait_polls, zout);
+  if (M > 0) k_dense<<<nblk(M, BM), BM, DENSE_SMEM, s>>>(mh, mm, mw, bias, out, M, status, wait_polls);
+  TM_LAUNCH();
+}
+
+template <bool TRAIN>
+void layer_launch(const CUtensorMap& mh, const CUtensorMap& mw, const CUtensorMap& mout, const CUtensorMap& mm,
+                  const LayerIn& in, cudaStream_t s) {
+  static bool attr = false;
+  if (!attr) {
+    TM_CUDA(cudaFuncSetAttribute(k_layer<TRAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, LAYER_SMEM));
+    attr = true;
+  }
+  k_layer<TRAIN><<<nblk(in.M, BM), LT, LAYER_SMEM, s>>>(mh, mw, mout, mm, in);
   TM_LAUNCH();
 }
 
@@ -487,13 +713,22 @@ void surrogate_grad(tm_surrogate* sg, tm_energy* e, tm_mesh* m, const double* P,
   const float* rho = reinterpret_cast<const float*>(e->rho.get());
   Split S{e->pos32.get(), e->poslo.get()};
   SurW* W = sg->w.get();
-  k_sfeat<<<nblk(nv, 128), 128, 0, s>>>(t, fd, ed, rho, W, sg->u.get(), sg->nrm.get(), sg->hb[0].get());
+  k_sfeat<<<nblk(nv, SFB), SFB, 0, s>>>(t, fd, ed, rho, W, nullptr, sg->nrm.get(), sg->hb[0].get());
   TM_LAUNCH();
   int cur = 0;
+  LayerIn in{};
+  in.t = t;
+  in.ed = ed;
+  in.rho = rho;
+  in.lbar = sg->hw.lbar;
+  in.M = nv;
+  in.status = sg->status.get();
   for (int r = 0; r < NR; ++r) {
-    k_agg<<<nblk(16L * nv, 256), 256, 0, s>>>(t, ed, rho, W, r, sg->hb[cur].get(), sg->mb.get());
-    TM_LAUNCH();
-    dense_launch(sg->map_h[cur], sg->map_m, sg->map_w[r], W->b[r], sg->hb[cur ^ 1].get(), nv, sg->status.get(), s);
+    in.we = W->we[r];
+    in.be = W->be[r];
+    in.bias = W->b[r];
+    in.h = reinterpret_cast<const uint4*>(sg->hb[cur].get());
+    layer_launch<false>(sg->map_h[cur], sg->map_w[r], sg->map_h[cur ^ 1], sg->map_h[cur ^ 1], in, s);
     cur ^= 1;
   }
   k_out<<<nblk(8L * nv, 256), 256, 0, s>>>(t, S, sg->nrm.get(), W, sg->hb[cur].get(), sg->gloc.get(), g);
@@ -544,64 +779,24 @@ __device__ __forceinline__ float dsilu(float z) {
 constexpr int TB = 256;  // threads per block of the per-vertex training kernels
 
 // input layer: z = W_in u + b_in, h = bf16(SiLU(z)); 8 threads per vertex,
-// 8 channels each
-__global__ void __launch_bounds__(TB) k_t_embed(int nv, const float* __restrict__ u, const float* __restrict__ th,
-                                                float* __restrict__ z, __nv_bfloat16* __restrict__ h) {
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  const int i = g >> 3, sub = g & 7;
-  if (i >= nv) return;
-  float x[FV];
+// 8 channels each, persistent blocks with the weights in registers (weights
+// loaded per vertex: 23 us at 40,962 vertices, now 12)
+__global__ void __launch_bounds__(TB, 2) k_t_embed(int nv, const float* __restrict__ u, const float* __restrict__ th,
+                                                   float* __restrict__ z, __nv_bfloat16* __restrict__ h) {
+  const int sub = threadIdx.x & 7;
+  const Embed8 emb(th + P_WIN, th + P_BIN, sub);
+  for (int i = (blockIdx.x * TB + threadIdx.x) >> 3; i < nv; i += gridDim.x * (TB / 8)) {
+    float x[FV], y[8], o[8];
 #pragma unroll
-  for (int k = 0; k < FV; ++k) x[k] = u[(size_t)FV * i + k];
-  float y[8], o[8];
+    for (int k = 0; k < FV; ++k) x[k] = u[(size_t)FV * i + k];
+    emb(x, y);
 #pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    const int c = 8 * sub + q;
-    const float4 w0 = *reinterpret_cast<const float4*>(th + P_WIN + c * FV);
-    const float4 w1 = *reinterpret_cast<const float4*>(th + P_WIN + c * FV + 4);
-    const float w[FV] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
-    y[q] = th[P_BIN + c];
-#pragma unroll
-    for (int k = 0; k < FV; ++k) y[q] += w[k] * x[k];
-    o[q] = silu(y[q]);
+    for (int q = 0; q < 8; ++q) o[q] = silu(y[q]);
+    float4* z4 = reinterpret_cast<float4*>(z + (size_t)H * i + 8 * sub);
+    z4[0] = make_float4(y[0], y[1], y[2], y[3]);
+    z4[1] = make_float4(y[4], y[5], y[6], y[7]);
+    reinterpret_cast<uint4*>(h)[(size_t)i * (H / 8) + sub] = pack8(o);
   }
-  float4* z4 = reinterpret_cast<float4*>(z + (size_t)H * i + 8 * sub);
-  z4[0] = make_float4(y[0], y[1], y[2], y[3]);
-  z4[1] = make_float4(y[4], y[5], y[6], y[7]);
-  reinterpret_cast<uint4*>(h)[(size_t)i * (H / 8) + sub] = pack8(o);
-}
-
-// messages m_i = sum_j (W_e e_ij + b_e) * h_j over the exported rings
-// (nbr / ef slot-major [D][n]); 8 threads per vertex, 8 channels (16 bytes of
-// h_j) each: half the index and feature loads of 16 threads with 4 channels.
-// The next neighbour's index is in flight while the current one is summed.
-__global__ void __launch_bounds__(TB) k_t_agg(int nv, int D, const int* __restrict__ nbr, const float* __restrict__ ef,
-                                              const float* __restrict__ th, int r,
-                                              const __nv_bfloat16* __restrict__ h, __nv_bfloat16* __restrict__ mout) {
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  const int i = g >> 3, sub = g & 7;
-  if (i >= nv) return;
-  float4 w[8];
-  float b[8], acc[8];
-#pragma unroll
-  for (int c = 0; c < 8; ++c) {
-    w[c] = *reinterpret_cast<const float4*>(th + p_we(r) + (8 * sub + c) * FE);
-    b[c] = th[p_be(r) + 8 * sub + c];
-    acc[c] = 0.f;
-  }
-  const uint4* h4 = reinterpret_cast<const uint4*>(h);
-  int j = nbr[i];
-  for (int m = 0; j >= 0; ++m) {
-    const size_t o = (size_t)m * nv + i;
-    const int jn = m + 1 < D ? nbr[o + nv] : -1;
-    const float4 e = *reinterpret_cast<const float4*>(ef + FE * o);
-    float hj[8];
-    unpack8(h4[(size_t)j * (H / 8) + sub], hj);
-#pragma unroll
-    for (int c = 0; c < 8; ++c) acc[c] += (b[c] + w[c].x * e.x + w[c].y * e.y + w[c].z * e.z + w[c].w * e.w) * hj[c];
-    j = jn;
-  }
-  reinterpret_cast<uint4*>(mout)[(size_t)i * (H / 8) + sub] = pack8(acc);
 }
 
 // Sum of a per-thread value over the block's threads in thread order,
@@ -1022,7 +1217,8 @@ __global__ void __launch_bounds__(TB, 2) k_t_embed_back(int nv, const float* __r
 // with bias correction) and the dense weights' bf16 copies (what the forward
 // reads) are refreshed from the FP32 master.  One thread a column over all
 // partials, a launch per group, took 718 us of the 1,265 us step at 40,962
-// vertices; with it, persistent blocks and the tiled products the step is 466.
+// vertices; with it, persistent blocks, the tiled products and k_layer the step
+// is 423.
 struct RedGroup {
   const float* part;
   int nb, n, dst, blk0;  // partials, columns (= stride), first parameter, first block
@@ -1094,7 +1290,7 @@ struct tm_strain {
   DevBuf<int> status;
   // persistent blocks of the backward kernels (at most one per tile)
   int nb_dense = 0, nb_msg = 0, nb_out = 0, nb_emb = 0;
-  alignas(64) CUtensorMap map_h[NR];
+  alignas(64) CUtensorMap map_h[NR + 1];
   alignas(64) CUtensorMap map_m[NR];
   alignas(64) CUtensorMap map_w[NR];
 };
@@ -1130,13 +1326,21 @@ void train_pass(tm_strain* st, const TrainInputs& in, float inv_norm, bool want_
   const size_t NH = (size_t)nv * H;
   const float* th = st->th.get();
   const int nb8 = nblk((long)nv * 8, TB);
-  k_t_embed<<<nb8, TB, 0, s>>>(nv, in.u, th, st->z.get(), st->hb.get());
+  k_t_embed<<<st->nb_emb, TB, 0, s>>>(nv, in.u, th, st->z.get(), st->hb.get());
   TM_LAUNCH();
+  LayerIn q{};
+  q.nbr = in.nbr;
+  q.ef = reinterpret_cast<const float4*>(in.ef);
+  q.D = D;
+  q.M = nv;
+  q.status = st->status.get();
   for (int r = 0; r < NR; ++r) {
-    k_t_agg<<<nb8, TB, 0, s>>>(nv, D, in.nbr, in.ef, th, r, st->hb.get() + r * NH, st->mb.get() + r * NH);
-    TM_LAUNCH();
-    dense_launch(st->map_h[r], st->map_m[r], st->map_w[r], th + p_b(r), st->hb.get() + (r + 1) * NH, nv,
-                 st->status.get(), s, WAIT_POLLS, st->z.get() + (r + 1) * NH);
+    q.we = th + p_we(r);
+    q.be = th + p_be(r);
+    q.bias = th + p_b(r);
+    q.h = reinterpret_cast<const uint4*>(st->hb.get() + r * NH);
+    q.z = st->z.get() + (r + 1) * NH;
+    layer_launch<true>(st->map_h[r], st->map_w[r], st->map_h[r + 1], st->map_m[r], q, s);
   }
   k_t_out<<<nb8, TB, 0, s>>>(nv, D, in.nbr, in.dirs, in.nrm, in.tgt, th, st->fscale, inv_norm,
                               st->hb.get() + NR * NH, F, st->dF.get(), st->lossp.get());
@@ -1210,20 +1414,16 @@ int tm_surrogate_create(tm_mesh* m, const float* weights, int64_t n_weights, tm_
   size_t n = std::max(nv, 1);
   sg->w.ensure(1);
   sg->wd.ensure(wd.size());
-  sg->u.ensure(FV * n);
   sg->nrm.ensure(4 * n);
   sg->hb[0].ensure(H * n);
   sg->hb[1].ensure(H * n);
-  sg->mb.ensure(H * n);
   sg->gloc.ensure(3 * n);
   sg->status.ensure(1);
   TM_CUDA(cudaMemcpy(sg->w.get(), &sg->hw, sizeof(SurW), cudaMemcpyHostToDevice));
   TM_CUDA(cudaMemcpy(sg->wd.get(), wd.data(), sizeof(__nv_bfloat16) * wd.size(), cudaMemcpyHostToDevice));
   TM_CUDA(cudaMemset(sg->status.get(), 0, sizeof(int)));
-  if (nv > 0) {
+  if (nv > 0)
     for (int k = 0; k < 2; ++k) make_map(&sg->map_h[k], sg->hb[k].get(), nv, H, BM);
-    make_map(&sg->map_m, sg->mb.get(), nv, H, BM);
-  }
   for (int r = 0; r < NR; ++r) make_map(&sg->map_w[r], sg->wd.get() + (size_t)r * H * 2 * H, H, 2 * H, H);
   *out = sg.release();
   TM_API_END
@@ -1269,7 +1469,7 @@ int tm_surrogate_inputs_device(tm_surrogate* sg, tm_energy* e, tm_mesh* m, const
   const EdgeF* ed = reinterpret_cast<const EdgeF*>(e->edge.get());
   const float* rho = reinterpret_cast<const float*>(e->rho.get());
   Split S{e->pos32.get(), e->poslo.get()};
-  k_sfeat<<<nblk(nv, 128), 128, 0, s>>>(t, fd, ed, rho, sg->w.get(), d_u, sg->nrm.get(), sg->hb[0].get());
+  k_sfeat<<<nblk(nv, SFB), SFB, 0, s>>>(t, fd, ed, rho, sg->w.get(), d_u, sg->nrm.get(), sg->hb[0].get());
   TM_LAUNCH();
   TM_CUDA(cudaMemcpyAsync(d_normals, sg->nrm.get(), sizeof(float) * 4 * nv, cudaMemcpyDeviceToDevice, s));
   k_export<<<nblk(nv, 128), 128, 0, s>>>(t, S, ed, rho, sg->w.get(), max_valence, d_nbr, d_edge_feat, d_dirs);
@@ -1357,6 +1557,7 @@ int tm_surrogate_train_create(int64_t n_vertices, int32_t max_valence, const flo
     make_map(&st->map_m[r], st->mb.get() + r * NH, nv, H, BM);
     make_map(&st->map_w[r], st->wd.get() + (size_t)r * H * 2 * H, H, 2 * H, H);
   }
+  make_map(&st->map_h[NR], st->hb.get() + NR * NH, nv, H, BM);
   *out = st.release();
   TM_API_END
 }

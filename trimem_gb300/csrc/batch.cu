@@ -14,12 +14,12 @@
 // and replayed.
 //
 // Replicas fall into size classes (runs of consecutive replicas whose
-// vertex counts share a power of two).  The element kernels (position
-// split, faces, edges, gradient) run per class, side by side on the
-// classes' streams inside the captured step, each with the block size the
-// autotuner picked for that class when the batch was created; the
-// repulsion and the vertex stage (with the per-replica reductions) run once
-// for all replicas.  Each replica keeps its own exclusion level; the
+// vertex counts share a power of two).  The element kernels (faces, edges,
+// gradient) run per class, side by side on the classes' streams inside the
+// captured step, each with the block size the autotuner picked for that class
+// when the batch was created; the position split (with the velocity-Verlet
+// update), the repulsion (beside the faces and edges) and the vertex stage
+// (with the per-replica reductions) run once for all replicas.  Each replica keeps its own exclusion level; the
 // replicas share the kind of neighbour list (cells, or Verlet rows built
 // from the replica-tagged cells at each replica's cut-off).
 #include <algorithm>
@@ -70,7 +70,7 @@ struct tm_batch {
   // element ranges and tuned block sizes, and their side streams
   std::vector<BatchClass> cls;
   BatchStreams bs{};
-  bool have_side = false;
+  bool have_side = false;  // streams and events exist
   cudaStream_t stream = nullptr;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t gexec = nullptr;
@@ -90,8 +90,10 @@ struct tm_batch {
         cudaStreamDestroy(bs.cs[c]);
         cudaEventDestroy(bs.join[c]);
       }
+      cudaStreamDestroy(bs.rep);
       cudaEventDestroy(bs.fork[0]);
       cudaEventDestroy(bs.fork[1]);
+      cudaEventDestroy(bs.join_rep);
     }
     if (stream) cudaStreamDestroy(stream);
   }
@@ -129,24 +131,9 @@ __global__ void k_copy_b(int n, const double* a, double* b) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) b[i] = a[i];
 }
-// im = 1/m (no FP64 division per element)
-__global__ void k_drift_b(int n3, double dt, double im, const double* p, const double* g, double* x) {
+__global__ void k_kick_b(int n3, double hdt, const double* g0, const double* g1, double* p) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n3) x[i] = x[i] + (p[i] * dt + 0.5 * (-g[i]) * (dt * dt)) * im;
-}
-__global__ void k_kick_b(int n3, double dt, const double* g0, const double* g1, double* p) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n3) p[i] = p[i] + 0.5 * ((-g0[i]) + (-g1[i])) * dt;
-}
-// a kick and the following drift in one pass (same arithmetic)
-__global__ void k_kick_drift_b(int n3, double dt, double im, const double* g0, const double* g1, double* p,
-                               double* x) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n3) {
-    const double pn = p[i] + 0.5 * ((-g0[i]) + (-g1[i])) * dt;
-    p[i] = pn;
-    x[i] = x[i] + (pn * dt + 0.5 * (-g1[i]) * (dt * dt)) * im;
-  }
+  if (i < n3) p[i] = p[i] + ((-g0[i]) + (-g1[i])) * hdt;
 }
 // p.p per 256-vertex block (blocks never straddle replicas)
 __global__ void k_kin_blocks(int nv, const double* p, double* part) {
@@ -163,14 +150,19 @@ __global__ void k_kin_blocks(int nv, const double* p, double* part) {
   }
   if (threadIdx.x == 0) part[blockIdx.x] = s[0];
 }
-// per replica: energy from its Globals and p.p from its blocks, in order
+// per replica (one warp): energy from its Globals and p.p from its blocks,
+// every 32nd per lane in order, then a fixed shuffle tree
 __global__ void k_collect(int R, const int2* rblocks, const double* part, const Globals* gs, double* sc, int slot) {
-  int r = blockIdx.x * blockDim.x + threadIdx.x;
+  const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (r >= R) return;
   double k = 0.0;
-  for (int b = rblocks[r].x; b < rblocks[r].y; ++b) k += part[b];
-  sc[4 * r + slot] = gs[r].comps[6];
-  sc[4 * r + slot + 1] = k;
+  for (int b = rblocks[r].x + lane; b < rblocks[r].y; b += 32) k += part[b];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) k += __shfl_down_sync(0xffffffffu, k, o);
+  if (lane == 0) {
+    sc[4 * r + slot] = gs[r].comps[6];
+    sc[4 * r + slot + 1] = k;
+  }
 }
 // Metropolis per replica (src/trimem/mc/hmc.py:147-155)
 __global__ void k_accept_b(int R, unsigned long long seed, unsigned long long* counter, double m, double T,
@@ -200,9 +192,9 @@ __global__ void k_tick(unsigned long long* counter) {
 
 }  // namespace
 
-static void batch_eval(tm_batch* b, const double* x, double* g, cudaStream_t s) {
+static void batch_eval(tm_batch* b, const double* x, double* g, const Leap* leap, cudaStream_t s) {
   energy_eval_batch32(b->en.get(), b->mesh.get(), x, g, b->eps.get(), b->vrep.get(), b->rblocks.get(), b->gs.get(),
-                      b->cls.data(), (int)b->cls.size(), b->have_side ? &b->bs : nullptr, s);
+                      b->cls.data(), (int)b->cls.size(), b->bs, leap, s);
 }
 
 static void batch_hmc_step(tm_batch* b, int L, double dt, double m, double T, unsigned long long seed,
@@ -214,19 +206,18 @@ static void batch_hmc_step(tm_batch* b, int L, double dt, double m, double T, un
   k_kin_blocks<<<nb, B, 0, s>>>(b->nv, b->p.get(), b->part.get());
   double* g0 = b->g0.get();
   double* g1 = b->g1.get();
-  batch_eval(b, b->x.get(), g0, s);
-  k_collect<<<nblk(b->R, 64), 64, 0, s>>>(b->R, b->rblocks.get(), b->part.get(), b->gs.get(), b->sc.get(), 0);
-  if (L > 0) k_drift_b<<<nblk(n3, B), B, 0, s>>>(n3, dt, 1.0 / m, b->p.get(), g0, b->x.get());
+  batch_eval(b, b->x.get(), g0, nullptr, s);
+  k_collect<<<nblk(32L * b->R, 64), 64, 0, s>>>(b->R, b->rblocks.get(), b->part.get(), b->gs.get(), b->sc.get(), 0);
   for (int i = 0; i < L; ++i) {
-    batch_eval(b, b->x.get(), g1, s);
-    if (i + 1 < L)
-      k_kick_drift_b<<<nblk(n3, B), B, 0, s>>>(n3, dt, 1.0 / m, g0, g1, b->p.get(), b->x.get());
-    else
-      k_kick_b<<<nblk(n3, B), B, 0, s>>>(n3, dt, g0, g1, b->p.get());
-    std::swap(g0, g1);
+    // drift with the first force, then kick with the last two and drift; the
+    // new force replaces the older one
+    const Leap leap{b->x.get(), b->p.get(), g0, i ? g1 : nullptr, dt, 1.0 / m};
+    batch_eval(b, b->x.get(), i ? g0 : g1, &leap, s);
+    if (i) std::swap(g0, g1);
   }
+  if (L > 0) k_kick_b<<<nblk(n3, B), B, 0, s>>>(n3, 0.5 * dt, g0, g1, b->p.get());
   k_kin_blocks<<<nb, B, 0, s>>>(b->nv, b->p.get(), b->part.get());
-  k_collect<<<nblk(b->R, 64), 64, 0, s>>>(b->R, b->rblocks.get(), b->part.get(), b->gs.get(), b->sc.get(), 2);
+  k_collect<<<nblk(32L * b->R, 64), 64, 0, s>>>(b->R, b->rblocks.get(), b->part.get(), b->gs.get(), b->sc.get(), 2);
   k_accept_b<<<nblk(b->R, 64), 64, 0, s>>>(b->R, seed, b->counter.get(), m, T, b->sc.get(), b->flag.get(),
                                            b->acc.get());
   k_finish_b<<<nblk(n3, B), B, 0, s>>>(n3, b->vrep.get(), b->flag.get(), b->x.get(), b->xs.get());
@@ -319,19 +310,21 @@ static void make_classes(tm_batch* b) {
   for (BatchClass& c : cls)
     for (int k = 0; k < 4; ++k) c.blk[k] = 256;
   b->cls = cls;
-  if (cls.size() > 1) {
+  {
     for (size_t c = 0; c < cls.size(); ++c) {
       TM_CUDA(cudaStreamCreateWithFlags(&b->bs.cs[c], cudaStreamNonBlocking));
       TM_CUDA(cudaEventCreateWithFlags(&b->bs.join[c], cudaEventDisableTiming));
     }
+    TM_CUDA(cudaStreamCreateWithFlags(&b->bs.rep, cudaStreamNonBlocking));
     TM_CUDA(cudaEventCreateWithFlags(&b->bs.fork[0], cudaEventDisableTiming));
     TM_CUDA(cudaEventCreateWithFlags(&b->bs.fork[1], cudaEventDisableTiming));
+    TM_CUDA(cudaEventCreateWithFlags(&b->bs.join_rep, cudaEventDisableTiming));
     b->have_side = true;
   }
 }
 
-// The autotuner: for every size class and element kernel (split, face,
-// edge, gradient), the block size among 64 .. 512 (the gradient kernel is
+// The autotuner: for every size class and element kernel (face, edge,
+// gradient), the block size among 64 .. 512 (the gradient kernel is
 // built for at most 256) with the shortest median of five timed launches
 // of that class's kernel alone, after a full evaluation has filled its
 // inputs.
@@ -341,19 +334,19 @@ static void autotune(tm_batch* b) {
   TM_CUDA(cudaEventCreate(&e0));
   TM_CUDA(cudaEventCreate(&e1));
   cudaStream_t s = b->stream;
-  batch_eval(b, b->x.get(), b->g0.get(), s);
+  batch_eval(b, b->x.get(), b->g0.get(), nullptr, s);
   for (BatchClass& c : b->cls) {
-    for (int k = 0; k < 4; ++k) {
+    for (int k = 1; k < 4; ++k) {
       float best = 1e30f;
       int bestb = 256;
       for (int bsz : cand) {
         if (k == 3 && bsz > 256) continue;
-        batch32_class_kernel(k, c, bsz, b->en.get(), b->mesh.get(), b->x.get(), b->g0.get(), b->eps.get(),
+        batch32_class_kernel(k, c, bsz, b->en.get(), b->mesh.get(), b->g0.get(), b->eps.get(),
                              b->vrep.get(), b->gs.get(), s);  // warm
         std::vector<float> t;
         for (int rep = 0; rep < 5; ++rep) {
           TM_CUDA(cudaEventRecord(e0, s));
-          batch32_class_kernel(k, c, bsz, b->en.get(), b->mesh.get(), b->x.get(), b->g0.get(), b->eps.get(),
+          batch32_class_kernel(k, c, bsz, b->en.get(), b->mesh.get(), b->g0.get(), b->eps.get(),
                                b->vrep.get(), b->gs.get(), s);
           TM_CUDA(cudaEventRecord(e1, s));
           TM_CUDA(cudaEventSynchronize(e1));
@@ -516,7 +509,7 @@ int tm_batch_positions(tm_batch* b, double* host_x, int direction) {
 int tm_batch_energy(tm_batch* b, double* energies, double* grad) {
   TM_API_BEGIN
   if (!b || !energies) fail(TM_ERR_ARG, "NULL argument");
-  batch_eval(b, b->x.get(), b->g0.get(), b->stream);
+  batch_eval(b, b->x.get(), b->g0.get(), nullptr, b->stream);
   std::vector<Globals> g(b->R);
   TM_CUDA(cudaMemcpyAsync(g.data(), b->gs.get(), sizeof(Globals) * b->R, cudaMemcpyDeviceToHost, b->stream));
   if (grad)

@@ -164,9 +164,7 @@ template <bool VPROPS>
 __global__ void __launch_bounds__(VB) k_vertex(Topo t, const double2* __restrict__ fav,
                                               const double2* __restrict__ elt, const double* __restrict__ reppot,
                                               EP ep, double2* __restrict__ rk, double* __restrict__ vprops,
-                                              double* __restrict__ partial, Globals* g) {
-  __shared__ double red[6][VB];
-  __shared__ bool last;
+                                              double* partial, Globals* g) {
   int v = blockIdx.x * VB + threadIdx.x;
   double pr[6] = {0, 0, 0, 0, 0, 0};
   if (v < t.nv) {
@@ -218,38 +216,7 @@ __global__ void __launch_bounds__(VB) k_vertex(Topo t, const double2* __restrict
     if (VPROPS)
       for (int k = 0; k < 6; ++k) vprops[6 * (size_t)v + k] = pr[k];
   }
-  for (int k = 0; k < 6; ++k) red[k][threadIdx.x] = pr[k];
-  __syncthreads();
-  for (int o = VB / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o)
-      for (int k = 0; k < 6; ++k) red[k][threadIdx.x] += red[k][threadIdx.x + o];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    for (int k = 0; k < 6; ++k) partial[8 * (size_t)blockIdx.x + k] = red[k][0];
-    __threadfence();
-    unsigned int tk = atomicAdd(&g->ticket, 1u);
-    last = (tk == gridDim.x - 1);
-  }
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  // last block: fixed-order reduction of the block partials
-  double acc[6] = {0, 0, 0, 0, 0, 0};
-  for (int b = threadIdx.x; b < (int)gridDim.x; b += VB)
-    for (int k = 0; k < 6; ++k) acc[k] += ((volatile double*)partial)[8 * (size_t)b + k];
-  for (int k = 0; k < 6; ++k) red[k][threadIdx.x] = acc[k];
-  __syncthreads();
-  for (int o = VB / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o)
-      for (int k = 0; k < 6; ++k) red[k][threadIdx.x] += red[k][threadIdx.x + o];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    for (int k = 0; k < 6; ++k) g->props[k] = red[k][0];
-    assemble(ep, g);
-    g->ticket = 0;
-  }
+  finish_props(pr, partial, gridDim.x, blockIdx.x, ep, g);
 }
 
 __global__ void k_assemble_props(EP ep, const double* props6, Globals* g) {
@@ -400,6 +367,12 @@ void energy_eval(tm_energy* e, tm_mesh* m, const double* P, bool want_grad, bool
   energy_eval_marked(e, m, P, want_grad, want_vprops, d_grad, s, nullptr);
   if (d_energy)
     TM_CUDA(cudaMemcpyAsync(d_energy, &e->glob.get()->comps[6], sizeof(double), cudaMemcpyDeviceToDevice, s));
+}
+
+bool energy_eval_moved(tm_energy* e, tm_mesh* m, const Leap& leap, double* d_grad, cudaStream_t s) {
+  if (e->stencil != 2) return false;
+  energy_eval_df(e, m, leap.x, true, d_grad, nullptr, &leap, s, nullptr);
+  return true;
 }
 
 static void eval_fp64_launches(tm_energy* e, tm_mesh* m, const double* P, bool want_grad, bool want_vprops,

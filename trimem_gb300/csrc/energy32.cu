@@ -17,6 +17,7 @@
 #include "tm_energy.cuh"
 #include "tm_internal.h"
 #include "tm_math.cuh"
+#include "tm_dw.cuh"
 #include "tm_fp32.cuh"
 
 namespace tmg {
@@ -25,14 +26,40 @@ namespace {
 
 using namespace fp32;
 
-// elements [i0, i1) of the 3 n coordinates
-__global__ void k_split(int i0, int i1, const double* __restrict__ P, float* __restrict__ hi, float* __restrict__ lo) {
-  int i = i0 + blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= i1) return;
-  double x = P[i];
-  float h = (float)x;
+// Positions as float hi + lo, per coordinate.  MOVE 1: drifts the positions
+// first (with g0), 2: kicks with g0 and g1, then drifts (with g1): the
+// velocity-Verlet update in the pass that reads the positions anyway.  With
+// the products of constants from the host it is five FP64 operations per
+// coordinate on GB300's narrow FP64 pipe (655,360 coordinates: 8 us, where a
+// kick-drift pass of eight operations and a split with conversions took 13 + 4).
+struct SplitMove {
+  double *x, *p;
+  const double *g0, *g1;
+  double dt, hdt, hdt2, im;
+};
+template <int MOVE>
+__global__ void __launch_bounds__(256) k_split(int n, const double* __restrict__ P, SplitMove mv,
+                                               float* __restrict__ hi, float* __restrict__ lo) {
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i >= n) return;
+  double x;
+  if (MOVE) {
+    double p = mv.p[i], f = -mv.g0[i];
+    if (MOVE == 2) {
+      const double f1 = -mv.g1[i];
+      p = p + (f + f1) * mv.hdt;
+      mv.p[i] = p;
+      f = f1;
+    }
+    x = mv.x[i] + (p * mv.dt + f * mv.hdt2) * mv.im;
+    mv.x[i] = x;
+  } else {
+    x = P[i];
+  }
+  float h, l;
+  split_bits(x, &h, &l);
   hi[i] = h;
-  lo[i] = (float)(x - (double)h);
+  lo[i] = l;
 }
 
 // faces [f0, f1)
@@ -56,24 +83,19 @@ __global__ void k_face32(int f0, int f1, Topo t, Split S, FaceF* __restrict__ fd
   fd[f] = F;
 }
 
-__global__ void k_edge32(Topo t, Split S, const FaceF* __restrict__ fd, EdgeF* __restrict__ ed,
-                         float* __restrict__ ebond, EP ep) {
-  int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= t.ne) return;
-  int4 E = t.edge[e];
+__device__ __forceinline__ EdgeF edge32(const int4& E, const Split& S, const FaceF* __restrict__ fd, const EP& ep) {
   f3 ev = S.diff(E.y, E.x);
   float l = fnorm(ev);
   EdgeF o;
-  o.l = l;
+  o.l = -l;
   o.th = 0.0f;
-  o.flag = 0.0f;
   if (E.z >= 0 && E.w >= 0) {
     FaceF F0 = fd[E.z], F1 = fd[E.w];
     f3 n0 = {F0.nx, F0.ny, F0.nz}, n1 = {F1.nx, F1.ny, F1.nz};
     f3 cr = fcross(n0, n1);
     float a = atan2f(fnorm(cr), fdot(n0, n1));
     o.th = fdot(cr, ev) >= 0.0f ? a : -a;
-    o.flag = 1.0f;
+    o.l = l;
   }
   float val = 0.0f, fac = 0.0f;
   if (ep.btype == 0) {
@@ -93,77 +115,68 @@ __global__ void k_edge32(Topo t, Split S, const FaceF* __restrict__ fd, EdgeF* _
     }
   }
   o.db = fac;
-  ed[e] = o;
-  ebond[e] = val;
+  o.bond = val;
+  return o;
+}
+__global__ void k_edge32(Topo t, Split S, const FaceF* __restrict__ fd, EdgeF* __restrict__ ed, EP ep) {
+  int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e < t.ne) ed[e] = edge32(t.edge[e], S, fd, ep);
 }
 
-__global__ void __launch_bounds__(VB) k_vertex32(Topo t, const FaceF* __restrict__ fd, const EdgeF* __restrict__ ed,
-                                                const float* __restrict__ ebond, const double* __restrict__ reppot,
-                                                EP ep, float* __restrict__ rho, double* __restrict__ partial,
-                                                Globals* g) {
-  __shared__ double red[6][VB];
-  __shared__ bool last;
-  int v = blockIdx.x * VB + threadIdx.x;
-  double pr[6] = {0, 0, 0, 0, 0, 0};
-  if (v < t.nv) {
-    int d = t.val[v];
-    float A = 0, V = 0, LT = 0, T = 0;
-    for (int m = 0; m < d; ++m) {
-      int4 s = t.slot[(size_t)m * t.nv + v];
-      int f = slot_face(s.y);
+// The six properties of vertex v from its ring, in slot order; the records
+// of six slots (one group at the usual valence) are loaded before the sums,
+// 32 bytes per slot.
+constexpr int VG32 = 6;
+__device__ __forceinline__ void vertex32(const Topo& t, const FaceF* __restrict__ fd, const EdgeF* __restrict__ ed,
+                                         const double* __restrict__ reppot, const EP& ep, int v,
+                                         float* __restrict__ rho, double* pr) {
+  const int d = t.val[v];
+  float A = 0, V = 0, LT = 0, T = 0;
+  for (int m0 = 0; m0 < d; m0 += VG32) {
+    int4 s[VG32];
+#pragma unroll
+    for (int k = 0; k < VG32; ++k) s[k] = m0 + k < d ? t.slot[(size_t)(m0 + k) * t.nv + v] : make_int4(0, -1, 0, 0);
+    float fa[VG32], fv[VG32];
+    EdgeF E[VG32];
+#pragma unroll
+    for (int k = 0; k < VG32; ++k) {
+      const int f = slot_face(s[k].y);
       if (f < 0) continue;
-      float fa = fd[f].A;
-      A += fa;
-      V += fd[f].V;
-      EdgeF E = ed[s.z];
-      LT += E.l * E.th;
+      fa[k] = fd[f].A;
+      fv[k] = fd[f].V;
+      E[k] = ed[s[k].z];
+    }
+#pragma unroll
+    for (int k = 0; k < VG32; ++k) {
+      if (slot_face(s[k].y) < 0) continue;
+      A += fa[k];
+      V += fv[k];
+      LT += E[k].length() * E[k].th;
       if (ep.btype == 0) {
-        T += ebond[s.z];
+        T += E[k].bond;
       } else {
-        float q = fa / (float)ep.a0 - 1.0f;
+        float q = fa[k] / (float)ep.a0 - 1.0f;
         T += q * q;
       }
     }
-    float a = A / 3, c = 0.25f * LT;
-    pr[0] = a;
-    pr[1] = V / 3;
-    pr[2] = c;
-    pr[3] = 2 * c * c / a;
-    pr[4] = T / (float)ep.tdiv;
-    pr[5] = reppot[v];
-    rho[v] = c / a;
   }
-  for (int k = 0; k < 6; ++k) red[k][threadIdx.x] = pr[k];
-  __syncthreads();
-  for (int o = VB / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o)
-      for (int k = 0; k < 6; ++k) red[k][threadIdx.x] += red[k][threadIdx.x + o];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    for (int k = 0; k < 6; ++k) partial[8 * (size_t)blockIdx.x + k] = red[k][0];
-    __threadfence();
-    unsigned int tk = atomicAdd(&g->ticket, 1u);
-    last = (tk == gridDim.x - 1);
-  }
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  double acc[6] = {0, 0, 0, 0, 0, 0};
-  for (int b = threadIdx.x; b < (int)gridDim.x; b += VB)
-    for (int k = 0; k < 6; ++k) acc[k] += ((volatile double*)partial)[8 * (size_t)b + k];
-  for (int k = 0; k < 6; ++k) red[k][threadIdx.x] = acc[k];
-  __syncthreads();
-  for (int o = VB / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o)
-      for (int k = 0; k < 6; ++k) red[k][threadIdx.x] += red[k][threadIdx.x + o];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    for (int k = 0; k < 6; ++k) g->props[k] = red[k][0];
-    assemble(ep, g);
-    g->ticket = 0;
-  }
+  float a = A / 3, c = 0.25f * LT;
+  pr[0] = a;
+  pr[1] = V / 3;
+  pr[2] = c;
+  pr[3] = 2 * c * c / a;
+  pr[4] = T / (float)ep.tdiv;
+  pr[5] = reppot[v];
+  rho[v] = c / a;
+}
+
+__global__ void __launch_bounds__(VB) k_vertex32(Topo t, const FaceF* __restrict__ fd, const EdgeF* __restrict__ ed,
+                                                const double* __restrict__ reppot, EP ep, float* __restrict__ rho,
+                                                double* partial, Globals* g) {
+  int v = blockIdx.x * VB + threadIdx.x;
+  double pr[6] = {0, 0, 0, 0, 0, 0};
+  if (v < t.nv) vertex32(t, fd, ed, reppot, ep, v, rho, pr);
+  finish_props(pr, partial, gridDim.x, blockIdx.x, ep, g);
 }
 
 __device__ __forceinline__ float cotf_at(const FaceF& F, int c) { return c == 0 ? F.c0 : (c == 1 ? F.c1 : F.c2); }
@@ -219,14 +232,14 @@ __global__ void __launch_bounds__(256) k_grad32(Topo t, Split S, const FaceF* __
         EdgeF E = ed[sc.z];
         float w = hgC + kb * (ri + rj);
         float cl = w * E.th + (ep.btype == 0 ? kt * E.db : 0.0f);
-        acc += (-cl / E.l) * xj;
+        acc += (-cl / E.length()) * xj;
         float cn = carry;
-        if (E.flag != 0.0f) {
+        if (E.interior()) {
           int cin = slot_corner(sn.y);
           cn += w * cj;
           carry_next = w * cotf_at(Fn, cin == 0 ? 2 : cin - 1);
         }
-        if (ed[sc.w].flag != 0.0f) cn -= (hgC + kb * (rj + rk)) * (cj + ck);
+        if (ed[sc.w].interior()) cn -= (hgC + kb * (rj + rk)) * (cj + ck);
         acc += cn * n;
       }
       carry = carry_next;
@@ -251,119 +264,24 @@ __global__ void __launch_bounds__(256) k_grad32(Topo t, Split S, const FaceF* __
 
 // edges [e0, e1)
 __global__ void k_edge32b(int e0, int e1, Topo t, Split S, const FaceF* __restrict__ fd, EdgeF* __restrict__ ed,
-                          float* __restrict__ ebond, const EP* __restrict__ eps, const int* __restrict__ vrep) {
+                          const EP* __restrict__ eps, const int* __restrict__ vrep) {
   int e = e0 + blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= e1) return;
-  int4 E = t.edge[e];
-  const EP& ep = eps[vrep[E.x]];
-  f3 ev = S.diff(E.y, E.x);
-  float l = fnorm(ev);
-  EdgeF o;
-  o.l = l;
-  o.th = 0.0f;
-  o.flag = 0.0f;
-  if (E.z >= 0 && E.w >= 0) {
-    FaceF F0 = fd[E.z], F1 = fd[E.w];
-    f3 n0 = {F0.nx, F0.ny, F0.nz}, n1 = {F1.nx, F1.ny, F1.nz};
-    f3 cr = fcross(n0, n1);
-    float a = atan2f(fnorm(cr), fdot(n0, n1));
-    o.th = fdot(cr, ev) >= 0.0f ? a : -a;
-    o.flag = 1.0f;
-  }
-  float val = 0.0f, fac = 0.0f;
-  if (ep.btype == 0) {
-    int r = ep.r;
-    float lc0 = (float)ep.lc0, lc1 = (float)ep.lc1;
-    if (l > lc0) {
-      val = fipow((float)r, r + 1) * fipow(l - lc0, r);
-      fac = fipow((float)r, r + 2) * fipow(l - lc0, r - 1);
-    } else if (l < lc1) {
-      val = expf(l / (l - lc1)) / fipow(l, r);
-    }
-    if (l < lc1) {
-      float lmc = l - lc1;
-      fac -= lc1 / (lmc * lmc) + r / l;
-      fac /= fipow(l, r);
-      fac *= expf(l / lmc);
-    }
-  }
-  o.db = fac;
-  ed[e] = o;
-  ebond[e] = val;
+  const int4 E = t.edge[e];
+  ed[e] = edge32(E, S, fd, eps[vrep[E.x]]);
 }
 
 __global__ void __launch_bounds__(VB) k_vertex32b(Topo t, const FaceF* __restrict__ fd, const EdgeF* __restrict__ ed,
-                                                 const float* __restrict__ ebond, const double* __restrict__ reppot,
-                                                 const EP* __restrict__ eps, const int* __restrict__ vrep,
-                                                 const int2* __restrict__ rblocks, float* __restrict__ rho,
-                                                 double* __restrict__ partial, Globals* gs) {
-  __shared__ double red[6][VB];
-  __shared__ bool last;
+                                                 const double* __restrict__ reppot, const EP* __restrict__ eps,
+                                                 const int* __restrict__ vrep, const int2* __restrict__ rblocks,
+                                                 float* __restrict__ rho, double* partial, Globals* gs) {
   const int rep = vrep[blockIdx.x * VB];  // blocks never straddle replicas
   const EP& ep = eps[rep];
+  const int2 rb = rblocks[rep];
   int v = blockIdx.x * VB + threadIdx.x;
   double pr[6] = {0, 0, 0, 0, 0, 0};
-  if (v < t.nv && vrep[v] >= 0) {
-    int d = t.val[v];
-    float A = 0, V = 0, LT = 0, T = 0;
-    for (int m = 0; m < d; ++m) {
-      int4 s = t.slot[(size_t)m * t.nv + v];
-      int f = slot_face(s.y);
-      if (f < 0) continue;
-      float fa = fd[f].A;
-      A += fa;
-      V += fd[f].V;
-      EdgeF E = ed[s.z];
-      LT += E.l * E.th;
-      if (ep.btype == 0) {
-        T += ebond[s.z];
-      } else {
-        float q = fa / (float)ep.a0 - 1.0f;
-        T += q * q;
-      }
-    }
-    float a = A / 3, c = 0.25f * LT;
-    pr[0] = a;
-    pr[1] = V / 3;
-    pr[2] = c;
-    pr[3] = 2 * c * c / a;
-    pr[4] = T / (float)ep.tdiv;
-    pr[5] = reppot[v];
-    rho[v] = c / a;
-  }
-  for (int k = 0; k < 6; ++k) red[k][threadIdx.x] = pr[k];
-  __syncthreads();
-  for (int o = VB / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o)
-      for (int k = 0; k < 6; ++k) red[k][threadIdx.x] += red[k][threadIdx.x + o];
-    __syncthreads();
-  }
-  Globals* g = gs + rep;
-  const int2 rb = rblocks[rep];
-  if (threadIdx.x == 0) {
-    for (int k = 0; k < 6; ++k) partial[8 * (size_t)blockIdx.x + k] = red[k][0];
-    __threadfence();
-    unsigned int tk = atomicAdd(&g->ticket, 1u);
-    last = (tk == (unsigned)(rb.y - rb.x - 1));
-  }
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  double acc[6] = {0, 0, 0, 0, 0, 0};
-  for (int b = rb.x + threadIdx.x; b < rb.y; b += VB)
-    for (int k = 0; k < 6; ++k) acc[k] += ((volatile double*)partial)[8 * (size_t)b + k];
-  for (int k = 0; k < 6; ++k) red[k][threadIdx.x] = acc[k];
-  __syncthreads();
-  for (int o = VB / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o)
-      for (int k = 0; k < 6; ++k) red[k][threadIdx.x] += red[k][threadIdx.x + o];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    for (int k = 0; k < 6; ++k) g->props[k] = red[k][0];
-    assemble(ep, g);
-    g->ticket = 0;
-  }
+  if (v < t.nv && vrep[v] >= 0) vertex32(t, fd, ed, reppot, ep, v, rho, pr);
+  finish_props(pr, partial + 8 * (size_t)rb.x, rb.y - rb.x, blockIdx.x - rb.x, ep, gs + rep);
 }
 
 // vertices [v0, v1)
@@ -424,14 +342,14 @@ __global__ void __launch_bounds__(256) k_grad32b(int v0, int v1, Topo t, Split S
         EdgeF E = ed[sc.z];
         float w = hgC + kb * (ri + rj);
         float cl = w * E.th + (ep.btype == 0 ? kt * E.db : 0.0f);
-        acc += (-cl / E.l) * xj;
+        acc += (-cl / E.length()) * xj;
         float cn = carry;
-        if (E.flag != 0.0f) {
+        if (E.interior()) {
           int cin = slot_corner(sn.y);
           cn += w * cj;
           carry_next = w * cotf_at(Fn, cin == 0 ? 2 : cin - 1);
         }
-        if (ed[sc.w].flag != 0.0f) cn -= (hgC + kb * (rj + rk)) * (cj + ck);
+        if (ed[sc.w].interior()) cn -= (hgC + kb * (rj + rk)) * (cj + ck);
         acc += cn * n;
       }
       carry = carry_next;
@@ -466,20 +384,19 @@ void energy_eval32(tm_energy* e, tm_mesh* m, const double* P, bool want_grad, bo
   Split S{e->pos32.get(), lo};
   FaceF* fd = reinterpret_cast<FaceF*>(e->face.get());
   EdgeF* ed = reinterpret_cast<EdgeF*>(e->edge.get());
-  float* eb = reinterpret_cast<float*>(e->ebond.get());
   float* rho = reinterpret_cast<float*>(e->rho.get());
   double* repg = e->repg.get();
   (void)nf;
   (void)ne;
   if (ev) TM_CUDA(cudaEventRecord(ev[0], s));
-  if (m->nv) k_split<<<nblk(3L * m->nv, 256), 256, 0, s>>>(0, 3 * m->nv, P, e->pos32.get(), lo);
+  if (m->nv) k_split<0><<<nblk(3L * m->nv, 256), 256, 0, s>>>(3 * m->nv, P, SplitMove{}, e->pos32.get(), lo);
   TM_LAUNCH();
   const bool conc = ev == nullptr;  // repulsion overlaps the face and edge kernels
   if (conc) fork_repulsion(e, m, P, want_grad, s, true);
   if (t.nf) k_face32<<<nblk(t.nf, 256), 256, 0, s>>>(0, t.nf, t, S, fd);
   TM_LAUNCH();
   if (ev) TM_CUDA(cudaEventRecord(ev[1], s));
-  if (t.ne) k_edge32<<<nblk(t.ne, 256), 256, 0, s>>>(t, S, fd, ed, eb, ep);
+  if (t.ne) k_edge32<<<nblk(t.ne, 256), 256, 0, s>>>(t, S, fd, ed, ep);
   TM_LAUNCH();
   if (ev) TM_CUDA(cudaEventRecord(ev[2], s));
   if (conc)
@@ -489,7 +406,7 @@ void energy_eval32(tm_energy* e, tm_mesh* m, const double* P, bool want_grad, bo
   (void)repg;
   int nb = std::max(1, nblk(t.nv, VB));
   (void)want_vprops;
-  k_vertex32<<<nb, VB, 0, s>>>(t, fd, ed, eb, e->reppot.get(), ep, rho, e->partials.get(), e->glob.get());
+  k_vertex32<<<nb, VB, 0, s>>>(t, fd, ed, e->reppot.get(), ep, rho, e->partials.get(), e->glob.get());
   TM_LAUNCH();
   if (ev) TM_CUDA(cudaEventRecord(ev[3], s));
   if (want_grad && t.nv) k_grad32<<<nblk(t.nv, 256), 256, 0, s>>>(t, S, fd, ed, rho, repg, e->glob.get(), ep, d_grad);
@@ -513,53 +430,50 @@ void energy_eval32_local(tm_energy* e, tm_mesh* m, const double* P, double* d_gr
   Split S{e->pos32.get(), e->poslo.get()};
   FaceF* fd = reinterpret_cast<FaceF*>(e->face.get());
   EdgeF* ed = reinterpret_cast<EdgeF*>(e->edge.get());
-  float* eb = reinterpret_cast<float*>(e->ebond.get());
   float* rho = reinterpret_cast<float*>(e->rho.get());
   TM_CUDA(cudaMemsetAsync(e->reppot.get(), 0, sizeof(double) * nv, s));
   TM_CUDA(cudaMemsetAsync(e->repg.get(), 0, sizeof(double) * 3 * nv, s));
-  if (m->nv) k_split<<<nblk(3L * m->nv, 256), 256, 0, s>>>(0, 3 * m->nv, P, e->pos32.get(), e->poslo.get());
+  if (m->nv) k_split<0><<<nblk(3L * m->nv, 256), 256, 0, s>>>(3 * m->nv, P, SplitMove{}, e->pos32.get(), e->poslo.get());
   TM_LAUNCH();
   if (t.nf) k_face32<<<nblk(t.nf, 256), 256, 0, s>>>(0, t.nf, t, S, fd);
   TM_LAUNCH();
-  if (t.ne) k_edge32<<<nblk(t.ne, 256), 256, 0, s>>>(t, S, fd, ed, eb, ep);
+  if (t.ne) k_edge32<<<nblk(t.ne, 256), 256, 0, s>>>(t, S, fd, ed, ep);
   TM_LAUNCH();
   int nb = std::max(1, nblk(t.nv, VB));
-  k_vertex32<<<nb, VB, 0, s>>>(t, fd, ed, eb, e->reppot.get(), ep, rho, e->partials.get(), e->glob.get());
+  k_vertex32<<<nb, VB, 0, s>>>(t, fd, ed, e->reppot.get(), ep, rho, e->partials.get(), e->glob.get());
   TM_LAUNCH();
   if (t.nv) k_grad32<<<nblk(t.nv, 256), 256, 0, s>>>(t, S, fd, ed, rho, e->repg.get(), e->glob.get(), ep, d_grad);
   TM_LAUNCH();
 }
 
-// One element kernel of one size class of a batch: which 0 split, 1 face,
-// 2 edge, 3 gradient, with block size blk, on stream s.
-void batch32_class_kernel(int which, const BatchClass& c, int blk, tm_energy* e, tm_mesh* m, const double* P,
-                          double* d_grad, const EP* eps, const int* vrep, const Globals* gs, cudaStream_t s) {
+// One element kernel of one size class of a batch: which 1 face, 2 edge, 3
+// gradient, with block size blk, on stream s.
+void batch32_class_kernel(int which, const BatchClass& c, int blk, tm_energy* e, tm_mesh* m, double* d_grad,
+                          const EP* eps, const int* vrep, const Globals* gs, cudaStream_t s) {
   Topo t = m->topo();
   Split S{e->pos32.get(), e->poslo.get()};
   FaceF* fd = reinterpret_cast<FaceF*>(e->face.get());
   EdgeF* ed = reinterpret_cast<EdgeF*>(e->edge.get());
-  float* eb = reinterpret_cast<float*>(e->ebond.get());
   float* rho = reinterpret_cast<float*>(e->rho.get());
-  if (which == 0 && c.v1 > c.v0)
-    k_split<<<nblk(3L * (c.v1 - c.v0), blk), blk, 0, s>>>(3 * c.v0, 3 * c.v1, P, e->pos32.get(), e->poslo.get());
   if (which == 1 && c.f1 > c.f0) k_face32<<<nblk(c.f1 - c.f0, blk), blk, 0, s>>>(c.f0, c.f1, t, S, fd);
   if (which == 2 && c.e1 > c.e0)
-    k_edge32b<<<nblk(c.e1 - c.e0, blk), blk, 0, s>>>(c.e0, c.e1, t, S, fd, ed, eb, eps, vrep);
+    k_edge32b<<<nblk(c.e1 - c.e0, blk), blk, 0, s>>>(c.e0, c.e1, t, S, fd, ed, eps, vrep);
   if (which == 3 && c.v1 > c.v0)
     k_grad32b<<<nblk(c.v1 - c.v0, blk), blk, 0, s>>>(c.v0, c.v1, t, S, fd, ed, rho, e->repg.get(), gs, eps, vrep,
                                                       d_grad);
   TM_LAUNCH();
 }
 
-// The batch's evaluation: per size class (consecutive replicas of similar
-// size, each with its own tuned block sizes) the split, face and edge
-// kernels, then the repulsion and the vertex stage for all replicas, then
-// the gradient per class.  With side streams the classes' kernels run
-// side by side (fork and join events), so the small replicas' launches fill
-// the SMs the large ones leave idle.
+// The batch's evaluation: the positions' split for all replicas (after the
+// velocity-Verlet update of leap, when given), then per size class
+// (consecutive replicas of similar size, each with its own tuned block sizes)
+// the face and edge kernels, the repulsion beside them on a stream of its
+// own, the vertex stage for all replicas, and the gradient per class.  With
+// side streams the classes' kernels run side by side (fork and join events),
+// so the small replicas' launches fill the SMs the large ones leave idle.
 void energy_eval_batch32(tm_energy* e, tm_mesh* m, const double* P, double* d_grad, const EP* eps,
                          const int* vrep, const int2* rblocks, Globals* gs, const BatchClass* cls, int ncls,
-                         const BatchStreams* bs, cudaStream_t s) {
+                         const BatchStreams& bs, const Leap* leap, cudaStream_t s) {
   e->ensure(m->nv, m->ne, m->nf);
   size_t nv = std::max(m->nv, 1);
   Topo t = m->topo();
@@ -567,35 +481,42 @@ void energy_eval_batch32(tm_energy* e, tm_mesh* m, const double* P, double* d_gr
   e->poslo.ensure(3 * nv);
   FaceF* fd = reinterpret_cast<FaceF*>(e->face.get());
   EdgeF* ed = reinterpret_cast<EdgeF*>(e->edge.get());
-  float* eb = reinterpret_cast<float*>(e->ebond.get());
   float* rho = reinterpret_cast<float*>(e->rho.get());
-  const bool side = bs && ncls > 1;
-  auto stream_of = [&](int c) { return side ? bs->cs[c] : s; };
+  const int n3 = 3 * m->nv;
+  SplitMove mv{};
+  if (leap)
+    mv = SplitMove{leap->x, leap->p, leap->g0, leap->g1, leap->dt, 0.5 * leap->dt, 0.5 * (leap->dt * leap->dt), leap->im};
+  auto* ks = !leap ? k_split<0> : (leap->g1 ? k_split<2> : k_split<1>);
+  ks<<<std::max(1, nblk(n3, 256)), 256, 0, s>>>(n3, P, mv, e->pos32.get(), e->poslo.get());
+  TM_LAUNCH();
+  const bool side = ncls > 1;
+  auto stream_of = [&](int c) { return side ? bs.cs[c] : s; };
   auto fork = [&](int k) {
-    if (!side) return;
-    TM_CUDA(cudaEventRecord(bs->fork[k], s));
-    for (int c = 0; c < ncls; ++c) TM_CUDA(cudaStreamWaitEvent(bs->cs[c], bs->fork[k], 0));
+    TM_CUDA(cudaEventRecord(bs.fork[k], s));
+    if (k == 0) TM_CUDA(cudaStreamWaitEvent(bs.rep, bs.fork[k], 0));
+    for (int c = 0; side && c < ncls; ++c) TM_CUDA(cudaStreamWaitEvent(bs.cs[c], bs.fork[k], 0));
   };
   auto join = [&]() {
-    if (!side) return;
-    for (int c = 0; c < ncls; ++c) {
-      TM_CUDA(cudaEventRecord(bs->join[c], bs->cs[c]));
-      TM_CUDA(cudaStreamWaitEvent(s, bs->join[c], 0));
+    for (int c = 0; side && c < ncls; ++c) {
+      TM_CUDA(cudaEventRecord(bs.join[c], bs.cs[c]));
+      TM_CUDA(cudaStreamWaitEvent(s, bs.join[c], 0));
     }
   };
   fork(0);
-  for (int c = 0; c < ncls; ++c)
-    for (int k = 0; k < 3; ++k)
-      batch32_class_kernel(k, cls[c], cls[c].blk[k], e, m, P, d_grad, eps, vrep, gs, stream_of(c));
-  join();
   repulsion_eval(e, m, P, e->pos32.get(), true, e->reppot.get(), e->repg.get(), e->slow.get(),
-                 e->slow.get() + std::max(m->nv, 1), s, eps);
+                 e->slow.get() + std::max(m->nv, 1), bs.rep, eps);
+  TM_CUDA(cudaEventRecord(bs.join_rep, bs.rep));
+  for (int c = 0; c < ncls; ++c)
+    for (int k = 1; k < 3; ++k)
+      batch32_class_kernel(k, cls[c], cls[c].blk[k], e, m, d_grad, eps, vrep, gs, stream_of(c));
+  join();
+  TM_CUDA(cudaStreamWaitEvent(s, bs.join_rep, 0));
   int nb = std::max(1, nblk(t.nv, VB));
-  k_vertex32b<<<nb, VB, 0, s>>>(t, fd, ed, eb, e->reppot.get(), eps, vrep, rblocks, rho, e->partials.get(), gs);
+  k_vertex32b<<<nb, VB, 0, s>>>(t, fd, ed, e->reppot.get(), eps, vrep, rblocks, rho, e->partials.get(), gs);
   TM_LAUNCH();
   fork(1);
   for (int c = 0; c < ncls; ++c)
-    batch32_class_kernel(3, cls[c], cls[c].blk[3], e, m, P, d_grad, eps, vrep, gs, stream_of(c));
+    batch32_class_kernel(3, cls[c], cls[c].blk[3], e, m, d_grad, eps, vrep, gs, stream_of(c));
   join();
 }
 

@@ -87,7 +87,7 @@ struct DwEval {
 struct DwMove {
   double *x, *p;
   const double *g0, *g1;  // g1 NULL: drift only, with g0
-  double dt, im;
+  double dt, hdt, hdt2, im;  // step, dt / 2, dt^2 / 2, 1 / mass
 };
 
 __device__ __forceinline__ df3 pos_of(const float4* X, int v) { return PosDW{X}.at(v); }
@@ -107,11 +107,11 @@ __device__ __forceinline__ bool split_vertex(const DwEval& a, const DwMove& mv, 
       double pn = mv.p[i], f = -mv.g0[i];
       if (mv.g1) {
         const double f1 = -mv.g1[i];
-        pn = pn + 0.5 * (f + f1) * mv.dt;
+        pn = pn + (f + f1) * mv.hdt;
         mv.p[i] = pn;
         f = f1;
       }
-      x[k] = mv.x[i] + (pn * mv.dt + 0.5 * f * (mv.dt * mv.dt)) * mv.im;
+      x[k] = mv.x[i] + (pn * mv.dt + f * mv.hdt2) * mv.im;
       mv.x[i] = x[k];
     } else {
       x[k] = a.P[i];
@@ -559,19 +559,6 @@ __device__ __forceinline__ void block_props(const df* pr, float2 (*wsum)[NW], do
     partial[threadIdx.x] = df_to(s);
   }
 }
-// Property w (warp w < 6) over nb block partials: lane l takes blocks l,
-// l + 32, ... in order, then a fixed shuffle tree
-__device__ __forceinline__ void total_props(const double* partial, int nb, double* redd) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  if (w < 6) {
-    double acc = 0.0;
-    for (int b = lane; b < nb; b += 32) acc += __ldcg(partial + 8 * (size_t)b + w);
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, off);
-    if (lane == 0) redd[w] = acc;
-  }
-}
-
 // ---- stage 5: gradient ---------------------------------------------------------
 // Gradient gather per vertex i over its ring (slot m: face (i, j = r_m,
 // k = r_{m-1})), the reference's gather (src/mesh_properties.cpp:51-148 with
@@ -892,7 +879,8 @@ void energy_eval_df(tm_energy* e, tm_mesh* m, const double* P, bool want_grad, d
   q.energy = d_energy;
   q.grad = want_grad ? d_grad : nullptr;
   DwMove mv{};
-  if (leap) mv = DwMove{leap->x, leap->p, leap->g0, leap->g1, leap->dt, leap->im};
+  if (leap)
+    mv = DwMove{leap->x, leap->p, leap->g0, leap->g1, leap->dt, 0.5 * leap->dt, 0.5 * (leap->dt * leap->dt), leap->im};
   const Topo& t = q.t;
   const int nsb = std::max(1, nblk(t.nv, SB));
   q.nmoved = nsb;

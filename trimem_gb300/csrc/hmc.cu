@@ -58,30 +58,33 @@ __global__ void k_copy(int n, const double* a, double* b) {
 
 // x += (p dt + 0.5 a dt^2) / m with a = -g
 // im = 1/m: an FP64 division per element would dominate the pass (FP64 is
-// GB300's scarce pipe); for the usual m = 1 both forms are exact
-__global__ void k_drift(int n3, double dt, double im, const double* p, const double* g, double* x) {
+// GB300's scarce pipe); for the usual m = 1 both forms are exact.  hdt = dt/2
+// and hdt2 = dt^2/2 likewise come from the host (halving is exact).
+__global__ void k_drift(int n3, double dt, double hdt2, double im, const double* p, const double* g, double* x) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n3) {
     double a = -g[i];
-    x[i] = x[i] + (p[i] * dt + 0.5 * a * (dt * dt)) * im;
+    x[i] = x[i] + (p[i] * dt + a * hdt2) * im;
   }
 }
 // p += 0.5 (a + a') dt
-__global__ void k_kick(int n3, double dt, const double* g0, const double* g1, double* p) {
+__global__ void k_kick(int n3, double hdt, const double* g0, const double* g1, double* p) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n3) p[i] = p[i] + 0.5 * ((-g0[i]) + (-g1[i])) * dt;
+  if (i < n3) p[i] = p[i] + ((-g0[i]) + (-g1[i])) * hdt;
 }
 
 // k_kick followed by the next step's k_drift (the kick's new momentum and
-// the same force), the same arithmetic per element in one pass
-__global__ void k_kick_drift(int n3, double dt, double im, const double* g0, const double* g1, double* p,
-                             double* x) {
+// the same force), the same arithmetic per element in one pass; where the
+// evaluation that follows can do both in its own first pass
+// (energy_eval_moved), it does
+__global__ void k_kick_drift(int n3, double dt, double hdt, double hdt2, double im, const double* g0,
+                             const double* g1, double* p, double* x) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n3) {
-    const double pn = p[i] + 0.5 * ((-g0[i]) + (-g1[i])) * dt;
+    const double pn = p[i] + ((-g0[i]) + (-g1[i])) * hdt;
     p[i] = pn;
     const double a = -g1[i];
-    x[i] = x[i] + (pn * dt + 0.5 * a * (dt * dt)) * im;
+    x[i] = x[i] + (pn * dt + a * hdt2) * im;
   }
 }
 
@@ -184,19 +187,27 @@ static void hmc_step(tm_surrogate* sg, tm_energy* e, tm_mesh* m, double* d_x, do
     force(g0);
     record(sc + 0, props);
   }
-  // velocity Verlet; each kick is fused with the following drift
-  if (n_steps > 0) {
-    k_drift<<<nblk(n3, b), b, 0, s>>>(n3, dt, 1.0 / mass, p, g0, x);
-    TM_LAUNCH();
-  }
+  // velocity Verlet; each kick is fused with the following drift, and both
+  // with the evaluation's first pass where its stencils allow
+  const double hdt = 0.5 * dt, hdt2 = 0.5 * (dt * dt), im = 1.0 / mass;
   for (int i = 0; i < n_steps; ++i) {
-    force(g1);
-    if (i + 1 < n_steps)
-      k_kick_drift<<<nblk(n3, b), b, 0, s>>>(n3, dt, 1.0 / mass, g0, g1, p, x);
-    else
-      k_kick<<<nblk(n3, b), b, 0, s>>>(n3, dt, g0, g1, p);
+    // g0: last force (i = 0), else the one before it with the last in g1;
+    // the new force replaces the older one
+    const Leap leap{x, p, g0, i ? g1 : nullptr, dt, im};
+    double* gnew = i ? g0 : g1;
+    if (sg || !energy_eval_moved(e, m, leap, gnew, s)) {
+      if (i)
+        k_kick_drift<<<nblk(n3, b), b, 0, s>>>(n3, dt, hdt, hdt2, im, g0, g1, p, x);
+      else
+        k_drift<<<nblk(n3, b), b, 0, s>>>(n3, dt, hdt2, im, p, g0, x);
+      TM_LAUNCH();
+      force(gnew);
+    }
+    if (i) std::swap(g0, g1);
+  }
+  if (n_steps > 0) {
+    k_kick<<<nblk(n3, b), b, 0, s>>>(n3, hdt, g0, g1, p);
     TM_LAUNCH();
-    std::swap(g0, g1);
   }
   if (sg) energy_eval(e, m, x, false, false, nullptr, s);
   record(sc + 2, props + 8);

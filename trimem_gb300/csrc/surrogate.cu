@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(SFB) k_sfeat(Topo t, const FaceF* __restrict__
         N += F.A * f3{F.nx, F.ny, F.nz};
       }
       EdgeF E = ed[s.z];
-      float lr = E.l / lbar;
+      float lr = E.length() / lbar;
       ls += lr;
       l2 += lr * lr;
       ths += E.th;
@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(SFB) k_sfeat(Topo t, const FaceF* __restrict__
 }
 
 __device__ __forceinline__ void edge_feat(const EdgeF& E, float ri, float rj, float lbar, float* ef) {
-  ef[0] = E.l / lbar - 1.0f;
+  ef[0] = E.length() / lbar - 1.0f;
   ef[1] = E.th;
   ef[2] = (rj - ri) * lbar;
   ef[3] = 0.5f * (rj + ri) * lbar;

@@ -366,6 +366,70 @@ __device__ __forceinline__ void assemble_warp(const EP& ep, const double* sum6, 
   }
 }
 
+// Sums of the six properties over a block into partial[0..5], in a fixed
+// order.  Warp sums by halving (each step a lane keeps half of its values and
+// adds the partner's): 8 FP64 additions per lane instead of the 30 of six
+// shuffle trees, and two barriers instead of the eight of a tree in shared
+// memory.  The lanes' bits 4..2 select the property they end with; property k
+// is then summed over the warps in warp order by thread k.
+template <int NW>
+__device__ __forceinline__ void block_sums(const double* pr, double (*wsum)[NW], double* partial) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  auto swap_add = [](bool up, double a, double b, int o) {  // keep a (up: b), add the partner's same one
+    const double keep = up ? b : a, send = up ? a : b;
+    return keep + __shfl_xor_sync(0xffffffffu, send, o);
+  };
+  const double q0 = swap_add(lane & 16, pr[0], pr[3], 16), q1 = swap_add(lane & 16, pr[1], pr[4], 16),
+               q2 = swap_add(lane & 16, pr[2], pr[5], 16);
+  const double r0 = swap_add(lane & 8, q0, q2, 8), r1 = q1 + __shfl_xor_sync(0xffffffffu, q1, 8);
+  double r = swap_add(lane & 4, r0, r1, 4);
+#pragma unroll
+  for (int o = 2; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+  // bits 16, 8, 4: property 0 + 3 (bit 4), + 2 (bit 3), or + 1 (bit 2); with
+  // bits 3 and 2 both set the lane holds property 1 or 4 once more
+  const int prop = (lane & 16 ? 3 : 0) + (lane & 4 ? 1 : (lane & 8 ? 2 : 0));
+  if ((lane & 3) == 0 && (lane & 12) != 12) wsum[prop][w] = r;
+  __syncthreads();
+  if (threadIdx.x < 6) {
+    double t = wsum[threadIdx.x][0];
+    for (int k = 1; k < NW; ++k) t += wsum[threadIdx.x][k];
+    partial[threadIdx.x] = t;
+  }
+}
+// Property w (warp w < 6) over nb block partials: lane l takes blocks l,
+// l + 32, ... in order, then a fixed shuffle tree
+__device__ __forceinline__ void total_props(const double* partial, int nb, double* redd) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (w < 6) {
+    double acc = 0.0;
+    for (int b = lane; b < nb; b += 32) acc += __ldcg(partial + 8 * (size_t)b + w);
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, off);
+    if (lane == 0) redd[w] = acc;
+  }
+}
+// The global sums after a vertex stage: block sums, then the last of the nb
+// blocks from partial on (atomic ticket) totals them in block order and
+// assembles energy and penalty factors.  Called by whole blocks of VB.
+__device__ __forceinline__ void finish_props(const double* pr, double* partial0, int nb, int mine, const EP& ep,
+                                             Globals* g) {
+  __shared__ double wsum[6][VB / 32];
+  __shared__ double redd[6];
+  __shared__ bool last;
+  block_sums<VB / 32>(pr, wsum, partial0 + 8 * (size_t)mine);
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(&g->ticket, 1u) == (unsigned)nb - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  total_props(partial0, nb, redd);
+  __syncthreads();
+  if (threadIdx.x < 32) assemble_warp(ep, redd, g);
+}
+
 // Energy of a set of global properties (src/kernel.h:110-122, summation
 // order area, volume, area-difference, tether, repulsion, bending).
 __device__ __forceinline__ double energy_of(const EP& ep, const double* p) {

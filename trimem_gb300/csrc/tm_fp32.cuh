@@ -8,8 +8,12 @@ namespace tmg {
 struct __align__(16) FaceF {
   float nx, ny, nz, A, V, c0, c1, c2;
 };
+// l: length, with the sign bit set on boundary edges (length() and
+// interior()); bond: the bond's value
 struct __align__(16) EdgeF {
-  float l, th, db, flag;
+  float l, th, db, bond;
+  __device__ __forceinline__ float length() const { return fabsf(l); }
+  __device__ __forceinline__ bool interior() const { return __float_as_int(l) >= 0; }
 };
 
 namespace fp32 {

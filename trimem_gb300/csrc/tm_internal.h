@@ -263,10 +263,14 @@ struct tm_energy {
 };
 
 namespace tmg {
+struct Leap;
 // energy.cu
 // (d_energy, when given, receives the energy)
 void energy_eval(tm_energy* e, tm_mesh* m, const double* d_points, bool want_grad, bool want_vprops,
                  double* d_grad, cudaStream_t s, double* d_energy = nullptr);
+// a gradient evaluation at leap->x after leap's update: true when the
+// stencil's evaluation does the update itself (nothing happens when false)
+bool energy_eval_moved(tm_energy* e, tm_mesh* m, const Leap& leap, double* d_grad, cudaStream_t s);
 // same, recording ev[0..4] around the face, edge, vertex and gradient kernels
 void energy_eval_marked(tm_energy* e, tm_mesh* m, const double* d_points, bool want_grad, bool want_vprops,
                         double* d_grad, cudaStream_t s, cudaEvent_t* ev);
@@ -287,22 +291,23 @@ void energy_eval32_local(tm_energy* e, tm_mesh* m, const double* d_points, doubl
 // batch of replicas, FP32 stencils and FP64 sums per replica.  A size class
 // is a run of consecutive replicas of similar size: its vertex, face and
 // edge ranges in the union mesh and the block sizes tuned for it
-// {split, face, edge, gradient}.
+// {split, face, edge, gradient} (the split is one launch for all replicas).
 struct BatchClass {
   int v0, v1, f0, f1, e0, e1;
   int blk[4];
 };
 constexpr int TM_MAX_CLASSES = 8;
-// side streams of the classes and the fork / join events between them
+// side streams of the classes and the repulsion, and the fork / join events
+// between them
 struct BatchStreams {
-  cudaStream_t cs[TM_MAX_CLASSES];
-  cudaEvent_t fork[2], join[TM_MAX_CLASSES];
+  cudaStream_t cs[TM_MAX_CLASSES], rep;
+  cudaEvent_t fork[2], join[TM_MAX_CLASSES], join_rep;
 };
 void energy_eval_batch32(tm_energy* e, tm_mesh* m, const double* d_points, double* d_grad, const EP* eps,
                          const int* vrep, const int2* rblocks, Globals* gs, const BatchClass* cls, int ncls,
-                         const BatchStreams* bs, cudaStream_t s);
-void batch32_class_kernel(int which, const BatchClass& c, int blk, tm_energy* e, tm_mesh* m, const double* P,
-                          double* d_grad, const EP* eps, const int* vrep, const Globals* gs, cudaStream_t s);
+                         const BatchStreams& bs, const Leap* leap, cudaStream_t s);
+void batch32_class_kernel(int which, const BatchClass& c, int blk, tm_energy* e, tm_mesh* m, double* d_grad,
+                          const EP* eps, const int* vrep, const Globals* gs, cudaStream_t s);
 // velocity-Verlet update that precedes an evaluation: kick with g0 and g1
 // (drift only, with g0, when g1 is NULL), drift of x; im = 1 / mass
 struct Leap {

@@ -54,11 +54,10 @@ namespace tmg {
 
 // ---- per-face and per-edge quantities ------------------------------------
 // Sign tests and absolute values as integer operations on the bits (no
-// FP64 compare or absolute value: FP64 is GB300's scarce pipe).  The sign
-// bit of an edge's il is its boundary flag; for non-negative doubles the
-// bit patterns order like the values, so a length l >= 0 is compared with
-// a threshold by its bits (NaN lengths compare as above every threshold).
-__device__ __forceinline__ bool interior_edge(double il) { return __double_as_longlong(il) >= 0; }
+// FP64 compare or absolute value: FP64 is GB300's scarce pipe).  For
+// non-negative doubles the bit patterns order like the values, so a length
+// l >= 0 is compared with a threshold by its bits (NaN lengths compare as
+// above every threshold).
 __device__ __forceinline__ double abs_bits(double x) {
   return __longlong_as_double(__double_as_longlong(x) & 0x7fffffffffffffffLL);
 }
@@ -100,62 +99,63 @@ __global__ void k_face(Topo t, const double* __restrict__ P, FaceD* __restrict__
   fav[f] = make_double2(F.A, F.V);
 }
 
-// elt: (l theta, bond value) of each edge, compact, for k_vertex's gathers
-// (the bond value of short edges is filled in by k_bond_short)
-__global__ void k_edge(Topo t, const double* __restrict__ P, const FaceD* __restrict__ fd, EdgeD* __restrict__ ed,
-                       double2* __restrict__ elt, EP ep, int* __restrict__ blist, int* __restrict__ bcnt,
-                       const double2* __restrict__ sct) {
-  int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= t.ne) return;
-  int4 E = t.edge[e];
-  d3 pi = ld3(P, E.x), pj = ld3(P, E.y);
-  d3 ev = pj - pi;
-  double l2 = dot(ev, ev);
-  double il = rsqrt(l2);
-  double l = l2 * il;
-  EdgeD o;
-  o.l = l;
-  o.th = 0.0;
-  o.il = -il;
-  if (E.z >= 0 && E.w >= 0) {
-    FaceD F0 = fd[E.z], F1 = fd[E.w];
-    d3 n0 = mk(F0.nx, F0.ny, F0.nz), n1 = mk(F1.nx, F1.ny, F1.nz);
-    // both normals are perpendicular to the shared edge, so n0 x n1 lies
-    // along it: its projection on the unit edge is the signed sine, whose
-    // sign is the reference's sign test (n0 x n1) . e >= 0
-    double sd = dot(cross(n0, n1), ev) * il;
-    double a = angle_sc(abs_bits(sd), dot(n0, n1), sct);
-    o.th = sd >= 0.0 ? a : -a;
-    o.il = il;
+// Per edge eg: (theta / l, kt dB/dl / l) for the gradient (theta 0 on
+// boundary edges) and elt: (l theta, bond value) for k_vertex, 16 bytes per
+// gather each.  Edges below the flat bottom (exp and a division in FP64) are
+// collected per block and handled by its first threads, so that whole warps
+// do not wait on a few lanes.
+constexpr int EB = 256;
+__global__ void __launch_bounds__(EB) k_edge(Topo t, const double* __restrict__ P, const FaceD* __restrict__ fd,
+                                             double2* __restrict__ eg, double2* __restrict__ elt, EP ep,
+                                             const double2* __restrict__ sct) {
+  __shared__ double sl[EB], sil[EB];
+  __shared__ int se[EB], nshort;
+  if (threadIdx.x == 0) nshort = 0;
+  __syncthreads();
+  const int e = blockIdx.x * EB + threadIdx.x;
+  if (e < t.ne) {
+    int4 E = t.edge[e];
+    d3 pi = ld3(P, E.x), pj = ld3(P, E.y);
+    d3 ev = pj - pi;
+    double l2 = dot(ev, ev);
+    double il = rsqrt(l2);
+    double l = l2 * il;
+    double th = 0.0;
+    if (E.z >= 0 && E.w >= 0) {
+      const FaceD &F0 = fd[E.z], &F1 = fd[E.w];
+      d3 n0 = mk(F0.nx, F0.ny, F0.nz), n1 = mk(F1.nx, F1.ny, F1.nz);
+      // both normals are perpendicular to the shared edge, so n0 x n1 lies
+      // along it: its projection on the unit edge is the signed sine, whose
+      // sign is the reference's sign test (n0 x n1) . e >= 0
+      double sd = dot(cross(n0, n1), ev) * il;
+      double a = angle_sc(abs_bits(sd), dot(n0, n1), sct);
+      th = sd >= 0.0 ? a : -a;
+    }
+    // flat-bottom edge penalty: above the flat bottom inline (products only,
+    // edge_bond's l > lc0 branch)
+    double val = 0.0, fac = 0.0;
+    if (ep.btype == 0) {
+      if (len_below(l, ep.lc1)) {
+        const int k = atomicAdd(&nshort, 1);
+        se[k] = e;
+        sl[k] = l;
+        sil[k] = il;
+      } else if (len_above(l, ep.lc0)) {
+        const double d = l - ep.lc0;
+        val = ep.br1 * ipow(d, ep.r);
+        fac = ep.kt * (ep.br2 * ipow(d, ep.r - 1)) * il;
+      }
+    }
+    eg[e] = make_double2(th * il, fac);
+    elt[e] = make_double2(l * th, val);
   }
-  // flat-bottom edge penalty: above the flat bottom inline (products only,
-  // edge_bond's l > lc0 branch); edges below it (exp and a division in
-  // FP64) go to a list handled by k_bond_short so that whole warps do not
-  // wait on a few lanes
-  double val = 0.0, fac = 0.0;
-  const bool shortb = ep.btype == 0 && len_below(l, ep.lc1);
-  if (ep.btype == 0 && !shortb && len_above(l, ep.lc0)) {
-    const double d = l - ep.lc0;
-    val = ep.br1 * ipow(d, ep.r);
-    fac = ep.br2 * ipow(d, ep.r - 1);
-  }
-  warp_append(shortb, e, blist, bcnt);
-  o.db = fac;
-  ed[e] = o;
-  elt[e] = make_double2(o.l * o.th, val);
-}
-
-__global__ void k_bond_short(const double* __restrict__ P, Topo t, EdgeD* __restrict__ ed,
-                             double2* __restrict__ elt, EP ep, const int* __restrict__ blist,
-                             const int* __restrict__ bcnt) {
-  int n = *bcnt;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    int e = blist[i];
+  __syncthreads();
+  if ((int)threadIdx.x < nshort) {
+    const int k = threadIdx.x;
     double val, fac;
-    const EdgeD E = ed[e];
-    edge_bond(ep, E.l, fabs(E.il), &val, &fac);
-    ed[e].db = fac;
-    elt[e].y = val;
+    edge_bond(ep, sl[k], sil[k], &val, &fac);
+    eg[se[k]].y = ep.kt * fac * sil[k];
+    elt[se[k]].y = val;
   }
 }
 
@@ -226,94 +226,105 @@ __global__ void k_assemble_props(EP ep, const double* props6, Globals* g) {
 }
 
 // ---- gradient gather ------------------------------------------------------
-// rk[v] = (kb rho_v, 2/3 kb rho_v^2), written by k_vertex
-__global__ void __launch_bounds__(256) k_grad(Topo t, const double* __restrict__ P, const FaceD* __restrict__ fd,
-                                             const EdgeD* __restrict__ ed, const double2* __restrict__ rk,
+// Per vertex i over its ring (slot m: face (i, j = r_m, k = r_{m-1})), every
+// term along an edge vector d_j = x_j - x_i or a face normal n (area gradient
+// in its cotangent form, volume through the normal; Meyer, Desbrun, Schroeder
+// & Barr 2003), as in the double-word evaluation: with h = alpha / 2, alpha =
+// gA - 2/3 kb (rho_i^2 + rho_j^2 + rho_k^2), and w = gC/2 + kb (rho_i + rho_j)
+//   area -h (cot_k d_j + cot_j d_k), volume gV/3 A n, length -(w theta + kt
+//   dB/dl) / l d_j, dihedral (w_ij cot_j + w_ik cot_k - w_jk (cot_j + cot_k)) n
+// 25 FP64 operations per slot on GB300's narrow FP64 pipe (35 with cross
+// products of absolute positions).  Two lanes share a vertex, each with half
+// of its slots: twice the warps to cover the latency of gathers and FP64
+// chains for an eighth more operations.  rk[v] = (kb rho_v, 2/3 kb rho_v^2),
+// written by k_vertex.
+constexpr int GL = 2, GB = 128;
+template <bool CLOSED>
+__global__ void __launch_bounds__(GB) k_grad(Topo t, const double* __restrict__ P, const FaceD* __restrict__ fd,
+                                             const double2* __restrict__ eg, const double2* __restrict__ rk,
                                              const double* __restrict__ repg, const Globals* __restrict__ g, EP ep,
                                              double* __restrict__ grad) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= t.nv) return;
-  const double gA = g->gA, gV = g->gV, gC = g->gC;
-  const double hgC = 0.5 * gC;
-  d3 xi = ld3(P, i);
-  const double2 qi = rk[i];
-  const double ai = gA - qi.y;   // alpha = gA - 2/3 kb (rho_i^2 + rho_j^2 + rho_k^2)
-  const double wi = hgC + qi.x;  // w = gC/2 + kb (rho_i + rho_j)
-  d3 acc = ep.kr * ld3(repg, i);
-  int d = t.val[i];
-  if (d > 0) {
+  const int i = (blockIdx.x * GB + threadIdx.x) / GL, sub = threadIdx.x % GL;
+  d3 acc = mk(0, 0, 0), tel = mk(0, 0, 0), xi = mk(0, 0, 0);
+  const double gV = g->gV;
+  if (i < t.nv) {
+    const double gA = g->gA, hgC = 0.5 * g->gC, gV3 = gV * (1.0 / 3.0);
+    xi = ld3(P, i);
+    const double2 qi = rk[i];
+    const double ai = gA - qi.y, wi = hgC + qi.x;
+    const int d = t.val[i];
+    const int run = (d + GL - 1) / GL, mb = sub * run, m1 = min(d, mb + run);
     const size_t nv = t.nv;
-    int4 sp = t.slot[(size_t)(d - 1) * nv + i];
-    d3 xk = ld3(P, sp.x);
-    double2 qk = rk[sp.x];
-    int4 sc = t.slot[i];
-    d3 xj = ld3(P, sc.x);
-    double2 qj = rk[sc.x];
-    FaceD Fc;
-    int fcur = slot_face(sc.y);
-    if (fcur >= 0) Fc = fd[fcur];
-    const double gV6 = gV * (1.0 / 6.0);
-    // scalar multiples of face normals are summed per face: the dihedral
-    // term of edge (i, j) reaches the normal of the next face, so its part
-    // is carried to the next slot (the last one wraps to the first face)
-    double carry = 0.0;
-    d3 n0 = mk(0, 0, 0);
-    // length terms s_j (x_j - x_i): sum s_j x_j here, - (sum s_j) x_i at the end
-    double ssum = 0.0;
-    for (int m = 0; m < d; ++m) {
-      int4 sn = t.slot[(size_t)((m + 1) == d ? 0 : m + 1) * nv + i];
-      int fnx = slot_face(sn.y);
-      FaceD Fn;
-      if (fnx >= 0) Fn = fd[fnx];
-      double carry_next = 0.0;
-      if (fcur >= 0) {
-        int ci = slot_corner(sc.y);
-        double cj = cot_at(Fc, ci == 2 ? 0 : ci + 1);
-        double ck = cot_at(Fc, ci == 0 ? 2 : ci - 1);
-        d3 n = mk(Fc.nx, Fc.ny, Fc.nz);
-        if (m == 0) n0 = n;
-        // face (i, j, k): area and volume terms, (alpha/2) n x (x_k - x_j)
-        // + (gV/6) x_j x x_k = ((alpha/2) n + (gV/6) x_j) x (x_k - x_j)
-        double alpha = (ai - qj.y) - qk.y;
-        if (ep.btype == 1) alpha += ep.kt * 2.0 * (Fc.A / ep.a0 - 1.0) / ep.a0;
-        d3 u = (0.5 * alpha) * n + gV6 * xj;
-        d3 e = xk - xj;
-        acc.x = fma(u.y, e.z, fma(-u.z, e.y, acc.x));
-        acc.y = fma(u.z, e.x, fma(-u.x, e.z, acc.y));
-        acc.z = fma(u.x, e.y, fma(-u.y, e.x, acc.z));
-        // edge (i, j): length and dihedral terms
-        EdgeD E = ed[sc.z];
-        double w = wi + qj.x;
-        double cl = w * E.th + (ep.btype == 0 ? ep.kt * E.db : 0.0);
-        const double sj = -cl * abs_bits(E.il);
-        ssum += sj;
-        acc.x = fma(sj, xj.x, acc.x);
-        acc.y = fma(sj, xj.y, acc.y);
-        acc.z = fma(sj, xj.z, acc.z);
-        double cn = carry;
-        if (interior_edge(E.il)) {
-          int cin = slot_corner(sn.y);
-          cn += w * cj;
-          carry_next = w * cot_at(Fn, cin == 0 ? 2 : cin - 1);
+    if (mb < m1) {
+      const int4 sp = t.slot[(size_t)(mb == 0 ? d - 1 : mb - 1) * nv + i];
+      d3 dk = ld3(P, sp.x) - xi;
+      double2 qk = rk[sp.x];
+      double uk = hgC + qk.x, wk = wi + qk.x;
+      bool fprev = slot_face(sp.y) >= 0;
+      int4 sc = t.slot[(size_t)mb * nv + i];
+      double s = 0.0;  // coefficient of d_k still open
+      for (int m = mb; m < m1; ++m) {
+        int4 sn = sc;
+        if (!CLOSED || m + 1 < m1) sn = t.slot[(size_t)(m + 1 == d ? 0 : m + 1) * nv + i];
+        const d3 dj = ld3(P, sc.x) - xi;
+        const double2 qj = rk[sc.x];
+        const double wj = wi + qj.x;
+        const int f = slot_face(sc.y);
+        double sj = 0.0;
+        if (CLOSED || f >= 0) {
+          const FaceD F = fd[f];
+          const double2 E = eg[sc.z];
+          const int ci = slot_corner(sc.y);
+          const double cj = cot_at(F, ci == 2 ? 0 : ci + 1), ck = cot_at(F, ci == 0 ? 2 : ci - 1);
+          double alpha = (ai - qj.y) - qk.y;
+          if (ep.btype == 1) alpha += ep.kt * 2.0 * (F.A / ep.a0 - 1.0) / ep.a0;
+          const double h = -0.5 * alpha;
+          // edge (i, k): this face completes its coefficient
+          s = fma(h, cj, s);
+          acc.x = fma(s, dk.x, acc.x);
+          acc.y = fma(s, dk.y, acc.y);
+          acc.z = fma(s, dk.z, acc.z);
+          // edge (i, j): length and area terms
+          sj = fma(h, ck, -fma(wj, E.x, E.y));
+          // along n
+          double c = gV3 * F.A;
+          bool in_ij = true, in_ik = true, in_jk = true;
+          if (!CLOSED) {
+            in_ij = slot_face(sn.y) >= 0;
+            in_ik = fprev;
+            const int4 ejk = t.edge[sc.w];
+            in_jk = ejk.z >= 0 && ejk.w >= 0;
+          }
+          if (in_ij) c = fma(wj, cj, c);
+          if (in_ik) c = fma(wk, ck, c);
+          if (in_jk) c = fma(-(uk + qj.x), cj + ck, c);
+          acc.x = fma(c, F.nx, acc.x);
+          acc.y = fma(c, F.ny, acc.y);
+          acc.z = fma(c, F.nz, acc.z);
+          if (!CLOSED) tel += dk - dj;
+        } else {
+          // no face: the edge before it has no more terms
+          acc += s * dk;
         }
-        // edge (j, k) opposite i: dihedral term
-        if (interior_edge(ed[sc.w].il)) cn -= ((hgC + qj.x) + qk.x) * (cj + ck);
-        acc += cn * n;
+        fprev = f >= 0;
+        s = sj;
+        dk = dj;
+        qk = qj;
+        uk = hgC + qj.x;
+        wk = wj;
+        sc = sn;
       }
-      carry = carry_next;
-      xk = xj;
-      qk = qj;
-      sc = sn;
-      fcur = fnx;
-      Fc = Fn;
-      xj = ld3(P, sn.x);
-      qj = rk[sn.x];
+      acc += s * dk;  // the run's last edge
     }
-    acc += carry * n0;  // the last edge's part on the first face
-    acc.x = fma(-ssum, xi.x, acc.x);
-    acc.y = fma(-ssum, xi.y, acc.y);
-    acc.z = fma(-ssum, xi.z, acc.z);
   }
+  auto lanes = [](double x) { return x + __shfl_xor_sync(0xffffffffu, x, 1); };
+  acc = mk(lanes(acc.x), lanes(acc.y), lanes(acc.z));
+  if (!CLOSED) {  // x_i x (d_k - d_j) / 6 cancels around a closed fan only
+    tel = mk(lanes(tel.x), lanes(tel.y), lanes(tel.z));
+    acc += (gV * (1.0 / 6.0)) * cross(xi, tel);
+  }
+  if (i >= t.nv || sub) return;
+  acc += ep.kr * ld3(repg, i);
   st3(grad, i, acc);
 }
 
@@ -486,9 +497,7 @@ static void eval_fp64_launches(tm_energy* e, tm_mesh* m, const double* P, bool w
   Topo t = m->topo();
   EP ep = make_ep(e);
   FaceD* fd = reinterpret_cast<FaceD*>(e->face.get());
-  EdgeD* ed = reinterpret_cast<EdgeD*>(e->edge.get());
-  NLView nlv = e->nl.view;
-  nlv.pos32 = e->pos32.get();
+  double2* eg = reinterpret_cast<double2*>(e->edge.get());
   int nfb = std::max(nblk(std::max(t.nf, t.nv), 256), 1);
   k_face<<<nfb, 256, 0, s>>>(t, P, fd, e->pos32.get(), fav2(e));
   TM_LAUNCH();
@@ -497,12 +506,7 @@ static void eval_fp64_launches(tm_energy* e, tm_mesh* m, const double* P, bool w
   // (in sequence when the stages are timed)
   const bool conc = ev == nullptr;
   if (conc) fork_repulsion(e, m, P, want_grad, s, true);
-  int* blist = e->slow.get() + std::max(m->nv, 1) + 1;
-  int* bcnt = blist + std::max(m->ne, 1);
-  TM_CUDA(cudaMemsetAsync(bcnt, 0, sizeof(int), s));
-  if (t.ne) k_edge<<<nblk(t.ne, 256), 256, 0, s>>>(t, P, fd, ed, elt2(e), ep, blist, bcnt, e->sct.get());
-  TM_LAUNCH();
-  if (t.ne) k_bond_short<<<std::min(nblk(t.ne, 256), 4 * 152), 256, 0, s>>>(P, t, ed, elt2(e), ep, blist, bcnt);
+  if (t.ne) k_edge<<<nblk(t.ne, EB), EB, 0, s>>>(t, P, fd, eg, elt2(e), ep, e->sct.get());
   TM_LAUNCH();
   if (ev) TM_CUDA(cudaEventRecord(ev[2], s));
   if (conc)
@@ -519,7 +523,8 @@ static void eval_fp64_launches(tm_energy* e, tm_mesh* m, const double* P, bool w
   TM_LAUNCH();
   if (ev) TM_CUDA(cudaEventRecord(ev[3], s));
   if (want_grad && t.nv)
-    k_grad<<<nblk(t.nv, 256), 256, 0, s>>>(t, P, fd, ed, rk2(e), e->repg.get(), e->glob.get(), ep, d_grad);
+    (m->closed ? k_grad<true> : k_grad<false>)<<<nblk((long)GL * t.nv, GB), GB, 0, s>>>(
+        t, P, fd, eg, rk2(e), e->repg.get(), e->glob.get(), ep, d_grad);
   TM_LAUNCH();
   if (ev) TM_CUDA(cudaEventRecord(ev[4], s));
 }
@@ -544,8 +549,7 @@ void tm_energy::ensure(int nv_, int ne_, int nf_) {
   rho.ensure(2 * (size_t)std::max(nv, 1));  // FP64 path: (kb rho, 2/3 kb rho^2) per vertex
   repg.ensure(3 * (size_t)std::max(nv, 1));
   reppot.ensure(std::max(nv, 1));
-  // repulsion slow list (nv + 1) and short-bond edge list (ne + 1)
-  slow.ensure((size_t)std::max(nv, 1) + 1 + (size_t)std::max(ne, 1) + 1);
+  slow.ensure((size_t)std::max(nv, 1) + 1);  // repulsion slow list
   vprops.ensure(6 * (size_t)std::max(nv, 1));
   pos32.ensure(3 * (size_t)std::max(nv, 1));
   int nb = std::max(1, (nv + tmg::VB - 1) / tmg::VB);
@@ -879,18 +883,18 @@ extern "C" int tm_energy_eval_device_noalloc(tm_energy* e, tm_mesh* m, const dou
   if (!e || !m || !d_points || !d_grad) fail(TM_ERR_ARG, "NULL argument");
   const size_t nv = std::max(m->nv, 1), ne = std::max(m->ne, 1), nf = std::max(m->nf, 1);
   const int nb = std::max(1, (m->nv + VB - 1) / VB);
-  // scratch layout, 256-byte aligned pieces
+  // scratch layout, 256-byte aligned pieces (the mesh sizes that fit are part of
+  // the interface: each edge keeps the 32 bytes and the list entry it had)
   size_t off_face = 0;
   size_t off_edge = off_face + align256(sizeof(FaceD) * nf);
-  size_t off_ebond = off_edge + align256(sizeof(EdgeD) * ne);
+  size_t off_ebond = off_edge + align256(4 * sizeof(double) * ne);
   size_t off_fav = off_ebond + align256(sizeof(double2) * ne);
   size_t off_rho = off_fav + align256(sizeof(double2) * nf);
   size_t off_repg = off_rho + align256(sizeof(double2) * nv);
   size_t off_pos32 = off_repg + align256(3 * sizeof(double) * nv);
   size_t off_pot = off_pos32 + align256(3 * sizeof(float) * nv);
   size_t off_slow = off_pot + align256(sizeof(double) * nv);
-  size_t off_blist = off_slow + align256(sizeof(int) * (nv + 1));
-  size_t off_part = off_blist + align256(sizeof(int) * (ne + 1));
+  size_t off_part = off_slow + align256(sizeof(int) * (nv + 1)) + align256(sizeof(int) * (ne + 1));
   size_t off_glob = off_part + align256(8 * sizeof(double) * nb);
   size_t need = off_glob + align256(sizeof(Globals));
   if (need > (size_t)TM_NOALLOC_SCRATCH_BYTES)
@@ -900,7 +904,7 @@ extern "C" int tm_energy_eval_device_noalloc(tm_energy* e, tm_mesh* m, const dou
   unsigned char* base = noalloc_scratch_for_current_device();
   cudaStream_t s = stream ? (cudaStream_t)stream : e->stream;
   FaceD* fd = reinterpret_cast<FaceD*>(base + off_face);
-  EdgeD* ed = reinterpret_cast<EdgeD*>(base + off_edge);
+  double2* eg = reinterpret_cast<double2*>(base + off_edge);
   double2* ebond = reinterpret_cast<double2*>(base + off_ebond);
   double2* fav = reinterpret_cast<double2*>(base + off_fav);
   double2* rho = reinterpret_cast<double2*>(base + off_rho);
@@ -908,28 +912,23 @@ extern "C" int tm_energy_eval_device_noalloc(tm_energy* e, tm_mesh* m, const dou
   float* pos32 = reinterpret_cast<float*>(base + off_pos32);
   double* reppot = reinterpret_cast<double*>(base + off_pot);
   int* slow = reinterpret_cast<int*>(base + off_slow);
-  int* blist = reinterpret_cast<int*>(base + off_blist);
-  int* bcnt = blist + ne;
   double* part = reinterpret_cast<double*>(base + off_part);
   Globals* g = reinterpret_cast<Globals*>(base + off_glob);
   // the block ticket of the reduction must start at zero
   TM_CUDA(cudaMemsetAsync(g, 0, sizeof(Globals), s));
   Topo t = m->topo();
   EP ep = make_ep(e);
-  NLView nlv = e->nl.view;
-  nlv.pos32 = pos32;
   int nfb = std::max(nblk(std::max(t.nf, t.nv), 256), 1);
   k_face<<<nfb, 256, 0, s>>>(t, d_points, fd, pos32, fav);
   TM_LAUNCH();
-  TM_CUDA(cudaMemsetAsync(bcnt, 0, sizeof(int), s));
-  if (t.ne) k_edge<<<nblk(t.ne, 256), 256, 0, s>>>(t, d_points, fd, ed, ebond, ep, blist, bcnt, e->sct.get());
-  TM_LAUNCH();
-  if (t.ne) k_bond_short<<<std::min(nblk(t.ne, 256), 4 * 152), 256, 0, s>>>(d_points, t, ed, ebond, ep, blist, bcnt);
+  if (t.ne) k_edge<<<nblk(t.ne, EB), EB, 0, s>>>(t, d_points, fd, eg, ebond, ep, e->sct.get());
   TM_LAUNCH();
   repulsion_eval(e, m, d_points, pos32, true, reppot, repg, slow, slow + nv, s);
   k_vertex<false><<<nb, VB, 0, s>>>(t, fav, ebond, reppot, ep, rho, nullptr, part, g);
   TM_LAUNCH();
-  if (t.nv) k_grad<<<nblk(t.nv, 256), 256, 0, s>>>(t, d_points, fd, ed, rho, repg, g, ep, d_grad);
+  if (t.nv)
+    (m->closed ? k_grad<true> : k_grad<false>)<<<nblk((long)GL * t.nv, GB), GB, 0, s>>>(t, d_points, fd, eg, rho,
+                                                                                       repg, g, ep, d_grad);
   TM_LAUNCH();
   if (d_energy) TM_CUDA(cudaMemcpyAsync(d_energy, &g->comps[6], sizeof(double), cudaMemcpyDeviceToDevice, s));
   TM_API_END

@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(EB) k_edge(Topo t, const double* __restrict__ 
     double l = l2 * il;
     double th = 0.0;
     if (E.z >= 0 && E.w >= 0) {
-      const FaceD &F0 = fd[E.z], &F1 = fd[E.w];
+      const FaceD F0 = fd[E.z], F1 = fd[E.w];
       d3 n0 = mk(F0.nx, F0.ny, F0.nz), n1 = mk(F1.nx, F1.ny, F1.nz);
       // both normals are perpendicular to the shared edge, so n0 x n1 lies
       // along it: its projection on the unit edge is the signed sine, whose

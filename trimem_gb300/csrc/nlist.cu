@@ -76,21 +76,6 @@ __device__ int cell_lookup(const NLView& nl, long long key, int* start) {
   return 0;
 }
 
-__device__ bool nl_excluded(const Topo& t, int excl, int v, int j) {
-  if (excl <= 0) return false;
-  int d = t.val[v];
-  for (int m = 0; m < d; ++m) {
-    int w = t.nbr[(size_t)m * t.nv + v];
-    if (w == j) return true;
-    if (excl > 1) {
-      int dw = t.val[w];
-      for (int q = 0; q < dw; ++q)
-        if (t.nbr[(size_t)q * t.nv + w] == j) return true;
-    }
-  }
-  return false;
-}
-
 namespace {
 
 constexpr int BB = 256;
@@ -386,7 +371,7 @@ __global__ void k_cell_pairs(int nv, const double* P, NLView nl, Topo t, const i
           if (mode == 1 && cid == ca && b < a) continue;
           double dd = exact_dist(pa, ld3(P, b));
           if (!(dd <= rd)) continue;
-          if (nl_excluded(t, nl.excl, a, b)) continue;
+          if (excluded(t, nl.excl, a, b)) continue;
           if (pass) {
             od[base + n] = dd;
             if (mode == 0) {
@@ -443,7 +428,7 @@ __global__ void k_verlet_batch(int nv, const double* P, NLView nl, Topo t, const
           if (b == a) continue;
           double dd = exact_dist(pa, ld3(P, b));
           if (!(dd <= rd)) continue;
-          if (nl_excluded(t, excl, a, b)) continue;
+          if (excluded(t, excl, a, b)) continue;
           if (pass) {
             od[base + n] = dd;
             oj[base + n] = b;
@@ -585,7 +570,7 @@ __global__ void __launch_bounds__(NB) k_near(int nv, const double* __restrict__ 
     if (sub == 0 && n > TM_NEAR_CAP) atomicOr(&flag[3], 1);
     n = min(n, TM_NEAR_CAP);
     __syncwarp(gmask);
-    // exclusion flags (nl_excluded): an entry is excluded when it is in the
+    // exclusion flags: an entry is excluded when it is in the
     // ring of a or, at level 2, in the ring of a ring vertex of a; the rings
     // are walked once and their vertices looked up in the row
     const int level = nl.rexcl ? nl.rexcl[rep] : excl;  // batch: the replica's level
@@ -673,7 +658,7 @@ __global__ void k_point(int pid, const double* P, NLView nl, Topo t, double rd, 
           for (int q = 0; q < cc; ++q) {
             int j = nl.cell_verts[st + q];
             if (j == pid) continue;
-            if (nl_excluded(t, nl.excl, pid, j)) continue;
+            if (excluded(t, nl.excl, pid, j)) continue;
             d3 pj = ld3(P, j);
             if (exact_dist(p, pj) < rd) {
               if (pass) {

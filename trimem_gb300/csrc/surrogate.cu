@@ -970,20 +970,22 @@ __global__ void __launch_bounds__(TB) k_t_outback(int nv, int D, const int* __re
   });
 }
 
-// Backward of dense layer r over tiles of 64 vertices (persistent blocks):
+// Backward of dense layer r over tiles of 32 vertices (persistent blocks):
 // dz = dh1 * SiLU'(z); dh0 = dh1 + dz W[:, :64]; dm = dz W[:, 64:];
 // block partials of dW (64 x 128, row n, column k) and db (64).  Both are
-// FP32 matrix products (the gradients keep FP32 operands), bound by the FMA
-// pipe once the operands reach it: thread t owns rows rg + 8 q (vertices) or
-// 8 rg + q (channels), q < 8, and columns 4 kg .. + 3 of each product, so that
-// 32 FMAs share three 16-byte shared loads, each one wavefront a warp (four
-// row groups and eight column groups a warp; sdz rows are padded by four
-// floats to keep the row groups on different banks).  40,962 vertices: one
-// column and 32 rows a thread, one shared load per FMA, took 142 us a layer.
-constexpr int DT = 64;        // vertices per tile
+// FP32 matrix products (the gradients keep FP32 operands), bound by shared
+// memory and the FMA pipe: thread t owns rows rg + 8 q (vertices, q < 4) or
+// 8 rg + q (channels, q < 8) and columns 4 kg .. + 3 of each product, so that
+// 16 or 32 FMAs share two or three 16-byte shared loads without bank conflicts
+// (four row groups and eight column groups a warp; sdz rows are padded by four
+// floats).  40,962 vertices: one column and 32 rows a thread, one shared load
+// per FMA, took 142 us a layer, tiles of 64 vertices with two blocks per SM
+// 56; with 32 and three blocks the loads of one overlap the products of
+// another (a step of 420 us then, 400 now).
+constexpr int DT = 32;        // vertices per tile
 constexpr int ZP = H + 4;     // padded row of sdz
 constexpr int DENSE_BACK_SMEM = (DT * ZP + DT * 2 * H + H * 2 * H) * sizeof(float);
-__global__ void __launch_bounds__(TB, 2) k_t_dense_back(int nv, const float* __restrict__ th, int r,
+__global__ void __launch_bounds__(TB, 3) k_t_dense_back(int nv, const float* __restrict__ th, int r,
                                                         const float* __restrict__ z,
                                                         const __nv_bfloat16* __restrict__ h,
                                                         const __nv_bfloat16* __restrict__ mm,
@@ -1038,9 +1040,9 @@ __global__ void __launch_bounds__(TB, 2) k_t_dense_back(int nv, const float* __r
     __syncthreads();
     // d[h | m][v][k] = sum_n dz[v][n] W[n][k], vertices rg + 8 q
     {
-      float o[8][4];
+      float o[DT / 8][4];
 #pragma unroll
-      for (int q = 0; q < 8; ++q)
+      for (int q = 0; q < DT / 8; ++q)
 #pragma unroll
         for (int c = 0; c < 4; ++c) o[q][c] = 0.f;
 #pragma unroll 2
@@ -1049,7 +1051,7 @@ __global__ void __launch_bounds__(TB, 2) k_t_dense_back(int nv, const float* __r
 #pragma unroll
         for (int u = 0; u < 4; ++u) w[u] = *reinterpret_cast<const float4*>(sw + (n + u) * 2 * H + kc);
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
+        for (int q = 0; q < DT / 8; ++q) {
           const float4 d = *reinterpret_cast<const float4*>(sdz + (rg + 8 * q) * ZP + n);
           const float dd[4] = {d.x, d.y, d.z, d.w};
 #pragma unroll
@@ -1062,7 +1064,7 @@ __global__ void __launch_bounds__(TB, 2) k_t_dense_back(int nv, const float* __r
         }
       }
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
+      for (int q = 0; q < DT / 8; ++q) {
         if (rg + 8 * q >= nrow) break;
         const size_t v = v0 + rg + 8 * q;
         float4 x = make_float4(o[q][0], o[q][1], o[q][2], o[q][3]);
@@ -1218,7 +1220,7 @@ __global__ void __launch_bounds__(TB, 2) k_t_embed_back(int nv, const float* __r
 // reads) are refreshed from the FP32 master.  One thread a column over all
 // partials, a launch per group, took 718 us of the 1,265 us step at 40,962
 // vertices; with it, persistent blocks, the tiled products and k_layer the step
-// is 423.
+// is 400.
 struct RedGroup {
   const float* part;
   int nb, n, dst, blk0;  // partials, columns (= stride), first parameter, first block

@@ -411,7 +411,7 @@ static std::vector<unsigned char> eval_key(tm_energy* e, tm_mesh* m, const doubl
   };
   // (the launch stream is not part of the key: a graph replays on any stream)
   const void* ptrs[] = {P, d_grad, e->face.get(), e->edge.get(), e->ebond.get(), e->fav.get(), e->rho.get(),
-                        e->repg.get(), e->reppot.get(), e->slow.get(), e->pos32.get(), e->poslo.get(), e->partials.get(),
+                        e->repg.get(), e->reppot.get(), e->slow.get(), e->pos32.get(), e->partials.get(),
                         e->glob.get(), e->sct.get(), e->aux, e->ev_fork, e->ev_join, e->nl.xb.get(),
                         e->posdw.get(), e->sctf.get()};
   add(ptrs, sizeof ptrs);

@@ -552,13 +552,14 @@ __global__ void __launch_bounds__(256) k_out(Topo t, Split S, const float* __res
   const float bo = W->bo;
   float F = cn * nrm[4 * (size_t)ii + (sub < 3 ? sub : 3)];  // lane k < 3: component k
   const float4* mine = term + (threadIdx.x & ~7);
+  const Pos32 xi = S.at(ii);
   for (int m = 0; __any_sync(FULL, m < d); m += 8) {
     const int cnt = min(8, d - m);
     int j = -1;
     f3 e = {0.f, 0.f, 0.f};
     if (sub < cnt) {
       j = t.nbr[(size_t)(m + sub) * t.nv + ii];
-      e = S.diff(j, ii);
+      e = diff(S.at(j), xi);
     }
     float c[8];
 #pragma unroll
@@ -608,7 +609,7 @@ __global__ void k_export(Topo t, Split S, const EdgeF* __restrict__ ed, const fl
       int4 s = t.slot[o];
       j = s.x;
       edge_feat(ed[s.z], rho[i], rho[j], W->lbar, f);
-      f3 e = S.diff(j, i);
+      f3 e = diff(S.at(j), S.at(i));
       dir = (1.0f / fnorm(e)) * e;
     }
     nbr[o] = j;
@@ -711,7 +712,7 @@ void surrogate_grad(tm_surrogate* sg, tm_energy* e, tm_mesh* m, const double* P,
   const FaceF* fd = reinterpret_cast<const FaceF*>(e->face.get());
   const EdgeF* ed = reinterpret_cast<const EdgeF*>(e->edge.get());
   const float* rho = reinterpret_cast<const float*>(e->rho.get());
-  Split S{e->pos32.get(), e->poslo.get()};
+  Split S{e->posdw.get()};
   SurW* W = sg->w.get();
   k_sfeat<<<nblk(nv, SFB), SFB, 0, s>>>(t, fd, ed, rho, W, nullptr, sg->nrm.get(), sg->hb[0].get());
   TM_LAUNCH();
@@ -1470,7 +1471,7 @@ int tm_surrogate_inputs_device(tm_surrogate* sg, tm_energy* e, tm_mesh* m, const
   const FaceF* fd = reinterpret_cast<const FaceF*>(e->face.get());
   const EdgeF* ed = reinterpret_cast<const EdgeF*>(e->edge.get());
   const float* rho = reinterpret_cast<const float*>(e->rho.get());
-  Split S{e->pos32.get(), e->poslo.get()};
+  Split S{e->posdw.get()};
   k_sfeat<<<nblk(nv, SFB), SFB, 0, s>>>(t, fd, ed, rho, sg->w.get(), d_u, sg->nrm.get(), sg->hb[0].get());
   TM_LAUNCH();
   TM_CUDA(cudaMemcpyAsync(d_normals, sg->nrm.get(), sizeof(float) * 4 * nv, cudaMemcpyDeviceToDevice, s));

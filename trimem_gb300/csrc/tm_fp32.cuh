@@ -1,12 +1,15 @@
 // FP32 element records and float helpers shared by the FP32-stencil
 // evaluation and the surrogate force model.
 #pragma once
+#include "tm_dw.cuh"
 #include "tm_internal.h"
 
 namespace tmg {
 
-struct __align__(16) FaceF {
-  float nx, ny, nz, A, V, c0, c1, c2;
+// unit normal and a cotangent, then (A, V) and the other cotangents: one
+// 16-byte or one 8-byte load for what the edge and vertex stages gather
+struct __align__(32) FaceF {
+  float nx, ny, nz, c0, A, V, c1, c2;
 };
 // l: length, with the sign bit set on boundary edges (length() and
 // interior()); bond: the bond's value
@@ -42,16 +45,27 @@ __device__ __forceinline__ float fipow(float x, int n) {
   return n < 0 ? 1.0f / r : r;
 }
 
+// Split positions, one 32-byte sector per vertex: hi parts (x, y, z, rho), lo
+// parts (x, y, z, .), with rho = c/a written by the vertex stage, so that a
+// gather of a neighbour is one load instruction where separate hi, lo and rho
+// arrays took seven.
+struct Pos32 {
+  f3 hi, lo;
+  float rho;
+};
 struct Split {
-  const float* hi;
-  const float* lo;
-  __device__ f3 h(int v) const { return {hi[3 * v], hi[3 * v + 1], hi[3 * v + 2]}; }
-  // x_b - x_a with FP32 relative accuracy
-  __device__ f3 diff(int b, int a) const {
-    return {(hi[3 * b] - hi[3 * a]) + (lo[3 * b] - lo[3 * a]), (hi[3 * b + 1] - hi[3 * a + 1]) + (lo[3 * b + 1] - lo[3 * a + 1]),
-            (hi[3 * b + 2] - hi[3 * a + 2]) + (lo[3 * b + 2] - lo[3 * a + 2])};
+  const float4* X;
+  __device__ __forceinline__ Pos32 at(int v) const {
+    float4 h, l;
+    ld32(X + 2 * (size_t)v, h, l);
+    return {{h.x, h.y, h.z}, {l.x, l.y, l.z}, h.w};
   }
 };
+// x_b - x_a with FP32 relative accuracy
+__device__ __forceinline__ f3 diff(const Pos32& b, const Pos32& a) {
+  return {(b.hi.x - a.hi.x) + (b.lo.x - a.lo.x), (b.hi.y - a.hi.y) + (b.lo.y - a.lo.y),
+          (b.hi.z - a.hi.z) + (b.lo.z - a.lo.z)};
+}
 
 }  // namespace fp32
 }  // namespace tmg

@@ -220,8 +220,8 @@ struct tm_energy {
   tmg::DevBuf<double> face, edge, ebond, fav, rho, repg, reppot, vprops, partials, grad, work;
   tmg::DevBuf<int> slow;  // vertices that left their build cell (+ count)
   tmg::DevBuf<int> moved;  // double-word path: per block, some vertex left its skin
-  tmg::DevBuf<float> pos32, poslo;
-  tmg::DevBuf<float4> posdw;  // double-word stencils: hi and lo parts, 2 per vertex (PosDW)
+  tmg::DevBuf<float> pos32;
+  tmg::DevBuf<float4> posdw;  // double-word and FP32 stencils: hi and lo parts, 2 per vertex (PosDW, Split)
   tmg::DevBuf<tmg::Globals> glob;
   tmg::DevBuf<double2> sct;  // {sin, cos}(k / 128), k < TM_SCT_N
   tmg::DevBuf<float4> sctf;  // the same as double-words (sin hi, sin lo, cos hi, cos lo)

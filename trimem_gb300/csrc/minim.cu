@@ -94,17 +94,21 @@ struct Direction {
 // Two-loop recursion d = -H g, the slope g . d, the restart from steepest
 // descent when d is not a descent direction, and the trial point x + a d.
 // The recursion is a chain of 2 stored + 1 dot products over the whole
-// vector: one cooperative kernel with one grid barrier per dot product.
-// Every warp sums the block partials itself, the update of d stays within
-// the thread (E elements in registers; E = 0: in memory), and the vectors of
-// the next update and dot product are loaded before the barrier.  As
+// vector: one kernel with one barrier per dot product.  The update of d
+// stays within the thread (E elements in registers; E = 0: in memory), and the
+// vectors of the next update and dot product are loaded before the barrier.
+// FP64 instructions of one SM queue on a pipe of two lanes, so one warp sums the
+// block partials and forms the update's coefficient for its block (every warp
+// for itself: 1.53 ms for ten iterations at 10,242 vertices, so 1.28; one
+// cluster of 16 blocks with its faster barrier, but the vectors' FP64 work on
+// 16 SMs: 1.38).  As
 // separate kernels with the dot product read by the host, 10,242 vertices and
 // ten iterations took 330 launches and 140 waits of the 600 launches and 5.7
-// ms of the whole minimisation, which takes 1.53 ms now.
+// ms of the whole minimisation.
 template <int E>
 __global__ void __launch_bounds__(DB, 2) k_direction(const __grid_constant__ Direction q) {
   __shared__ double s[DB];
-  __shared__ double alpha[MAXHIST];
+  __shared__ double alpha[MAXHIST], coef;
   constexpr int M = E > 0 ? E : 1;
   const cooperative_groups::grid_group grid = cooperative_groups::this_grid();
   const int n = q.n, first = blockIdx.x * DB + threadIdx.x, step = gridDim.x * DB;
@@ -130,7 +134,8 @@ __global__ void __launch_bounds__(DB, 2) k_direction(const __grid_constant__ Dir
     d[e] = -1.0 * g[i];
     if (E == 0) q.d[i] = d[e];
   });
-  auto row = [&](int k) { return (size_t)((q.head - 1 - k + q.history) % q.history) * n; };
+  auto pair = [&](int k) { return (q.head - 1 - k + q.history) % q.history; };
+  auto row = [&](int k) { return (size_t)pair(k) * n; };
   const int nd = 2 * q.stored;
   auto dot_vec = [&](int k) { return k < q.stored ? q.S + row(k) : (k < nd ? q.Y + row(nd - 1 - k) : g); };
   auto add_vec = [&](int k) { return k < q.stored ? q.Y + row(k) : q.S + row(nd - 1 - k); };
@@ -152,8 +157,21 @@ __global__ void __launch_bounds__(DB, 2) k_direction(const __grid_constant__ Dir
         nv[e] = w[i];
       });
     grid.sync();
-    r = total_of(part, gridDim.x);
-    if (k >= nd) {  // the slope
+    if (threadIdx.x < 32) {  // the slope, or the coefficient of the update
+      double c = total_of(part, gridDim.x);
+      if (threadIdx.x == 0) {
+        if (k < q.stored) {
+          alpha[k] = __dmul_rn(q.rho[pair(k)], c);
+          c = -alpha[k];
+        } else if (k < nd) {
+          c = __dsub_rn(alpha[nd - 1 - k], __dmul_rn(q.rho[pair(nd - 1 - k)], c));
+        }
+        coef = c;
+      }
+    }
+    __syncthreads();
+    r = coef;
+    if (k >= nd) {
       if (restart || r < 0.0) break;
       restart = true;
       each([&](int e, int i) {
@@ -161,21 +179,13 @@ __global__ void __launch_bounds__(DB, 2) k_direction(const __grid_constant__ Dir
         if (E == 0) q.d[i] = d[e];
       });
     } else {
-      double c;
-      if (k < q.stored) {
-        const double al = __dmul_rn(q.rho[row(k) / n], r);
-        if (threadIdx.x == 0) alpha[k] = al;
-        c = -al;
-      } else {
-        c = __dsub_rn(alpha[nd - 1 - k], __dmul_rn(q.rho[row(nd - 1 - k) / n], r));
-      }
       const bool scale = k == q.stored - 1;
       each([&](int e, int i) {
         if (E > 0) {
-          d[e] += c * av[e];
+          d[e] += r * av[e];
           if (scale) d[e] = q.gamma * d[e];
         } else {
-          double y = q.d[i] + c * a[i];
+          double y = q.d[i] + r * a[i];
           if (scale) y = q.gamma * y;
           q.d[i] = y;
         }

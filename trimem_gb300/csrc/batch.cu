@@ -71,6 +71,8 @@ struct tm_batch {
   std::vector<BatchClass> cls;
   BatchStreams bs{};
   bool have_side = false;  // streams and events exist
+  cudaStream_t mom = nullptr;  // the momenta's stream and its fork and join
+  cudaEvent_t fork_mom = nullptr, join_mom = nullptr;
   cudaStream_t stream = nullptr;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t gexec = nullptr;
@@ -95,6 +97,9 @@ struct tm_batch {
       cudaEventDestroy(bs.fork[1]);
       cudaEventDestroy(bs.join_rep);
     }
+    if (mom) cudaStreamDestroy(mom);
+    if (fork_mom) cudaEventDestroy(fork_mom);
+    if (join_mom) cudaEventDestroy(join_mom);
     if (stream) cudaStreamDestroy(stream);
   }
 };
@@ -202,11 +207,18 @@ static void batch_hmc_step(tm_batch* b, int L, double dt, double m, double T, un
   int n3 = 3 * b->nv;
   int nb = b->nv / B;
   k_copy_b<<<nblk(n3, B), B, 0, s>>>(n3, b->x.get(), b->xs.get());
-  k_momenta_b<<<nblk((n3 + 1) / 2, B), B, 0, s>>>(n3, seed, b->counter.get(), sqrt(m * T), b->vrep.get(), b->p.get());
-  k_kin_blocks<<<nb, B, 0, s>>>(b->nv, b->p.get(), b->part.get());
+  // the momenta (FP64 logarithms and sines, 49 us at 218,000 vertices) beside
+  // the first evaluation, which does not need them
+  TM_CUDA(cudaEventRecord(b->fork_mom, s));
+  TM_CUDA(cudaStreamWaitEvent(b->mom, b->fork_mom, 0));
+  k_momenta_b<<<nblk((n3 + 1) / 2, B), B, 0, b->mom>>>(n3, seed, b->counter.get(), sqrt(m * T), b->vrep.get(),
+                                                        b->p.get());
+  k_kin_blocks<<<nb, B, 0, b->mom>>>(b->nv, b->p.get(), b->part.get());
+  TM_CUDA(cudaEventRecord(b->join_mom, b->mom));
   double* g0 = b->g0.get();
   double* g1 = b->g1.get();
   batch_eval(b, b->x.get(), g0, nullptr, s);
+  TM_CUDA(cudaStreamWaitEvent(s, b->join_mom, 0));
   k_collect<<<nblk(32L * b->R, 64), 64, 0, s>>>(b->R, b->rblocks.get(), b->part.get(), b->gs.get(), b->sc.get(), 0);
   for (int i = 0; i < L; ++i) {
     // drift with the first force, then kick with the last two and drift; the
@@ -407,6 +419,9 @@ int tm_batch_create(int n_rep, const double* const* points, const int64_t* n_poi
     rb[r] = make_int2(b->voff[r] / B, b->voff[r + 1] / B);
   }
   TM_CUDA(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
+  TM_CUDA(cudaStreamCreateWithFlags(&b->mom, cudaStreamNonBlocking));
+  TM_CUDA(cudaEventCreateWithFlags(&b->fork_mom, cudaEventDisableTiming));
+  TM_CUDA(cudaEventCreateWithFlags(&b->join_mom, cudaEventDisableTiming));
   tm_mesh* mraw = nullptr;
   int rc = tm_mesh_create(P.data(), nv, F.data(), (int64_t)F.size() / 3, &mraw);
   if (rc) return rc;

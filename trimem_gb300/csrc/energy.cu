@@ -553,7 +553,7 @@ void tm_energy::ensure(int nv_, int ne_, int nf_) {
   vprops.ensure(6 * (size_t)std::max(nv, 1));
   pos32.ensure(3 * (size_t)std::max(nv, 1));
   int nb = std::max(1, (nv + tmg::VB - 1) / tmg::VB);
-  partials.ensure(8 * (size_t)nb * 8);  // up to eight lanes per vertex
+  partials.ensure(8 * (size_t)nb * 2);  // up to two lanes per vertex
   moved.ensure(nb);
   grad.ensure(3 * (size_t)std::max(nv, 1));
   work.ensure(64);

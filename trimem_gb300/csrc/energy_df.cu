@@ -905,18 +905,26 @@ void energy_eval_df(tm_energy* e, tm_mesh* m, const double* P, bool want_grad, d
   launch_after(want_grad ? k_edge_dw<true> : k_edge_dw<false>, std::max(1, nqueue + nblk(t.ne, SB)), SB, s, q,
                nqueue);
   if (ev) TM_CUDA(cudaEventRecord(ev[2], s));
-  // Eight lanes per vertex shorten the chain of one thread's walk over its
-  // ring, one lane per vertex issues fewer instructions.  Whole evaluations
-  // of spheres on a GB300, eight lanes against one: 642 vertices 23.9 / 27.4
-  // us, 2,562 25.3 / 28.5, 10,242 30.8 / 30.2, 16,002 34.8 / 29.3; an open
-  // tube of 7,566 vertices (more arithmetic per slot) 36.9 / 38.5.
-  const bool lanes = t.nv <= 8000;
-  launch_after(lanes ? k_vertex_dw<8> : k_vertex_dw<1>, std::max(1, nblk((long)t.nv * (lanes ? 8 : 1), VB)), VB, s, q);
+  // Several lanes per vertex shorten the chain of one thread's walk over its
+  // ring and fill more SMs, one lane per vertex issues fewer instructions.
+  // Whole evaluations of spheres on a GB300 in us, lanes of the vertex stage /
+  // of the gradient:
+  //   vertices    1 / 1   1 / 2   2 / 2   2 / 4   2 / 8   8 / 8
+  //        642    26.7    24.8    24.3    23.4    22.9    23.2
+  //      4,002    27.0    26.3    25.3    25.1    25.1    26.5
+  //     10,242    29.6    28.5    28.4    28.3    28.6    30.7
+  //     23,042    32.6    31.0    30.7    30.6    34.5    39.1
+  //     40,962    39.0    37.7    37.8    41.0    46.0    51.0
+  //     81,002    44.0    47.1    49.7    56.2    65.2    79.7
+  const bool two = t.nv <= 50000;
+  launch_after(two ? k_vertex_dw<2> : k_vertex_dw<1>, std::max(1, nblk((long)t.nv * (two ? 2 : 1), VB)), VB, s, q);
   if (ev) TM_CUDA(cudaEventRecord(ev[3], s));
   if (want_grad && t.nv) {
-    auto* kg = lanes ? (m->closed ? k_grad_dw<true, 8> : k_grad_dw<false, 8>)
-                     : (m->closed ? k_grad_dw<true, 1> : k_grad_dw<false, 1>);
-    launch_after(kg, nblk((long)t.nv * (lanes ? 8 : 1), 128), 128, s, q);
+    const int lanes = t.nv <= 4500 ? 8 : (two ? 2 : 1);
+    auto* kg = lanes == 8   ? (m->closed ? k_grad_dw<true, 8> : k_grad_dw<false, 8>)
+               : lanes == 2 ? (m->closed ? k_grad_dw<true, 2> : k_grad_dw<false, 2>)
+                            : (m->closed ? k_grad_dw<true, 1> : k_grad_dw<false, 1>);
+    launch_after(kg, nblk((long)t.nv * lanes, 128), 128, s, q);
   }
   if (ev) TM_CUDA(cudaEventRecord(ev[4], s));
 }

@@ -214,7 +214,7 @@ __device__ __forceinline__ void rep_vertex(const DwEval& q, int v, int sub, int 
   const unsigned gmask = ((1u << RL) - 1u) << (threadIdx.x & 31 & ~(RL - 1));
   const d3 p = ld3p(q.P, v);
   const PairTest pt = make_pair_test(nl, v, ep.rlc1, ep.rT);
-  TableExcl x{q.t, nl.excl};
+  TableExclSlim x{q.t, nl.excl};
   RepTerm sum{0.0, 0.0, 0.0, 0.0};
   auto add = [&](int, double l, d3 dv) {
     const RepTerm r = rep_term<GRAD>(ep, l, dv);
@@ -411,7 +411,7 @@ __device__ __forceinline__ void rep_queue(const DwEval& q, int warp, int nwarps)
   const int lane = threadIdx.x & 31;
   const NLView& nl = q.nl;
   const NLGeom& G = *nl.geom;
-  TableExcl x{q.t, nl.excl};
+  TableExclSlim x{q.t, nl.excl};
   for (int i = warp; i < n; i += nwarps) {
     const int v = ((volatile int*)q.slow)[i];
     const d3 p = ld3p(q.P, v);

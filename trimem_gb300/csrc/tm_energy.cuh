@@ -107,6 +107,27 @@ __device__ __forceinline__ bool excluded(const T& t, int excl, int v, int j) {
   return rings_meet(t, excl, v, j, -3, -3, -4, -4);
 }
 
+// The same test one vertex at a time: few registers, for the double-word face
+// kernel, whose repulsion hardly ever makes the test and whose faces pay for
+// its registers (64 instead of 56: 86.2 us an evaluation of 163,842 vertices
+// against 84).
+struct TableExclSlim {
+  const Topo& t;
+  int excl;
+  __device__ bool operator()(int v, int j) const {
+    const int d = t.val[v], dj = excl > 1 ? t.val[j] : 0;
+#pragma unroll 1
+    for (int m = 0; m < d; ++m) {
+      const int w = t.nbr[(size_t)m * t.nv + v];
+      if (w == j) return true;
+#pragma unroll 1
+      for (int q = 0; q < dj; ++q)
+        if (t.nbr[(size_t)q * t.nv + j] == w) return true;
+    }
+    return false;
+  }
+};
+
 struct TableExcl {  // exclusion on the current topology tables
   const Topo& t;
   int excl;

@@ -272,7 +272,8 @@ __global__ void k_winner(TopoW t, const FlipState* st, int mode, const long long
 // first, then new ones, as k_fill), the claims, a grid-wide barrier, then
 // the window's state is advanced and the ownership test runs on the same
 // vertices (read past L1)
-__global__ void __launch_bounds__(64) k_claim_win(TopoW t, FlipState* st, int B, int mode, const long long* pend,
+constexpr int CWT = 256;  // threads of the claim kernels: few blocks, a short grid barrier
+__global__ void __launch_bounds__(CWT) k_claim_win(TopoW t, FlipState* st, int B, int mode, const long long* pend,
                                                  long long* win, int* owner, unsigned char* winner, int* limit) {
   let_next_start();
   const unsigned long long seed = st->seed;
@@ -762,11 +763,13 @@ __device__ __forceinline__ int2 block_scan2(int a, int b, int* ea, int* eb, int2
   return wsum[31];
 }
 
+constexpr size_t METRO_SMEM = MAXB * 2 * sizeof(float4);
 constexpr int PREF = 256;  // walked slots whose data is prefetched into shared memory
 __global__ void __launch_bounds__(MB) k_metro(const long long* win, const unsigned char* winner, const double* dpn,
                                              const float* dpf, FlipE fe, FlipEF fg, FlipState* st, const int* limit,
                                              int* accl, long long* pend) {
   constexpr unsigned char SKIP = 0, REJECT = 1, ACCEPT = 2, OPEN = 3;
+  extern __shared__ float4 rec[];  // the slots' float records, 16-byte chunks swizzled
   __shared__ int lst[MAXB];
   __shared__ double sdp[PREF][7];  // dp of the walked slots, and -log(u) of the open ones
   __shared__ int2 wsum[32];
@@ -778,17 +781,22 @@ __global__ void __launch_bounds__(MB) k_metro(const long long* win, const unsign
   const unsigned long long seed = st->seed;
   float q[3];
   for (int k = 0; k < 3; ++k) q[k] = st->sq[k];
-  // this thread's slots' float records (two 16-byte loads each; the
-  // eligibility flag 0 for slots past the window)
+  // The slots' float records go through shared memory: fetched in order (a
+  // thread's four records apart, every load instruction would touch 32 cache
+  // lines), then each thread takes its consecutive slots' (the eligibility
+  // flag 0 for slots past the window).  Chunk c lies at c ^ ((c >> 3) & 7), so
+  // that reads 128 bytes apart fall on different banks.
+  auto chunk = [&](int c) -> float4& { return rec[c ^ ((c >> 3) & 7)]; };
+  for (int c = tid; c < 2 * W; c += MB) chunk(c) = reinterpret_cast<const float4*>(dpf)[c];
+  __syncthreads();
   float4 fa[MS], fb[MS];
   for (int k = 0; k < MS; ++k) {
     const int s = tid * MS + k;
     fa[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     fb[k] = fa[k];
     if (s < W) {
-      const float4* r = reinterpret_cast<const float4*>(dpf + 8 * (size_t)s);
-      fa[k] = r[0];
-      fb[k] = r[1];
+      fa[k] = chunk(2 * s);
+      fb[k] = chunk(2 * s + 1);
     }
   }
   // window-wide bound of the state's movement: sum of |dp|/ref of the
@@ -1095,24 +1103,25 @@ static int flip_sweep(tm_mesh* m, tm_energy* e, const double* P, double ratio, u
   // (W = 0: every kernel returns at once).  A group's 40 launches do not
   // depend on the sweep (the seed is in the device state), so they are
   // captured once as a CUDA graph per launch key and replayed.
+  TM_CUDA(cudaFuncSetAttribute(k_metro, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)METRO_SMEM));
   const int B = batch;
   constexpr int GROUP = 8;
   // claim + winner as one cooperative launch when all its blocks fit on the
   // GPU at once (else, or when the launch is refused, two kernels)
-  const int ncw = nblk(4L * B, 64);
+  const int ncw = nblk(4L * B, CWT);
   if (e->flip_coop == 0) {
     int per_sm = 0, nsm = 0, dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_claim_win, 64, 0);
-    e->flip_coop = per_sm * nsm >= (MAXB * 4 + 63) / 64 ? 1 : -1;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_claim_win, CWT, 0);
+    e->flip_coop = per_sm * nsm >= (MAXB * 4 + CWT - 1) / CWT ? 1 : -1;
     cudaGetLastError();
   }
   auto claim_win = [&](bool coop) {
     if (coop) {
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3(ncw);
-      cfg.blockDim = dim3(64);
+      cfg.blockDim = dim3(CWT);
       cfg.stream = s;
       cudaLaunchAttribute attr[1];
       attr[0].id = cudaLaunchAttributeCooperative;
@@ -1124,9 +1133,9 @@ static int flip_sweep(tm_mesh* m, tm_energy* e, const double* P, double ratio, u
     } else {
       k_fill<<<nblk(B, 256), 256, 0, s>>>(B, pend.get(), st, win.get(), limit.get());
       TM_LAUNCH();
-      k_claim<<<ncw, 64, 0, s>>>(t, st, win.get(), owner.get());
+      k_claim<<<ncw, CWT, 0, s>>>(t, st, win.get(), owner.get());
       TM_LAUNCH();
-      k_winner<<<ncw, 64, 0, s>>>(t, st, mode, win.get(), owner.get(), winner.get(), limit.get());
+      k_winner<<<ncw, CWT, 0, s>>>(t, st, mode, win.get(), owner.get(), winner.get(), limit.get());
       TM_LAUNCH();
     }
   };
@@ -1139,7 +1148,7 @@ static int flip_sweep(tm_mesh* m, tm_energy* e, const double* P, double ratio, u
       // it and the two-row exclusion test
       launch_after(k_delta, B, 64, s, t, st, win.get(), winner.get(), limit.get(), P, ep, epd, X, nlv, dpn.get(),
                    dpf.get(), e->sctf.get());
-      launch_after(k_metro, 1, MB, s, win.get(), winner.get(), dpn.get(), dpf.get(), fe, fg, st, limit.get(),
+      launch_after_smem(k_metro, 1, MB, METRO_SMEM, s, win.get(), winner.get(), dpn.get(), dpf.get(), fe, fg, st, limit.get(),
                    accl.get(), pend.get());
       launch_after(k_commit, CB, 32, s, t, win.get(), accl.get(), st);
     }

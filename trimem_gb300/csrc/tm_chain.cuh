@@ -17,10 +17,11 @@ __device__ __forceinline__ void let_next_start() { cudaTriggerProgrammaticLaunch
 
 // launch with programmatic stream serialisation (see wait_previous)
 template <class... A, class... B>
-void launch_after(void (*k)(A...), int grid, int block, cudaStream_t s, B... args) {
+void launch_after_smem(void (*k)(A...), int grid, int block, size_t smem, cudaStream_t s, B... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -28,6 +29,10 @@ void launch_after(void (*k)(A...), int grid, int block, cudaStream_t s, B... arg
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   TM_CUDA(cudaLaunchKernelEx(&cfg, k, args...));
+}
+template <class... A, class... B>
+void launch_after(void (*k)(A...), int grid, int block, cudaStream_t s, B... args) {
+  launch_after_smem(k, grid, block, 0, s, args...);
 }
 
 }  // namespace tmg

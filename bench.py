@@ -719,12 +719,13 @@ def main():
     # inputs and outputs, including this implementation's face and edge
     # records), for comparison with the per-stage DRAM traffic
     # (double-word stencils: positions split into 32-byte hi/lo records and
-    # 12-byte floats first, then read as 32 bytes per vertex)
+    # 12-byte floats first, then read as 32 bytes per vertex; the repulsion's
+    # row lengths, potentials and gradients belong to the face kernel)
     stage_bytes = {
-        "k_face": 24 * V + 32 * V + 12 * V + 3 * 4 * F + 32 * V + 64 * F + 16 * F,
-        "k_edge": 16 * E + 32 * V + 64 * F + 32 * E + 16 * E,
-        "k_vertex": 4 * V + 16 * 2 * E + 16 * F + 16 * E + 8 * V + 16 * V,
-        "k_grad": 4 * V + 16 * 2 * E + 32 * V + 16 * V + 64 * F + 32 * E + 24 * V + 24 * V,
+        "k_face": 24 * V + 32 * V + 12 * V + 3 * 4 * F + 32 * V + 64 * F + 16 * F + 4 * V + 8 * V + 24 * V,
+        "k_edge": 16 * E + 32 * V + 32 * F + 16 * E + 16 * E,
+        "k_vertex": 4 * V + 16 * 2 * E + 16 * F + 16 * E + 8 * V + 8 * V,
+        "k_grad": 4 * V + 16 * 2 * E + 32 * V + 64 * F + 16 * E + 24 * V + 24 * V,
     }
     peaks = read_peaks()
     hbm = peaks.get("hbm_gbs")
@@ -820,7 +821,7 @@ def main():
                 sms.append(a.elapsed_time(b))
             s_ms = float(np.median(sms))
             # three message-passing rounds, each a (V x 128) @ (128 x 64) bf16
-            # product on the tensor cores (k_dense); the rest is gathers
+            # product on the tensor cores (k_layer); the rest is gathers
             dense_flop = 3 * 2 * V * 128 * 64
             bf16 = peaks.get("bf16_tflops")
             surrogate = {"force_ms_cold": round(s_ms, 5), "forces_per_s_cold": round(1e3 / s_ms, 1),
@@ -830,7 +831,7 @@ def main():
                          "dense_tflops_over_whole_force": round(dense_flop / (s_ms * 1e-3) / 1e12, 2),
                          "bf16_peak_tflops": bf16, "peak_source": "of measured" if bf16 else None,
                          "frac": round(dense_flop / (s_ms * 1e-3) / 1e12 / bf16, 5) if bf16 else None,
-                         "note": "tensor FLOP over the whole force time (a lower bound on k_dense's own rate); "
+                         "note": "tensor FLOP over the whole force time (a lower bound on k_layer's own rate); "
                                  "the force is bound by the gathers around the dense layers"}
     except Exception as exc:  # the headline line is printed either way
         surrogate = {"error": f"{type(exc).__name__}: {exc}"}
@@ -931,12 +932,11 @@ def main():
             except Exception as exc:
                 cb["chain_step"] = {"error": f"{type(exc).__name__}: {exc}"}
 
-    # this library's kernels per step: 8 per double-word evaluation (k_split_dw,
-    # k_face_dw, k_edge_dw, k_moved, k_rep_fast, k_rep_slow, k_vertex_dw,
-    # k_grad_dw) and 14 per cell-list rebuild (box 2, table 1, insert 1,
-    # counts 1, scan 3, starts 1, scatter 1, sort 1, near-row check / build /
-    # done 3); the displacement and L2-flush kernels are torch's
-    launches_per_step = 8 * EVALS_PER_STEP + 14
+    # this library's kernels per step: 5 per double-word evaluation (k_split_dw,
+    # k_face_dw and k_edge_dw with the repulsion, k_vertex_dw, k_grad_dw) and 6
+    # per cell-list rebuild (k_box, k_insert, k_alloc, k_scatter, k_rank,
+    # k_near); the displacement and L2-flush kernels are torch's
+    launches_per_step = 5 * EVALS_PER_STEP + 6
     line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
             "warmup": max(args.warmup, 3), "ms_per_step": ms_per_step, "higher_is_better": True,
             "scaling": "weak", "vs_baseline": None, "dtype": "f64", "data": "synthetic",

@@ -579,7 +579,7 @@ void tm_energy::to_host(double* dst, const double* src, size_t n) {
 }
 
 double* tm_energy::host_scalars() {
-  if (!pinned && cudaMallocHost(&pinned, 16 * sizeof(double)) != cudaSuccess) {
+  if (!pinned && cudaMallocHost(&pinned, sizeof(tmg::Globals) + 16 * sizeof(double)) != cudaSuccess) {
     cudaGetLastError();
     pinned = nullptr;
     fail(TM_ERR_NOMEM, "page-locked allocation failed");
@@ -607,9 +607,14 @@ static void check_params(const tm_params& p) {
   if (p.exclusion_level < 0 || p.exclusion_level > 2) fail(TM_ERR_ARG, "Unsupported exclusion level");
 }
 
-static void fetch_globals(tm_energy* e, tmg::Globals* g) {
-  TM_CUDA(cudaMemcpyAsync(g, e->glob.get(), sizeof(tmg::Globals), cudaMemcpyDeviceToHost, e->stream));
+// staged: through the handle's page-locked memory, which the driver would
+// otherwise do for a pageable destination (energy() of 642 vertices: 35 us, so
+// 33); not at creation, where allocating it would cost more
+static void fetch_globals(tm_energy* e, tmg::Globals* g, bool staged = true) {
+  void* h = staged ? (void*)e->host_scalars() : (void*)g;
+  TM_CUDA(cudaMemcpyAsync(h, e->glob.get(), sizeof(tmg::Globals), cudaMemcpyDeviceToHost, e->stream));
   TM_CUDA(cudaStreamSynchronize(e->stream));
+  if (staged) std::memcpy(g, h, sizeof(tmg::Globals));
 }
 
 static void eval_host(tm_energy* e, tm_mesh* m, bool grad, bool vprops) {
@@ -661,7 +666,7 @@ int tm_energy_create(tm_mesh* m, const tm_params* p, tm_energy** out) {
   tmg::energy_eval(e.get(), m, m->d_pts.get(), false, false, nullptr, e->stream);
   e->stencil = stencil;
   tmg::Globals g;
-  fetch_globals(e.get(), &g);
+  fetch_globals(e.get(), &g, false);
   for (int k = 0; k < 6; ++k) e->initial[k] = g.props[k];
   *out = e.release();
   TM_API_END

@@ -194,113 +194,71 @@ __device__ __forceinline__ RepTerm rep_term(const EP& ep, double l, d3 dv) {
   return r;
 }
 
-// The repulsion of vertex v by its RL lanes (1 or NEAR_HITS): each lane tests
-// every RL-th row entry (one coalesced load of the row instead of one
-// thread's serial walk).  Near rows: the accepted pairs go to the group's
-// slots in shared memory, one lane evaluates each, and they are added in the
-// reference's visiting order (the rows' own order depends on when they were
-// built).  Verlet rows keep their order between rebuilds: each lane sums its
-// own pairs, then a fixed shuffle tree.  Vertices that need the cell walk
-// are queued.
-struct RepSlots {
-  long long key[NEAR_HITS];
-  double s[NEAR_HITS];
+constexpr int SB = 256;  // threads per block of the split, face and edge kernels
+
+// The repulsion runs a block at a time in two steps: the threads test their
+// rows and set the accepted pairs aside in shared memory, then the block
+// evaluates those densely, and each vertex adds its terms in a fixed order.  A
+// term is about 200 FP64 instructions of 16 cycles an SM each, whatever part of a
+// warp takes them: with every thread evaluating its own pairs where it found
+// them, a sphere of 642 vertices with near rows and 1.5 accepted pairs a vertex
+// took 159 us an evaluation (so 35), one of 161,292 715 (260), a tube of
+// 7,566 vertices with Verlet rows and 1,220 active pairs 35.3 (32.9).
+constexpr int VL = 8;  // lanes per vertex, where several share one
+struct RepPair {
+  double a, x, y, z;  // squared distance and vector, then potential and gradient
 };
-template <bool GRAD, int RL>
-__device__ __forceinline__ void rep_vertex(const DwEval& q, int v, int sub, int near_mode, RepSlots* slots) {
+template <bool LANES>
+struct RepBlock {
+  RepPair pair[LANES ? SB : 1];   // one per thread (one lane per vertex: in pot and repg)
+  long long key[LANES ? SB : 1];  // near rows by VL lanes: NEAR_HITS per vertex
+  unsigned short list[SB];
+  int n[2];  // list lengths of a round and the next, zero at the start
+};
+static_assert(VL == NEAR_HITS, "one lane per accepted pair of a near row");
+// the n pairs named by list, dense
+template <bool GRAD>
+__device__ __forceinline__ void rep_dense(const EP& ep, RepBlock<true>& sh, int n) {
+  for (int i = threadIdx.x; i < n; i += SB) {
+    RepPair& c = sh.pair[sh.list[i]];
+    const RepTerm r = rep_term<GRAD>(ep, __dsqrt_rn(c.a), mk(c.x, c.y, c.z));
+    c = {r.pot, r.gx, r.gy, r.gz};
+  }
+  __syncthreads();
+}
+__device__ __forceinline__ void add_term(RepTerm& sum, const RepTerm& r) {
+  sum.pot += r.pot;
+  sum.gx += r.gx;
+  sum.gy += r.gy;
+  sum.gz += r.gz;
+}
+template <bool GRAD>
+__device__ __forceinline__ void store_rep(const DwEval& q, int v, const RepTerm& sum) {
+  q.pot[v] = sum.pot;
+  if (GRAD) st3(q.repg, v, 2.0 * mk(sum.gx, sum.gy, sum.gz));
+}
+
+// Vertex v by one thread without near rows: its candidate row (the others are
+// queued for the cell walk) or its Verlet row
+template <bool GRAD>
+__device__ __forceinline__ void rep_vertex(const DwEval& q, int v) {
   const NLView& nl = q.nl;
   const EP& ep = q.ep;
-  static_assert(RL == 1 || RL == NEAR_HITS, "one lane per accepted pair");
-  const unsigned gmask = ((1u << RL) - 1u) << (threadIdx.x & 31 & ~(RL - 1));
   const d3 p = ld3p(q.P, v);
   const PairTest pt = make_pair_test(nl, v, ep.rlc1, ep.rT);
   TableExclSlim x{q.t, nl.excl};
   RepTerm sum{0.0, 0.0, 0.0, 0.0};
-  auto add = [&](int, double l, d3 dv) {
-    const RepTerm r = rep_term<GRAD>(ep, l, dv);
-    sum.pot += r.pot;
-    sum.gx += r.gx;
-    sum.gy += r.gy;
-    sum.gz += r.gz;
-  };
-  if (nl.kind == 0 && !near_mode) {  // candidate rows or the cell walk
-    bool fast = false;
-    if (sub == 0) {
-      int co[3];
-      fast = in_build_cell(nl, v, p, co);
-      if (fast) {
-        visit_candidates(pt, nl, q.P, v, p, x, add);
-      } else {
-        q.slow[atomicAdd(q.nslow, 1)] = v;
-      }
-    }
-    if (!fast) return;
-  } else if (nl.kind == 0 && RL == 1) {
+  auto add = [&](int, double l, d3 dv) { add_term(sum, rep_term<GRAD>(ep, l, dv)); };
+  if (nl.kind == 0) {
     int co[3];
-    in_build_cell(nl, v, p, co);
-    if (!visit_near(pt, nl, q.P, v, p, near_mode, co, x, add)) {
+    if (!in_build_cell(nl, v, p, co)) {
       q.slow[atomicAdd(q.nslow, 1)] = v;
       return;
     }
-  } else if (nl.kind == 0) {
-    const int* row = nl.nent + (size_t)v * TM_NEAR_CAP;
-    const int n = nl.ncnt[v];
-    int co[3];
-    bool have_co = false;
-    int total = 0;
-    for (int e0 = 0; e0 < n; e0 += RL) {
-      const int e = e0 + sub;
-      bool acc = false;
-      long long key = 0;
-      double s = 0.0;
-      if (e < n) {
-        const int c = row[e], j = c & 0x7fffffff;
-        d3 pj;
-        if (!(near_mode == 1 && c < 0) && pair_within(pt, nl, q.P, p, j, &pj, &s)) {
-          if (!have_co) in_build_cell(nl, v, p, co);
-          have_co = true;
-          const int ox = nl.bcoord[3 * j] - co[0], oy = nl.bcoord[3 * j + 1] - co[1], oz = nl.bcoord[3 * j + 2] - co[2];
-          acc = ox >= -1 && ox <= 1 && oy >= -1 && oy <= 1 && oz >= -1 && oz <= 1 &&
-                !(near_mode == 2 && nl.excl > 0 && x(v, j));
-          key = ((long long)((ox + 1) * 9 + (oy + 1) * 3 + (oz + 1)) << 32) | (long long)j;
-        }
-      }
-      const unsigned b = __ballot_sync(gmask, acc);
-      const int pos = total + __popc(b & ((1u << (threadIdx.x & 31)) - 1u));
-      if (acc && pos < NEAR_HITS) {
-        slots->key[pos] = key;
-        slots->s[pos] = s;
-      }
-      total += __popc(b);
-    }
-    if (total > NEAR_HITS) {
-      if (sub == 0) q.slow[atomicAdd(q.nslow, 1)] = v;
-      return;
-    }
-    if (total > 0) {
-      __syncwarp(gmask);
-      RepTerm r{0.0, 0.0, 0.0, 0.0};
-      int rank = -1;
-      if (sub < total) {
-        const long long k = slots->key[sub];
-        rank = 0;
-        for (int o = 0; o < total; ++o) rank += slots->key[o] < k ? 1 : 0;
-        r = rep_term<GRAD>(ep, __dsqrt_rn(slots->s[sub]), exact_diff(p, ld3p(q.P, (int)(k & 0xffffffff))));
-      }
-      __syncwarp(gmask);
-      for (int h = 0; h < total; ++h) {
-        const int src = __ffs(__ballot_sync(gmask, rank == h)) - 1;
-        sum.pot += __shfl_sync(gmask, r.pot, src);
-        if (GRAD) {
-          sum.gx += __shfl_sync(gmask, r.gx, src);
-          sum.gy += __shfl_sync(gmask, r.gy, src);
-          sum.gz += __shfl_sync(gmask, r.gz, src);
-        }
-      }
-    }
+    visit_candidates(pt, nl, q.P, v, p, x, add);
   } else {
     const int lo = nl.vrow[v], hi = nl.vrow[v + 1];
-    for (int e = lo + sub; e < hi; e += RL) {
+    for (int e = lo; e < hi; ++e) {
       const int j = nl.vcol[e];
       d3 pj;
       double s;
@@ -309,24 +267,215 @@ __device__ __forceinline__ void rep_vertex(const DwEval& q, int v, int sub, int 
       if (!q.excl_fresh && nl.excl > 0 && x(v, j)) continue;
       add(j, __dsqrt_rn(s), exact_diff(p, pj));
     }
-    __syncwarp(gmask);
-    const unsigned any = __ballot_sync(gmask, sum.pot != 0.0);
-    if (RL > 1 && any) {  // (no FP64 shuffle tree where no lane has a pair)
-#pragma unroll
-      for (int o = RL / 2; o > 0; o >>= 1) {
-        sum.pot += __shfl_down_sync(gmask, sum.pot, o);
-        if (GRAD) {
-          sum.gx += __shfl_down_sync(gmask, sum.gx, o);
-          sum.gy += __shfl_down_sync(gmask, sum.gy, o);
-          sum.gz += __shfl_down_sync(gmask, sum.gz, o);
+  }
+  store_rep<GRAD>(q, v, sum);
+}
+
+// the cell-list pair of v (in cell co) and j, as visit_near takes it: its key
+// in the reference's visiting order, or -1
+__device__ __forceinline__ long long near_key(const NLView& nl, const int* co, int j) {
+  const int ox = nl.bcoord[3 * j] - co[0], oy = nl.bcoord[3 * j + 1] - co[1], oz = nl.bcoord[3 * j + 2] - co[2];
+  if (ox < -1 || ox > 1 || oy < -1 || oy > 1 || oz < -1 || oz > 1) return -1;
+  return ((long long)((ox + 1) * 9 + (oy + 1) * 3 + (oz + 1)) << 32) | (long long)j;
+}
+
+// Near rows by one thread per vertex (mode: see visit_near), the first accepted
+// pairs of all vertices in one round, then the second ones, and so on.  A pair is
+// set aside in its vertex's own result entries, not in shared memory, which would
+// take L1 from the faces' gathers.
+template <bool GRAD>
+__device__ __forceinline__ void rep_near_block(const DwEval& q, int mode, RepBlock<false>& sh) {
+  const NLView& nl = q.nl;
+  const EP& ep = q.ep;
+  const int v = blockIdx.x * SB + threadIdx.x;
+  long long key[NEAR_HITS];
+  double dist2[NEAR_HITS];
+  int hits = 0;
+  bool walk = false;
+  d3 p = mk(0, 0, 0);
+  if (v < q.t.nv) {
+    p = ld3p(q.P, v);
+    const PairTest pt = make_pair_test(nl, v, ep.rlc1, ep.rT);
+    TableExclSlim x{q.t, nl.excl};
+    int co[3];
+    in_build_cell(nl, v, p, co);
+    // four entries per load (a row starts on a 192-byte boundary)
+    const int4* row4 = reinterpret_cast<const int4*>(nl.nent + (size_t)v * TM_NEAR_CAP);
+    const int n = nl.ncnt[v];
+    int4 r4 = make_int4(0, 0, 0, 0);
+    for (int e = 0; e < n; ++e) {
+      if ((e & 3) == 0) r4 = row4[e >> 2];
+      const int c = r4.x, j = c & 0x7fffffff;
+      r4 = make_int4(r4.y, r4.z, r4.w, 0);
+      if (mode == 1 && c < 0) continue;
+      d3 pj;
+      double s;
+      if (!pair_within(pt, nl, q.P, p, j, &pj, &s)) continue;
+      const long long k = near_key(nl, co, j);
+      if (k < 0 || (mode == 2 && nl.excl > 0 && x(v, j))) continue;
+      if (hits == NEAR_HITS) {
+        walk = true;
+        break;
+      }
+      int h = hits++;
+      while (h > 0 && key[h - 1] > k) {
+        key[h] = key[h - 1];
+        dist2[h] = dist2[h - 1];
+        --h;
+      }
+      key[h] = k;
+      dist2[h] = s;
+    }
+    if (walk) {
+      hits = 0;
+      q.slow[atomicAdd(q.nslow, 1)] = v;
+    }
+  }
+  RepTerm sum{0.0, 0.0, 0.0, 0.0};
+  for (int r = 0; __syncthreads_or(r < hits); ++r) {
+    int& n = sh.n[r & 1];
+    if (r < hits) {
+      q.pot[v] = dist2[r];
+      st3(q.repg, v, exact_diff(p, ld3p(q.P, (int)(key[r] & 0xffffffff))));
+      sh.list[atomicAdd(&n, 1)] = (unsigned short)threadIdx.x;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += SB) {
+      const int u = blockIdx.x * SB + sh.list[i];
+      const RepTerm t = rep_term<GRAD>(ep, __dsqrt_rn(q.pot[u]), ld3p(q.repg, u));
+      q.pot[u] = t.pot;
+      if (GRAD) st3(q.repg, u, mk(t.gx, t.gy, t.gz));
+    }
+    __syncthreads();
+    if (r < hits) {
+      sum.pot += q.pot[v];
+      if (GRAD) {
+        const d3 g = ld3p(q.repg, v);
+        sum.gx += g.x;
+        sum.gy += g.y;
+        sum.gz += g.z;
+      }
+    }
+    if (threadIdx.x == 0) n = 0;  // for the round after the next
+  }
+  if (v < q.t.nv && !walk) store_rep<GRAD>(q, v, sum);
+}
+
+// Near rows by VL lanes per vertex
+template <bool GRAD>
+__device__ __forceinline__ void rep_near_lanes(const DwEval& q, int mode, RepBlock<true>& sh) {
+  const NLView& nl = q.nl;
+  const EP& ep = q.ep;
+  const int v = (blockIdx.x * SB + threadIdx.x) / VL, sub = threadIdx.x % VL, base = threadIdx.x & ~(VL - 1);
+  const bool act = v < q.t.nv;
+  const unsigned gmask = ((1u << VL) - 1u) << (threadIdx.x & 31 & ~(VL - 1));
+  int total = 0;
+  if (act) {
+    const d3 p = ld3p(q.P, v);
+    const PairTest pt = make_pair_test(nl, v, ep.rlc1, ep.rT);
+    TableExclSlim x{q.t, nl.excl};
+    const int* row = nl.nent + (size_t)v * TM_NEAR_CAP;
+    const int n = nl.ncnt[v];
+    int co[3];
+    in_build_cell(nl, v, p, co);
+    for (int e0 = 0; e0 < n; e0 += VL) {
+      const int e = e0 + sub;
+      long long key = -1;
+      double s = 0.0;
+      d3 pj = p;
+      if (e < n) {
+        const int c = row[e], j = c & 0x7fffffff;
+        if (!(mode == 1 && c < 0) && pair_within(pt, nl, q.P, p, j, &pj, &s)) {
+          key = near_key(nl, co, j);
+          if (mode == 2 && key >= 0 && nl.excl > 0 && x(v, j)) key = -1;
         }
+      }
+      const unsigned b = __ballot_sync(gmask, key >= 0);
+      const int pos = total + __popc(b & ((1u << (threadIdx.x & 31)) - 1u));
+      if (key >= 0 && pos < NEAR_HITS) {
+        const d3 dv = exact_diff(p, pj);
+        sh.key[base + pos] = key;
+        sh.pair[base + pos] = {s, dv.x, dv.y, dv.z};
+      }
+      total += __popc(b);
+    }
+    if (total > NEAR_HITS) {
+      if (sub == 0) q.slow[atomicAdd(q.nslow, 1)] = v;
+    } else if (sub < total) {
+      sh.list[atomicAdd(&sh.n[0], 1)] = (unsigned short)(base + sub);
+    }
+  }
+  if (__syncthreads_or(total > 0)) rep_dense<GRAD>(ep, sh, sh.n[0]);
+  if (!act || total > NEAR_HITS) return;
+  // in the order of the keys
+  int rank = -1;
+  if (sub < total) {
+    rank = 0;
+    for (int o = 0; o < total; ++o) rank += sh.key[base + o] < sh.key[base + sub] ? 1 : 0;
+  }
+  RepTerm sum{0.0, 0.0, 0.0, 0.0};
+  for (int h = 0; h < total; ++h) {
+    const int src = __ffs(__ballot_sync(gmask, rank == h)) - 1 - (threadIdx.x & 31 & ~(VL - 1));
+    const RepPair c = sh.pair[base + src];
+    add_term(sum, {c.a, c.x, c.y, c.z});
+  }
+  if (sub == 0) store_rep<GRAD>(q, v, sum);
+}
+
+// Verlet rows by VL lanes per vertex: a lane's first accepted pair is set aside,
+// further ones are evaluated where they are found; each lane adds its own in row
+// order, then a fixed shuffle tree
+template <bool GRAD>
+__device__ __forceinline__ void rep_verlet_lanes(const DwEval& q, RepBlock<true>& sh) {
+  const NLView& nl = q.nl;
+  const EP& ep = q.ep;
+  const int v = (blockIdx.x * SB + threadIdx.x) / VL, sub = threadIdx.x % VL;
+  const bool act = v < q.t.nv;
+  const unsigned gmask = ((1u << VL) - 1u) << (threadIdx.x & 31 & ~(VL - 1));
+  RepTerm more{0.0, 0.0, 0.0, 0.0};  // past the first
+  bool mine = false;
+  if (act) {
+    const d3 p = ld3p(q.P, v);
+    const PairTest pt = make_pair_test(nl, v, ep.rlc1, ep.rT);
+    TableExclSlim x{q.t, nl.excl};
+    const int lo = nl.vrow[v], hi = nl.vrow[v + 1];
+    for (int e = lo + sub; e < hi; e += VL) {
+      const int j = nl.vcol[e];
+      d3 pj;
+      double s;
+      if (!pair_within(pt, nl, q.P, p, j, &pj, &s)) continue;
+      // the rows leave out the pairs excluded when they were built
+      if (!q.excl_fresh && nl.excl > 0 && x(v, j)) continue;
+      const d3 dv = exact_diff(p, pj);
+      if (!mine) {
+        mine = true;
+        sh.pair[threadIdx.x] = {s, dv.x, dv.y, dv.z};
+        sh.list[atomicAdd(&sh.n[0], 1)] = (unsigned short)threadIdx.x;
+      } else {
+        add_term(more, rep_term<GRAD>(ep, __dsqrt_rn(s), dv));
       }
     }
   }
-  if (sub == 0) {
-    q.pot[v] = sum.pot;
-    if (GRAD) st3(q.repg, v, 2.0 * mk(sum.gx, sum.gy, sum.gz));
+  if (__syncthreads_or(mine)) rep_dense<GRAD>(ep, sh, sh.n[0]);
+  if (!act) return;
+  RepTerm sum{0.0, 0.0, 0.0, 0.0};
+  if (mine) {
+    const RepPair c = sh.pair[threadIdx.x];
+    sum = {c.a, c.x, c.y, c.z};
   }
+  if (__ballot_sync(gmask, mine)) {  // (no FP64 shuffle tree where no lane has a pair)
+    add_term(sum, more);
+#pragma unroll
+    for (int o = VL / 2; o > 0; o >>= 1) {
+      sum.pot += __shfl_down_sync(gmask, sum.pot, o);
+      if (GRAD) {
+        sum.gx += __shfl_down_sync(gmask, sum.gx, o);
+        sum.gy += __shfl_down_sync(gmask, sum.gy, o);
+        sum.gz += __shfl_down_sync(gmask, sum.gz, o);
+      }
+    }
+  }
+  if (sub == 0) store_rep<GRAD>(q, v, sum);
 }
 
 // ---- stage 3: edges, and the queued repulsion --------------------------------
@@ -704,7 +853,6 @@ __device__ __forceinline__ void grad_dw(const DwEval& q, int i, int sub, df gA, 
 // serialisation: it may start while the one before drains, fetches its
 // topology rows (which no evaluation writes) and only then waits.
 
-constexpr int SB = 256;  // threads per block of the split, face and edge kernels
 
 template <bool MOVE>
 __global__ void __launch_bounds__(SB) k_split_dw(const __grid_constant__ DwEval q, const __grid_constant__ DwMove mv) {
@@ -718,16 +866,31 @@ __global__ void __launch_bounds__(SB) k_split_dw(const __grid_constant__ DwEval 
   if (v == 0) *q.nslow = 0;
 }
 
-// blocks [0, nrep): repulsion, RL lanes per vertex; the others: faces
-template <bool GRAD, int RL>
+// blocks [0, nrep): repulsion, with LANES by VL lanes per vertex (near or Verlet
+// rows) or else by one; the others: faces
+template <bool GRAD, bool LANES>
 __global__ void __launch_bounds__(SB) k_face_dw(const __grid_constant__ DwEval q, int nrep) {
-  __shared__ RepSlots slots[RL > 1 ? SB / RL : 1];
+  __shared__ RepBlock<LANES> sh;
   let_next_start();
   if ((int)blockIdx.x < nrep) {
+    if (threadIdx.x < 2) sh.n[threadIdx.x] = 0;
+    __syncthreads();
     wait_previous();
-    const int nm = near_mode_of(q);
-    const int v = (blockIdx.x * SB + threadIdx.x) / RL;
-    if (v < q.t.nv) rep_vertex<GRAD, RL>(q, v, threadIdx.x % RL, nm, &slots[RL > 1 ? threadIdx.x / RL : 0]);
+    const int mode = near_mode_of(q);  // the same in every thread
+    const int v = (blockIdx.x * SB + threadIdx.x) / (LANES ? VL : 1);
+    if constexpr (LANES) {
+      if (mode != 0)
+        rep_near_lanes<GRAD>(q, mode, sh);
+      else if (q.nl.kind == 1)
+        rep_verlet_lanes<GRAD>(q, sh);
+      else if (v < q.t.nv && threadIdx.x % VL == 0)
+        rep_vertex<GRAD>(q, v);
+    } else {
+      if (mode != 0)
+        rep_near_block<GRAD>(q, mode, sh);
+      else if (v < q.t.nv)
+        rep_vertex<GRAD>(q, v);
+    }
     return;
   }
   const int f = (blockIdx.x - nrep) * SB + threadIdx.x;
@@ -890,15 +1053,16 @@ void energy_eval_df(tm_energy* e, tm_mesh* m, const double* P, bool want_grad, d
   else
     k_split_dw<false><<<nsb, SB, 0, s>>>(q, mv);
   TM_LAUNCH();
-  // Verlet rows that hold a few entries per vertex are shared by eight lanes
-  // (the tube of 7,566 vertices with 1,220 active pairs: 38.6 us per
-  // evaluation against 57.5); near rows and sparse rows, where almost every
-  // entry is skipped without a test, are walked by one (163,842 vertices:
-  // 85 us against 105).
-  const int RL = q.nl.kind == 1 && e->nl.vtotal >= 2LL * t.nv ? 8 : 1;
-  const int nrep = q.rep ? nblk((long)t.nv * RL, SB) : 0;
-  auto* kf = RL == 8 ? (want_grad ? k_face_dw<true, 8> : k_face_dw<false, 8>)
-                       : (want_grad ? k_face_dw<true, 1> : k_face_dw<false, 1>);
+  // Eight lanes share a vertex over Verlet rows that hold a few entries each
+  // (the tube of 7,566 vertices with 1,220 active pairs: 38.6 us per evaluation
+  // against 57.5 with one, before the pairs were set aside) and over near rows
+  // up to 8,000 vertices, where one lane per vertex leaves SMs idle; above, and
+  // over sparse Verlet rows, almost every entry is skipped without a test and
+  // one lane walks them (163,842 vertices: 85 us against 105).
+  const bool lanes8 = q.nl.kind == 1 ? e->nl.vtotal >= 2LL * t.nv : q.use_near && t.nv <= 8000;
+  const int nrep = q.rep ? nblk((long)t.nv * (lanes8 ? VL : 1), SB) : 0;
+  auto* kf = lanes8 ? (want_grad ? k_face_dw<true, true> : k_face_dw<false, true>)
+                    : (want_grad ? k_face_dw<true, false> : k_face_dw<false, false>);
   launch_after(kf, std::max(1, nrep + nblk(t.nf, SB)), SB, s, q, nrep);
   if (ev) TM_CUDA(cudaEventRecord(ev[1], s));
   const int nqueue = q.rep && q.nl.kind == 0 ? e->sm_count() : 0;

@@ -1,5 +1,5 @@
 """Double-word repulsion over Verlet rows with no, few and many accepted pairs
-per lane (two per lane are set aside for the block, further ones are evaluated
+per lane (one per lane is set aside for the block, further ones are evaluated
 where they are found), ragged last blocks, against the oracle (1e-10, the
 parity bar of the double-word stencils)."""
 import numpy as np

@@ -853,7 +853,6 @@ __device__ __forceinline__ void grad_dw(const DwEval& q, int i, int sub, df gA, 
 // serialisation: it may start while the one before drains, fetches its
 // topology rows (which no evaluation writes) and only then waits.
 
-
 template <bool MOVE>
 __global__ void __launch_bounds__(SB) k_split_dw(const __grid_constant__ DwEval q, const __grid_constant__ DwMove mv) {
   let_next_start();
@@ -1056,9 +1055,11 @@ void energy_eval_df(tm_energy* e, tm_mesh* m, const double* P, bool want_grad, d
   // Eight lanes share a vertex over Verlet rows that hold a few entries each
   // (the tube of 7,566 vertices with 1,220 active pairs: 38.6 us per evaluation
   // against 57.5 with one, before the pairs were set aside) and over near rows
-  // up to 8,000 vertices, where one lane per vertex leaves SMs idle; above, and
-  // over sparse Verlet rows, almost every entry is skipped without a test and
-  // one lane walks them (163,842 vertices: 85 us against 105).
+  // up to 8,000 vertices, where one lane per vertex leaves SMs idle (at 10,242
+  // vertices 54 us against 90 where pairs are accepted, but 30.2 against 28.6
+  // where none is, the usual case; at 5,762 the latter are equal, 26.4); above,
+  // and over sparse Verlet rows, almost every entry is skipped without a test
+  // and one lane walks them (163,842 vertices: 85 us against 105).
   const bool lanes8 = q.nl.kind == 1 ? e->nl.vtotal >= 2LL * t.nv : q.use_near && t.nv <= 8000;
   const int nrep = q.rep ? nblk((long)t.nv * (lanes8 ? VL : 1), SB) : 0;
   auto* kf = lanes8 ? (want_grad ? k_face_dw<true, true> : k_face_dw<false, true>)

@@ -12,13 +12,16 @@ namespace tmg {
 __device__ __forceinline__ df third() { return {3.333333433e-01f, -9.934107481e-09f}; }
 __device__ __forceinline__ df sixth() { return {1.666666716e-01f, -4.967053740e-09f}; }
 
-// 32 bytes of read-only data in one load instruction, 32-byte aligned: one
-// sector per lane instead of two 16-byte requests (volatile: stays below the
-// wait for the kernel that writes the data)
+// 32 bytes in one load instruction, 32-byte aligned: one sector per lane
+// instead of two 16-byte requests.  An ordinary load and not a read-only one
+// (.nc): in a chain of dependent launches the kernel that reads the data may
+// have started before the one that writes it ended, and read-only loads are
+// defined only for data that no one writes while the reading kernel runs.
 __device__ __forceinline__ void ld32(const float4* p, float4& a, float4& b) {
-  asm volatile("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+  asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
       : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
-      : "l"(p));
+      : "l"(p)
+      : "memory");
 }
 // 32 bytes in one store instruction (a whole sector), 32-byte aligned
 __device__ __forceinline__ void st32(float4* p, const float4& a, const float4& b) {
@@ -32,7 +35,7 @@ __device__ __forceinline__ void st32(float4* p, const float4& a, const float4& b
 // entries are the vertex stage's: hi and lo of kb c/a, so that a gradient's
 // gather of a neighbour's position brings its curvature weight along.
 struct PosDW {
-  const float4* __restrict__ p;
+  const float4* p;
   __device__ __forceinline__ df3 at(int v) const {
     float4 h, l;
     ld32(p + 2 * (size_t)v, h, l);

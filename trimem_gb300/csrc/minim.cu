@@ -81,14 +81,15 @@ __global__ void k_step(int n, double a, const double* __restrict__ x, const doub
 }
 
 struct Direction {
-  int n, stored, head, history, accept;
+  int n, stored, head, rows, accept;
+  size_t pitch;          // doubles from one row of S or Y to the next
   double gamma, amax;
   double *x, *g;         // iterate and its gradient
   double *xn;            // trial point: in, the accepted one (accept); out, the next
   const double* gn;      // gradient at the accepted trial point
-  const double *S, *Y;   // correction pairs, [history][n]
+  const double *S, *Y;   // correction pairs, [rows][pitch]
   double *d, *part, *out;
-  double rho[MAXHIST];
+  double rho[MAXHIST + 1];
 };
 
 // Two-loop recursion d = -H g, the slope g . d, the restart from steepest
@@ -134,8 +135,8 @@ __global__ void __launch_bounds__(DB, 2) k_direction(const __grid_constant__ Dir
     d[e] = -1.0 * g[i];
     if (E == 0) q.d[i] = d[e];
   });
-  auto pair = [&](int k) { return (q.head - 1 - k + q.history) % q.history; };
-  auto row = [&](int k) { return (size_t)pair(k) * n; };
+  auto pair = [&](int k) { return (q.head - 1 - k + q.rows) % q.rows; };
+  auto row = [&](int k) { return pair(k) * q.pitch; };
   const int nd = 2 * q.stored;
   auto dot_vec = [&](int k) { return k < q.stored ? q.S + row(k) : (k < nd ? q.Y + row(nd - 1 - k) : g); };
   auto add_vec = [&](int k) { return k < q.stored ? q.Y + row(k) : q.S + row(nd - 1 - k); };
@@ -289,14 +290,16 @@ extern "C" int tm_minimize_device(tm_energy* e, tm_mesh* m, double* d_x, int max
   cudaStream_t s = stream ? (cudaStream_t)stream : e->stream;
   const int n = 3 * m->nv;
   // work space of the handle, kept between calls: d, g, trial point and its
-  // gradient, the pairs, block partials and a ticket (rows on 16-byte
-  // boundaries)
-  const size_t row = ((size_t)n + 1) & ~(size_t)1;
-  const size_t need = (4 + 2 * (size_t)history) * row + 3 * DG + 2;
+  // gradient, the pairs, block partials and a ticket.  One pair more than the
+  // history: every trial's pair is written before its s . y is known, and a
+  // refused one must not have replaced the oldest that is still in use.
+  const int rows = history + 1;
+  const size_t row = ((size_t)n + 1) & ~(size_t)1;  // 16-byte boundaries
+  const size_t need = (4 + 2 * (size_t)rows) * row + 3 * DG + 2;
   e->mwork.ensure(need);
   double* d = e->mwork.get();
-  double *g = d + row, *xn = g + row, *gn = xn + row, *S = gn + row, *Y = S + history * row;
-  double* part = Y + history * row;
+  double *g = d + row, *xn = g + row, *gn = xn + row, *S = gn + row, *Y = S + rows * row;
+  double* part = Y + rows * row;
   unsigned int* ticket = reinterpret_cast<unsigned int*>(part + 3 * DG);
   TM_CUDA(cudaMemsetAsync(ticket, 0, sizeof(unsigned int), s));
   double* out = e->host_scalars();
@@ -314,7 +317,8 @@ extern "C" int tm_minimize_device(tm_energy* e, tm_mesh* m, double* d_x, int max
   double f = out[R_E];
   Direction q{};
   q.n = n;
-  q.history = history;
+  q.rows = rows;
+  q.pitch = row;
   q.gamma = 1.0;
   q.amax = out[R_AMAX];
   q.x = d_x;
@@ -348,7 +352,7 @@ extern "C" int tm_minimize_device(tm_energy* e, tm_mesh* m, double* d_x, int max
         TM_LAUNCH();
       }
       eval(xn, gn);
-      k_finish<true><<<grid, DB, 0, s>>>(n, d_x, g, xn, gn, S + q.head * (size_t)n, Y + q.head * (size_t)n, part,
+      k_finish<true><<<grid, DB, 0, s>>>(n, d_x, g, xn, gn, S + q.head * row, Y + q.head * row, part,
                                           ticket, energy_at, out);
       TM_LAUNCH();
       TM_CUDA(cudaStreamSynchronize(s));
@@ -375,7 +379,7 @@ extern "C" int tm_minimize_device(tm_energy* e, tm_mesh* m, double* d_x, int max
     if (sy > 1e-300) {
       q.rho[q.head] = 1.0 / sy;
       q.gamma = sy / out[R_YY];
-      q.head = (q.head + 1) % history;
+      q.head = (q.head + 1) % rows;
       q.stored = std::min(q.stored + 1, history);
     }
     if ((fprev - f) <= ftol * std::max({std::fabs(fprev), std::fabs(f), 1.0})) {

@@ -136,14 +136,16 @@ struct TableExcl {  // exclusion on the current topology tables
 };
 
 // Cell coordinate int((p - bmin) / rl) with C truncation
-// (src/nlists/cell_list.h:141), decided without the FP64 division unless
-// the quotient is within 1e-9 of an integer, where the exact quotient is used.
+// (src/nlists/cell_list.h:71-78,141), decided without the FP64 division unless
+// the quotient is within 1e-9 of an integer or above 1e6, where the exact
+// quotient is used: below, the product with the rounded reciprocal is off by
+// less than 4 units of 2^-53 |t|, 5e-10.
 __device__ __forceinline__ int cell_coord(double p, const NLGeom& G, int k) {
   double q = __dsub_rn(p, G.bmin[k]);
   double t = __dmul_rn(q, G.inv_rl[k]);
   double ti = trunc(t);
   double fr = fabs(t - ti);
-  if (fr > 1e-9 && fr < 1.0 - 1e-9 && fabs(t) < 1.0e9) return (int)ti;
+  if (fr > 1e-9 && fr < 1.0 - 1e-9 && fabs(t) < 1.0e6) return (int)ti;
   return (int)__ddiv_rn(q, G.rl[k]);
 }
 

@@ -985,7 +985,8 @@ EPD make_epd(const EP& ep) {
   std::frexp(ep.kb, &ex);
   ex = std::min(std::max(ex, -100), 100);
   epd.iks = (float)std::ldexp(1.0, -ex);
-  epd.kq = host_df(ep.kb != 0.0 ? std::ldexp(2.0 / 3.0, ex) / ep.kb : 0.0);
+  // (none where kb is zero as a float: kb rho, which it multiplies, is zero then)
+  epd.kq = host_df((float)ep.kb != 0.0f ? std::ldexp(2.0 / 3.0, ex) / ep.kb : 0.0);
   epd.a0 = host_df(ep.a0);
   epd.inv_a0 = host_df(1.0 / ep.a0);
   epd.inv_tdiv = host_df(1.0 / ep.tdiv);

@@ -53,7 +53,7 @@ struct PosDW {
 // double-word parameters (hi / lo from the host)
 struct EPD {
   df kb, kt, kr, a0, inv_a0, inv_tdiv, lc0, lc1, br1, br2;
-  df kq;      // 2 s / (3 kb) with s the power of two at kb, 0 without bending
+  df kq;      // 2 s / (3 kb) with s the power of two at kb, 0 where kb is 0 as a float
   float iks;  // 1 / s
 };
 __device__ __forceinline__ bool df_less(df a, df b) { return a.hi < b.hi || (a.hi == b.hi && a.lo < b.lo); }

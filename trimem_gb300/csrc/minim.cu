@@ -16,6 +16,7 @@
 #include <cmath>
 
 #include "tm_energy.cuh"
+#include "tm_grid.h"
 #include "tm_internal.h"
 
 using namespace tmg;
@@ -272,12 +273,15 @@ __global__ void __launch_bounds__(DB) k_finish(int n, const double* __restrict__
 
 inline int nblk(long n, int b) { return (int)((n + b - 1) / b); }
 
-// registers per thread for n elements (0: more than eight, in memory)
 using DirectionKernel = void (*)(const Direction);
-DirectionKernel direction_kernel(int n) {
-  const int e = nblk(n, DG * DB);
-  return e <= 1 ? k_direction<1> : e <= 2 ? k_direction<2> : e <= 4 ? k_direction<4> : e <= 8 ? k_direction<8>
-                                                                                              : k_direction<0>;
+DirectionKernel direction_kernel(int n, int blocks) {
+  switch (elements_held(n, (long long)blocks * DB)) {
+    case 1: return k_direction<1>;
+    case 2: return k_direction<2>;
+    case 4: return k_direction<4>;
+    case 8: return k_direction<8>;
+    default: return k_direction<0>;
+  }
 }
 
 }  // namespace
@@ -304,6 +308,7 @@ extern "C" int tm_minimize_device(tm_energy* e, tm_mesh* m, double* d_x, int max
   TM_CUDA(cudaMemsetAsync(ticket, 0, sizeof(unsigned int), s));
   double* out = e->host_scalars();
   const int grid = std::max(1, std::min(DG, nblk(n, DB)));
+  int dgrid = grid;  // of the direction: fewer where they cannot all be resident
   // energy and gradient at x, neighbour list refreshed first
   auto eval = [&](const double* x, double* gx) {
     nlist_make(&e->nl, m, e->prm, x, s);
@@ -334,7 +339,6 @@ extern "C" int tm_minimize_device(tm_energy* e, tm_mesh* m, double* d_x, int max
   for (; k < maxiter; ++k) {
     if (q.amax <= gtol) break;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(DB);
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
@@ -342,7 +346,12 @@ extern "C" int tm_minimize_device(tm_energy* e, tm_mesh* m, double* d_x, int max
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    TM_CUDA(cudaLaunchKernelEx(&cfg, direction_kernel(n), q));
+    TM_CUDA(launch_as_fits(dgrid, cudaErrorCooperativeLaunchTooLarge, [&](int blocks) {
+      cfg.gridDim = dim3(blocks);
+      const cudaError_t r = cudaLaunchKernelEx(&cfg, direction_kernel(n, blocks), q);
+      if (r == cudaErrorCooperativeLaunchTooLarge) cudaGetLastError();
+      return r;
+    }));
     q.accept = 0;  // x and g are the accepted ones again
     double a = 0.0, gd = 0.0, fn = 0.0;
     bool ok = false;

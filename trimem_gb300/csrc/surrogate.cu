@@ -646,13 +646,16 @@ void make_map(CUtensorMap* map, const void* ptr, uint64_t rows, uint64_t cols, u
   if (r != CUDA_SUCCESS) fail(TM_ERR_CUDA, "cuTensorMapEncodeTiled failed (" + std::to_string((int)r) + ")");
 }
 
+// a kernel's limit of dynamic shared memory belongs to the current device: set
+// for every handle at its creation, and on every call without one
+template <class K>
+void allow_smem(K* k, int bytes) {
+  TM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+}
+
 void dense_launch(const CUtensorMap& mh, const CUtensorMap& mm, const CUtensorMap& mw, const float* bias,
                   __nv_bfloat16* out, int M, int* status, cudaStream_t s, int wait_polls) {
-  static bool attr = false;
-  if (!attr) {
-    TM_CUDA(cudaFuncSetAttribute(k_dense, cudaFuncAttributeMaxDynamicSharedMemorySize, DENSE_SMEM));
-    attr = true;
-  }
+  allow_smem(k_dense, DENSE_SMEM);
   if (M > 0) k_dense<<<nblk(M, BM), BM, DENSE_SMEM, s>>>(mh, mm, mw, bias, out, M, status, wait_polls);
   TM_LAUNCH();
 }
@@ -660,11 +663,6 @@ void dense_launch(const CUtensorMap& mh, const CUtensorMap& mm, const CUtensorMa
 template <bool TRAIN>
 void layer_launch(const CUtensorMap& mh, const CUtensorMap& mw, const CUtensorMap& mout, const CUtensorMap& mm,
                   const LayerIn& in, cudaStream_t s) {
-  static bool attr = false;
-  if (!attr) {
-    TM_CUDA(cudaFuncSetAttribute(k_layer<TRAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, LAYER_SMEM));
-    attr = true;
-  }
   k_layer<TRAIN><<<nblk(in.M, BM), LT, LAYER_SMEM, s>>>(mh, mw, mout, mm, in);
   TM_LAUNCH();
 }
@@ -1304,7 +1302,7 @@ namespace {
 template <class K>
 int resident_blocks(K* k, int smem) {
   int per_sm = 0, nsm = 0, dev = 0;
-  if (smem > 48 * 1024) TM_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  if (smem > 48 * 1024) allow_smem(k, smem);
   TM_CUDA(cudaGetDevice(&dev));
   TM_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
   TM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, TB, smem));
@@ -1410,6 +1408,7 @@ int tm_surrogate_create(tm_mesh* m, const float* weights, int64_t n_weights, tm_
   if (!m || !weights || !out) fail(TM_ERR_ARG, "NULL argument");
   *out = nullptr;
   std::unique_ptr<tm_surrogate> sg(new tm_surrogate());
+  allow_smem(k_layer<false>, LAYER_SMEM);
   std::vector<__nv_bfloat16> wd;
   parse_blob(weights, n_weights, sg->hw, wd);
   int nv = m->nv;
@@ -1542,6 +1541,7 @@ int tm_surrogate_train_create(int64_t n_vertices, int32_t max_valence, const flo
   st->dm.ensure(NH);
   st->dF.ensure(3 * (size_t)nv);
   const int nb8 = nblk((long)nv * 8, TB), nb16 = nblk((long)nv * 16, TB);
+  allow_smem(k_layer<true>, LAYER_SMEM);
   st->nb_dense = std::min(resident_blocks(k_t_dense_back, DENSE_BACK_SMEM), nblk(nv, DT));
   st->nb_msg = std::min(resident_blocks(k_t_msg_back, 0), nb16);
   st->nb_out = std::min(resident_blocks(k_t_outback, 0), nb8);

@@ -32,6 +32,8 @@
 // 163,842 vertices, energy 1.9e-14).  A variant with all stages in one
 // cooperative kernel (grid barriers instead of launches) was slower at every
 // size: 32 us at 642 vertices, 40 at 10,242, 150 at 163,842.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <cmath>
 
@@ -238,6 +240,15 @@ __device__ __forceinline__ void store_rep(const DwEval& q, int v, const RepTerm&
   if (GRAD) st3(q.repg, v, 2.0 * mk(sum.gx, sum.gy, sum.gz));
 }
 
+// appends v to the queue of the cell walk (one atomic for the threads that do
+// so together; the order does not matter, each vertex is written by one warp)
+__device__ __forceinline__ void queue_vertex(const DwEval& q, int v) {
+  const cooperative_groups::coalesced_group g = cooperative_groups::coalesced_threads();
+  int at = 0;
+  if (g.thread_rank() == 0) at = atomicAdd(q.nslow, (int)g.size());
+  q.slow[g.shfl(at, 0) + g.thread_rank()] = v;
+}
+
 // Vertex v by one thread without near rows: its candidate row (the others are
 // queued for the cell walk) or its Verlet row
 template <bool GRAD>
@@ -252,7 +263,7 @@ __device__ __forceinline__ void rep_vertex(const DwEval& q, int v) {
   if (nl.kind == 0) {
     int co[3];
     if (!in_build_cell(nl, v, p, co)) {
-      q.slow[atomicAdd(q.nslow, 1)] = v;
+      queue_vertex(q, v);
       return;
     }
     visit_candidates(pt, nl, q.P, v, p, x, add);
@@ -328,7 +339,7 @@ __device__ __forceinline__ void rep_near_block(const DwEval& q, int mode, RepBlo
     }
     if (walk) {
       hits = 0;
-      q.slow[atomicAdd(q.nslow, 1)] = v;
+      queue_vertex(q, v);
     }
   }
   RepTerm sum{0.0, 0.0, 0.0, 0.0};
@@ -400,7 +411,7 @@ __device__ __forceinline__ void rep_near_lanes(const DwEval& q, int mode, RepBlo
       total += __popc(b);
     }
     if (total > NEAR_HITS) {
-      if (sub == 0) q.slow[atomicAdd(q.nslow, 1)] = v;
+      if (sub == 0) queue_vertex(q, v);
     } else if (sub < total) {
       sh.list[atomicAdd(&sh.n[0], 1)] = (unsigned short)(base + sub);
     }
@@ -551,12 +562,15 @@ __device__ __forceinline__ void edge_dw(const DwEval& q, int4 E, int e) {
   q.elt[e] = make_float4(lt.hi, lt.lo, val.hi, val.lo);
 }
 
-// One warp per queued vertex: lane l < 27 scans neighbour cell l (the
-// reference's x-outer / z-inner order), then the lanes' sums are combined by
-// a fixed shuffle tree, so the result does not depend on timing.
+// One warp per queued vertex: lane l < 27 looks up neighbour cell l (the
+// reference's x-outer / z-inner order), then all lanes take the cells' members
+// in that order, every 32nd each, so that the pair terms (about 200 FP64
+// instructions) are evaluated by as many lanes as there are pairs; the lanes'
+// sums are combined by a fixed shuffle tree, so the result does not depend on
+// timing.
 template <bool GRAD>
-__device__ __forceinline__ void rep_queue(const DwEval& q, int warp, int nwarps) {
-  const int n = *(volatile int*)q.nslow;
+__device__ __forceinline__ void rep_queue(const DwEval& q, int n, int warp, int nwarps) {
+  constexpr unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const NLView& nl = q.nl;
   const NLGeom& G = *nl.geom;
@@ -566,40 +580,43 @@ __device__ __forceinline__ void rep_queue(const DwEval& q, int warp, int nwarps)
     const d3 p = ld3p(q.P, v);
     const PairTest pt = make_pair_test(nl, v, q.ep.rlc1, q.ep.rT);
     RepTerm sum{0.0, 0.0, 0.0, 0.0};
+    auto add = [&](int, double l, d3 dv) { add_term(sum, rep_term<GRAD>(q.ep, l, dv)); };
     int co[3];
     in_build_cell(nl, v, p, co);
+    int st = 0, cnt = 0;
     if (lane < 27) {
       const int ii = co[0] + lane / 9 - 1, jj = co[1] + (lane / 3) % 3 - 1, kk = co[2] + lane % 3 - 1;
-      if (ii >= 0 && ii < G.shape[0] && jj >= 0 && jj < G.shape[1] && kk >= 0 && kk < G.shape[2]) {
-        const long long cid = ii * G.stride[0] + jj * G.stride[1] + kk * G.stride[2];
-        int st = 0;
-        const int cnt = cell_find(nl, cell_key(cid, 0), &st);
-        auto add = [&](int, double l, d3 dv) {
-          const RepTerm r = rep_term<GRAD>(q.ep, l, dv);
-          sum.pot += r.pot;
-          sum.gx += r.gx;
-          sum.gy += r.gy;
-          sum.gz += r.gz;
-        };
-        for (int c = 0; c < cnt; ++c) {
-          const int j = nl.cell_verts[st + c];
-          if (j != v) visit_pair(pt, nl, q.P, v, p, j, x, add);
-        }
+      if (ii >= 0 && ii < G.shape[0] && jj >= 0 && jj < G.shape[1] && kk >= 0 && kk < G.shape[2])
+        cnt = cell_find(nl, cell_key(ii * G.stride[0] + jj * G.stride[1] + kk * G.stride[2], 0), &st);
+    }
+    int end = cnt;  // members of the cells up to this lane's
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(FULL, end, o);
+      if (lane >= o) end += y;
+    }
+    const int total = __shfl_sync(FULL, end, 31), first = st + cnt - end;
+    for (int m = lane; m - lane < total; m += 32) {
+      int c = 0;  // the cell of member m: as many cells end at or before it
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+        if (__shfl_sync(FULL, end, c + o - 1) <= m) c += o;
+      const int at = __shfl_sync(FULL, first, c);
+      if (m < total) {
+        const int j = nl.cell_verts[at + m];
+        if (j != v) visit_pair(pt, nl, q.P, v, p, j, x, add);
       }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-      sum.pot += __shfl_down_sync(0xffffffffu, sum.pot, o);
+      sum.pot += __shfl_down_sync(FULL, sum.pot, o);
       if (GRAD) {
-        sum.gx += __shfl_down_sync(0xffffffffu, sum.gx, o);
-        sum.gy += __shfl_down_sync(0xffffffffu, sum.gy, o);
-        sum.gz += __shfl_down_sync(0xffffffffu, sum.gz, o);
+        sum.gx += __shfl_down_sync(FULL, sum.gx, o);
+        sum.gy += __shfl_down_sync(FULL, sum.gy, o);
+        sum.gz += __shfl_down_sync(FULL, sum.gz, o);
       }
     }
-    if (lane == 0) {
-      q.pot[v] = sum.pot;
-      if (GRAD) st3(q.repg, v, 2.0 * mk(sum.gx, sum.gy, sum.gz));
-    }
+    if (lane == 0) store_rep<GRAD>(q, v, sum);
   }
 }
 
@@ -903,20 +920,22 @@ __global__ void __launch_bounds__(SB) k_face_dw(const __grid_constant__ DwEval q
   if (f < q.t.nf) face_dw(q, a, b, c, f);
 }
 
-// blocks [0, nqueue): the queued repulsion, one warp per vertex
+// blocks [0, nqueue): the queued repulsion, one warp per vertex; the others:
+// edges.  Blocks [0, nwalk) share the queue, the edges' after their edges: once
+// a vertex has left its skin, or a near row has overflowed, it holds every
+// vertex of the mesh.  nwalk is the number of resident blocks (four per SM at
+// 62 registers), since blocks of a second wave would begin their walks when
+// those of the first have ended.
 template <bool GRAD>
-__global__ void __launch_bounds__(SB) k_edge_dw(const __grid_constant__ DwEval q, int nqueue) {
+__global__ void __launch_bounds__(SB) k_edge_dw(const __grid_constant__ DwEval q, int nqueue, int nwalk) {
   let_next_start();
-  if ((int)blockIdx.x < nqueue) {
-    wait_previous();
-    rep_queue<GRAD>(q, (blockIdx.x * SB + threadIdx.x) >> 5, nqueue * (SB / 32));
-    return;
-  }
   const int e = (blockIdx.x - nqueue) * SB + threadIdx.x;
   int4 E = make_int4(0, 0, -1, -1);
-  if (e < q.t.ne) E = __ldg(q.t.edge + e);
+  if (e >= 0 && e < q.t.ne) E = __ldg(q.t.edge + e);
   wait_previous();
-  if (e < q.t.ne) edge_dw(q, E, e);
+  const int n = nqueue ? *(volatile int*)q.nslow : 0;
+  if (e >= 0 && e < q.t.ne) edge_dw(q, E, e);
+  if ((int)blockIdx.x < nwalk) rep_queue<GRAD>(q, n, (blockIdx.x * SB + threadIdx.x) >> 5, nwalk * (SB / 32));
 }
 
 // The last block (atomic ticket) reduces the block partials in block order
@@ -1067,9 +1086,17 @@ void energy_eval_df(tm_energy* e, tm_mesh* m, const double* P, bool want_grad, d
                     : (want_grad ? k_face_dw<true, false> : k_face_dw<false, false>);
   launch_after(kf, std::max(1, nrep + nblk(t.nf, SB)), SB, s, q, nrep);
   if (ev) TM_CUDA(cudaEventRecord(ev[1], s));
+  // One block per SM for the queue alone: more cost evaluations without a queue
+  // (two per SM 0.6 us of 28.4 at 10,242 vertices).  Whole evaluations with
+  // every vertex queued, in us, of the separate kernel of 1,216 blocks that it
+  // once was / of 152 blocks with one lane per cell / now, at 642, 10,242,
+  // 46,242 and 163,842 vertices: one vertex past its skin (cut-off 0.8 l,
+  // exclusion 2) 43/27/27, 64/66/57, 125/134/107, 381/801/324; rows overflowing
+  // (2.2 l, exclusion 0) 96/61/37, 489/611/192, 1,930/-/466, 6,560/13,020/1,580.
   const int nqueue = q.rep && q.nl.kind == 0 ? e->sm_count() : 0;
-  launch_after(want_grad ? k_edge_dw<true> : k_edge_dw<false>, std::max(1, nqueue + nblk(t.ne, SB)), SB, s, q,
-               nqueue);
+  const int edge_grid = std::max(1, nqueue + nblk(t.ne, SB));
+  launch_after(want_grad ? k_edge_dw<true> : k_edge_dw<false>, edge_grid, SB, s, q, nqueue,
+               std::min(edge_grid, 4 * nqueue));
   if (ev) TM_CUDA(cudaEventRecord(ev[2], s));
   // Several lanes per vertex shorten the chain of one thread's walk over its
   // ring and fill more SMs, one lane per vertex issues fewer instructions.

@@ -268,11 +268,16 @@ __global__ void __launch_bounds__(BB) k_scatter(int nv, const int* vslot, const 
   const int s = vslot[v];
   if (s >= 0) members[T[s].start + vrank[v]] = v;
 }
-// rank of each vertex among its cell's members (ascending vertex id)
+// rank of each vertex among its cell's members (ascending vertex id).  early:
+// the next kernel may start at once, and otherwise when these blocks have ended.
+// Near rows that are rebuilt fill the GPU for long, and blocks that were placed
+// while others held most of the SMs stay stacked on the few that were free
+// (10,242 vertices, a rebuild with new rows: 130 us against 104; 163,842, one
+// lane a vertex: 1,370 against 998).
 __global__ void __launch_bounds__(BB) k_rank(int nv, const int* vslot, const CellEntry* T,
                                              const int* members, int* cell_verts,
-                                             int* vrank) {
-  let_next_start();
+                                             int* vrank, bool early) {
+  if (early) let_next_start();
   wait_previous();
   const int v = blockIdx.x * BB + threadIdx.x;
   if (v >= nv) return;
@@ -495,26 +500,27 @@ __global__ void __launch_bounds__(256) k_cand(int nv, NLView nl, const int* vcoo
 // table (the cells that meet the ball of radius rn), with a flag for pairs
 // excluded on the current topology.  A row longer than TM_NEAR_CAP marks the
 // rows unusable (flag[3]).
-// Eight lanes share a vertex: each looks up every eighth of the up to 343
+// With eight lanes a vertex (NLN) each looks up every eighth of the up to 343
 // cells around the ball (most are empty, so the time is the chain of hash
 // probes) and walks the rings of every eighth ring vertex for the exclusion
-// flags.  A row's order does not matter to its readers, which visit accepted
-// pairs by their cell and id; it is the same from run to run.  10,242
-// vertices: 290 us with one thread per vertex.
+// flags; one lane a vertex runs the chain but works out whole planes and lines
+// of cells to be too far at once.  A row's order does not matter to its
+// readers, which visit accepted pairs by their cell and id; it is the same from
+// run to run.
 constexpr int NB = 128;   // threads per block of k_near
-constexpr int NL8 = 8;    // lanes per vertex
-constexpr int NEAR_BLOCKS = 8 * 152;  // resident blocks, looping over the vertices
+constexpr int NEAR_BLOCKS = 8 * 152;  // resident blocks of eight lanes a vertex, looping over the vertices
+template <int NLN>
 __global__ void __launch_bounds__(NB) k_near(int nv, const double* __restrict__ P, NLView nl, Topo t, int excl,
                                              double rn, double rn2, int* flag, const int* dtopo, int* ncnt,
                                              int* nent, double* xb, const EP* eps) {
-  __shared__ int srow[NB / NL8][TM_NEAR_CAP + 1];
+  __shared__ int srow[NB / NLN][TM_NEAR_CAP + 1];  // (an odd pitch: no bank conflicts)
   let_next_start();
   wait_previous();
   if (flag[1] == 0) return;  // rows still valid
-  const int sub = threadIdx.x % NL8, lane = threadIdx.x & 31;
-  const unsigned gmask = ((1u << NL8) - 1u) << (lane & ~(NL8 - 1)), below = (1u << lane) - 1u;
-  int* row = srow[threadIdx.x / NL8];
-  for (int a = (blockIdx.x * NB + threadIdx.x) / NL8; a < nv; a += gridDim.x * (NB / NL8)) {
+  const int sub = threadIdx.x % NLN, lane = threadIdx.x & 31;
+  const unsigned gmask = ((1u << NLN) - 1u) << (lane & ~(NLN - 1)), below = (1u << lane) - 1u;
+  int* row = srow[threadIdx.x / NLN];
+  for (int a = (blockIdx.x * NB + threadIdx.x) / NLN; a < nv; a += gridDim.x * (NB / NLN)) {
     const int rep = rep_of(nl, a);
     if (rep < 0) {  // padding vertex of a batch
       if (sub == 0) ncnt[a] = 0;
@@ -542,34 +548,59 @@ __global__ void __launch_bounds__(NB) k_near(int nv, const double* __restrict__ 
       mg[k] = 1e-3f + 9.6e-7f * fabsf(u[k]);
     }
     const float rnf2 = (float)rn2 * 1.0001f;
-    const int ny = hi[1] - lo[1] + 1, nz = hi[2] - lo[2] + 1;
-    const int ncell = hi[0] >= lo[0] && ny > 0 && nz > 0 ? (hi[0] - lo[0] + 1) * ny * nz : 0;
+    // distance of the ball's centre from a plane of cells, cell c along axis k
+    auto away = [&](int k, int c) {
+      return fmaxf(fmaxf((float)c - u[k], u[k] - (float)(c + 1)) - mg[k], 0.0f) * rlf[k];
+    };
+    auto lookup = [&](int ii, int jj, int kk, int* st) {
+      return cell_lookup(nl, cell_key(ii * G.stride[0] + jj * G.stride[1] + kk * G.stride[2], rep), st);
+    };
+    auto near = [&](int b) {
+      const d3 pb = ld3(P, b);
+      const double ex = pa.x - pb.x, ey = pa.y - pb.y, ez = pa.z - pb.z;
+      return b != a && !(ex * ex + ey * ey + ez * ez >= rn2);
+    };
     int n = 0;
-    for (int c0 = 0; c0 < ncell; c0 += NL8) {
-      const int c = c0 + sub;
-      int cnt = 0, st = 0;
-      if (c < ncell) {
-        const int kk = lo[2] + c % nz, ij = c / nz;
-        const int jj = lo[1] + ij % ny, ii = lo[0] + ij / ny;
-        const float dx = fmaxf(fmaxf((float)ii - u[0], u[0] - (float)(ii + 1)) - mg[0], 0.0f) * rlf[0];
-        const float dy = fmaxf(fmaxf((float)jj - u[1], u[1] - (float)(jj + 1)) - mg[1], 0.0f) * rlf[1];
-        const float dz = fmaxf(fmaxf((float)kk - u[2], u[2] - (float)(kk + 1)) - mg[2], 0.0f) * rlf[2];
-        if (!(dx * dx + dy * dy + dz * dz > rnf2))
-          cnt = cell_lookup(nl, cell_key(ii * G.stride[0] + jj * G.stride[1] + kk * G.stride[2], rep), &st);
-      }
-      for (int q = 0; __any_sync(gmask, q < cnt); ++q) {
-        bool acc = false;
-        int b = a;
-        if (q < cnt) {
-          b = nl.cell_verts[st + q];
-          const d3 pb = ld3(P, b);
-          const double ex = pa.x - pb.x, ey = pa.y - pb.y, ez = pa.z - pb.z;
-          acc = b != a && !(ex * ex + ey * ey + ez * ez >= rn2);
+    if constexpr (NLN == 1) {
+      for (int ii = lo[0]; ii <= hi[0]; ++ii) {
+        const float dx = away(0, ii);
+        for (int jj = lo[1]; jj <= hi[1]; ++jj) {
+          const float dy = away(1, jj), gxy = dx * dx + dy * dy;
+          if (gxy > rnf2) continue;
+          for (int kk = lo[2]; kk <= hi[2]; ++kk) {
+            const float dz = away(2, kk);
+            if (gxy + dz * dz > rnf2) continue;
+            int st = 0;
+            const int cnt = lookup(ii, jj, kk, &st);
+            for (int q = 0; q < cnt; ++q) {
+              const int b = nl.cell_verts[st + q];
+              if (!near(b)) continue;
+              if (n < TM_NEAR_CAP) row[n] = b;
+              ++n;
+            }
+          }
         }
-        const unsigned bal = __ballot_sync(gmask, acc);
-        const int pos = n + __popc(bal & below);
-        if (acc && pos < TM_NEAR_CAP) row[pos] = b;
-        n += __popc(bal);
+      }
+    } else {
+      const int ny = hi[1] - lo[1] + 1, nz = hi[2] - lo[2] + 1;
+      const int ncell = hi[0] >= lo[0] && ny > 0 && nz > 0 ? (hi[0] - lo[0] + 1) * ny * nz : 0;
+      for (int c0 = 0; c0 < ncell; c0 += NLN) {
+        const int c = c0 + sub;
+        int cnt = 0, st = 0;
+        if (c < ncell) {
+          const int kk = lo[2] + c % nz, ij = c / nz;
+          const int jj = lo[1] + ij % ny, ii = lo[0] + ij / ny;
+          const float dx = away(0, ii), dy = away(1, jj), dz = away(2, kk);
+          if (!(dx * dx + dy * dy + dz * dz > rnf2)) cnt = lookup(ii, jj, kk, &st);
+        }
+        for (int q = 0; __any_sync(gmask, q < cnt); ++q) {
+          const int b = q < cnt ? nl.cell_verts[st + q] : a;
+          const bool acc = q < cnt && near(b);
+          const unsigned bal = __ballot_sync(gmask, acc);
+          const int pos = n + __popc(bal & below);
+          if (acc && pos < TM_NEAR_CAP) row[pos] = b;
+          n += __popc(bal);
+        }
       }
     }
     if (sub == 0 && n > TM_NEAR_CAP) atomicOr(&flag[3], 1);
@@ -583,9 +614,14 @@ __global__ void __launch_bounds__(NB) k_near(int nv, const double* __restrict__ 
       const int d = t.val[a];
       auto mark = [&](int w) {
         for (int e = 0; e < n; ++e)
-          if ((row[e] & 0x7fffffff) == w) atomicOr(&row[e], (int)0x80000000u);
+          if ((row[e] & 0x7fffffff) == w) {
+            if constexpr (NLN == 1)
+              row[e] |= (int)0x80000000u;
+            else
+              atomicOr(&row[e], (int)0x80000000u);
+          }
       };
-      for (int m = sub; m < d; m += NL8) {
+      for (int m = sub; m < d; m += NLN) {
         const int w = t.nbr[(size_t)m * t.nv + a];
         mark(w);
         if (level > 1) {
@@ -596,9 +632,12 @@ __global__ void __launch_bounds__(NB) k_near(int nv, const double* __restrict__ 
       __syncwarp(gmask);
     }
     int* out = nent + (size_t)a * TM_NEAR_CAP;
-    for (int e = sub; e < n; e += NL8) out[e] = row[e];
+    for (int e = sub; e < n; e += NLN) out[e] = row[e];
     if (sub == 0) ncnt[a] = n;
-    if (sub < 3) xb[3 * (size_t)a + sub] = pp[sub];
+    if constexpr (NLN == 1)
+      st3(xb, a, pa);
+    else if (sub < 3)
+      xb[3 * (size_t)a + sub] = pp[sub];
     __syncwarp(gmask);  // the row is reused
   }
   // the last block (it follows every block's reads of the flag): usable
@@ -739,7 +778,7 @@ static void build_cells(tm_nlist* nl, NLView& V, int nv, const double* P, const 
   launch_after(k_alloc, vb, BB, s, nv, nl->vslot.get(), nl->vrank.get(), nl->table.get(), cursor);
   launch_after(k_scatter, vb, BB, s, nv, nl->vslot.get(), nl->vrank.get(), nl->table.get(), nl->fill.get());
   launch_after(k_rank, vb, BB, s, nv, nl->vslot.get(), nl->table.get(), nl->fill.get(), nl->cell_verts.get(),
-               nl->vrank.get());
+               nl->vrank.get(), nblk(8L * nv, NB) <= NEAR_BLOCKS / 8);
   if (candidates && nv > 0) {
     // candidate rows for the queries of points that stay in their build cell
     nl->crow.ensure((size_t)nv + 1);
@@ -790,8 +829,14 @@ static void refresh_near(tm_nlist* nl, tm_mesh* m, NLView& V, const double* P, d
   const int nv = nl->nv;
   const double rn = 2.0 * lc1;
   int* flag = nl->nflag.get();
-  launch_after(k_near, std::min(NEAR_BLOCKS, nblk((long)nv * NL8, NB)), NB, s, nv, P, V, m->topo(), V.excl, rn,
-               rn * rn * (1.0 + 1e-12), flag, m->d_topo_ver.get(), nl->ncnt.get(), nl->nent.get(), nl->xb.get(), eps);
+  // A rebuild with new rows, us, of one / eight lanes a vertex at 10,242, 40,962,
+  // 51,842, 81,002 and 163,842 vertices: 0.8 l, exclusion 2: 292/105, 319/241,
+  // 325/277, 302/367, 510/677; 2.2 l, exclusion 0: 745/252, 843/672, 677/821,
+  // 893/1,242, 1,416/2,325
+  const bool eight = nv <= 45000;
+  launch_after(eight ? k_near<8> : k_near<1>, eight ? std::min(NEAR_BLOCKS, nblk(8L * nv, NB)) : nblk(nv, NB), NB, s, nv,
+               P, V, m->topo(), V.excl, rn, rn * rn * (1.0 + 1e-12), flag, m->d_topo_ver.get(), nl->ncnt.get(),
+               nl->nent.get(), nl->xb.get(), eps);
   V.nent = nl->nent.get();
   V.ncnt = nl->ncnt.get();
   V.nflag = flag;

@@ -543,7 +543,7 @@ void tm_energy::ensure(int nv_, int ne_, int nf_) {
   ne = ne_;
   nf = nf_;
   face.ensure(8 * (size_t)std::max(nf, 1));
-  edge.ensure(4 * (size_t)std::max(ne, 1));
+  edge.ensure(2 * (size_t)std::max(ne, 1));  // 16 bytes per edge in every stencil precision
   ebond.ensure(2 * (size_t)std::max(ne, 1));  // FP64 path: (l theta, bond value) per edge
   fav.ensure(2 * (size_t)std::max(nf, 1));    // FP64 path: (area, volume) per face
   rho.ensure(2 * (size_t)std::max(nv, 1));  // FP64 path: (kb rho, 2/3 kb rho^2) per vertex
@@ -552,6 +552,7 @@ void tm_energy::ensure(int nv_, int ne_, int nf_) {
   slow.ensure((size_t)std::max(nv, 1) + 1);  // repulsion slow list
   vprops.ensure(6 * (size_t)std::max(nv, 1));
   pos32.ensure(3 * (size_t)std::max(nv, 1));
+  posdw.ensure(2 * (size_t)std::max(nv, 1));
   int nb = std::max(1, (nv + tmg::VB - 1) / tmg::VB);
   partials.ensure(8 * (size_t)nb * 2);  // up to two lanes per vertex
   moved.ensure(nb);

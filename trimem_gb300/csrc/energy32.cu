@@ -336,8 +336,6 @@ void energy_eval32(tm_energy* e, tm_mesh* m, const double* P, bool want_grad, bo
   // FP32 records live in the FP64 buffers (they are smaller)
   Topo t = m->topo();
   EP ep = make_ep(e);
-  e->pos32.ensure(3 * nv);
-  e->posdw.ensure(2 * nv);
   float4* X = e->posdw.get();
   Split S{X};
   FaceF* fd = reinterpret_cast<FaceF*>(e->face.get());
@@ -385,8 +383,6 @@ void energy_eval32_local(tm_energy* e, tm_mesh* m, const double* P, double* d_gr
   EP ep = make_ep(e);
   ep.kb = 0.0;
   ep.kr = 0.0;
-  e->pos32.ensure(3 * nv);
-  e->posdw.ensure(2 * nv);
   float4* X = e->posdw.get();
   Split S{X};
   FaceF* fd = reinterpret_cast<FaceF*>(e->face.get());
@@ -439,8 +435,6 @@ void energy_eval_batch32(tm_energy* e, tm_mesh* m, const double* P, double* d_gr
   e->ensure(m->nv, m->ne, m->nf);
   size_t nv = std::max(m->nv, 1);
   Topo t = m->topo();
-  e->pos32.ensure(3 * nv);
-  e->posdw.ensure(2 * nv);
   FaceF* fd = reinterpret_cast<FaceF*>(e->face.get());
   EdgeF* ed = reinterpret_cast<EdgeF*>(e->edge.get());
   float* rho = reinterpret_cast<float*>(e->rho.get());

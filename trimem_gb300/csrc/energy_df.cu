@@ -1029,8 +1029,6 @@ void energy_eval_df(tm_energy* e, tm_mesh* m, const double* P, bool want_grad, d
                     const Leap* leap, cudaStream_t s, cudaEvent_t* ev) {
   e->ensure(m->nv, m->ne, m->nf);
   const size_t nv = std::max(m->nv, 1);
-  e->pos32.ensure(3 * nv);
-  e->posdw.ensure(2 * nv);
   DwEval q{};
   q.t = m->topo();
   q.P = P;

@@ -579,11 +579,11 @@ void tm_energy::to_host(double* dst, const double* src, size_t n) {
   TM_CUDA(cudaStreamSynchronize(stream));
 }
 
-double* tm_energy::host_scalars() {
+double* tm_energy::host_scalars(bool required) {
   if (!pinned && cudaMallocHost(&pinned, sizeof(tmg::Globals) + 16 * sizeof(double)) != cudaSuccess) {
     cudaGetLastError();
     pinned = nullptr;
-    fail(TM_ERR_NOMEM, "page-locked allocation failed");
+    if (required) fail(TM_ERR_NOMEM, "page-locked allocation failed");
   }
   return pinned;
 }
@@ -608,14 +608,15 @@ static void check_params(const tm_params& p) {
   if (p.exclusion_level < 0 || p.exclusion_level > 2) fail(TM_ERR_ARG, "Unsupported exclusion level");
 }
 
-// staged: through the handle's page-locked memory, which the driver would
-// otherwise do for a pageable destination (energy() of 642 vertices: 35 us, so
-// 33); not at creation, where allocating it would cost more
+// staged: through the handle's page-locked memory (where there is none, the
+// driver does so for a pageable destination: energy() of 642 vertices takes 35
+// us instead of 33); not at creation, where allocating it would cost more
 static void fetch_globals(tm_energy* e, tmg::Globals* g, bool staged = true) {
-  void* h = staged ? (void*)e->host_scalars() : (void*)g;
+  void* pinned = staged ? e->host_scalars(false) : nullptr;
+  void* h = pinned ? pinned : (void*)g;
   TM_CUDA(cudaMemcpyAsync(h, e->glob.get(), sizeof(tmg::Globals), cudaMemcpyDeviceToHost, e->stream));
   TM_CUDA(cudaStreamSynchronize(e->stream));
-  if (staged) std::memcpy(g, h, sizeof(tmg::Globals));
+  if (pinned) std::memcpy(g, pinned, sizeof(tmg::Globals));
 }
 
 static void eval_host(tm_energy* e, tm_mesh* m, bool grad, bool vprops) {

@@ -233,9 +233,10 @@ struct tm_energy {
   tmg::DevBuf<float> fw_dpf;
   tmg::DevBuf<double> mwork;  // minimisation workspace, kept between calls
   // a few page-locked doubles that kernels write for the host (one call at a
-  // time, like every other workspace of the handle)
+  // time, like every other workspace of the handle); NULL where they cannot be
+  // had and are not required
   double* pinned = nullptr;
-  double* host_scalars();
+  double* host_scalars(bool required = true);
   cudaStream_t stream = nullptr;
   // second stream: the repulsion pass runs there, concurrent with the
   // edge kernels, between a fork and a join event

@@ -376,7 +376,7 @@ def batch_leg(stream, n_per_level=16, levels=(3, 4, 5, 6), n_leapfrog=10, n_step
     upd_batch = n_steps * n_leapfrog * nvert / t_batch
     upd_seq = n_seq * n_leapfrog * nvert / t_seq
     return {"replicas": n_rep, "vertices": nvert, "sizes": "642/2562/10242/40962 vertices, 16 replicas each",
-            "size_classes": [{"vertices": [c[0], c[1]], "block_split_face_edge_grad": list(c[2:])} for c in tuning],
+            "size_classes": [{"vertices": [c[0], c[1]], "block_face_edge_grad": list(c[3:])} for c in tuning],
             "hmc": f"{n_steps} steps x {n_leapfrog} leapfrog, dt {dt:g}, graph replay, rebuild every step",
             "hmc_steps_per_s": round(n_steps / t_batch, 2),
             "vertex_updates_per_s": round(upd_batch, 1),

@@ -212,7 +212,9 @@ int tm_hmc_step_device(tm_energy* e, tm_mesh* m, double* d_x, double mass, doubl
  * backtracking line search; the cell list is rebuilt at every evaluation
  * like the reference's refresh = 1.  Stops when max |gradient| <= gtol, the
  * relative energy decrease of a step is <= ftol, no decrease is found, or
- * after maxiter iterations. */
+ * after maxiter iterations.  The handle keeps the workspace, (6 + 2 history)
+ * x 3 n_vertices doubles (102 MB at 163,842 vertices and history 10), for
+ * later minimisations until it is destroyed. */
 int tm_minimize_device(tm_energy* e, tm_mesh* m, double* d_x, int maxiter, int history, double gtol, double ftol,
                        int32_t* iterations, double* energy, void* stream);
 
@@ -308,8 +310,9 @@ int tm_batch_create(int n_rep, const double* const* points, const int64_t* n_poi
                     const int64_t* n_faces, const tm_params* params, tm_batch** out);
 int tm_batch_destroy(tm_batch* b);
 /* the size classes: their number, and per class (up to 8) six ints: first
- * and end vertex of its range, tuned block sizes of the split, face, edge
- * and gradient kernels */
+ * and end vertex of its range, block size of the split (one launch for all
+ * replicas, 256) and the tuned block sizes of the face, edge and gradient
+ * kernels */
 int tm_batch_tuning(tm_batch* b, int32_t* n_classes, int32_t* info);
 int tm_batch_layout(tm_batch* b, int64_t* n_total, int64_t* offsets);
 /* direction 0: device -> host_x, 1: host_x -> device; host_x is n_total x 3 */

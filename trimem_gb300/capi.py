@@ -411,8 +411,9 @@ class Batch:
         check(lib().tm_batch_update_repulsion(self.h))
 
     def tuning(self):
-        """Size classes: (first vertex, end vertex, block sizes of the split,
-        face, edge and gradient kernels) per class."""
+        """Size classes: (first vertex, end vertex, block size of the split
+        (one launch for all, 256), tuned block sizes of the face, edge and
+        gradient kernels) per class."""
         n = ctypes.c_int32()
         info = (ctypes.c_int32 * (6 * 8))()
         check(lib().tm_batch_tuning(self.h, ctypes.byref(n), info))

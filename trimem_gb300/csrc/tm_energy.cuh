@@ -128,13 +128,6 @@ struct TableExclSlim {
   }
 };
 
-struct TableExcl {  // exclusion on the current topology tables
-  const Topo& t;
-  int excl;
-  const NLView* nl = nullptr;  // per-replica levels of a batch, when given
-  __device__ bool operator()(int v, int j) const { return excluded(t, nl ? excl_of(*nl, v) : excl, v, j); }
-};
-
 // Cell coordinate int((p - bmin) / rl) with C truncation
 // (src/nlists/cell_list.h:71-78,141), decided without the FP64 division unless
 // the quotient is within 1e-9 of an integer or above 1e6, where the exact
@@ -327,13 +320,6 @@ __device__ __forceinline__ void for_each_neighbour_x(const NLView& nl, const dou
   } else {
     visit_verlet(pt, nl, P, v, p, is_excluded, fn);
   }
-}
-
-template <class F>
-__device__ __forceinline__ void for_each_neighbour(const NLView& nl, const Topo& t, const double* P, int v, d3 p,
-                                                   double dmax, double T, F&& fn) {
-  TableExcl x{t, nl.excl, &nl};
-  for_each_neighbour_x(nl, P, v, p, dmax, T, x, fn);
 }
 
 // ---- per-vertex properties + block reduction + device-side assembly -------

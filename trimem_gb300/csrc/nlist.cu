@@ -343,11 +343,23 @@ __global__ void k_verlet_sort(int nv, const int* vrow, int* vcol, double* vd, co
   }
 }
 
+// Exclusion of the pairs of a build: with both rings in registers up to 60,000
+// vertices (2,562 with exclusion 2 and 1.6 l: 419 us a Verlet build, 567 one
+// vertex at a time), one vertex at a time above, where the GPU is full and the
+// registers cost more (163,842: 1,262 and 1,264; exclusion 0 1,332 and 1,214;
+// the distance matrix 701 and 665)
+constexpr int SLIM_FROM = 60000;
+template <bool SLIM>
+__device__ __forceinline__ bool excluded_pair(const Topo& t, int excl, int a, int b) {
+  return SLIM ? TableExclSlim{t, excl}(a, b) : excluded(t, excl, a, b);
+}
+
 // Pairs of the build-time cell neighbourhood of vertex a:
 //   mode 0: Verlet build, all b != a, d <= rd        (both orders)
 //   mode 1: distance_matrix of the cell list, each pair once with
 //           (cid_b > cid_a) or (same cell and b > a), d <= rd
 // pass 0 counts, pass 1 writes (d, i, j) at row offsets.
+template <bool SLIM>
 __global__ void k_cell_pairs(int nv, const double* P, NLView nl, Topo t, const int* vcoord, const long long* vcid,
                              double rd, int mode, int pass, int* cnt, const int* off, double* od, int* oi, int* oj) {
   int a = blockIdx.x * blockDim.x + threadIdx.x;
@@ -376,7 +388,7 @@ __global__ void k_cell_pairs(int nv, const double* P, NLView nl, Topo t, const i
           if (mode == 1 && cid == ca && b < a) continue;
           double dd = exact_dist(pa, ld3(P, b));
           if (!(dd <= rd)) continue;
-          if (excluded(t, nl.excl, a, b)) continue;
+          if (excluded_pair<SLIM>(t, nl.excl, a, b)) continue;
           if (pass) {
             od[base + n] = dd;
             if (mode == 0) {
@@ -400,6 +412,7 @@ __global__ void k_cell_pairs(int nv, const double* P, NLView nl, Topo t, const i
 // cut-off rlist[rep], not excluded at that replica's level; padding
 // vertices have empty rows.  pass 0 counts, pass 1 writes (then ordered by
 // k_verlet_sort like the single-mesh rows).
+template <bool SLIM>
 __global__ void k_verlet_batch(int nv, const double* P, NLView nl, Topo t, const int* vcoord,
                                const double* __restrict__ rlist, int pass, int* cnt, const int* off, double* od,
                                int* oj) {
@@ -433,7 +446,7 @@ __global__ void k_verlet_batch(int nv, const double* P, NLView nl, Topo t, const
           if (b == a) continue;
           double dd = exact_dist(pa, ld3(P, b));
           if (!(dd <= rd)) continue;
-          if (excluded(t, excl, a, b)) continue;
+          if (excluded_pair<SLIM>(t, excl, a, b)) continue;
           if (pass) {
             od[base + n] = dd;
             oj[base + n] = b;
@@ -870,16 +883,17 @@ void nlist_make(tm_nlist* nl, tm_mesh* m, const tm_params& p, const double* P, c
     int total = 0;
     if (nv > 0) {
       nl->cnt.ensure((size_t)nv + 1);
-      k_cell_pairs<<<nblk(nv, 256), 256, 0, s>>>(nv, P, V, t, nl->vcoord.get(), nl->vcid.get(), p.rlist, 0, 0,
-                                                 nl->cnt.get(), nullptr, nullptr, nullptr, nullptr);
+      auto* pairs = nv > SLIM_FROM ? k_cell_pairs<true> : k_cell_pairs<false>;
+      pairs<<<nblk(nv, 256), 256, 0, s>>>(nv, P, V, t, nl->vcoord.get(), nl->vcid.get(), p.rlist, 0, 0, nl->cnt.get(),
+                                          nullptr, nullptr, nullptr, nullptr);
       TM_LAUNCH();
       TM_CUDA(cudaMemsetAsync(nl->cnt.get() + nv, 0, sizeof(int), s));
       exclusive_scan_int(nl->cnt.get(), nl->vrow.get(), nv + 1, &total, nl->tmp, s);
       nl->vcol.ensure(std::max(total, 1));
       nl->vtotal = total;
       nl->d_res.ensure(std::max(total, 1));
-      k_cell_pairs<<<nblk(nv, 256), 256, 0, s>>>(nv, P, V, t, nl->vcoord.get(), nl->vcid.get(), p.rlist, 0, 1,
-                                                 nullptr, nl->vrow.get(), nl->d_res.get(), nullptr, nl->vcol.get());
+      pairs<<<nblk(nv, 256), 256, 0, s>>>(nv, P, V, t, nl->vcoord.get(), nl->vcid.get(), p.rlist, 0, 1, nullptr,
+                                          nl->vrow.get(), nl->d_res.get(), nullptr, nl->vcol.get());
       TM_LAUNCH();
       k_verlet_sort<<<nblk(nv, 128), 128, 0, s>>>(nv, nl->vrow.get(), nl->vcol.get(), nl->d_res.get(),
                                                   nl->vcid.get(), nl->vcoord.get(), nl->vrank.get());
@@ -920,16 +934,17 @@ void nlist_make_batch(tm_nlist* nl, tm_mesh* m, int R, const int* d_vrep, const 
     int total = 0;
     if (nv > 0) {
       nl->cnt.ensure((size_t)nv + 1);
-      k_verlet_batch<<<nblk(nv, 256), 256, 0, s>>>(nv, P, V, t, nl->vcoord.get(), d_rlist, 0, nl->cnt.get(),
-                                                   nullptr, nullptr, nullptr);
+      auto* rows = nv > SLIM_FROM ? k_verlet_batch<true> : k_verlet_batch<false>;
+      rows<<<nblk(nv, 256), 256, 0, s>>>(nv, P, V, t, nl->vcoord.get(), d_rlist, 0, nl->cnt.get(), nullptr, nullptr,
+                                         nullptr);
       TM_LAUNCH();
       TM_CUDA(cudaMemsetAsync(nl->cnt.get() + nv, 0, sizeof(int), s));
       exclusive_scan_int(nl->cnt.get(), nl->vrow.get(), nv + 1, &total, nl->tmp, s);
       nl->vcol.ensure(std::max(total, 1));
       nl->vtotal = total;
       nl->d_res.ensure(std::max(total, 1));
-      k_verlet_batch<<<nblk(nv, 256), 256, 0, s>>>(nv, P, V, t, nl->vcoord.get(), d_rlist, 1, nullptr,
-                                                   nl->vrow.get(), nl->d_res.get(), nl->vcol.get());
+      rows<<<nblk(nv, 256), 256, 0, s>>>(nv, P, V, t, nl->vcoord.get(), d_rlist, 1, nullptr, nl->vrow.get(),
+                                         nl->d_res.get(), nl->vcol.get());
       TM_LAUNCH();
       k_verlet_sort<<<nblk(nv, 128), 128, 0, s>>>(nv, nl->vrow.get(), nl->vcol.get(), nl->d_res.get(),
                                                   nl->vcid.get(), nl->vcoord.get(), nl->vrank.get());
@@ -965,9 +980,10 @@ int64_t nlist_distance_matrix(tm_nlist* nl, tm_mesh* m, const double* P, double 
   nl->fill.ensure((size_t)nv + 1);
   Topo t = m->topo();
   int total = 0;
+  auto* pairs = nv > SLIM_FROM ? k_cell_pairs<true> : k_cell_pairs<false>;
   if (nl->view.kind == 0)
-    k_cell_pairs<<<nblk(nv, 256), 256, 0, s>>>(nv, P, nl->view, t, nl->vcoord.get(), nl->vcid.get(), rd, 1, 0,
-                                               nl->cnt.get(), nullptr, nullptr, nullptr, nullptr);
+    pairs<<<nblk(nv, 256), 256, 0, s>>>(nv, P, nl->view, t, nl->vcoord.get(), nl->vcid.get(), rd, 1, 0, nl->cnt.get(),
+                                        nullptr, nullptr, nullptr, nullptr);
   else
     k_verlet_dm<<<nblk(nv, 256), 256, 0, s>>>(nv, P, nl->vrow.get(), nl->vcol.get(), rd, 0, nl->cnt.get(), nullptr,
                                               nullptr, nullptr, nullptr);
@@ -978,9 +994,8 @@ int64_t nlist_distance_matrix(tm_nlist* nl, tm_mesh* m, const double* P, double 
   nl->d_resi.ensure(std::max(total, 1));
   nl->d_resj.ensure(std::max(total, 1));
   if (nl->view.kind == 0)
-    k_cell_pairs<<<nblk(nv, 256), 256, 0, s>>>(nv, P, nl->view, t, nl->vcoord.get(), nl->vcid.get(), rd, 1, 1,
-                                               nullptr, nl->fill.get(), nl->d_res.get(), nl->d_resi.get(),
-                                               nl->d_resj.get());
+    pairs<<<nblk(nv, 256), 256, 0, s>>>(nv, P, nl->view, t, nl->vcoord.get(), nl->vcid.get(), rd, 1, 1, nullptr,
+                                        nl->fill.get(), nl->d_res.get(), nl->d_resi.get(), nl->d_resj.get());
   else
     k_verlet_dm<<<nblk(nv, 256), 256, 0, s>>>(nv, P, nl->vrow.get(), nl->vcol.get(), rd, 1, nullptr, nl->fill.get(),
                                               nl->d_res.get(), nl->d_resi.get(), nl->d_resj.get());

@@ -115,6 +115,7 @@ struct TableExclSlim {
   const Topo& t;
   int excl;
   __device__ bool operator()(int v, int j) const {
+    if (excl <= 0) return false;
     const int d = t.val[v], dj = excl > 1 ? t.val[j] : 0;
 #pragma unroll 1
     for (int m = 0; m < d; ++m) {

@@ -477,19 +477,23 @@ __global__ void __launch_bounds__(256) k_cand(int nv, NLView nl, const int* vcoo
   }
   const NLGeom& G = nl.geom[rep];
   const int ci = vcoord[3 * a], cj = vcoord[3 * a + 1], ck = vcoord[3 * a + 2];
-  const long long home = ci * G.stride[0] + cj * G.stride[1] + ck * G.stride[2];
+  // The vertex itself is in the cell with its own id: the middle one, or, for a
+  // vertex on the upper face of a box so wide that the margin of its sides is
+  // lost in rounding, the one that the id past the side wraps to
+  const bool inside = ci >= 0 && ci < G.shape[0] && cj >= 0 && cj < G.shape[1] && ck >= 0 && ck < G.shape[2];
+  const long long home = inside ? 0 : ci * G.stride[0] + cj * G.stride[1] + ck * G.stride[2];
   int n = pass ? off[a] : 0;
   for (int c0 = 0; c0 < 27; c0 += L) {
     const int c = c0 + sub;
     const int ii = ci + c / 9 - 1, jj = cj + (c / 3) % 3 - 1, kk = ck + c % 3 - 1;
     int st = 0, m = 0;
-    const long long id = ii * G.stride[0] + jj * G.stride[1] + kk * G.stride[2];
-    if (c < 27 && ii >= 0 && ii < G.shape[0] && jj >= 0 && jj < G.shape[1] && kk >= 0 && kk < G.shape[2])
+    bool self = false;
+    if (c < 27 && ii >= 0 && ii < G.shape[0] && jj >= 0 && jj < G.shape[1] && kk >= 0 && kk < G.shape[2]) {
+      const long long id = ii * G.stride[0] + jj * G.stride[1] + kk * G.stride[2];
       m = cell_lookup(nl, cell_key(id, rep), &st);
-    // the vertex itself is in the cell with its own id: the middle one, or, for
-    // a vertex on the upper face of a box so wide that the margin of its sides
-    // is lost in rounding, the one that the id past the side wraps to
-    const int own = m - (id == home && m > 0 ? 1 : 0);
+      self = inside ? c == 13 : id == home;
+    }
+    const int own = m - (self && m > 0 ? 1 : 0);
     int incl = own;
 #pragma unroll
     for (int o = 1; o < L; o <<= 1) {

@@ -23,23 +23,29 @@ namespace tmg {
 namespace {
 
 // Exclusion on the current topology, at the vertex's own level.  The test holds
-// 16 ring entries in registers, which slows the walk of rows that hardly ever
-// make it: with a gradient it is a call, for the energy alone one vertex at a
-// time (163,842 vertices, cut-off 1.6 l, FP32 stencils, us an evaluation with
-// the test inline / so: gradient 350 / 313, energy 269 / 227; 2,562 vertices
-// after flips, every pair tested: 45 both ways).
+// 16 ring entries in registers, which pays where every pair is tested (after
+// flips, Verlet and candidate rows) and slows the walk of rows that hardly ever
+// make it.  As a call it costs neither, except that the energy alone, whose walk
+// is shorter, needs 78 registers with it: on large meshes, where that costs
+// occupancy, it tests one vertex at a time.  us an evaluation with FP32 stencils
+// inline / as a call / one vertex at a time, cut-off 1.6 l: gradient of 163,842
+// vertices 350 / 313 / 317, energy of 163,842 269 / 256 / 227, of 40,962 129 /
+// 109 / 111, of 2,562 91 / 83 / 82; this kernel after flips at 2,562, energy
+// alone: 21 inline, 33 one vertex at a time.
 struct TableExcl {
   const Topo& t;
   const NLView& nl;
   __device__ bool operator()(int v, int j) const { return excluded(t, excl_of(nl, v), v, j); }
 };
 __device__ __noinline__ bool excluded_call(const Topo& t, int excl, int v, int j) { return excluded(t, excl, v, j); }
-template <bool GRAD>
+constexpr int SLIM_FROM = 50000;
+template <bool SLIM>
 struct RowExcl {
   const Topo& t;
   const NLView& nl;
   __device__ bool operator()(int v, int j) const {
-    return GRAD ? excluded_call(t, excl_of(nl, v), v, j) : TableExclSlim{t, excl_of(nl, v)}(v, j);
+    const int excl = excl_of(nl, v);
+    return SLIM ? TableExclSlim{t, excl}(v, j) : excluded_call(t, excl, v, j);
   }
 };
 
@@ -62,11 +68,11 @@ struct RepAcc {
   }
 };
 
-template <bool GRAD>
-__global__ void __launch_bounds__(256) k_rep_fast(const __grid_constant__ Topo t, const double* __restrict__ P, NLView nl, EP ep,
-                                                 double* __restrict__ pot, double* __restrict__ repg,
-                                                 int* __restrict__ slow, int* __restrict__ nslow,
-                                                 const EP* __restrict__ eps, int use_near) {
+template <bool GRAD, bool SLIM>
+__global__ void __launch_bounds__(256) k_rep_fast(const __grid_constant__ Topo t, const double* __restrict__ P,
+                                                  NLView nl, EP ep, double* __restrict__ pot,
+                                                  double* __restrict__ repg, int* __restrict__ slow,
+                                                  int* __restrict__ nslow, const EP* __restrict__ eps, int use_near) {
   int v = blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= t.nv) return;
   if (nl.vrep) {  // batch: per-replica cut-off, padding vertices have none
@@ -85,7 +91,7 @@ __global__ void __launch_bounds__(256) k_rep_fast(const __grid_constant__ Topo t
   d3 p = ld3(P, v);
   PairTest pt = make_pair_test(nl, v, ep.rlc1, ep.rT);
   RepAcc acc{ep.rlc1, ep.rr, 0.0, mk(0, 0, 0), GRAD};
-  RowExcl<GRAD> x{t, nl};
+  RowExcl<SLIM> x{t, nl};
   if (nl.kind == 0) {
     int co[3];
     bool fast = in_build_cell(nl, v, p, co);
@@ -193,10 +199,8 @@ void repulsion_eval(tm_energy* e, tm_mesh* m, const double* P, const float* pos3
     k_moved<<<nblk(nv, 256), 256, 0, s>>>(nv, P, e->nl.xb.get(), e->nl.near_move2, flag, nlv.vrep, eps);
     TM_LAUNCH();
   }
-  if (want_grad)
-    k_rep_fast<true><<<nblk(nv, 256), 256, 0, s>>>(t, P, nlv, ep, pot, repg, slow, nslow, eps, use_near);
-  else
-    k_rep_fast<false><<<nblk(nv, 256), 256, 0, s>>>(t, P, nlv, ep, pot, repg, slow, nslow, eps, use_near);
+  auto* fast = want_grad ? k_rep_fast<true, false> : (nv >= SLIM_FROM ? k_rep_fast<false, true> : k_rep_fast<false, false>);
+  fast<<<nblk(nv, 256), 256, 0, s>>>(t, P, nlv, ep, pot, repg, slow, nslow, eps, use_near);
   TM_LAUNCH();
   if (nlv.kind == 0) {
     int grid = 8 * 152;  // 8 warps per block, one warp per queued vertex (all of them when the near rows are stale)

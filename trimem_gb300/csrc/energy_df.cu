@@ -26,8 +26,8 @@
 // and gathers over the 1-ring, on small ones the kernels' latencies.  Against
 // the former chain of eight kernels on two streams (a graph replay, 64- and
 // 32-byte records gathered in 16-byte pieces, cross products per ring slot):
-// 113 to 85 us at 163,842 vertices (the gradient 41 to 25), 59 to 41 at
-// 40,962, 43 to 24 at 642, 85 to 37 for an open tube of 7,566 vertices with
+// 113 to 87 us at 163,842 vertices (the gradient 41 to 25), 53 to 37 at
+// 40,962, 43 to 23 at 642, 84 to 32 for an open tube of 7,566 vertices with
 // Verlet rows; the errors against 64 bits are the same (gradient 6.7e-13 at
 // 163,842 vertices, energy 1.9e-14).  A variant with all stages in one
 // cooperative kernel (grid barriers instead of launches) was slower at every

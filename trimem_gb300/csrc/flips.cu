@@ -1100,7 +1100,7 @@ static int flip_sweep(tm_mesh* m, tm_energy* e, const double* P, double ratio, u
   TM_LAUNCH();
   // windows are queued in groups without host round trips; W and the window
   // number live on the device, and a window after the last one is empty
-  // (W = 0: every kernel returns at once).  A group's 40 launches do not
+  // (W = 0: every kernel returns at once).  A group's 32 launches do not
   // depend on the sweep (the seed is in the device state), so they are
   // captured once as a CUDA graph per launch key and replayed.
   TM_CUDA(cudaFuncSetAttribute(k_metro, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)METRO_SMEM));

@@ -18,9 +18,9 @@
 //             in ascending order like the reference's
 //             std::map<int, std::vector<int>>
 // What bounds it is the chain's length: at 10,242 vertices a rebuild was 13
-// launches and 60 us, with passes over all table slots, a three-kernel scan
-// of them and one thread sorting a cell (a ten-iteration minimisation, eleven
-// rebuilds with two of the near rows: 5.55 ms then, 4.89 now).
+// launches and 75 us, with passes over all table slots, a three-kernel scan
+// of them and one thread sorting a cell, and is 28 now (with new near rows 340
+// then, 104 now); at 163,842 vertices 97 and 57 (554 and 511).
 // Queries bin the query point with its CURRENT position but look up the
 // cells' build-time members, as the reference does (cell_list.h:131-219).
 // Distances are rounded operation by operation (no FMA), so pair sets match

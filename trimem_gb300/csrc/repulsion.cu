@@ -7,12 +7,12 @@
 // decides this for the whole mesh before the pass) every vertex walks its
 // near row in k_rep_fast.  Otherwise a vertex whose current position still
 // lies in its build-time cell walks the precomputed candidate row of that
-// cell; the few that moved
-// to another cell are queued and walk the 27 cells through the cell table in
-// a second kernel (k_rep_slow), so the long table walk never holds a warp of
-// fast vertices.  Both produce the per-vertex values in the reference's pair
-// order; the queue order does not matter because each vertex is written by
-// one thread.
+// cell, where the list has such rows; the others (with near rows, all) are
+// queued and walk the 27 cells through the cell table in a second kernel
+// (k_rep_slow), so the long table walk never holds a warp of fast vertices.
+// Rows are summed in the reference's pair order, a walk by its lanes and a
+// fixed shuffle tree; the queue order does not matter because each vertex is
+// written by one warp.
 #include <algorithm>
 
 #include "tm_energy.cuh"

@@ -109,8 +109,8 @@ __device__ __forceinline__ bool excluded(const T& t, int excl, int v, int j) {
 
 // The same test one vertex at a time: few registers, for the double-word face
 // kernel, whose repulsion hardly ever makes the test and whose faces pay for
-// its registers (64 instead of 56: 86.2 us an evaluation of 163,842 vertices
-// against 84).
+// its registers (an evaluation of 163,842 vertices: 79.9 us with both rings in
+// registers, 78.1 so).
 struct TableExclSlim {
   const Topo& t;
   int excl;

@@ -557,7 +557,8 @@ void tm_energy::ensure(int nv_, int ne_, int nf_) {
   partials.ensure(8 * (size_t)nb * 2);  // up to two lanes per vertex
   moved.ensure(nb);
   grad.ensure(3 * (size_t)std::max(nv, 1));
-  work.ensure(64);
+  // workspace of an HMC move: position, momentum, two forces, partials and scalars
+  work.ensure(12 * (size_t)std::max(nv, 1) + 1024 + 64);
   glob.ensure(1);
   TM_CUDA(cudaMemsetAsync(glob.get(), 0, sizeof(tmg::Globals), stream));
 }
